@@ -491,7 +491,8 @@ static void isl_ensure( HostWorld* W )
 		dgrow( h.log, 0, (size_t)d.bodyCap + d.jointCap );
 		h.logCap = d.bodyCap + d.jointCap;
 	}
-	cudaMemcpy( W->islDev, &h, sizeof( DIslands ), cudaMemcpyHostToDevice );
+	cudaMemcpyAsync( W->islDev, &h, sizeof( DIslands ), cudaMemcpyHostToDevice, W->stream );
+	cudaStreamSynchronize( W->stream );
 	d.isl = W->islDev;
 	d.islFlag = h.flag;
 	d.islPos = h.pos;
@@ -3588,13 +3589,18 @@ static void cb_ensure( HostWorld* W )
 	W->graphDirty = true;
 }
 
+// The hooks' copies go through the world's stream: a pageable copy on the
+// default stream may return before its transfer, and the world's stream does
+// not wait for it.
 static void upload_rejected( HostWorld* W, std::vector<unsigned long long>& rejected )
 {
 	std::sort( rejected.begin(), rejected.end() );
 	int n = (int)rejected.size();
 	if ( n > 0 )
-		cudaMemcpy( W->d.cbReject, rejected.data(), sizeof( unsigned long long ) * n, cudaMemcpyHostToDevice );
-	cudaMemcpy( &W->d.sc->cbReject, &n, sizeof( int ), cudaMemcpyHostToDevice );
+		cudaMemcpyAsync( W->d.cbReject, rejected.data(), sizeof( unsigned long long ) * n, cudaMemcpyHostToDevice,
+						 W->stream );
+	cudaMemcpyAsync( &W->d.sc->cbReject, &n, sizeof( int ), cudaMemcpyHostToDevice, W->stream );
+	cudaStreamSynchronize( W->stream ); // the sources are the caller's
 }
 
 static int listed_count( HostWorld* W )
@@ -3639,10 +3645,11 @@ static void pair_filter_hook( void* context )
 		return;
 	if ( kept > 0 )
 	{
-		cudaMemcpy( d.pairVal, s1.data(), sizeof( int ) * kept, cudaMemcpyHostToDevice );
-		cudaMemcpy( d.pairValAlt, s2.data(), sizeof( int ) * kept, cudaMemcpyHostToDevice );
+		cudaMemcpyAsync( d.pairVal, s1.data(), sizeof( int ) * kept, cudaMemcpyHostToDevice, W->stream );
+		cudaMemcpyAsync( d.pairValAlt, s2.data(), sizeof( int ) * kept, cudaMemcpyHostToDevice, W->stream );
 	}
-	cudaMemcpy( &d.sc->newPairCount, &kept, sizeof( int ), cudaMemcpyHostToDevice );
+	cudaMemcpyAsync( &d.sc->newPairCount, &kept, sizeof( int ), cudaMemcpyHostToDevice, W->stream );
+	cudaStreamSynchronize( W->stream ); // the sources are locals
 }
 
 // solver.c:270-280: continuous candidates (static shape, fast shape)
