@@ -531,7 +531,7 @@ def run_batched(args, torch):
                     "links; gravity tilted U[-15,15] deg; seed %d), dt=1/60, 4 substeps" % (worlds, seed),
         "worlds": worlds, "bodies": c["awake_bodies"], "touching": c["touching"], "joints": c["joints"],
         "ms_per_step": bms, "world_steps_per_s": batched_ws, "body_steps_per_s": c["awake_bodies"] * 1000.0 / bms,
-        "autotune": {"solver_variant": ["auto", "cluster", "grid512", "grid256"][chosen[0]],
+        "autotune": {"solver_variant": ["auto", "few_parts", "one_block_per_sm", "two_blocks_per_sm"][chosen[0]],
                      "leaf_order_period": chosen[1], "tuning_steps": taken},
         "frame": frames, "status": st,
         "plain": {"sample_worlds": len(sample), "ms_per_world_step": float(np.mean(pms)),

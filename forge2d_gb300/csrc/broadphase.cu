@@ -647,6 +647,13 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 						 w.sortHist, &w.sc->barrierCount, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder );
 	if ( hs != st )
 		cudaStreamWaitEvent( st, s.sideJoin[0], 0 );
+	// the solver's body order follows the leaf order, beside the pair search
+	if ( s.side[3] )
+	{
+		cudaEventRecord( s.sideFork, st );
+		cudaStreamWaitEvent( s.side[3], s.sideFork, 0 );
+	}
+	launch_solver_order( w, s, s.side[3] ? s.side[3] : st );
 	k_wide_refit<<<( ( w.shapeCap + WIDE - 1 ) / WIDE + 7 ) / 8, BP_THREADS, 0, st>>>( w );
 	k_find_pairs<<<( w.shapeCap + FIND_WARPS - 1 ) / FIND_WARPS, BP_THREADS, 0, st>>>( w );
 	k_clamp_pairs<<<1, 1, 0, st>>>( w );

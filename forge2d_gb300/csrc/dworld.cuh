@@ -88,6 +88,16 @@
 // (new pairs are sorted by key), so it is refreshed periodically.
 #define ORDER_REBUILD_PERIOD 8
 
+// Substeps of one solver launch, at most (rows of DWorld::dsub per body).
+#define FLOW_SUBSTEPS 8
+// Blocks of the solver launch, at most, and rows of a contact constraint.
+#define SOLVER_MAX_PARTS 320
+#define KROWS 11
+// Bodies per part of the solver, at least (and in worlds that deal small
+// worlds to many blocks).
+#define SOLVER_MIN_CHUNK 64
+#define SOLVER_SMALL_CHUNK 8
+
 // Per-step scalars kept in device memory so that no launch needs a host
 // round trip.
 struct DScalars
@@ -98,7 +108,6 @@ struct DScalars
 	int opCount;
 	int touchingCount;
 	int colorCount[F2D_COLORS];
-	int colorStart[F2D_COLORS + 1];
 	int overflowCount;
 	int overflowJointCount;
 	int fastCount;
@@ -140,7 +149,7 @@ struct DScalars
 	// creation stamp of the next new contact (the bodies' contact lists are
 	// newest first); non-static bodies in the awake set (worlds without
 	// island records); destroy calls: collected contacts, end events
-	int solveBarriers; // grid barriers the last grid-wide solver launch passed
+	int orderTotal; // bodies with a place in the solver's spatial order
 	unsigned long long stampBase;
 	int awakeOrderCount;
 	int apiCount, apiEndCount;
@@ -419,19 +428,10 @@ struct DWorld
 	unsigned long long* opScan; // look-back state of the op output scans
 
 	// ---------------- constraints (by slot, grouped by colour) ----------------
-	int* slotContact;
 	int* overflowList; // contact ids in overflow-array order
-	int2* kIndex;	   // indexA indexB (-1 static)
-	float4* kMass;	   // invMassA invIA invMassB invIB
-	float4* kNormal;   // normal.x normal.y friction tangentSpeed
-	float4* kMisc;	   // restitution rollingResistance rollingMass rollingImpulse
-	float4* kSoft;	   // biasRate massScale impulseScale pointCount(bits)
-	float4* kAnch1;	   // anchorA1.xy anchorB1.xy
-	float4* kAnch2;	   // anchorA2.xy anchorB2.xy
-	float4* kP1;	   // baseSeparation normalMass tangentMass relativeVelocity (point 1)
-	float4* kP2;	   // same, point 2
-	float4* kImp;	   // normalImpulse1 normalImpulse2 tangentImpulse1 tangentImpulse2
-	float2* kTot;	   // totalNormalImpulse1 totalNormalImpulse2
+	int slotCap;	   // constraint slots (contacts, padded to groups of 32 per part and colour)
+	float4* kRow;	   // constraint rows (dsolve.cuh)
+	int2* slotPlace;   // per contact: bin (part and colour; the part of an overflow contact) and place in it
 
 	// ---------------- joints (by joint id) ----------------
 	int2* jbody;
@@ -454,17 +454,29 @@ struct DWorld
 	float4* jprepM; // invMassA invIA invMassB invIB
 	int2* jindex;	// solver body indices
 	int* overflowJoints;
-	// overflow levels (solver scratch): body owner per level round, level
-	// per overflow constraint, constraints in level order beyond the
-	// shared-memory list
 	int* npBucket; // narrowphase: contact ids by manifold class, NP_CLASSES x contactCap
 	DIslands* isl;  // islands and solver sets (sleeping worlds only, else null)
 	int* islFlag;	// device copies of isl->flag and isl->pos (scan arguments)
 	int* islPos;
 	unsigned long long *islNcKeys, *islNcKeysAlt; // copies of isl->ncKeys, ncKeysAlt (sort arguments)
-	int* ovfOwner; // bodyCap
-	int* ovfLevel; // contactCap + jointCap
-	int* ovfOrder; // contactCap + jointCap
+	// solver scratch
+	unsigned long long* orderState; // look-back state of the body order
+	int* bodyPos;	 // place in the spatial order of the bodies with constraints, or -2 - place
+	int* bodyAt;	 // the inverse
+	int4* bodyOrd;	 // colour bits (and those with restitution << 11, shared flag), overflow constraints, those with
+					 // restitution, head of the body's overflow list
+	float4* bodyInt; // [2*id+k] velocity change xy, linear damping, angular change; angular damping, flags
+	float4* dsub;	 // delta rows after each substep of a launch, FLOW_SUBSTEPS x bodyCap
+	int2* jointPlace; // per joint: bin and place in it
+	int* jointSlots;  // joint ids by part and colour
+	int* ovfItems;	  // overflow constraints (joints, then contacts, in list order) by part, unordered
+	int* ovfSorted;	  // the same in ascending order
+	int4* ovfRank;	  // ranks of an overflow constraint on its bodies (all, with restitution)
+	int* ovfNext;	  // links of the bodies' overflow lists
+	// constraints per part and colour, and per part overflow constraints (one
+	// block of memory), and their starts
+	int *binContacts, *binJoints, *binOverflow;
+	int *binContactStart, *binJointStart, *binOverflowStart;
 	int* pendingJointOps; // joint ids whose colour must be assigned at next step
 	int pendingJointCount;
 

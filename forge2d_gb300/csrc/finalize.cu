@@ -467,11 +467,12 @@ __global__ void k_continuous( DWorld w, int listOnly )
 // solver.c:1758-1818 hit events
 __global__ void k_hit_events( DWorld w )
 {
-	int n = w.sc->touchingCount;
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x )
+	int n = w.sc->contactIdCount;
+	for ( int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x )
 	{
-		int c = w.slotContact[k];
-		if ( ( w.cflags[c] & CF_HIT_EVENT ) == 0 )
+		// contacts in the graph
+		int flags = w.cflags[c];
+		if ( ( flags & CF_USED ) == 0 || ( flags & CF_HIT_EVENT ) == 0 || w.ccolor[c] < 0 )
 			continue;
 		float4 mn = w.mnorm[c];
 		int count = __float_as_int( mn.w );

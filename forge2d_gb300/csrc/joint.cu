@@ -1,11 +1,11 @@
-// Joint preparation and the per-colour joint slot lists of the solver.
+// Joint preparation of the solver.
 // Reference: packages/forge2d/third_party/box2d/src/joint.c:1346-1390
 // (softness clamp, type dispatch), revolute_joint.c:195-259,
 // weld_joint.c:83-140, distance_joint.c:158-205, prismatic_joint.c:279-346,
 // wheel_joint.c:183-262, motor_joint.c:99-160, mouse_joint.c:77-128.
 #include "joint.cuh"
 
-__global__ void k_prepare_joints( DWorld w, float h, float inv_h, Soft jointSoft )
+__global__ void k_prepare_joints( DWorld w, float h, Soft jointSoft )
 {
 	int n = w.jointCount;
 	for ( int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x )
@@ -180,60 +180,7 @@ __global__ void k_prepare_joints( DWorld w, float h, float inv_h, Soft jointSoft
 	}
 }
 
-__global__ void k_joint_count( DWorld w, int* cnt )
+void launch_prepare_joints( DWorld& w, cudaStream_t st, float h, Soft jointSoft )
 {
-	int n = w.jointCount;
-	for ( int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x )
-	{
-		int c = w.jcolor[j];
-		if ( ( w.jflags[j] & JF_USED ) && c >= 0 && c < F2D_OVERFLOW )
-			atomicAdd( cnt + c, 1 );
-	}
-}
-
-__global__ void k_joint_offsets( int* cnt, int* start )
-{
-	if ( threadIdx.x != 0 || blockIdx.x != 0 )
-		return;
-	int s = 0;
-	for ( int c = 0; c < F2D_OVERFLOW; ++c )
-	{
-		start[c] = s;
-		s += cnt[c];
-		cnt[c] = 0;
-	}
-	start[F2D_OVERFLOW] = s;
-}
-
-__global__ void k_joint_fill( DWorld w, int* cnt, const int* start, int* slots )
-{
-	int n = w.jointCount;
-	for ( int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x )
-	{
-		int c = w.jcolor[j];
-		if ( ( w.jflags[j] & JF_USED ) && c >= 0 && c < F2D_OVERFLOW )
-			slots[start[c] + atomicAdd( cnt + c, 1 )] = j;
-	}
-}
-
-__global__ void k_zero_small( int* p, int n )
-{
-	if ( threadIdx.x < n )
-		p[threadIdx.x] = 0;
-}
-
-void launch_prepare_joints( DWorld& w, StepScratch& s, cudaStream_t st, float h, float inv_h, Soft jointSoft )
-{
-	int* slots = s.tmpB;
-	int* start = s.tmpB + w.jointCap;
-	int* cnt = start + F2D_COLORS + 4;
-	k_zero_small<<<1, 32, 0, st>>>( cnt, F2D_COLORS );
-	if ( w.jointCount > 0 )
-	{
-		k_prepare_joints<<<grid_for( w.jointCount ), 256, 0, st>>>( w, h, inv_h, jointSoft );
-		k_joint_count<<<grid_for( w.jointCount ), 256, 0, st>>>( w, cnt );
-	}
-	k_joint_offsets<<<1, 1, 0, st>>>( cnt, start );
-	if ( w.jointCount > 0 )
-		k_joint_fill<<<grid_for( w.jointCount ), 256, 0, st>>>( w, cnt, start, slots );
+	k_prepare_joints<<<grid_for( w.jointCount ), 256, 0, st>>>( w, h, jointSoft );
 }

@@ -1079,4 +1079,3 @@ template <class BA> __device__ void mouse_solve( const DWorld& w, const BA& ba, 
 	jstate_store( ba, idx.y, vB, wB );
 }
 
-void launch_prepare_joints( DWorld& w, StepScratch& s, cudaStream_t st, float h, float inv_h, Soft jointSoft );

@@ -31,10 +31,10 @@ struct StepScratch
 	float4* bounds;
 	int boundsBlocks;
 	int shapeIdBits;
-	int solverBlocks;  // persistent solver grid (co-resident)
-	int solverThreads;
-	int clusterCapacity; // bodies the cluster solver takes (0: cooperative solver only)
-	int solverBlocks256; // grid of the 256-thread variant of the grid-wide solver
+	int solverBlocks;  // solver grid, one block per SM (co-resident)
+	bool smallParts;   // the solver deals small worlds' bodies to many blocks too
+	int subSteps;		// of the step being enqueued
+	int solverBlocks2; // solver grid, two blocks per SM
 	int solverVariant;	 // SOLVER_* (the autotuner's choice; results never depend on it)
 	int ptBlocks;		 // co-resident grid of the tree rebuild's cooperative levels
 	cudaEvent_t evSolveStart; // recorded right before the cooperative solver launch when non-null
@@ -49,10 +49,10 @@ struct StepScratch
 };
 
 // solver variants: same arithmetic, different launch shapes
-#define SOLVER_AUTO 0	 // cluster solver up to 2e4 bodies, else grid-wide with 512-thread blocks
-#define SOLVER_CLUSTER 1 // one thread-block cluster (when the bodies fit its shared memory)
-#define SOLVER_GRID512 2 // grid-wide, one 512-thread block per SM
-#define SOLVER_GRID256 3 // grid-wide, two 256-thread blocks per SM
+#define SOLVER_AUTO 0		// one block per SM
+#define SOLVER_FEW_PARTS 1	// the same; worlds of up to four times the size are one part
+#define SOLVER_ONE_PER_SM 2 // the same as AUTO
+#define SOLVER_TWO_PER_SM 3 // two blocks of half the threads per SM
 
 // A host hook runs between launches when the world has user callbacks
 // (the stream is synchronised by the hook itself).
@@ -97,7 +97,9 @@ void launch_explode( DWorld& w, cudaStream_t st, int* hit, unsigned long long ma
 void launch_isl_fix_flags( DWorld& w, cudaStream_t st, int n );
 void launch_learned_warm_start( DWorld& w, cudaStream_t st );
 void launch_record_samples( DWorld& w, cudaStream_t st );
-int solver_cluster_capacity();
+void launch_solver_order( DWorld& w, StepScratch& s, cudaStream_t st );
+struct Soft;
+void launch_prepare_joints( DWorld& w, cudaStream_t st, float h, Soft jointSoft );
 // the reference's broadphase trees and the move array (proxytree.cu)
 int pt_large_blocks();
 void launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st );

@@ -15,6 +15,7 @@
 // b2 [64], b3 [8]. Features and targets are normalised with per-column mean
 // and 1/std held with the model.
 #include "../../include/forge2d_gb300.h"
+#include "dsolve.cuh"
 #include "dworld.cuh"
 #include "kernels.cuh"
 
@@ -503,7 +504,8 @@ __global__ void __launch_bounds__( MLP_THREADS ) k_mlp_warm_start( DWorld w, con
 				float friction = w.newFeat[(size_t)i * MLP_IN + 11];
 				ni = fmaxf( ni, 0.0f );
 				ti = fminf( fmaxf( ti, -friction * ni ), friction * ni );
-				float4 imp = w.kImp[kj.x];
+				float4* row = krow( w, kj.x, KR_IMP );
+				float4 imp = *row;
 				if ( kj.y == 0 )
 				{
 					imp.x = ni;
@@ -514,7 +516,7 @@ __global__ void __launch_bounds__( MLP_THREADS ) k_mlp_warm_start( DWorld w, con
 					imp.y = ni;
 					imp.w = ti;
 				}
-				w.kImp[kj.x] = imp;
+				*row = imp;
 			}
 		}
 		__syncwarp();
@@ -532,7 +534,7 @@ __global__ void k_record_samples( DWorld w )
 		if ( slot >= w.sampleCap )
 			return;
 		int2 kj = w.newPoint[i];
-		int c = w.slotContact[kj.x];
+		int c = __float_as_int( krow( w, kj.x, KR_HEAD )->z );
 		float4 im = w.mpI[2 * c + kj.y];
 		float* o = w.samples + (size_t)slot * MLP_SAMPLE;
 		for ( int f = 0; f < MLP_IN; ++f )

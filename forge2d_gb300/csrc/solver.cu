@@ -4,26 +4,16 @@
 // src/solver.c:929-1160): prepare joints and contacts; per substep integrate
 // velocities, warm start (overflow joints, overflow contacts, then graph
 // colours 0..10), solve, integrate positions, relax; then restitution and
-// impulse storage. All of it runs in one persistent cooperative kernel: the
-// colour stages are separated by grid barriers (bounded spins that raise an
-// error bit instead of hanging), the serial overflow constraints run on one
-// thread between two barriers, and within a colour one thread solves one
-// constraint (bodies within a colour are disjoint, so the slot order inside
-// a colour does not change any result).
-//
-// Constraint arithmetic: graph-colour constraints follow the operand order of
-// the reference's SIMD lanes (contact_solver.c:1438-2120, separate mul and
-// add, SSE2 min/max/blend semantics); overflow constraints follow its scalar
-// functions (contact_solver.c:24-510). Built with -fmad=false the results
-// are bit-identical to the reference C code.
+// impulse storage. After the set-up launches all of it runs in one persistent
+// launch in which no stage waits for the whole device: the constraints are a
+// data flow over the bodies (k_solve).
 #include "dscan.cuh"
 #include "dsync.cuh"
 
-#include <cooperative_groups.h>
+#include "dsolve.cuh"
 #include "dworld.cuh"
 #include "joint.cuh"
 #include "kernels.cuh"
-
 
 struct SolveParams
 {
@@ -34,104 +24,362 @@ struct SolveParams
 	float restitutionThreshold;
 	float maxLinearSpeed, maxAngularSpeed;
 	fv2 gravity;
-	int subSteps;
+	int subSteps;	 // of this launch
+	int restitution; // this launch ends the step: restitution and impulse storage
 	int enableWarmStarting;
+	int parts;	  // blocks of the solver launch
+	int minChunk; // bodies per part, at least
+	int onePart;  // up to this many bodies with constraints make one part
+	int slots;	  // bodies whose rows fit a block's shared memory
 };
 
-// ---------------------------------------------------------------------------
-// constraint slots: overflow first (overflow-array order), then colours
-// ---------------------------------------------------------------------------
-// Colour occupancy of the touching contacts: per-block counts in shared
-// memory, one global add per colour and block.
-__global__ void k_count_colors( DWorld w, int* fill )
+#define FLOW_SENTINEL 0xffffffffu
+#define FLOW_SPIN_LIMIT ( 1 << 20 )
+#define FLOW_REST_SHIFT 11		  // bodyOrd.x: colour bits, then the bits of colours with restitution,
+#define FLOW_GLOBAL ( 1 << 22 )	  // and whether the body's row is shared between blocks
+#define FLOW_COLOURS ( ( 1 << F2D_OVERFLOW ) - 1 )
+#define BI_AWAKE 1 // bodyInt flags
+#define BI_FAST_ROT 2
+
+__device__ __forceinline__ bool body_awake( int f )
 {
-	__shared__ int cnt[F2D_OVERFLOW];
-	if ( threadIdx.x < F2D_OVERFLOW )
-		cnt[threadIdx.x] = 0;
+	return ( f & ( BF_USED | BF_ENABLED | BF_ASLEEP ) ) == ( BF_USED | BF_ENABLED ) && body_type( f ) != 0;
+}
+
+// ---------------------------------------------------------------------------
+// parts: bodies in spatial order, dealt to the solver's blocks in runs
+// ---------------------------------------------------------------------------
+
+// Position of every body with graph constraints (as of the last step's
+// colours) in the order of the broadphase tree's leaves, which follow a
+// Morton curve: one launch, tiles chained by decoupled look-back. bodyPos is
+// the position, or -2 - position for a body without constraints, which gets no
+// place of its own. The order only decides where a constraint is solved,
+// never what it computes.
+#define ORDER_THREADS 1024
+#define ORDER_ITEMS 4
+#define ORDER_TILE ( ORDER_THREADS * ORDER_ITEMS )
+__global__ void __launch_bounds__( ORDER_THREADS ) k_body_order( DWorld w )
+{
+	__shared__ int smem[32];
+	__shared__ int s_tile, s_prefix;
+	const int n = w.sc->treeLeafCount;
+	unsigned long long* state = w.orderState;
+	if ( threadIdx.x == 0 )
+		s_tile = (int)atomicAdd( (unsigned*)state, 1u );
 	__syncthreads();
-	int n = w.sc->contactIdCount;
-	for ( int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x )
+	const int tile = s_tile;
+	const int base = tile * ORDER_TILE;
+	if ( base >= n )
+	{
+		if ( tile == 0 && threadIdx.x == 0 )
+			w.sc->orderTotal = 0;
+		return;
+	}
+	int body[ORDER_ITEMS], flag[ORDER_ITEMS];
+	int sum = 0;
+#pragma unroll
+	for ( int k = 0; k < ORDER_ITEMS; ++k )
+	{
+		int i = base + threadIdx.x * ORDER_ITEMS + k;
+		body[k] = -1;
+		flag[k] = 0;
+		if ( i < n )
+		{
+			int s = w.leafShape[i];
+			int b = w.shapeBody[s];
+			if ( w.headShape[b] == s )
+			{
+				body[k] = b;
+				flag[k] = w.colorMask[b] != 0u ? 1 : 0;
+			}
+		}
+		sum += flag[k];
+	}
+	int aggregate;
+	int excl = block_exclusive_scan_1024( sum, smem, &aggregate );
+	if ( threadIdx.x == 0 )
+	{
+		const unsigned long long AGG = 1ull, PREFIX = 2ull;
+		int prefix = 0;
+		if ( tile > 0 )
+		{
+			st_release_u64( state + 1 + tile, ( AGG << 32 ) | (unsigned)aggregate );
+			long long spins = 0;
+			for ( int j = tile - 1; j >= 0; )
+			{
+				unsigned long long v = ld_acquire_u64( state + 1 + j );
+				if ( ( v >> 32 ) == 0ull )
+				{
+					if ( ++spins > F2D_SPIN_LIMIT )
+					{
+						atomicOr( &w.sc->error, ERR_BARRIER_TIMEOUT );
+						break;
+					}
+					continue;
+				}
+				prefix += (int)(unsigned)( v & 0xffffffffull );
+				if ( ( v >> 32 ) == PREFIX )
+					break;
+				j -= 1;
+			}
+		}
+		st_release_u64( state + 1 + tile, ( PREFIX << 32 ) | (unsigned)( prefix + aggregate ) );
+		s_prefix = prefix;
+		if ( base + ORDER_TILE >= n )
+			w.sc->orderTotal = prefix + aggregate;
+	}
+	__syncthreads();
+	excl += s_prefix;
+#pragma unroll
+	for ( int k = 0; k < ORDER_ITEMS; ++k )
+	{
+		if ( body[k] >= 0 )
+			w.bodyPos[body[k]] = flag[k] ? excl : -2 - excl;
+		if ( flag[k] )
+			w.bodyAt[excl] = body[k];
+		excl += flag[k];
+	}
+}
+
+// Bodies per part: positions are dealt to the blocks in runs of this length.
+__device__ __forceinline__ int part_chunk( const DWorld& w, const SolveParams& p )
+{
+	int n = w.sc->orderTotal;
+	int chunk = max( p.minChunk, ( n + p.parts - 1 ) / p.parts );
+	return max( n <= p.onePart ? n : chunk, 1 );
+}
+
+__device__ __forceinline__ int body_part( const DWorld& w, const SolveParams& p, int chunk, int b )
+{
+	int pos = w.bodyPos[b];
+	pos = pos >= 0 ? pos : -2 - pos;
+	return min( max( pos, 0 ) / chunk, p.parts - 1 );
+}
+
+// Part of the constraint between two bodies (-1 static): the lower of the
+// bodies' parts, so that of two neighbouring parts only the higher one's
+// bodies are shared. Shared bodies are marked.
+__device__ __forceinline__ int constraint_part( const DWorld& w, const SolveParams& p, int chunk, int a, int b )
+{
+	int pa = a >= 0 ? body_part( w, p, chunk, a ) : 0x7fffffff;
+	int pb = b >= 0 ? body_part( w, p, chunk, b ) : 0x7fffffff;
+	int part = min( min( pa, pb ), p.parts - 1 );
+	if ( a >= 0 && pa != part )
+		atomicOr( (int*)( w.bodyOrd + a ), FLOW_GLOBAL );
+	if ( b >= 0 && pb != part )
+		atomicOr( (int*)( w.bodyOrd + b ), FLOW_GLOBAL );
+	return part;
+}
+
+__device__ __forceinline__ int dynamic_index( const DWorld& w, int b )
+{
+	return body_type( w.bflags[b] ) == 0 ? -1 : b;
+}
+
+// Counts the constraints per part and colour and gives each its place there;
+// per body, the factors of a substep's velocity integration (solver.c:65-130;
+// they are the same in every substep).
+__global__ void k_solver_count( DWorld w, SolveParams p )
+{
+	const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+	const int chunk = part_chunk( w, p );
+	const int nc = w.sc->contactIdCount;
+	for ( int c = tid; c < nc; c += stride )
 	{
 		int col = w.ccolor[c];
-		if ( col >= 0 && col < F2D_OVERFLOW && ( w.cflags[c] & CF_USED ) )
-			atomicAdd( cnt + col, 1 );
+		if ( col < 0 || ( w.cflags[c] & CF_USED ) == 0 )
+			continue;
+		int2 bd = w.cbody[c];
+		int part = constraint_part( w, p, chunk, dynamic_index( w, bd.x ), dynamic_index( w, bd.y ) );
+		if ( col < F2D_OVERFLOW )
+		{
+			int bin = part * F2D_OVERFLOW + col;
+			w.slotPlace[c] = make_int2( bin, atomicAdd( w.binContacts + bin, 1 ) );
+		}
+		else
+			w.slotPlace[c] = make_int2( part, atomicAdd( w.binOverflow + part, 1 ) );
+	}
+	for ( int j = tid; j < w.jointCount; j += stride )
+	{
+		int col = w.jcolor[j];
+		if ( ( w.jflags[j] & JF_USED ) == 0 || col < 0 )
+			continue;
+		int2 bd = w.jbody[j];
+		int part = constraint_part( w, p, chunk, dynamic_index( w, bd.x ), dynamic_index( w, bd.y ) );
+		if ( col < F2D_OVERFLOW )
+		{
+			int bin = part * F2D_OVERFLOW + col;
+			w.jointPlace[j] = make_int2( bin, atomicAdd( w.binJoints + bin, 1 ) );
+		}
+		else
+			w.jointPlace[j] = make_int2( part, atomicAdd( w.binOverflow + part, 1 ) );
+	}
+	for ( int b = tid; b < w.bodyCount; b += stride )
+	{
+		float4 m = w.massv[b];
+		float4 dmp = w.damp[b];
+		float4 f = w.force[b];
+		int flags = w.bflags[b];
+		float h = p.h;
+		float linearDamping = 1.0f / ( 1.0f + h * dmp.x );
+		float angularDamping = 1.0f / ( 1.0f + h * dmp.y );
+		float gravityScale = m.x > 0.0f ? dmp.z : 0.0f;
+		fv2 g = p.gravity;
+		if ( w.subCount > 0 )
+		{
+			float2 gb = w.bodyGravity[b];
+			g = mk( gb.x, gb.y );
+		}
+		fv2 lvd = vadd( vscale( h * m.x, mk( f.x, f.y ) ), vscale( h * gravityScale, g ) );
+		float avd = h * m.y * f.z;
+		int bits = ( body_awake( flags ) ? BI_AWAKE : 0 ) | ( ( flags & BF_FAST_ROT ) ? BI_FAST_ROT : 0 );
+		w.bodyInt[2 * (size_t)b] = make_float4( lvd.x, lvd.y, linearDamping, avd );
+		w.bodyInt[2 * (size_t)b + 1] = make_float4( angularDamping, __int_as_float( bits ), 0.0f, 0.0f );
+		// the solver counts a body's operations in its row's last word
+		if ( __float_as_int( w.vel[b].w ) != 0 )
+			w.vel[b].w = 0.0f;
+	}
+}
+
+// Exclusive prefix over n bins in shared memory (256 threads): plain counts,
+// or groups of 32.
+__device__ __forceinline__ int bin_prefix( const int* bins, int n, int* out, bool groups, int* smem )
+{
+	int per = ( n + 255 ) / 256;
+	int lo = threadIdx.x * per, hi = min( lo + per, n );
+	int sum = 0;
+	for ( int i = lo; i < hi; ++i )
+	{
+		int v = bins[i];
+		sum += groups ? ( v + 31 ) >> 5 : v;
+	}
+	int total;
+	int at = block_exclusive_scan_1024( sum, smem, &total );
+	for ( int i = lo; i < hi; ++i )
+	{
+		out[i] = at;
+		int v = bins[i];
+		at += groups ? ( v + 31 ) >> 5 : v;
 	}
 	__syncthreads();
-	if ( threadIdx.x < F2D_OVERFLOW && cnt[threadIdx.x] > 0 )
-		atomicAdd( fill + threadIdx.x, cnt[threadIdx.x] );
+	return total;
 }
 
-__global__ void k_zero_ints( int* p, int n )
+// Notes a constraint on a body, for the ranks of the solver's data flow: its
+// colour, or overflow constraint `e` (its place in the serial order: joints,
+// then contacts) in the body's list.
+__device__ __forceinline__ void flow_note( const DWorld& w, int b, int colour, int e, int side, bool restitution )
 {
-	for ( int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x )
-		p[i] = 0;
-}
-
-__global__ void k_color_offsets( DWorld w, int* fill )
-{
-	if ( blockIdx.x != 0 || threadIdx.x != 0 )
+	if ( b < 0 )
 		return;
-	int start = w.sc->overflowCount;
-	for ( int c = 0; c < F2D_OVERFLOW; ++c )
+	int* o = (int*)( w.bodyOrd + b );
+	if ( colour < F2D_OVERFLOW )
 	{
-		w.sc->colorStart[c] = start;
-		w.sc->colorCount[c] = fill[c];
-		start += fill[c];
-		fill[c] = 0;
+		atomicOr( o, ( 1 << colour ) | ( restitution ? 1 << ( FLOW_REST_SHIFT + colour ) : 0 ) );
+		return;
 	}
-	w.sc->colorStart[F2D_OVERFLOW] = start;
-	w.sc->colorCount[F2D_OVERFLOW] = w.sc->overflowCount;
-	w.sc->touchingCount = start;
+	atomicAdd( o + 1, 1 );
+	if ( restitution )
+		atomicAdd( o + 2, 1 );
+	// list heads are keys + 1, 0 when empty
+	w.ovfNext[2 * (size_t)e + side] = atomicExch( o + 3, ( ( e << 2 ) | ( restitution ? 2 : 0 ) | side ) + 1 );
 }
 
-// Constraint slots: overflow contacts first (overflow-array order), then
-// each colour's contacts in a contiguous range. Inside a colour the slot
-// order is arbitrary (no two constraints of a colour share a dynamic body);
-// each block reserves its range with one global add per colour.
-__global__ void k_fill_slots( DWorld w, int* fill )
+// Constraint rows of every contact in the graph (contact_solver.c:1438-1669
+// and :24-156, identical expressions in both), grouped by part and colour,
+// overflow contacts first in overflow-array order; the joints' lists.
+__global__ void __launch_bounds__( 256 ) k_solver_prepare( DWorld w, SolveParams p )
 {
-	__shared__ int cnt[F2D_OVERFLOW], base[F2D_OVERFLOW];
-	int n = w.sc->contactIdCount;
-	int nov = w.sc->overflowCount;
-	for ( int i = blockIdx.x * blockDim.x + threadIdx.x; i < nov; i += gridDim.x * blockDim.x )
-		w.slotContact[i] = w.overflowList[i];
-	int stride = gridDim.x * blockDim.x;
-	for ( int c0 = blockIdx.x * blockDim.x; c0 < n; c0 += stride )
+	extern __shared__ int dynBins[];
+	__shared__ int smem[32];
+	const int bins = p.parts * F2D_OVERFLOW;
+	int* sContact = dynBins;
+	int* sJoint = dynBins + bins;
+	int* sOverflow = dynBins + 2 * bins;
+	const int novf = w.sc->overflowCount, novfJ = w.sc->overflowJointCount;
+	const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+	bin_prefix( w.binContacts, bins, sContact, true, smem );
+	if ( w.jointCount > 0 )
+		bin_prefix( w.binJoints, bins, sJoint, false, smem );
+	if ( novf + novfJ > 0 )
+		bin_prefix( w.binOverflow, p.parts, sOverflow, false, smem );
+	const int firstGroup = ( novf + 31 ) >> 5;
+	if ( blockIdx.x == 0 )
 	{
+		// the bins' starts for the solver, and the colours' sizes
+		__shared__ int colour[F2D_OVERFLOW];
 		if ( threadIdx.x < F2D_OVERFLOW )
-			cnt[threadIdx.x] = 0;
+			colour[threadIdx.x] = 0;
 		__syncthreads();
-		int c = c0 + threadIdx.x;
-		int col = -1, rank = 0;
-		if ( c < n )
+		for ( int i = threadIdx.x; i < bins; i += blockDim.x )
 		{
-			col = w.ccolor[c];
-			if ( col >= 0 && col < F2D_OVERFLOW && ( w.cflags[c] & CF_USED ) )
-				rank = atomicAdd( cnt + col, 1 );
-			else
-				col = -1;
+			w.binContactStart[i] = firstGroup + sContact[i];
+			if ( w.jointCount > 0 )
+				w.binJointStart[i] = sJoint[i];
+			atomicAdd( colour + i % F2D_OVERFLOW, w.binContacts[i] );
 		}
+		if ( novf + novfJ > 0 )
+			for ( int i = threadIdx.x; i < p.parts; i += blockDim.x )
+				w.binOverflowStart[i] = sOverflow[i];
 		__syncthreads();
-		if ( threadIdx.x < F2D_OVERFLOW )
-			base[threadIdx.x] = cnt[threadIdx.x] > 0 ? atomicAdd( fill + threadIdx.x, cnt[threadIdx.x] ) : 0;
-		__syncthreads();
-		if ( col >= 0 )
-			w.slotContact[w.sc->colorStart[col] + base[col] + rank] = c;
-		__syncthreads();
+		if ( threadIdx.x == 0 )
+		{
+			int total = novf;
+			for ( int c = 0; c < F2D_OVERFLOW; ++c )
+			{
+				w.sc->colorCount[c] = colour[c];
+				total += colour[c];
+			}
+			w.sc->colorCount[F2D_OVERFLOW] = novf;
+			w.sc->touchingCount = total;
+		}
 	}
-}
-
-// contact_solver.c:1438-1669 / :24-156 (identical expressions in both)
-__global__ void k_prepare_contacts( DWorld w, SolveParams p )
-{
-	int n = w.sc->touchingCount;
-	float warmStartScale = p.enableWarmStarting ? 1.0f : 0.0f;
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x )
+	// joints: the solver's lists (their rows are prepared by joint.cu)
+	for ( int j = tid; j < w.jointCount; j += stride )
 	{
-		int c = w.slotContact[k];
+		int col = w.jcolor[j];
+		if ( ( w.jflags[j] & JF_USED ) == 0 || col < 0 || col >= F2D_OVERFLOW )
+			continue;
+		int2 pl = w.jointPlace[j];
+		w.jointSlots[sJoint[pl.x] + pl.y] = j;
+		int2 bd = w.jbody[j];
+		flow_note( w, dynamic_index( w, bd.x ), col, 0, 0, false );
+		flow_note( w, dynamic_index( w, bd.y ), col, 0, 1, false );
+	}
+	for ( int e = tid; e < novfJ; e += stride )
+	{
+		int j = w.overflowJoints[e];
+		int2 pl = w.jointPlace[j];
+		w.ovfItems[sOverflow[pl.x] + pl.y] = e;
+		int2 bd = w.jbody[j];
+		flow_note( w, dynamic_index( w, bd.x ), F2D_OVERFLOW, e, 0, false );
+		flow_note( w, dynamic_index( w, bd.y ), F2D_OVERFLOW, e, 1, false );
+	}
+	float warmStartScale = p.enableWarmStarting ? 1.0f : 0.0f;
+	const int nc = w.sc->contactIdCount;
+	for ( int c = tid; c < nc; c += stride )
+	{
+		const int col = w.ccolor[c];
+		if ( col < 0 || ( w.cflags[c] & CF_USED ) == 0 )
+			continue;
+		int2 pl = w.slotPlace[c];
+		int k;
+		if ( col < F2D_OVERFLOW )
+			k = 32 * ( firstGroup + sContact[pl.x] ) + pl.y;
+		else
+		{
+			k = w.coverflowIndex[c];
+			w.ovfItems[sOverflow[pl.x] + pl.y] = novfJ + k;
+		}
+		if ( k < 0 || k >= w.slotCap )
+		{
+			atomicOr( &w.sc->error, ERR_CONTACT_CAPACITY );
+			continue;
+		}
 		int2 bd = w.cbody[c];
-		int ia = body_type( w.bflags[bd.x] ) == 0 ? -1 : bd.x;
-		int ib = body_type( w.bflags[bd.y] ) == 0 ? -1 : bd.y;
+		int ia = dynamic_index( w, bd.x );
+		int ib = dynamic_index( w, bd.y );
 		float4 cm = w.cmass[c];
 		float mA = cm.x, iA = cm.y, mB = cm.z, iB = cm.w;
 		// constraint_graph.c:139-181: a static side carries zero mass
@@ -161,16 +409,18 @@ __global__ void k_prepare_contacts( DWorld w, SolveParams p )
 		}
 		float kk = iA + iB;
 		float rollingMass = kk > 0.0f ? 1.0f / kk : 0.0f;
-		Soft soft = ( ia < 0 || ib < 0 ) ? p.staticSoft : p.contactSoft;
 		float4 mn = w.mnorm[c];
 		fv2 normal = mk( mn.x, mn.y );
 		int pointCount = __float_as_int( mn.w );
 		float4 cmat = w.cmat[c];
-		w.kIndex[k] = make_int2( ia, ib );
-		w.kMass[k] = make_float4( mA, iA, mB, iB );
-		w.kNormal[k] = make_float4( normal.x, normal.y, cmat.x, cmat.w );
-		w.kMisc[k] = make_float4( cmat.y, cmat.z, rollingMass, warmStartScale * mn.z );
-		w.kSoft[k] = make_float4( soft.biasRate, soft.massScale, soft.impulseScale, __int_as_float( pointCount ) );
+		flow_note( w, ia, col, novfJ + k, 0, cmat.y != 0.0f );
+		flow_note( w, ib, col, novfJ + k, 1, cmat.y != 0.0f );
+		float4* row = krow( w, k, 0 );
+		row[32 * KR_HEAD] = make_float4( __int_as_float( ia ), __int_as_float( ib ), __int_as_float( c ),
+										 __int_as_float( pointCount ) );
+		row[32 * KR_MASS] = make_float4( mA, iA, mB, iB );
+		row[32 * KR_NORMAL] = make_float4( normal.x, normal.y, cmat.x, cmat.w );
+		row[32 * KR_MISC] = make_float4( cmat.y, cmat.z, rollingMass, warmStartScale * mn.z );
 		fv2 tangent = vright( normal );
 		float4 anch[2], pp[2];
 		float ni[2], ti[2];
@@ -227,60 +477,157 @@ __global__ void k_prepare_contacts( DWorld w, SolveParams p )
 				}
 			}
 		}
-		w.kAnch1[k] = anch[0];
-		w.kAnch2[k] = anch[1];
-		w.kP1[k] = pp[0];
-		w.kP2[k] = pp[1];
-		w.kImp[k] = make_float4( ni[0], ni[1], ti[0], ti[1] );
-		w.kTot[k] = make_float2( 0.0f, 0.0f );
+		row[32 * KR_ANCH1] = anch[0];
+		row[32 * KR_ANCH2] = anch[1];
+		row[32 * KR_P1] = pp[0];
+		row[32 * KR_P2] = pp[1];
+		row[32 * KR_IMP] = make_float4( ni[0], ni[1], ti[0], ti[1] );
+		row[32 * KR_TOT] = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
 	}
 }
 
-// ---------------------------------------------------------------------------
-// body state access: static bodies read as the identity state and are never
-// written (contact_solver.c:1184-1222)
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ BState load_state( const DWorld& w, int i )
+// The operation counts at zero and the substep deltas unwritten again, for
+// the next launch of a step with more than FLOW_SUBSTEPS substeps.
+__global__ void k_solver_refill( DWorld w, int subSteps )
 {
-	BState s;
-	if ( i < 0 )
+	const float sentinel = __uint_as_float( FLOW_SENTINEL );
+	for ( int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.bodyCount; b += gridDim.x * blockDim.x )
 	{
-		s.vx = s.vy = s.w = 0.0f;
-		s.dpx = s.dpy = 0.0f;
-		s.dqc = 1.0f;
-		s.dqs = 0.0f;
-		return s;
+		w.vel[b].w = 0.0f;
+		for ( int s = 0; s < subSteps; ++s )
+			w.dsub[(size_t)s * w.bodyCount + b] = make_float4( sentinel, sentinel, sentinel, sentinel );
 	}
-	float4 v = __ldcg( w.vel + i );
-	float4 d = __ldcg( w.delta + i );
-	s.vx = v.x;
-	s.vy = v.y;
-	s.w = v.z;
-	s.dpx = d.x;
-	s.dpy = d.y;
-	s.dqc = d.z;
-	s.dqs = d.w;
-	return s;
 }
 
-__device__ __forceinline__ void store_vel( const DWorld& w, int i, const BState& s )
+// ---------------------------------------------------------------------------
+// The solver proper: constraints as a data flow over the bodies' velocity
+// rows, in one persistent launch.
+//
+// The reference runs its stages (per substep: warm start, solve, relax; then
+// restitution) one after another, each as overflow joints, overflow contacts
+// and the colours 0..10 in turn (solver.c:929-1160). All that order decides is
+// in which order a body meets its constraints: two constraints without a
+// common non-static body commute. So no stage is separated from the next by a
+// barrier here. Every body's velocity row carries, in its fourth word, the
+// number of constraint operations the body has been through in this launch; a
+// constraint with the body's rank r among its d constraints runs its stage-s
+// operation when that count reads s * d + r, and stores the row back with the
+// count one higher. The row travels as one 16-byte relaxed access, so a row
+// that shows the awaited count also shows its velocity, and no fence is
+// needed. The per-substep position deltas go through rows written once per
+// launch (filled with a pattern no delta has), which a reader polls the same
+// way. Velocity integration is done by a body's first warm start, position
+// integration by its last solve; bodies without constraints are integrated by
+// a thread of their own.
+//
+// The bodies are dealt to the blocks in runs of their spatial order, and a
+// constraint is solved in the (lower) part of its bodies. A body whose
+// constraints all lie in one part lives in that block's shared memory for the
+// launch; only bodies on the parts' borders go through global memory (L2).
+// A warp takes up to 32 constraints of one part and colour at a time, which
+// touch disjoint bodies, waits for all their bodies and runs them together.
+//
+// No wait is endless: every warp takes its groups in the order (stage,
+// overflow joints, overflow contacts, colour), each waits only for operations
+// that precede it in that order, and all blocks are resident, so the first
+// unfinished group of that order is always at the head of its warp and its
+// wait ends. Polls are counted all the same: a warp that makes no progress
+// for FLOW_SPIN_LIMIT polls raises the timeout bit and leaves, as do the
+// others when they see the bit.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float4 unpack_row( unsigned long long lo, unsigned long long hi )
 {
-	if ( i < 0 )
-		return;
-	__stcg( w.vel + i, make_float4( s.vx, s.vy, s.w, 0.0f ) );
+	return make_float4( __uint_as_float( (unsigned)lo ), __uint_as_float( (unsigned)( lo >> 32 ) ),
+						__uint_as_float( (unsigned)hi ), __uint_as_float( (unsigned)( hi >> 32 ) ) );
 }
 
-// Body state access of the solver stages. GBodies reads and writes the device
-// rows through L2 (.cg); CBodies reads and writes the copy of the body rows
-// held in the distributed shared memory of a thread-block cluster (body b in
-// block b % F2D_CLUSTER of the cluster, slot b / F2D_CLUSTER; see
-// k_solve_cluster). Static bodies (index < 0) read as the identity state and
-// are never written.
-struct GBodies
+__device__ __forceinline__ float4 ld_row( const float4* p )
 {
-	float4* vel;
-	float4* delta;
+	unsigned long long lo, hi;
+	asm volatile( "{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+				  : "=l"( lo ), "=l"( hi )
+				  : "l"( p )
+				  : "memory" );
+	return unpack_row( lo, hi );
+}
+
+__device__ __forceinline__ float4 ld_row_shared( unsigned a )
+{
+	unsigned long long lo, hi;
+	asm volatile( "{ .reg .b128 t; ld.relaxed.cta.shared::cta.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+				  : "=l"( lo ), "=l"( hi )
+				  : "r"( a )
+				  : "memory" );
+	return unpack_row( lo, hi );
+}
+
+__device__ __forceinline__ void st_row( float4* p, float4 v )
+{
+	unsigned long long lo = __float_as_uint( v.x ) | ( (unsigned long long)__float_as_uint( v.y ) << 32 );
+	unsigned long long hi = __float_as_uint( v.z ) | ( (unsigned long long)__float_as_uint( v.w ) << 32 );
+	asm volatile( "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"( p ), "l"( lo ),
+				  "l"( hi )
+				  : "memory" );
+}
+
+__device__ __forceinline__ void st_row_shared( unsigned a, float4 v )
+{
+	unsigned long long lo = __float_as_uint( v.x ) | ( (unsigned long long)__float_as_uint( v.y ) << 32 );
+	unsigned long long hi = __float_as_uint( v.z ) | ( (unsigned long long)__float_as_uint( v.w ) << 32 );
+	asm volatile( "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.cta.shared::cta.b128 [%0], t; }" ::"r"( a ), "l"( lo ),
+				  "l"( hi )
+				  : "memory" );
+}
+
+// Body rows: `slot` is the body's place in this block's shared memory, or
+// FLOW_NO_SLOT for a body in global memory.
+#define FLOW_NO_SLOT 0xffff
+struct Rows
+{
+	unsigned base; // shared address: velocities of all slots, then per delta row all slots
+	unsigned stride; // bytes from one row kind to the next
+	float4* vels;
+	float4* deltas;
+	float4* dsub;
+	size_t cap;
+	__device__ __forceinline__ float4 vel( int b, int slot ) const
+	{
+		return slot != FLOW_NO_SLOT ? ld_row_shared( base + 16u * (unsigned)slot ) : ld_row( vels + b );
+	}
+	__device__ __forceinline__ void put_vel( int b, int slot, float4 v ) const
+	{
+		if ( slot != FLOW_NO_SLOT )
+			st_row_shared( base + 16u * (unsigned)slot, v );
+		else
+			st_row( vels + b, v );
+	}
+	// delta after s substeps of the launch
+	__device__ __forceinline__ float4 delta( int s, int b, int slot ) const
+	{
+		if ( slot != FLOW_NO_SLOT )
+			return ld_row_shared( base + stride * (unsigned)( 1 + s ) + 16u * (unsigned)slot );
+		return s == 0 ? __ldcg( deltas + b ) : ld_row( dsub + ( s - 1 ) * cap + b );
+	}
+	__device__ __forceinline__ void put_delta( int s, bool last, int b, int slot, float4 d ) const
+	{
+		if ( slot != FLOW_NO_SLOT )
+			st_row_shared( base + stride * (unsigned)( 1 + s ) + 16u * (unsigned)slot, d );
+		else
+		{
+			st_row( dsub + ( s - 1 ) * cap + b, d );
+			if ( last )
+				__stcg( deltas + b, d );
+		}
+	}
+};
+
+// The two bodies of a joint or overflow contact, in registers: what their
+// functions load and store. Static bodies (index < 0) read as the identity
+// state and are never written (contact_solver.c:1184-1222).
+struct PairBodies
+{
+	int ia, ib;
+	mutable BState a, b;
 	__device__ __forceinline__ BState load( int i ) const
 	{
 		BState s;
@@ -292,661 +639,31 @@ struct GBodies
 			s.dqs = 0.0f;
 			return s;
 		}
-		float4 v = __ldcg( vel + i );
-		float4 d = __ldcg( delta + i );
-		s.vx = v.x;
-		s.vy = v.y;
-		s.w = v.z;
-		s.dpx = d.x;
-		s.dpy = d.y;
-		s.dqc = d.z;
-		s.dqs = d.w;
-		return s;
+		return i == ia ? a : b;
 	}
 	__device__ __forceinline__ void store( int i, const BState& s ) const
 	{
-		if ( i >= 0 )
-			__stcg( vel + i, make_float4( s.vx, s.vy, s.w, 0.0f ) );
-	}
-};
-
-#define F2D_CLUSTER 16
-
-__device__ __forceinline__ unsigned dsm_map( unsigned localAddr, unsigned rank )
-{
-	unsigned r;
-	asm volatile( "mapa.shared::cluster.u32 %0, %1, %2;" : "=r"( r ) : "r"( localAddr ), "r"( rank ) );
-	return r;
-}
-
-__device__ __forceinline__ float4 dsm_ld4( unsigned addr )
-{
-	float4 v;
-	asm volatile( "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-				  : "=f"( v.x ), "=f"( v.y ), "=f"( v.z ), "=f"( v.w )
-				  : "r"( addr )
-				  : "memory" );
-	return v;
-}
-
-__device__ __forceinline__ void dsm_st4( unsigned addr, float4 v )
-{
-	asm volatile( "st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"( addr ), "f"( v.x ), "f"( v.y ), "f"( v.z ),
-				  "f"( v.w )
-				  : "memory" );
-}
-
-struct CBodies
-{
-	unsigned base; // shared::cta address of this block's slots (vel, delta per slot)
-	__device__ __forceinline__ unsigned addr( int i ) const
-	{
-		return dsm_map( base + 32u * (unsigned)( i / F2D_CLUSTER ), (unsigned)( i % F2D_CLUSTER ) );
-	}
-	__device__ __forceinline__ BState load( int i ) const
-	{
-		BState s;
 		if ( i < 0 )
-		{
-			s.vx = s.vy = s.w = 0.0f;
-			s.dpx = s.dpy = 0.0f;
-			s.dqc = 1.0f;
-			s.dqs = 0.0f;
-			return s;
-		}
-		unsigned a = addr( i );
-		float4 v = dsm_ld4( a );
-		float4 d = dsm_ld4( a + 16u );
-		s.vx = v.x;
-		s.vy = v.y;
-		s.w = v.z;
-		s.dpx = d.x;
-		s.dpy = d.y;
-		s.dqc = d.z;
-		s.dqs = d.w;
-		return s;
-	}
-	__device__ __forceinline__ void store( int i, const BState& s ) const
-	{
-		if ( i >= 0 )
-			dsm_st4( addr( i ), make_float4( s.vx, s.vy, s.w, 0.0f ) );
+			return;
+		BState& t = i == ia ? a : b;
+		t.vx = s.vx;
+		t.vy = s.vy;
+		t.w = s.w;
 	}
 };
 
-__device__ __forceinline__ float lmax( float a, float b )
+// Velocity integration over a substep (solver.c:65-130) with the factors of
+// k_solver_count.
+__device__ __forceinline__ void integrate_velocity( const DWorld& w, const SolveParams& p, int b, BState& s )
 {
-	return a > b ? a : b;
-}
-__device__ __forceinline__ float lmin( float a, float b )
-{
-	return a < b ? a : b;
-}
-
-// A graph-colour constraint held in registers for the whole solver launch:
-// its static rows are read once, its impulses accumulate in place and are
-// written back once (see k_solve).
-struct Lane
-{
-	int2 idx;
-	float4 ms;	 // invMassA invIA invMassB invIB
-	float4 nm;	 // normal.xy friction tangentSpeed
-	float4 sf;	 // biasRate massScale impulseScale pointCount
-	float4 misc; // restitution rollingResistance rollingMass rollingImpulse
-	float4 imp;	 // normalImpulse1 normalImpulse2 tangentImpulse1 tangentImpulse2
-	float2 tot;	 // totalNormalImpulse1 totalNormalImpulse2
-	float4 an[2];
-	float4 pt[2];
-};
-
-__device__ __forceinline__ void lane_load( const DWorld& w, int k, Lane& L )
-{
-	L.idx = w.kIndex[k];
-	L.ms = w.kMass[k];
-	L.nm = w.kNormal[k];
-	L.sf = w.kSoft[k];
-	L.misc = __ldcg( w.kMisc + k );
-	L.imp = __ldcg( w.kImp + k );
-	L.tot = __ldcg( w.kTot + k );
-	L.an[0] = w.kAnch1[k];
-	L.an[1] = w.kAnch2[k];
-	L.pt[0] = w.kP1[k];
-	L.pt[1] = w.kP2[k];
-}
-
-__device__ __forceinline__ void lane_store( const DWorld& w, int k, const Lane& L )
-{
-	__stcg( w.kImp + k, L.imp );
-	__stcg( w.kTot + k, L.tot );
-	__stcg( w.kMisc + k, L.misc );
-}
-
-// contact_solver.c:1671-1727
-template <class BA> __device__ __forceinline__ void lane_warm( const BA& ba, const Lane& L )
-{
-	BState A = ba.load( L.idx.x ), B = ba.load( L.idx.y );
-	const float4 ms = L.ms, nm = L.nm;
-	float tx = nm.y;
-	float ty = 0.0f - nm.x;
-	float nis[2] = { L.imp.x, L.imp.y };
-	float tis[2] = { L.imp.z, L.imp.w };
-	for ( int j = 0; j < 2; ++j )
-	{
-		float rAx = L.an[j].x, rAy = L.an[j].y, rBx = L.an[j].z, rBy = L.an[j].w;
-		float Px = nis[j] * nm.x + tis[j] * tx;
-		float Py = nis[j] * nm.y + tis[j] * ty;
-		A.w = A.w - ms.y * ( rAx * Py - rAy * Px );
-		A.vx = A.vx - ms.x * Px;
-		A.vy = A.vy - ms.x * Py;
-		B.w = B.w + ms.w * ( rBx * Py - rBy * Px );
-		B.vx = B.vx + ms.z * Px;
-		B.vy = B.vy + ms.z * Py;
-	}
-	A.w = A.w - ms.y * L.misc.w;
-	B.w = B.w + ms.w * L.misc.w;
-	ba.store( L.idx.x, A );
-	ba.store( L.idx.y, B );
-}
-
-// contact_solver.c:1729-1967
-template <class BA>
-__device__ __forceinline__ void lane_solve( const BA& ba, Lane& L, float inv_h, float minBiasVel, bool useBias )
-{
-	BState A = ba.load( L.idx.x ), B = ba.load( L.idx.y );
-	const float4 ms = L.ms, nm = L.nm, sf = L.sf;
-	float4 misc = L.misc;
-	float biasRate, massScale, impulseScale;
-	if ( useBias )
-	{
-		biasRate = sf.x;
-		massScale = sf.y;
-		impulseScale = sf.z;
-	}
-	else
-	{
-		biasRate = 0.0f;
-		massScale = 1.0f;
-		impulseScale = 0.0f;
-	}
-	float totalNormalImpulse = 0.0f;
-	float dpx = B.dpx - A.dpx;
-	float dpy = B.dpy - A.dpy;
-	float nis[2] = { L.imp.x, L.imp.y };
-	float tis[2] = { L.imp.z, L.imp.w };
-	float tots[2] = { L.tot.x, L.tot.y };
-	for ( int j = 0; j < 2; ++j )
-	{
-		float rAx = L.an[j].x, rAy = L.an[j].y, rBx = L.an[j].z, rBy = L.an[j].w;
-		float rsAx = A.dqc * rAx - A.dqs * rAy;
-		float rsAy = A.dqs * rAx + A.dqc * rAy;
-		float rsBx = B.dqc * rBx - B.dqs * rBy;
-		float rsBy = B.dqs * rBx + B.dqc * rBy;
-		float dsx = dpx + ( rsBx - rsAx );
-		float dsy = dpy + ( rsBy - rsAy );
-		float s = ( nm.x * dsx + nm.y * dsy ) + L.pt[j].x;
-		bool mask = s > 0.0f;
-		float specBias = s * inv_h;
-		float softBias = lmax( biasRate * s, minBiasVel );
-		float bias = mask ? specBias : softBias;
-		float pointMassScale = mask ? 1.0f : massScale;
-		float pointImpulseScale = mask ? 0.0f : impulseScale;
-		float dvx = ( B.vx - B.w * rBy ) - ( A.vx - A.w * rAy );
-		float dvy = ( B.vy + B.w * rBx ) - ( A.vy + A.w * rAx );
-		float vn = dvx * nm.x + dvy * nm.y;
-		float negImpulse = L.pt[j].y * ( pointMassScale * ( vn + bias ) ) + pointImpulseScale * nis[j];
-		float newImpulse = lmax( nis[j] - negImpulse, 0.0f );
-		float impulse = newImpulse - nis[j];
-		nis[j] = newImpulse;
-		tots[j] = tots[j] + newImpulse;
-		totalNormalImpulse = totalNormalImpulse + newImpulse;
-		float Px = impulse * nm.x;
-		float Py = impulse * nm.y;
-		A.vx = A.vx - ms.x * Px;
-		A.vy = A.vy - ms.x * Py;
-		A.w = A.w - ms.y * ( rAx * Py - rAy * Px );
-		B.vx = B.vx + ms.z * Px;
-		B.vy = B.vy + ms.z * Py;
-		B.w = B.w + ms.w * ( rBx * Py - rBy * Px );
-	}
-	float tx = nm.y;
-	float ty = 0.0f - nm.x;
-	for ( int j = 0; j < 2; ++j )
-	{
-		float rAx = L.an[j].x, rAy = L.an[j].y, rBx = L.an[j].z, rBy = L.an[j].w;
-		float dvx = ( B.vx - B.w * rBy ) - ( A.vx - A.w * rAy );
-		float dvy = ( B.vy + B.w * rBx ) - ( A.vy + A.w * rAx );
-		float vt = dvx * tx + dvy * ty;
-		vt = vt - nm.w;
-		float negImpulse = L.pt[j].z * vt;
-		float maxFriction = nm.z * nis[j];
-		float newImpulse = tis[j] - negImpulse;
-		newImpulse = lmax( 0.0f - maxFriction, lmin( newImpulse, maxFriction ) );
-		float impulse = newImpulse - tis[j];
-		tis[j] = newImpulse;
-		float Px = impulse * tx;
-		float Py = impulse * ty;
-		A.vx = A.vx - ms.x * Px;
-		A.vy = A.vy - ms.x * Py;
-		A.w = A.w - ms.y * ( rAx * Py - rAy * Px );
-		B.vx = B.vx + ms.z * Px;
-		B.vy = B.vy + ms.z * Py;
-		B.w = B.w + ms.w * ( rBx * Py - rBy * Px );
-	}
-	{
-		float deltaLambda = misc.z * ( A.w - B.w );
-		float lambda = misc.w;
-		float maxLambda = misc.y * totalNormalImpulse;
-		float nb = -maxLambda;
-		float r = lmax( nb, lmin( lambda + deltaLambda, maxLambda ) );
-		misc.w = r;
-		deltaLambda = r - lambda;
-		A.w = A.w - ms.y * deltaLambda;
-		B.w = B.w + ms.w * deltaLambda;
-	}
-	L.imp = make_float4( nis[0], nis[1], tis[0], tis[1] );
-	L.tot = make_float2( tots[0], tots[1] );
-	L.misc = misc;
-	ba.store( L.idx.x, A );
-	ba.store( L.idx.y, B );
-}
-
-// contact_solver.c:1969-2076 (lanes with restitution 0 are unchanged)
-template <class BA> __device__ __forceinline__ void lane_restitution( const BA& ba, Lane& L, float threshold )
-{
-	float restitution = L.misc.x;
-	if ( restitution == 0.0f )
+	float4 r0 = w.bodyInt[2 * (size_t)b], r1 = w.bodyInt[2 * (size_t)b + 1];
+	int flags = __float_as_int( r1.y );
+	if ( ( flags & BI_AWAKE ) == 0 )
 		return;
-	BState A = ba.load( L.idx.x ), B = ba.load( L.idx.y );
-	const float4 ms = L.ms, nm = L.nm;
-	float nis[2] = { L.imp.x, L.imp.y };
-	float tots[2] = { L.tot.x, L.tot.y };
-	for ( int j = 0; j < 2; ++j )
-	{
-		bool mask1 = ( L.pt[j].w + threshold ) > 0.0f;
-		bool mask2 = tots[j] == 0.0f;
-		float mass = ( mask1 || mask2 ) ? 0.0f : L.pt[j].y;
-		float rAx = L.an[j].x, rAy = L.an[j].y, rBx = L.an[j].z, rBy = L.an[j].w;
-		float dvx = ( B.vx - B.w * rBy ) - ( A.vx - A.w * rAy );
-		float dvy = ( B.vy + B.w * rBx ) - ( A.vy + A.w * rAx );
-		float vn = dvx * nm.x + dvy * nm.y;
-		float negImpulse = mass * ( vn + restitution * L.pt[j].w );
-		float newImpulse = lmax( nis[j] - negImpulse, 0.0f );
-		float impulse = newImpulse - nis[j];
-		nis[j] = newImpulse;
-		float Px = impulse * nm.x;
-		float Py = impulse * nm.y;
-		A.vx = A.vx - ms.x * Px;
-		A.vy = A.vy - ms.x * Py;
-		A.w = A.w - ms.y * ( rAx * Py - rAy * Px );
-		B.vx = B.vx + ms.z * Px;
-		B.vy = B.vy + ms.z * Py;
-		B.w = B.w + ms.w * ( rBx * Py - rBy * Px );
-	}
-	L.imp.x = nis[0];
-	L.imp.y = nis[1];
-	ba.store( L.idx.x, A );
-	ba.store( L.idx.y, B );
-}
-
-// contact_solver.c:160-225
-template <class BA> static __device__ void warm_overflow( const DWorld& w, const BA& ba, int k )
-{
-	int2 idx = w.kIndex[k];
-	BState A = ba.load( idx.x ), B = ba.load( idx.y );
-	float4 ms = w.kMass[k];
-	float4 nm = w.kNormal[k];
-	float4 imp = __ldcg( w.kImp + k );
-	float4 misc = __ldcg( w.kMisc + k );
-	int count = __float_as_int( w.kSoft[k].w );
-	fv2 normal = mk( nm.x, nm.y );
-	fv2 tangent = vright( normal );
-	fv2 vA = mk( A.vx, A.vy ), vB = mk( B.vx, B.vy );
-	float wA = A.w, wB = B.w;
-	float4 an[2] = { w.kAnch1[k], w.kAnch2[k] };
-	float nis[2] = { imp.x, imp.y };
-	float tis[2] = { imp.z, imp.w };
-	for ( int j = 0; j < count; ++j )
-	{
-		fv2 rA = mk( an[j].x, an[j].y ), rB = mk( an[j].z, an[j].w );
-		fv2 P = vadd( vscale( nis[j], normal ), vscale( tis[j], tangent ) );
-		wA -= ms.y * vcross( rA, P );
-		vA = vmuladd( vA, -ms.x, P );
-		wB += ms.w * vcross( rB, P );
-		vB = vmuladd( vB, ms.z, P );
-	}
-	wA -= ms.y * misc.w;
-	wB += ms.w * misc.w;
-	A.vx = vA.x;
-	A.vy = vA.y;
-	A.w = wA;
-	B.vx = vB.x;
-	B.vy = vB.y;
-	B.w = wB;
-	ba.store( idx.x, A );
-	ba.store( idx.y, B );
-}
-
-// contact_solver.c:227-380
-template <class BA>
-static __device__ void solve_overflow( const DWorld& w, const BA& ba, int k, float inv_h, float pushout, bool useBias )
-{
-	int2 idx = w.kIndex[k];
-	BState A = ba.load( idx.x ), B = ba.load( idx.y );
-	float4 ms = w.kMass[k];
-	float mA = ms.x, iA = ms.y, mB = ms.z, iB = ms.w;
-	float4 nm = w.kNormal[k];
-	float4 sf = w.kSoft[k];
-	float4 misc = __ldcg( w.kMisc + k );
-	float4 imp = __ldcg( w.kImp + k );
-	float2 tot = __ldcg( w.kTot + k );
-	int count = __float_as_int( sf.w );
-	fv2 vA = mk( A.vx, A.vy ), vB = mk( B.vx, B.vy );
-	float wA = A.w, wB = B.w;
-	frot dqA, dqB;
-	dqA.c = A.dqc;
-	dqA.s = A.dqs;
-	dqB.c = B.dqc;
-	dqB.s = B.dqs;
-	fv2 dp = vsub( mk( B.dpx, B.dpy ), mk( A.dpx, A.dpy ) );
-	fv2 normal = mk( nm.x, nm.y );
-	fv2 tangent = vright( normal );
-	float friction = nm.z;
-	float totalNormalImpulse = 0.0f;
-	float4 an[2] = { w.kAnch1[k], w.kAnch2[k] };
-	float4 pt[2] = { w.kP1[k], w.kP2[k] };
-	float nis[2] = { imp.x, imp.y };
-	float tis[2] = { imp.z, imp.w };
-	float tots[2] = { tot.x, tot.y };
-	for ( int j = 0; j < count; ++j )
-	{
-		fv2 rA = mk( an[j].x, an[j].y ), rB = mk( an[j].z, an[j].w );
-		fv2 ds = vadd( dp, vsub( rrot( dqB, rB ), rrot( dqA, rA ) ) );
-		float s = pt[j].x + vdot( ds, normal );
-		float velocityBias = 0.0f;
-		float massScale = 1.0f;
-		float impulseScale = 0.0f;
-		if ( s > 0.0f )
-			velocityBias = s * inv_h;
-		else if ( useBias )
-		{
-			velocityBias = fmax_s( sf.x * s, -pushout );
-			massScale = sf.y;
-			impulseScale = sf.z;
-		}
-		fv2 vrA = vadd( vA, vcrossSV( wA, rA ) );
-		fv2 vrB = vadd( vB, vcrossSV( wB, rB ) );
-		float vn = vdot( vsub( vrB, vrA ), normal );
-		float impulse = -pt[j].y * massScale * ( vn + velocityBias ) - impulseScale * nis[j];
-		float newImpulse = fmax_s( nis[j] + impulse, 0.0f );
-		impulse = newImpulse - nis[j];
-		nis[j] = newImpulse;
-		tots[j] += newImpulse;
-		totalNormalImpulse += newImpulse;
-		fv2 P = vscale( impulse, normal );
-		vA = vmulsub( vA, mA, P );
-		wA -= iA * vcross( rA, P );
-		vB = vmuladd( vB, mB, P );
-		wB += iB * vcross( rB, P );
-	}
-	for ( int j = 0; j < count; ++j )
-	{
-		fv2 rA = mk( an[j].x, an[j].y ), rB = mk( an[j].z, an[j].w );
-		fv2 vrB = vadd( vB, vcrossSV( wB, rB ) );
-		fv2 vrA = vadd( vA, vcrossSV( wA, rA ) );
-		float vt = vdot( vsub( vrB, vrA ), tangent ) - nm.w;
-		float impulse = pt[j].z * ( -vt );
-		float maxFriction = friction * nis[j];
-		float newImpulse = fclamp_s( tis[j] + impulse, -maxFriction, maxFriction );
-		impulse = newImpulse - tis[j];
-		tis[j] = newImpulse;
-		fv2 P = vscale( impulse, tangent );
-		vA = vmulsub( vA, mA, P );
-		wA -= iA * vcross( rA, P );
-		vB = vmuladd( vB, mB, P );
-		wB += iB * vcross( rB, P );
-	}
-	{
-		float deltaLambda = -misc.z * ( wB - wA );
-		float lambda = misc.w;
-		float maxLambda = misc.y * totalNormalImpulse;
-		misc.w = fclamp_s( lambda + deltaLambda, -maxLambda, maxLambda );
-		deltaLambda = misc.w - lambda;
-		wA -= iA * deltaLambda;
-		wB += iB * deltaLambda;
-	}
-	__stcg( w.kImp + k, make_float4( nis[0], nis[1], tis[0], tis[1] ) );
-	__stcg( w.kTot + k, make_float2( tots[0], tots[1] ) );
-	__stcg( w.kMisc + k, misc );
-	A.vx = vA.x;
-	A.vy = vA.y;
-	A.w = wA;
-	B.vx = vB.x;
-	B.vy = vB.y;
-	B.w = wB;
-	ba.store( idx.x, A );
-	ba.store( idx.y, B );
-}
-
-// contact_solver.c:382-478
-template <class BA> static __device__ void restitution_overflow( const DWorld& w, const BA& ba, int k, float threshold )
-{
-	float4 misc = __ldcg( w.kMisc + k );
-	float restitution = misc.x;
-	if ( restitution == 0.0f )
-		return;
-	int2 idx = w.kIndex[k];
-	BState A = ba.load( idx.x ), B = ba.load( idx.y );
-	float4 ms = w.kMass[k];
-	float mA = ms.x, iA = ms.y, mB = ms.z, iB = ms.w;
-	float4 nm = w.kNormal[k];
-	int count = __float_as_int( w.kSoft[k].w );
-	float4 imp = __ldcg( w.kImp + k );
-	float2 tot = __ldcg( w.kTot + k );
-	fv2 vA = mk( A.vx, A.vy ), vB = mk( B.vx, B.vy );
-	float wA = A.w, wB = B.w;
-	fv2 normal = mk( nm.x, nm.y );
-	float4 an[2] = { w.kAnch1[k], w.kAnch2[k] };
-	float4 pt[2] = { w.kP1[k], w.kP2[k] };
-	float nis[2] = { imp.x, imp.y };
-	float tots[2] = { tot.x, tot.y };
-	for ( int j = 0; j < count; ++j )
-	{
-		if ( pt[j].w > -threshold || tots[j] == 0.0f )
-			continue;
-		fv2 rA = mk( an[j].x, an[j].y ), rB = mk( an[j].z, an[j].w );
-		fv2 vrB = vadd( vB, vcrossSV( wB, rB ) );
-		fv2 vrA = vadd( vA, vcrossSV( wA, rA ) );
-		float vn = vdot( vsub( vrB, vrA ), normal );
-		float impulse = -pt[j].y * ( vn + restitution * pt[j].w );
-		float newImpulse = fmax_s( nis[j] + impulse, 0.0f );
-		impulse = newImpulse - nis[j];
-		nis[j] = newImpulse;
-		tots[j] += impulse;
-		fv2 P = vscale( impulse, normal );
-		vA = vmulsub( vA, mA, P );
-		wA -= iA * vcross( rA, P );
-		vB = vmuladd( vB, mB, P );
-		wB += iB * vcross( rB, P );
-	}
-	__stcg( w.kImp + k, make_float4( nis[0], nis[1], imp.z, imp.w ) );
-	__stcg( w.kTot + k, make_float2( tots[0], tots[1] ) );
-	A.vx = vA.x;
-	A.vy = vA.y;
-	A.w = wA;
-	B.vx = vB.x;
-	B.vy = vB.y;
-	B.w = wB;
-	ba.store( idx.x, A );
-	ba.store( idx.y, B );
-}
-
-// ---------------------------------------------------------------------------
-// Overflow levels. The reference solves the overflow joints and then the
-// overflow contacts one after another on its main thread (solver.c:1008-1009,
-// 1027-1028, 1055-1056, 1077). Here those constraints are split into levels:
-// constraint e (joints first, then contacts, each in overflow-array order)
-// joins level r when every earlier overflow constraint that shares a
-// non-static body with it sits in a level below r (as-soon-as-possible
-// scheduling of each body's constraint order). Constraints of one level touch
-// disjoint bodies and every body meets its constraints in the serial order,
-// so one block solving the levels one after another, with a block barrier
-// between levels, produces the serial sweep's values bit for bit.
-#define OVF_MAX_LEVELS 64	 // rounds of level assignment; the rest go serial
-#define OVF_SMEM_ITEMS 3072 // level-ordered list kept in shared memory
-
-struct OvfPlan
-{
-	const int* order; // constraints in level order
-	int levels;		  // parallel levels
-	int n;			  // overflow joints + contacts
-	int nj;			  // overflow joints
-};
-
-static __device__ __forceinline__ int2 ovf_bodies( const DWorld& w, int e, int nj )
-{
-	return e < nj ? w.jindex[w.overflowJoints[e]] : w.kIndex[e - nj];
-}
-
-// All threads of one block. Writes the level-ordered list into order (n
-// entries) and the level starts into levelStart (OVF_MAX_LEVELS + 1 entries,
-// shared memory). Constraints left after OVF_MAX_LEVELS rounds follow in
-// ascending order as one serial tail.
-static __device__ OvfPlan ovf_schedule( const DWorld& w, int* order, int* levelStart )
-{
-	__shared__ int sPos;
-	OvfPlan plan;
-	plan.nj = w.sc->overflowJointCount;
-	plan.n = plan.nj + w.sc->overflowCount;
-	plan.order = order;
-	const int n = plan.n, nj = plan.nj;
-	int* level = w.ovfLevel;
-	int* owner = w.ovfOwner;
-	for ( int e = threadIdx.x; e < n; e += blockDim.x )
-		__stcg( level + e, -1 );
-	if ( threadIdx.x == 0 )
-	{
-		sPos = 0;
-		levelStart[0] = 0;
-	}
-	__syncthreads();
-	int r = 0;
-	while ( r < OVF_MAX_LEVELS && sPos < n )
-	{
-		for ( int e = threadIdx.x; e < n; e += blockDim.x )
-			if ( __ldcg( level + e ) < 0 )
-			{
-				int2 b = ovf_bodies( w, e, nj );
-				if ( b.x >= 0 )
-					__stcg( owner + b.x, 0x7fffffff );
-				if ( b.y >= 0 )
-					__stcg( owner + b.y, 0x7fffffff );
-			}
-		__syncthreads();
-		for ( int e = threadIdx.x; e < n; e += blockDim.x )
-			if ( __ldcg( level + e ) < 0 )
-			{
-				int2 b = ovf_bodies( w, e, nj );
-				if ( b.x >= 0 )
-					atomicMin( owner + b.x, e );
-				if ( b.y >= 0 )
-					atomicMin( owner + b.y, e );
-			}
-		__syncthreads();
-		for ( int e = threadIdx.x; e < n; e += blockDim.x )
-			if ( __ldcg( level + e ) < 0 )
-			{
-				int2 b = ovf_bodies( w, e, nj );
-				bool first = ( b.x < 0 || __ldcg( owner + b.x ) == e ) && ( b.y < 0 || __ldcg( owner + b.y ) == e );
-				if ( first )
-				{
-					__stcg( level + e, r );
-					order[atomicAdd( &sPos, 1 )] = e;
-				}
-			}
-		__syncthreads();
-		r += 1;
-		if ( threadIdx.x == 0 )
-			levelStart[r] = sPos;
-		__syncthreads();
-	}
-	plan.levels = r;
-	if ( threadIdx.x == 0 && sPos < n )
-	{
-		int pos = sPos;
-		for ( int e = 0; e < n; ++e )
-			if ( __ldcg( level + e ) < 0 )
-				order[pos++] = e;
-	}
-	__syncthreads();
-	return plan;
-}
-
-// kind 0 warm start, 1 solve, 2 relax, 3 restitution (contacts only)
-template <class BA>
-static __device__ __forceinline__ void ovf_item( const DWorld& w, const BA& ba, int e, int nj, int kind,
-												  const SolveParams& p )
-{
-	if ( e < nj )
-	{
-		int j = w.overflowJoints[e];
-		if ( kind == 0 )
-			joint_warm_start( w, ba, j );
-		else if ( kind < 3 )
-			joint_solve( w, ba, j, p.h, p.inv_h, kind == 1 );
-		return;
-	}
-	int k = e - nj;
-	if ( kind == 0 )
-		warm_overflow( w, ba, k );
-	else if ( kind < 3 )
-		solve_overflow( w, ba, k, p.inv_h, p.pushout, kind == 1 );
-	else
-		restitution_overflow( w, ba, k, p.restitutionThreshold );
-}
-
-// All threads of the scheduling block: the overflow constraints level by
-// level, then the serial tail on thread 0.
-template <class BA>
-static __device__ void ovf_stage( const DWorld& w, const BA& ba, const OvfPlan& plan, const int* levelStart, int kind,
-								  const SolveParams& p )
-{
-	for ( int l = 0; l < plan.levels; ++l )
-	{
-		int end = levelStart[l + 1];
-		for ( int i = levelStart[l] + threadIdx.x; i < end; i += blockDim.x )
-			ovf_item( w, ba, plan.order[i], plan.nj, kind, p );
-		__syncthreads();
-	}
-	if ( threadIdx.x == 0 )
-		for ( int i = levelStart[plan.levels]; i < plan.n; ++i )
-			ovf_item( w, ba, plan.order[i], plan.nj, kind, p );
-	__syncthreads();
-}
-
-__device__ __forceinline__ void integrate_velocity( const DWorld& w, int b, const SolveParams& p )
-{
-	float4 v4 = w.vel[b];
-	float4 m = w.massv[b];
-	float4 dmp = w.damp[b];
-	float4 f = w.force[b];
-	float h = p.h;
+	fv2 v = vmuladd( mk( r0.x, r0.y ), r0.z, mk( s.vx, s.vy ) );
+	float wv = r0.w + r1.x * s.w;
 	float maxLinearSpeedSq = p.maxLinearSpeed * p.maxLinearSpeed;
 	float maxAngularSpeedSq = p.maxAngularSpeed * p.maxAngularSpeed;
-	fv2 v = mk( v4.x, v4.y );
-	float wv = v4.z;
-	float linearDamping = 1.0f / ( 1.0f + h * dmp.x );
-	float angularDamping = 1.0f / ( 1.0f + h * dmp.y );
-	float gravityScale = m.x > 0.0f ? dmp.z : 0.0f;
-	fv2 g = p.gravity;
-	if ( w.subCount > 0 )
-	{
-		float2 gb = w.bodyGravity[b];
-		g = mk( gb.x, gb.y );
-	}
-	fv2 lvd = vadd( vscale( h * m.x, mk( f.x, f.y ) ), vscale( h * gravityScale, g ) );
-	float avd = h * m.y * f.z;
-	v = vmuladd( lvd, linearDamping, v );
-	wv = avd + angularDamping * wv;
-	int flags = w.bflags[b];
 	bool capped = false;
 	if ( vdot( v, v ) > maxLinearSpeedSq )
 	{
@@ -954,319 +671,646 @@ __device__ __forceinline__ void integrate_velocity( const DWorld& w, int b, cons
 		v = vscale( ratio, v );
 		capped = true;
 	}
-	if ( wv * wv > maxAngularSpeedSq && ( flags & BF_FAST_ROT ) == 0 )
+	if ( wv * wv > maxAngularSpeedSq && ( flags & BI_FAST_ROT ) == 0 )
 	{
 		float ratio = p.maxAngularSpeed / fabs_s( wv );
 		wv *= ratio;
 		capped = true;
 	}
 	if ( capped )
-		w.bflags[b] = flags | BF_SPEED_CAPPED;
-	w.vel[b] = make_float4( v.x, v.y, wv, 0.0f );
+		w.bflags[b] = __ldcg( w.bflags + b ) | BF_SPEED_CAPPED;
+	s.vx = v.x;
+	s.vy = v.y;
+	s.w = wv;
 }
 
-__device__ __forceinline__ bool body_awake( int f )
+// Position integration over a substep (solver.c:182-200)
+__device__ __forceinline__ float4 integrate_position( const DWorld& w, const SolveParams& p, int b, const BState& s )
 {
-	return ( f & ( BF_USED | BF_ENABLED | BF_ASLEEP ) ) == ( BF_USED | BF_ENABLED ) && body_type( f ) != 0;
-}
-
-template <class BA> __device__ __forceinline__ void lane_op( const BA& ba, Lane& L, int kind, const SolveParams& p )
-{
-	if ( kind == 0 )
-		lane_warm( ba, L );
-	else if ( kind == 1 )
-		lane_solve( ba, L, p.inv_h, p.minBiasVel, true );
-	else if ( kind == 2 )
-		lane_solve( ba, L, p.inv_h, p.minBiasVel, false );
-	else
-		lane_restitution( ba, L, p.restitutionThreshold );
-}
-
-template <class BA>
-__device__ __forceinline__ void joint_colour_stage( const DWorld& w, const BA& ba, int c, int kind, const SolveParams& p,
-													int gtid, int gstride, const int* jointSlots, const int* sJStart )
-{
-	int start = sJStart[c];
-	int count = sJStart[c + 1] - start;
-	for ( int k = gtid; k < count; k += gstride )
-	{
-		int j = jointSlots[start + k];
-		if ( kind == 0 )
-			joint_warm_start( w, ba, j );
-		else if ( kind == 1 )
-			joint_solve( w, ba, j, p.h, p.inv_h, true );
-		else if ( kind == 2 )
-			joint_solve( w, ba, j, p.h, p.inv_h, false );
-	}
+	int flags = __float_as_int( w.bodyInt[2 * (size_t)b + 1].y );
+	if ( ( flags & BI_AWAKE ) == 0 )
+		return make_float4( s.dpx, s.dpy, s.dqc, s.dqs );
+	frot dq;
+	dq.c = s.dqc;
+	dq.s = s.dqs;
+	dq = rintegrate( dq, p.h * s.w );
+	fv2 dp = vmuladd( mk( s.dpx, s.dpy ), p.h, mk( s.vx, s.vy ) );
+	return make_float4( dp.x, dp.y, dq.c, dq.s );
 }
 
 // Manifold write-back of one constraint (contact_solver.c:480-509 overflow,
 // :2078-2120 graph lanes; graph lanes store both points, zeros for a
 // one-point manifold).
-__device__ __forceinline__ void store_manifold( const DWorld& w, int k, float4 imp, float2 tot, float rolling,
-												float rv1, float rv2, int count, bool lane )
+__device__ __forceinline__ void store_manifold( const DWorld& w, int c, float4 imp, float4 tot, float rolling, float rv1,
+												float rv2, bool both )
 {
-	int c = w.slotContact[k];
 	w.mpI[2 * c + 0] = make_float4( imp.x, imp.z, tot.x, rv1 );
-	if ( lane || count > 1 )
+	if ( both )
 		w.mpI[2 * c + 1] = make_float4( imp.y, imp.w, tot.y, rv2 );
-	float4 mn = w.mnorm[c];
-	mn.z = rolling;
-	w.mnorm[c] = mn;
+	w.mnorm[c].z = rolling;
 }
 
-__device__ __forceinline__ void store_manifold_global( const DWorld& w, int k, bool lane )
+// One block's work: its groups of constraints in colour order (a colour's
+// joints, then its contacts) and its overflow constraints.
+#define FLOW_KINDS ( 2 * F2D_OVERFLOW ) // joints of colour c at 2c, contacts at 2c + 1
+#define FLOW_LIST 2048					// groups whose kind is looked up in shared memory
+struct FlowPart
 {
-	float4 imp = __ldcg( w.kImp + k );
-	float2 tot = __ldcg( w.kTot + k );
-	float4 misc = __ldcg( w.kMisc + k );
-	store_manifold( w, k, imp, tot, misc.w, w.kP1[k].w, w.kP2[k].w, __float_as_int( w.kSoft[k].w ), lane );
-}
+	int groupStart[FLOW_KINDS + 1]; // first group of each kind within the part
+	int first[FLOW_KINDS];			// its first joint slot / group of rows
+	int count[FLOW_KINDS];
+	int overflow, overflowFirst; // overflow constraints and their place in ovfSorted
+	unsigned char kind[FLOW_LIST];
+};
 
-// Colour-c constraint slots beyond the register-resident first stride of
-// slots: consecutive threads take consecutive slots (coalesced row loads);
-// their impulses go through the constraint rows between stages.
-template <class BA>
-__device__ __forceinline__ void colour_lanes_extra( const DWorld& w, const BA& ba, int c, const int* sStart,
-													const int* sCount, int novf, int tid, int stride, int kind,
-													const SolveParams& p )
+__device__ __forceinline__ void flow_part( const DWorld& w, const SolveParams& p, int part, FlowPart& f )
 {
-	int lo = max( sStart[c], novf + stride ), hi = sStart[c] + sCount[c];
-	for ( int k = lo + tid; k < hi; k += stride )
+	const int novf = w.sc->overflowCount + w.sc->overflowJointCount;
+	if ( threadIdx.x < FLOW_KINDS )
 	{
-		Lane L;
-		if ( kind == 0 )
-		{
-			// warm start reads no softness or point rows and changes no impulse
-			L.idx = w.kIndex[k];
-			L.ms = w.kMass[k];
-			L.nm = w.kNormal[k];
-			L.misc = __ldcg( w.kMisc + k );
-			L.imp = __ldcg( w.kImp + k );
-			L.an[0] = w.kAnch1[k];
-			L.an[1] = w.kAnch2[k];
-			lane_warm( ba, L );
-			continue;
-		}
-		lane_load( w, k, L );
-		lane_op( ba, L, kind, p );
-		if ( kind == 3 )
-			__stcg( w.kImp + k, L.imp );
-		else
-			lane_store( w, k, L );
+		int k = threadIdx.x, bin = part * F2D_OVERFLOW + ( k >> 1 );
+		bool contacts = k & 1;
+		f.first[k] = contacts ? w.binContactStart[bin] : ( w.jointCount > 0 ? w.binJointStart[bin] : 0 );
+		f.count[k] = contacts ? w.binContacts[bin] : ( w.jointCount > 0 ? w.binJoints[bin] : 0 );
 	}
-}
-
-// Tail colours: the highest active colours, without joints, holding at most
-// TAIL_MAX constraints together. Block 0 runs them one after another with
-// block barriers in between; the grid then needs one barrier for all of
-// them instead of one per colour. A constraint's colour and its colour's
-// place in the order are unchanged, so results are too.
-#define TAIL_MAX 1024
-
-__device__ __forceinline__ int tail_first_colour( const int* sCount, const int* sJStart, unsigned activeMask )
-{
-	int first = F2D_OVERFLOW, colours = 0, total = 0;
-	for ( int c = F2D_OVERFLOW - 1; c >= 0; --c )
+	if ( threadIdx.x == FLOW_KINDS )
 	{
-		if ( ( activeMask & ( 1u << c ) ) == 0 )
-			continue;
-		if ( sJStart[c + 1] > sJStart[c] || total + sCount[c] > TAIL_MAX )
-			break;
-		total += sCount[c];
-		first = c;
-		colours += 1;
+		f.overflow = novf > 0 ? w.binOverflow[part] : 0;
+		f.overflowFirst = novf > 0 ? w.binOverflowStart[part] : 0;
 	}
-	return colours >= 2 ? first : F2D_OVERFLOW;
-}
-
-template <class BA>
-__device__ void tail_stage( const DWorld& w, const BA& ba, const int* sStart, const int* sCount, int first,
-							unsigned activeMask, int kind, const SolveParams& p )
-{
-	for ( int c = first; c < F2D_OVERFLOW; ++c )
-	{
-		if ( ( activeMask & ( 1u << c ) ) == 0 )
-			continue;
-		for ( int k = sStart[c] + threadIdx.x; k < sStart[c] + sCount[c]; k += blockDim.x )
-		{
-			Lane L;
-			if ( kind == 0 )
-			{
-				L.idx = w.kIndex[k];
-				L.ms = w.kMass[k];
-				L.nm = w.kNormal[k];
-				L.misc = __ldcg( w.kMisc + k );
-				L.imp = __ldcg( w.kImp + k );
-				L.an[0] = w.kAnch1[k];
-				L.an[1] = w.kAnch2[k];
-				lane_warm( ba, L );
-				continue;
-			}
-			lane_load( w, k, L );
-			lane_op( ba, L, kind, p );
-			if ( kind == 3 )
-				__stcg( w.kImp + k, L.imp );
-			else
-				lane_store( w, k, L );
-		}
-		__syncthreads();
-	}
-}
-
-// The persistent solver. Graph-colour constraint slots (after the overflow
-// slots) are dealt to threads round-robin over the blocks: thread t of block
-// b owns colour slot r = t * gridDim.x + b (and r + gridDim.x * blockDim.x,
-// ... when the graph holds more constraints than the grid has threads). The
-// first owned constraint lives in registers for the whole launch; a colour
-// stage then costs one load and one store of each of its two bodies.
-template <int THREADS>
-__global__ void __launch_bounds__( THREADS ) k_solve( DWorld w, SolveParams p, const int* jointSlots,
-													  const int* jointStart )
-{
-	__shared__ int sStart[F2D_COLORS], sCount[F2D_COLORS], sJStart[F2D_OVERFLOW + 1];
-	if ( threadIdx.x < F2D_COLORS )
-	{
-		sStart[threadIdx.x] = w.sc->colorStart[threadIdx.x];
-		sCount[threadIdx.x] = w.sc->colorCount[threadIdx.x];
-	}
-	if ( threadIdx.x <= F2D_OVERFLOW )
-		sJStart[threadIdx.x] = jointStart[threadIdx.x];
 	__syncthreads();
-
-	int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-	int gstride = gridDim.x * blockDim.x;
-	unsigned epoch = 0;
-	const GBodies gb = { w.vel, w.delta };
-	int nb = w.bodyCount;
-	int novf = w.sc->overflowCount;
-	int novfJ = w.sc->overflowJointCount;
-	int nColour = w.sc->touchingCount - novf;
-	bool serialStage = novf > 0 || novfJ > 0;
-	unsigned activeMask = 0;
-	for ( int c = 0; c < F2D_OVERFLOW; ++c )
-		if ( sCount[c] > 0 || sJStart[c + 1] > sJStart[c] )
-			activeMask |= 1u << c;
-	// block 0 solves the overflow constraints, level by level
-	__shared__ int sLevelStart[OVF_MAX_LEVELS + 1];
-	__shared__ int sOrder[OVF_SMEM_ITEMS];
-	OvfPlan plan = {};
-	if ( serialStage && blockIdx.x == 0 )
-		plan = ovf_schedule( w, novf + novfJ <= OVF_SMEM_ITEMS ? sOrder : w.ovfOrder, sLevelStart );
-
-	// tail colours run in block 0; their constraints stay in global memory
-	const int tailFirst = tail_first_colour( sCount, sJStart, activeMask );
-	const int tailSlot = tailFirst < F2D_OVERFLOW ? sStart[tailFirst] : novf + nColour;
-
-	const int r0 = threadIdx.x * gridDim.x + blockIdx.x;
-	Lane L0;
-	int col0 = -1;
-	if ( r0 < nColour && novf + r0 < tailSlot )
+	if ( threadIdx.x == 0 )
 	{
-		int k0 = novf + r0;
-		lane_load( w, k0, L0 );
-		for ( int c = 0; c < F2D_OVERFLOW; ++c )
-			if ( k0 >= sStart[c] && k0 < sStart[c] + sCount[c] )
-				col0 = c;
-	}
-
-	for ( int sub = 0; sub < p.subSteps; ++sub )
-	{
-		for ( int b = gtid; b < nb; b += gstride )
-			if ( body_awake( w.bflags[b] ) )
-				integrate_velocity( w, b, p );
-		if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-			return;
-		for ( int kind = 0; kind < 3; ++kind )
+		int at = 0;
+		for ( int k = 0; k < FLOW_KINDS; ++k )
 		{
-			if ( kind == 2 )
-			{
-				// integrate positions (solver.c:182-200)
-				for ( int b = gtid; b < nb; b += gstride )
-				{
-					if ( !body_awake( w.bflags[b] ) )
-						continue;
-					float4 v = __ldcg( w.vel + b );
-					float4 d = __ldcg( w.delta + b );
-					frot dq;
-					dq.c = d.z;
-					dq.s = d.w;
-					dq = rintegrate( dq, p.h * v.z );
-					fv2 dp = vmuladd( mk( d.x, d.y ), p.h, mk( v.x, v.y ) );
-					__stcg( w.delta + b, make_float4( dp.x, dp.y, dq.c, dq.s ) );
-				}
-				if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-					return;
-			}
-			if ( serialStage )
-			{
-				if ( blockIdx.x == 0 )
-					ovf_stage( w, gb, plan, sLevelStart, kind, p );
-				if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-					return;
-			}
-			for ( int c = 0; c < tailFirst; ++c )
-			{
-				if ( ( activeMask & ( 1u << c ) ) == 0 )
-					continue;
-				joint_colour_stage( w, gb, c, kind, p, gtid, gstride, jointSlots, sJStart );
-				if ( col0 == c )
-					lane_op( gb, L0, kind, p );
-				colour_lanes_extra( w, gb, c, sStart, sCount, novf, gtid, gstride, kind, p );
-				if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-					return;
-			}
-			if ( tailFirst < F2D_OVERFLOW )
-			{
-				if ( blockIdx.x == 0 )
-					tail_stage( w, gb, sStart, sCount, tailFirst, activeMask, kind, p );
-				if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-					return;
-			}
+			f.groupStart[k] = at;
+			at += ( f.count[k] + 31 ) >> 5;
 		}
+		f.groupStart[FLOW_KINDS] = at;
 	}
-	// restitution: overflow then colours (solver.c:1103-1117)
-	if ( novf > 0 )
+	// overflow constraints in their serial order: each counts the smaller ones
+	for ( int i = threadIdx.x; i < f.overflow; i += blockDim.x )
 	{
-		if ( blockIdx.x == 0 )
-			ovf_stage( w, gb, plan, sLevelStart, 3, p );
-		if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-			return;
+		int e = w.ovfItems[f.overflowFirst + i], rank = 0;
+		for ( int j = 0; j < f.overflow; ++j )
+			rank += w.ovfItems[f.overflowFirst + j] < e ? 1 : 0;
+		w.ovfSorted[f.overflowFirst + rank] = e;
 	}
-	for ( int c = 0; c < tailFirst; ++c )
+	__syncthreads();
+	for ( int g = threadIdx.x; g < min( f.groupStart[FLOW_KINDS], FLOW_LIST ); g += blockDim.x )
 	{
-		if ( sCount[c] == 0 )
-			continue;
-		if ( col0 == c )
-			lane_op( gb, L0, 3, p );
-		colour_lanes_extra( w, gb, c, sStart, sCount, novf, gtid, gstride, 3, p );
-		if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-			return;
+		int k = 0;
+		while ( k < FLOW_KINDS - 1 && g >= f.groupStart[k + 1] )
+			k += 1;
+		f.kind[g] = (unsigned char)k;
 	}
-	if ( tailFirst < F2D_OVERFLOW )
-	{
-		if ( blockIdx.x == 0 )
-			tail_stage( w, gb, sStart, sCount, tailFirst, activeMask, 3, p );
-		if ( !grid_barrier( &w.sc->barrierCount, &w.sc->error, epoch ) )
-			return;
-	}
-	// store impulses into the manifolds
-	for ( int k = gtid; k < novf; k += gstride )
-		store_manifold_global( w, k, false );
-	if ( col0 >= 0 )
-		store_manifold( w, novf + r0, L0.imp, L0.tot, L0.misc.w, L0.pt[0].w, L0.pt[1].w,
-						__float_as_int( L0.sf.w ), true );
-	for ( int k = novf + gstride + gtid; k < novf + nColour; k += gstride )
-		store_manifold_global( w, k, true );
-	// tail constraints below the extras' range had no register lane
-	for ( int k = tailSlot + gtid; k < min( novf + gstride, novf + nColour ); k += gstride )
-		store_manifold_global( w, k, true );
-	if ( blockIdx.x == 0 && threadIdx.x == 0 )
-		w.sc->solveBarriers = (int)epoch; // grid barriers this launch passed
+	__syncthreads();
 }
 
-// A launch of nothing but grid barriers on the solver's grid: the per-barrier
-// latency that bounds the stages of k_solve from below.
+// Rank of overflow constraint e on body b among the body's overflow
+// constraints, from the body's (unordered) list; .y among those with
+// restitution.
+__device__ __forceinline__ int2 overflow_rank( const DWorld& w, int e, int b, int limit )
+{
+	int2 r = make_int2( 0, 0 );
+	if ( b < 0 )
+		return r;
+	int key = w.bodyOrd[b].w - 1;
+	for ( int guard = 0; key >= 0 && guard < limit; ++guard )
+	{
+		if ( ( key >> 2 ) < e )
+		{
+			r.x += 1;
+			r.y += ( key >> 1 ) & 1;
+		}
+		key = w.ovfNext[2 * (size_t)( key >> 2 ) + ( key & 1 )] - 1;
+	}
+	return r;
+}
+
+// A constraint's view of one body: KR_REF packs the bodies (x, y), their
+// slots (z, 16 bits each) and per body, 9 bits from bit 0 and bit 16 of w: the
+// colour's rank among the body's colours, their number, and whether overflow
+// constraints lead them.
+__device__ __forceinline__ int ref_bits( const int4& ord, int colour )
+{
+	unsigned bits = (unsigned)ord.x & FLOW_COLOURS;
+	return __popc( bits & ( ( 1u << colour ) - 1u ) ) | ( __popc( bits ) << 4 ) | ( ord.y > 0 ? 256 : 0 );
+}
+
+// A body has a slot when its constraints all lie in this part and its place
+// fits the shared memory.
+__device__ __forceinline__ int body_slot( const DWorld& w, const int4& ord, int b, int firstPos, int slots )
+{
+	int pos = w.bodyPos[b];
+	if ( pos < 0 || ( ord.x & FLOW_GLOBAL ) || pos - firstPos >= slots )
+		return FLOW_NO_SLOT;
+	return pos - firstPos;
+}
+
+// Loads the rows of a contact constraint (all of them, or those its warm
+// start needs).
+__device__ __forceinline__ void load_lane( const float4* row, Lane& L, bool all )
+{
+	L.ms = row[32 * KR_MASS];
+	L.nm = row[32 * KR_NORMAL];
+	L.misc = row[32 * KR_MISC];
+	L.imp = row[32 * KR_IMP];
+	L.an[0] = row[32 * KR_ANCH1];
+	L.an[1] = row[32 * KR_ANCH2];
+	if ( all )
+	{
+		L.pt[0] = row[32 * KR_P1];
+		L.pt[1] = row[32 * KR_P2];
+		L.tot = row[32 * KR_TOT];
+	}
+}
+
+__device__ __forceinline__ void store_lane( float4* row, const Lane& L )
+{
+	row[32 * KR_IMP] = L.imp;
+	row[32 * KR_TOT] = L.tot;
+	row[32 * KR_MISC] = L.misc;
+}
+
+// One constraint's pair of bodies and where their rows are.
+struct FlowPair
+{
+	int ia, ib;		  // -1 static
+	int slotA, slotB; // FLOW_NO_SLOT: global
+	int rankA, rankB, degA, degB;
+};
+
+// What a waiting constraint has seen of its bodies.
+struct FlowSeen
+{
+	float4 vA, vB, dA, dB;
+	bool okA, okB, okD;
+};
+
+// One poll of the rows a constraint still waits for; true when it has all.
+// `ds`: substep delta rows, -1 when the operation needs none.
+__device__ __forceinline__ bool flow_poll( const Rows& rows, const FlowPair& q, int wantA, int wantB, int ds, FlowSeen& s )
+{
+	float4 a, b;
+	if ( !s.okA )
+		a = rows.vel( q.ia, q.slotA );
+	if ( !s.okB )
+		b = rows.vel( q.ib, q.slotB );
+	if ( !s.okD && ds >= 0 )
+	{
+		s.dA = s.dB = make_float4( 0.0f, 0.0f, 1.0f, 0.0f );
+		if ( q.ia >= 0 )
+			s.dA = rows.delta( ds, q.ia, q.slotA );
+		if ( q.ib >= 0 )
+			s.dB = rows.delta( ds, q.ib, q.slotB );
+		s.okD = __float_as_uint( s.dA.x ) != FLOW_SENTINEL && __float_as_uint( s.dB.x ) != FLOW_SENTINEL;
+	}
+	if ( !s.okA )
+	{
+		s.vA = a;
+		s.okA = __float_as_int( a.w ) == wantA;
+	}
+	if ( !s.okB )
+	{
+		s.vB = b;
+		s.okB = __float_as_int( b.w ) == wantB;
+	}
+	return s.okA && s.okB && ( s.okD || ds < 0 );
+}
+
+__device__ __forceinline__ void flow_expect( const FlowPair& q, FlowSeen& s )
+{
+	s.okA = q.ia < 0;
+	s.okB = q.ib < 0;
+	if ( s.okA )
+		s.vA = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
+	if ( s.okB )
+		s.vB = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
+}
+
+__device__ __forceinline__ void flow_states( const FlowPair& q, const FlowSeen& s, PairBodies& ba )
+{
+	ba.ia = q.ia;
+	ba.ib = q.ib;
+	ba.a = { s.vA.x, s.vA.y, s.vA.z, s.dA.x, s.dA.y, s.dA.z, s.dA.w };
+	ba.b = { s.vB.x, s.vB.y, s.vB.z, s.dB.x, s.dB.y, s.dB.z, s.dB.w };
+}
+
+// The velocity rows back with their counts one higher; after a body's last
+// solve of a substep, its new delta.
+__device__ __forceinline__ void flow_publish( const DWorld& w, const SolveParams& p, const Rows& rows, const FlowPair& q,
+											  const PairBodies& ba, int wantA, int wantB, int sub, bool solve )
+{
+	if ( q.ia >= 0 )
+		rows.put_vel( q.ia, q.slotA, make_float4( ba.a.vx, ba.a.vy, ba.a.w, __int_as_float( wantA + 1 ) ) );
+	if ( q.ib >= 0 )
+		rows.put_vel( q.ib, q.slotB, make_float4( ba.b.vx, ba.b.vy, ba.b.w, __int_as_float( wantB + 1 ) ) );
+	if ( solve )
+	{
+		const bool last = sub == p.subSteps - 1;
+		if ( q.ia >= 0 && q.rankA == q.degA - 1 )
+			rows.put_delta( sub + 1, last, q.ia, q.slotA, integrate_position( w, p, q.ia, ba.a ) );
+		if ( q.ib >= 0 && q.rankB == q.degB - 1 )
+			rows.put_delta( sub + 1, last, q.ib, q.slotB, integrate_position( w, p, q.ib, ba.b ) );
+	}
+}
+
+// Counts a poll without progress; true when the wait is to be given up.
+__device__ __forceinline__ bool flow_give_up( const DWorld& w, int& spins )
+{
+	spins += 1;
+	if ( ( spins & 1023 ) != 0 )
+		return false;
+	bool out = spins >= FLOW_SPIN_LIMIT;
+	if ( out && ( threadIdx.x & 31 ) == 0 )
+		atomicOr( &w.sc->error, F2D_ERR_BARRIER_TIMEOUT );
+	return __any_sync( 0xffffffffu, out || ( ld_relaxed_s32( &w.sc->error ) & F2D_ERR_BARRIER_TIMEOUT ) );
+}
+
+// One warp's groups first, first + stride, ... of the part's colours, through
+// every stage.
+__device__ __forceinline__ void solve_colours( const DWorld& w, const SolveParams& p, const Rows& rows, const FlowPart& f,
+											   int firstPos, int slots, int first, int stride )
+{
+	const int lane = threadIdx.x & 31;
+	const int nGroups = f.groupStart[FLOW_KINDS];
+	const int stages = 3 * p.subSteps; // restitution is stage `stages`
+	const int lastStage = p.restitution ? stages : stages - 1;
+	if ( first >= nGroups )
+		return;
+	const bool single = first + stride >= nGroups; // the group stays in registers
+
+	Lane L;
+	float4* row = nullptr;
+	int joint = -1; // joint of this lane, -1 in a group of contacts
+	bool item = false;
+	FlowPair q = { -1, -1, FLOW_NO_SLOT, FLOW_NO_SLOT, 0, 0, 1, 1 };
+	FlowSeen s;
+	s.dA = s.dB = make_float4( 0.0f, 0.0f, 1.0f, 0.0f );
+	s.okD = false;
+
+	for ( int stage = 0; stage <= lastStage; ++stage )
+	{
+		const int sub = stage / 3;
+		const bool rest = stage == stages;
+		const int op = rest ? 3 : stage - 3 * sub; // 0 warm start, 1 solve, 2 relax, 3 restitution
+		for ( int g = first; g < nGroups; g += stride )
+		{
+			if ( !single || stage == 0 || rest )
+			{
+				// open the group
+				int k = 0;
+				if ( g < FLOW_LIST )
+					k = f.kind[g];
+				else
+					while ( k < FLOW_KINDS - 1 && g >= f.groupStart[k + 1] )
+						k += 1;
+				const int gk = g - f.groupStart[k];
+				item = 32 * gk + lane < f.count[k];
+				joint = -1;
+				if ( k & 1 )
+				{
+					row = w.kRow + (size_t)( f.first[k] + gk ) * ( KROWS * 32 ) + lane;
+					load_lane( row, L, op != 0 || single );
+				}
+				else
+					joint = w.jointSlots[f.first[k] + ( item ? 32 * gk + lane : 0 )];
+				if ( joint < 0 && stage > 0 && !rest )
+				{
+					float4 r = row[32 * KR_REF];
+					q.ia = __float_as_int( r.x );
+					q.ib = __float_as_int( r.y );
+					q.slotA = __float_as_int( r.z ) & 0xffff;
+					q.slotB = (unsigned)__float_as_int( r.z ) >> 16;
+					int bits = __float_as_int( r.w );
+					q.rankA = bits & 15;
+					q.degA = ( bits >> 4 ) & 15;
+					q.rankB = ( bits >> 16 ) & 15;
+					q.degB = ( bits >> 20 ) & 15;
+					if ( item && ( bits & 256 ) )
+					{
+						int lead = w.bodyOrd[q.ia].y;
+						q.rankA += lead;
+						q.degA += lead;
+					}
+					if ( item && ( bits & ( 256 << 16 ) ) )
+					{
+						int lead = w.bodyOrd[q.ib].y;
+						q.rankB += lead;
+						q.degB += lead;
+					}
+				}
+				else if ( item )
+				{
+					if ( joint < 0 )
+					{
+						float4 h = row[32 * KR_HEAD];
+						q.ia = __float_as_int( h.x );
+						q.ib = __float_as_int( h.y );
+					}
+					else
+					{
+						int2 idx = w.jindex[joint];
+						q.ia = idx.x;
+						q.ib = idx.y;
+					}
+					const int colour = k >> 1;
+					int4 oa = make_int4( 0, 0, 0, 0 ), ob = oa;
+					if ( q.ia >= 0 )
+						oa = w.bodyOrd[q.ia];
+					if ( q.ib >= 0 )
+						ob = w.bodyOrd[q.ib];
+					q.slotA = q.ia >= 0 ? body_slot( w, oa, q.ia, firstPos, slots ) : FLOW_NO_SLOT;
+					q.slotB = q.ib >= 0 ? body_slot( w, ob, q.ib, firstPos, slots ) : FLOW_NO_SLOT;
+					q.degA = oa.y + __popc( oa.x & FLOW_COLOURS );
+					q.degB = ob.y + __popc( ob.x & FLOW_COLOURS );
+					unsigned below = ( 1u << colour ) - 1u;
+					int shift = rest ? FLOW_REST_SHIFT : 0;
+					q.rankA = ( rest ? oa.z : oa.y ) + __popc( ( (unsigned)oa.x >> shift ) & below );
+					q.rankB = ( rest ? ob.z : ob.y ) + __popc( ( (unsigned)ob.x >> shift ) & below );
+					if ( joint < 0 && !single && stage == 0 )
+						row[32 * KR_REF] = make_float4(
+							__int_as_float( q.ia ), __int_as_float( q.ib ), __int_as_float( q.slotA | ( q.slotB << 16 ) ),
+							__int_as_float( ref_bits( oa, colour ) | ( ref_bits( ob, colour ) << 16 ) ) );
+				}
+				if ( rest )
+					item = item && joint < 0 && L.misc.x != 0.0f; // contacts that have some
+				if ( !item )
+					q.ia = q.ib = -1;
+				s.okD = false;
+			}
+			else if ( op == 2 )
+				s.okD = false; // relaxing reads the substep's new deltas
+
+			// wait for the operations before this one on every body of the group
+			// (the restitution counts follow the last relax stage's)
+			const int wantA = stage * q.degA + q.rankA, wantB = stage * q.degB + q.rankB;
+			// deltas: none for restitution and a contact's warm start
+			const int ds = rest || ( op == 0 && joint < 0 ) ? -1 : sub + ( op == 2 ? 1 : 0 );
+			flow_expect( q, s );
+			for ( int spins = 0; !__all_sync( 0xffffffffu, flow_poll( rows, q, wantA, wantB, ds, s ) ); )
+				if ( flow_give_up( w, spins ) )
+					return;
+
+			if ( item )
+			{
+				PairBodies ba;
+				flow_states( q, s, ba );
+				if ( op == 0 )
+				{
+					if ( q.ia >= 0 && q.rankA == 0 )
+						integrate_velocity( w, p, q.ia, ba.a );
+					if ( q.ib >= 0 && q.rankB == 0 )
+						integrate_velocity( w, p, q.ib, ba.b );
+				}
+				if ( joint < 0 )
+				{
+					Soft soft = ( q.ia < 0 || q.ib < 0 ) ? p.staticSoft : p.contactSoft;
+					if ( op == 0 )
+						lane_warm( ba.a, ba.b, L );
+					else if ( op == 3 )
+						lane_restitution( ba.a, ba.b, L, p.restitutionThreshold );
+					else
+						lane_solve( ba.a, ba.b, L, soft, p.inv_h, p.minBiasVel, op == 1 );
+				}
+				else if ( op == 0 )
+					joint_warm_start( w, ba, joint );
+				else
+					joint_solve( w, ba, joint, p.h, p.inv_h, op == 1 );
+				flow_publish( w, p, rows, q, ba, wantA, wantB, sub, op == 1 );
+				// the step's last operation of a contact hands its impulses over
+				if ( joint < 0 )
+				{
+					if ( p.restitution && ( rest || ( stage == stages - 1 && L.misc.x == 0.0f ) ) )
+						store_manifold( w, __float_as_int( row[32 * KR_HEAD].z ), L.imp, L.tot, L.misc.w, L.pt[0].w, L.pt[1].w,
+										true );
+					else if ( op != 0 && ( !single || stage == stages - 1 ) )
+						store_lane( row, L );
+				}
+			}
+			__syncwarp();
+		}
+	}
+}
+
+// Overflow constraints: each lane goes through its own, first, first +
+// stride, ... of the part's list, at its own pace; a round polls for all
+// lanes and runs those that are ready.
+__device__ __forceinline__ void solve_overflows( const DWorld& w, const SolveParams& p, const Rows& rows,
+												 const FlowPart& f, int firstPos, int slots, int first, int stride )
+{
+	const int stages = 3 * p.subSteps;
+	const int novfJ = w.sc->overflowJointCount, limit = 2 * ( novfJ + w.sc->overflowCount );
+	const bool single = first + stride >= f.overflow;
+	Lane L;
+	float4* row = nullptr;
+	int joint = -1, contact = -1, points = 0;
+	FlowPair q = { -1, -1, FLOW_NO_SLOT, FLOW_NO_SLOT, 0, 0, 1, 1 };
+	FlowSeen s;
+	s.dA = s.dB = make_float4( 0.0f, 0.0f, 1.0f, 0.0f );
+	int i = first, stage = 0;
+	bool act = i < f.overflow, fresh = true;
+	for ( int spins = 0;; )
+	{
+		const bool rest = stage == stages;
+		const int sub = stage / 3;
+		const int op = rest ? 3 : stage - 3 * sub;
+		bool fire = false;
+		if ( act )
+		{
+			if ( fresh )
+			{
+				int e = w.ovfSorted[f.overflowFirst + i];
+				joint = e < novfJ ? w.overflowJoints[e] : -1;
+				if ( joint >= 0 )
+				{
+					int2 idx = w.jindex[joint];
+					q.ia = idx.x;
+					q.ib = idx.y;
+				}
+				else
+				{
+					row = krow( w, e - novfJ, 0 );
+					load_lane( row, L, true );
+					float4 h = row[32 * KR_HEAD];
+					q.ia = __float_as_int( h.x );
+					q.ib = __float_as_int( h.y );
+					contact = __float_as_int( h.z );
+					points = __float_as_int( h.w );
+				}
+				int4 oa = make_int4( 0, 0, 0, 0 ), ob = oa;
+				if ( q.ia >= 0 )
+					oa = w.bodyOrd[q.ia];
+				if ( q.ib >= 0 )
+					ob = w.bodyOrd[q.ib];
+				q.slotA = q.ia >= 0 ? body_slot( w, oa, q.ia, firstPos, slots ) : FLOW_NO_SLOT;
+				q.slotB = q.ib >= 0 ? body_slot( w, ob, q.ib, firstPos, slots ) : FLOW_NO_SLOT;
+				q.degA = oa.y + __popc( oa.x & FLOW_COLOURS );
+				q.degB = ob.y + __popc( ob.x & FLOW_COLOURS );
+				if ( stage == 0 )
+				{
+					int2 ra = overflow_rank( w, e, q.ia, limit ), rb = overflow_rank( w, e, q.ib, limit );
+					w.ovfRank[e] = make_int4( ra.x, rb.x, ra.y, rb.y );
+				}
+				int4 o = w.ovfRank[e];
+				q.rankA = rest ? o.z : o.x;
+				q.rankB = rest ? o.w : o.y;
+				fresh = false;
+				s.okD = false;
+				flow_expect( q, s );
+			}
+			const int wantA = stage * q.degA + q.rankA, wantB = stage * q.degB + q.rankB;
+			const int ds = rest || ( op == 0 && joint < 0 ) ? -1 : sub + ( op == 2 ? 1 : 0 );
+			fire = flow_poll( rows, q, wantA, wantB, ds, s );
+			if ( fire )
+			{
+				PairBodies ba;
+				flow_states( q, s, ba );
+				if ( op == 0 )
+				{
+					if ( q.ia >= 0 && q.rankA == 0 )
+						integrate_velocity( w, p, q.ia, ba.a );
+					if ( q.ib >= 0 && q.rankB == 0 )
+						integrate_velocity( w, p, q.ib, ba.b );
+				}
+				if ( joint < 0 )
+				{
+					Soft soft = ( q.ia < 0 || q.ib < 0 ) ? p.staticSoft : p.contactSoft;
+					if ( op == 0 )
+						warm_overflow( ba.a, ba.b, L, points );
+					else if ( op == 3 )
+						restitution_overflow( ba.a, ba.b, L, points, p.restitutionThreshold );
+					else
+						solve_overflow( ba.a, ba.b, L, points, soft, p.inv_h, p.pushout, op == 1 );
+				}
+				else if ( op == 0 )
+					joint_warm_start( w, ba, joint );
+				else
+					joint_solve( w, ba, joint, p.h, p.inv_h, op == 1 );
+				flow_publish( w, p, rows, q, ba, wantA, wantB, sub, op == 1 );
+				if ( joint < 0 )
+				{
+					if ( p.restitution && ( rest || ( stage == stages - 1 && L.misc.x == 0.0f ) ) )
+						store_manifold( w, contact, L.imp, L.tot, L.misc.w, L.pt[0].w, L.pt[1].w, points > 1 );
+					else if ( op != 0 && ( !single || stage == stages - 1 ) )
+						store_lane( row, L );
+				}
+				// this lane's next operation
+				if ( !single )
+				{
+					fresh = true;
+					i += stride;
+					if ( i >= f.overflow )
+					{
+						i = first;
+						stage += 1;
+					}
+				}
+				else
+				{
+					stage += 1;
+					if ( stage % 3 == 2 )
+						s.okD = false; // relaxing reads the substep's new deltas
+					flow_expect( q, s );
+				}
+				if ( stage >= stages )
+				{
+					// restitution: contacts that have some
+					fresh = true;
+					act = false;
+					while ( stage == stages && p.restitution && i < f.overflow )
+					{
+						int e = w.ovfSorted[f.overflowFirst + i];
+						if ( e >= novfJ && krow( w, e - novfJ, KR_MISC )->x != 0.0f )
+						{
+							act = true;
+							break;
+						}
+						i += stride;
+					}
+				}
+			}
+		}
+		if ( !__any_sync( 0xffffffffu, act ) )
+			return;
+		if ( __any_sync( 0xffffffffu, fire ) )
+			spins = 0;
+		else if ( flow_give_up( w, spins ) )
+			return;
+	}
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__( THREADS ) k_solve( DWorld w, SolveParams p )
+{
+	extern __shared__ float4 sbody[]; // velocities of all slots, deltas at the start, deltas after each substep
+	__shared__ FlowPart f;
+	const int part = blockIdx.x;
+	const int chunk = part_chunk( w, p );
+	const int firstPos = part * chunk;
+	const int mine = max( min( min( w.sc->orderTotal - firstPos, chunk ), p.slots ), 0 );
+	const float sentinel = __uint_as_float( FLOW_SENTINEL );
+	for ( int t = threadIdx.x; t < mine; t += THREADS )
+	{
+		int b = w.bodyAt[firstPos + t];
+		float4 v = __ldcg( w.vel + b );
+		v.w = 0.0f;
+		sbody[t] = v;
+		sbody[p.slots + t] = __ldcg( w.delta + b );
+		for ( int k = 0; k < p.subSteps; ++k )
+			sbody[( 2 + k ) * p.slots + t] = make_float4( sentinel, sentinel, sentinel, sentinel );
+	}
+	flow_part( w, p, part, f );
+	// bodies no constraint holds: all substeps at once, nothing to wait for
+	// (the last blocks first: a small world's parts are the first ones)
+	for ( int b = ( gridDim.x - 1 - blockIdx.x ) * THREADS + threadIdx.x; b < w.bodyCount; b += gridDim.x * THREADS )
+	{
+		int4 o = w.bodyOrd[b];
+		if ( ( o.x & FLOW_COLOURS ) != 0 || o.y != 0 ||
+			 ( __float_as_int( w.bodyInt[2 * (size_t)b + 1].y ) & BI_AWAKE ) == 0 )
+			continue;
+		float4 v = w.vel[b], d = w.delta[b];
+		BState s = { v.x, v.y, v.z, d.x, d.y, d.z, d.w };
+		for ( int sub = 0; sub < p.subSteps; ++sub )
+		{
+			integrate_velocity( w, p, b, s );
+			d = integrate_position( w, p, b, s );
+			s.dpx = d.x;
+			s.dpy = d.y;
+			s.dqc = d.z;
+			s.dqs = d.w;
+		}
+		w.vel[b] = make_float4( s.vx, s.vy, s.w, 0.0f );
+		w.delta[b] = d;
+	}
+	const Rows rows = { (unsigned)__cvta_generic_to_shared( sbody ), 16u * (unsigned)p.slots, w.vel, w.delta, w.dsub,
+						(size_t)w.bodyCount };
+	const int warp = threadIdx.x >> 5, warps = THREADS / 32;
+	// a quarter of the warps at most is kept for the overflow constraints,
+	// whose chains would hold up the colour groups of a warp that had both
+	const int ovfWarps = min( warps / 4, f.overflow );
+	if ( warp < warps - ovfWarps )
+		solve_colours( w, p, rows, f, firstPos, mine, warp, warps - ovfWarps );
+	else
+		solve_overflows( w, p, rows, f, firstPos, mine, ( threadIdx.x & 31 ) * ovfWarps + warp - ( warps - ovfWarps ),
+						 32 * ovfWarps );
+	__syncthreads();
+	for ( int t = threadIdx.x; t < mine; t += THREADS )
+	{
+		int b = w.bodyAt[firstPos + t];
+		int4 o = w.bodyOrd[b];
+		if ( ( o.x & FLOW_GLOBAL ) || ( ( o.x & FLOW_COLOURS ) == 0 && o.y == 0 ) )
+			continue;
+		float4 v = sbody[t];
+		w.vel[b] = make_float4( v.x, v.y, v.z, 0.0f );
+		w.delta[b] = sbody[( 1 + p.subSteps ) * p.slots + t];
+	}
+}
+
+// A launch of nothing but grid barriers on one block per SM: what a barrier
+// per stage would cost at least.
 __global__ void __launch_bounds__( 512 ) k_barrier_probe( unsigned* counter, int* err, int n )
 {
 	unsigned epoch = 0;
@@ -1294,266 +1338,58 @@ float solver_barrier_probe( StepScratch& s, cudaStream_t st, unsigned* counter, 
 }
 
 // ---------------------------------------------------------------------------
-// Cluster solver: the same stages on one thread-block cluster of F2D_CLUSTER
-// blocks, for worlds whose body rows fit the cluster's shared memory. The
-// body velocities and substep deltas live in distributed shared memory (body
-// b in block b % F2D_CLUSTER, slot b / F2D_CLUSTER) for the whole launch, and
-// the stages are separated by the hardware cluster barrier, so a colour stage
-// costs shared-memory round trips instead of L2 round trips and a grid-wide
-// barrier. Constraint rows stream from L2; a colour's constraint k is always
-// handled by the same thread, which therefore reads back its own impulses.
-// ---------------------------------------------------------------------------
-#define CLUSTER_THREADS 512
-#define CLUSTER_SOLVER_MAX_BODIES 20000
-
-__device__ __forceinline__ void integrate_velocity_smem( const DWorld& w, int b, float4& v4, const SolveParams& p )
-{
-	float4 m = w.massv[b];
-	float4 dmp = w.damp[b];
-	float4 f = w.force[b];
-	float h = p.h;
-	float maxLinearSpeedSq = p.maxLinearSpeed * p.maxLinearSpeed;
-	float maxAngularSpeedSq = p.maxAngularSpeed * p.maxAngularSpeed;
-	fv2 v = mk( v4.x, v4.y );
-	float wv = v4.z;
-	float linearDamping = 1.0f / ( 1.0f + h * dmp.x );
-	float angularDamping = 1.0f / ( 1.0f + h * dmp.y );
-	float gravityScale = m.x > 0.0f ? dmp.z : 0.0f;
-	fv2 g = p.gravity;
-	if ( w.subCount > 0 )
-	{
-		float2 gb = w.bodyGravity[b];
-		g = mk( gb.x, gb.y );
-	}
-	fv2 lvd = vadd( vscale( h * m.x, mk( f.x, f.y ) ), vscale( h * gravityScale, g ) );
-	float avd = h * m.y * f.z;
-	v = vmuladd( lvd, linearDamping, v );
-	wv = avd + angularDamping * wv;
-	int flags = w.bflags[b];
-	bool capped = false;
-	if ( vdot( v, v ) > maxLinearSpeedSq )
-	{
-		float ratio = p.maxLinearSpeed / vlen( v );
-		v = vscale( ratio, v );
-		capped = true;
-	}
-	if ( wv * wv > maxAngularSpeedSq && ( flags & BF_FAST_ROT ) == 0 )
-	{
-		float ratio = p.maxAngularSpeed / fabs_s( wv );
-		wv *= ratio;
-		capped = true;
-	}
-	if ( capped )
-		w.bflags[b] = flags | BF_SPEED_CAPPED;
-	v4 = make_float4( v.x, v.y, wv, 0.0f );
-}
-
-__global__ void __launch_bounds__( CLUSTER_THREADS ) k_solve_cluster( DWorld w, SolveParams p, const int* jointSlots,
-																	  const int* jointStart )
-{
-	extern __shared__ float4 sbody[]; // per slot: vel, delta
-	__shared__ int sStart[F2D_COLORS], sCount[F2D_COLORS], sJStart[F2D_OVERFLOW + 1];
-	cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-	const int rank = (int)cl.block_rank();
-	if ( threadIdx.x < F2D_COLORS )
-	{
-		sStart[threadIdx.x] = w.sc->colorStart[threadIdx.x];
-		sCount[threadIdx.x] = w.sc->colorCount[threadIdx.x];
-	}
-	if ( threadIdx.x <= F2D_OVERFLOW )
-		sJStart[threadIdx.x] = jointStart[threadIdx.x];
-	const int nb = w.bodyCount;
-	const int slots = ( nb + F2D_CLUSTER - 1 ) / F2D_CLUSTER;
-	for ( int sl = threadIdx.x; sl < slots; sl += blockDim.x )
-	{
-		int b = sl * F2D_CLUSTER + rank;
-		if ( b < nb )
-		{
-			sbody[2 * sl] = __ldcg( w.vel + b );
-			sbody[2 * sl + 1] = __ldcg( w.delta + b );
-		}
-	}
-	cl.sync();
-
-	const int stride = F2D_CLUSTER * blockDim.x;
-	const int tid = rank * blockDim.x + threadIdx.x;
-	const CBodies cb = { (unsigned)__cvta_generic_to_shared( sbody ) };
-	const int novf = w.sc->overflowCount;
-	const int novfJ = w.sc->overflowJointCount;
-	const int nColour = w.sc->touchingCount - novf;
-	const bool serialStage = novf > 0 || novfJ > 0;
-	unsigned activeMask = 0;
-	for ( int c = 0; c < F2D_OVERFLOW; ++c )
-		if ( sCount[c] > 0 || sJStart[c + 1] > sJStart[c] )
-			activeMask |= 1u << c;
-	// block 0 of the cluster solves the overflow constraints, level by level
-	__shared__ int sLevelStart[OVF_MAX_LEVELS + 1];
-	__shared__ int sOrder[OVF_SMEM_ITEMS];
-	OvfPlan plan = {};
-	if ( serialStage && rank == 0 )
-		plan = ovf_schedule( w, novf + novfJ <= OVF_SMEM_ITEMS ? sOrder : w.ovfOrder, sLevelStart );
-	// colour slot r = threadIdx.x * F2D_CLUSTER + rank (+ stride ...) belongs to
-	// this thread; the first one stays in registers for the whole launch
-	const int r0 = threadIdx.x * F2D_CLUSTER + rank;
-	Lane L0;
-	int col0 = -1;
-	if ( r0 < nColour )
-	{
-		int k0 = novf + r0;
-		lane_load( w, k0, L0 );
-		for ( int c = 0; c < F2D_OVERFLOW; ++c )
-			if ( k0 >= sStart[c] && k0 < sStart[c] + sCount[c] )
-				col0 = c;
-	}
-
-	for ( int sub = 0; sub < p.subSteps; ++sub )
-	{
-		for ( int sl = threadIdx.x; sl < slots; sl += blockDim.x )
-		{
-			int b = sl * F2D_CLUSTER + rank;
-			if ( b < nb && body_awake( w.bflags[b] ) )
-				integrate_velocity_smem( w, b, sbody[2 * sl], p );
-		}
-		cl.sync();
-		for ( int kind = 0; kind < 3; ++kind )
-		{
-			if ( kind == 2 )
-			{
-				// integrate positions (solver.c:182-200)
-				for ( int sl = threadIdx.x; sl < slots; sl += blockDim.x )
-				{
-					int b = sl * F2D_CLUSTER + rank;
-					if ( b >= nb || !body_awake( w.bflags[b] ) )
-						continue;
-					float4 v = sbody[2 * sl];
-					float4 d = sbody[2 * sl + 1];
-					frot dq;
-					dq.c = d.z;
-					dq.s = d.w;
-					dq = rintegrate( dq, p.h * v.z );
-					fv2 dp = vmuladd( mk( d.x, d.y ), p.h, mk( v.x, v.y ) );
-					sbody[2 * sl + 1] = make_float4( dp.x, dp.y, dq.c, dq.s );
-				}
-				cl.sync();
-			}
-			if ( serialStage )
-			{
-				if ( rank == 0 )
-					ovf_stage( w, cb, plan, sLevelStart, kind, p );
-				cl.sync();
-			}
-			for ( int c = 0; c < F2D_OVERFLOW; ++c )
-			{
-				if ( ( activeMask & ( 1u << c ) ) == 0 )
-					continue;
-				joint_colour_stage( w, cb, c, kind, p, tid, stride, jointSlots, sJStart );
-				if ( col0 == c )
-					lane_op( cb, L0, kind, p );
-				colour_lanes_extra( w, cb, c, sStart, sCount, novf, tid, stride, kind, p );
-				cl.sync();
-			}
-		}
-	}
-	// restitution: overflow then colours (solver.c:1103-1117)
-	if ( novf > 0 )
-	{
-		if ( rank == 0 )
-			ovf_stage( w, cb, plan, sLevelStart, 3, p );
-		cl.sync();
-	}
-	for ( int c = 0; c < F2D_OVERFLOW; ++c )
-	{
-		if ( sCount[c] == 0 )
-			continue;
-		if ( col0 == c )
-			lane_op( cb, L0, 3, p );
-		colour_lanes_extra( w, cb, c, sStart, sCount, novf, tid, stride, 3, p );
-		cl.sync();
-	}
-	// body rows back to the device, impulses into the manifolds
-	for ( int sl = threadIdx.x; sl < slots; sl += blockDim.x )
-	{
-		int b = sl * F2D_CLUSTER + rank;
-		if ( b < nb )
-		{
-			__stcg( w.vel + b, sbody[2 * sl] );
-			__stcg( w.delta + b, sbody[2 * sl + 1] );
-		}
-	}
-	for ( int k = tid; k < novf; k += stride )
-		store_manifold_global( w, k, false );
-	if ( col0 >= 0 )
-		store_manifold( w, novf + r0, L0.imp, L0.tot, L0.misc.w, L0.pt[0].w, L0.pt[1].w,
-						__float_as_int( L0.sf.w ), true );
-	for ( int k = novf + stride + tid; k < novf + nColour; k += stride )
-		store_manifold_global( w, k, true );
-	// no block leaves while another may still address its shared memory
-	cl.sync();
-}
-
-// Largest body count the cluster solver takes on this device (0 when a
-// cluster of F2D_CLUSTER blocks with that much shared memory cannot run).
-int solver_cluster_capacity()
-{
-	int dev = 0, optin = 0;
-	cudaGetDevice( &dev );
-	cudaDeviceGetAttribute( &optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev );
-	cudaFuncAttributes fa = {};
-	if ( cudaFuncGetAttributes( &fa, k_solve_cluster ) != cudaSuccess )
-	{
-		cudaGetLastError();
-		return 0;
-	}
-	int dyn = optin - (int)fa.sharedSizeBytes - 256; // less the static shared memory and a margin
-	if ( dyn < 32 * 64 )
-		return 0;
-	if ( cudaFuncSetAttribute( k_solve_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 ) != cudaSuccess ||
-		 cudaFuncSetAttribute( k_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn ) != cudaSuccess )
-	{
-		cudaGetLastError();
-		return 0;
-	}
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3( F2D_CLUSTER );
-	cfg.blockDim = dim3( CLUSTER_THREADS );
-	cfg.dynamicSmemBytes = (size_t)dyn;
-	cudaLaunchAttribute attr;
-	attr.id = cudaLaunchAttributeClusterDimension;
-	attr.val.clusterDim.x = F2D_CLUSTER;
-	attr.val.clusterDim.y = 1;
-	attr.val.clusterDim.z = 1;
-	cfg.attrs = &attr;
-	cfg.numAttrs = 1;
-	int clusters = 0;
-	if ( cudaOccupancyMaxActiveClusters( &clusters, k_solve_cluster, &cfg ) != cudaSuccess || clusters < 1 )
-	{
-		cudaGetLastError();
-		return 0;
-	}
-	return ( dyn / 32 ) * F2D_CLUSTER;
-}
-
-// ---------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------
-// Co-resident grid of the grid-wide solver: one block of 512 threads or two
-// of 256 per SM (the cooperative launch checks co-residency).
-template <int THREADS> static int grid_blocks( int perSMWanted )
+#define SOLVER_ROWS_SMEM ( 120 * 1024 ) // body rows a block keeps, at most; the rest caches constraint rows
+// Threads per SM: twelve warps. Measured (100k pile at its densest, 25k pile,
+// 820-box pyramid; us per launch): 256 threads 425, 187, 129; 320: 327, 172,
+// 121; 384: 312, 172, 119; 512: 335, 198, 133; 768: 467, 257, 150. More warps
+// cost registers (spills from 512 on) and issue slots (waiting warps poll);
+// fewer leave too many groups to a warp.
+#define SOLVER_THREADS 384
+// A world of up to this many bodies with constraints is one part: no body is
+// shared (pyramids of 55, 210, 465 boxes: 66, 76, 104 us as one part; 66, 111,
+// 109 us in parts of 64). Larger worlds take parts of at least SOLVER_MIN_CHUNK = 64 bodies (820
+// boxes: 111 us against 165 us as one part; 2k-6k piles: parts of 64 bodies
+// 138, 139 us, of 256 bodies 150, 152 us).
+#define SOLVER_ONE_PART 400
+
+static size_t solver_smem( int slots, int subSteps )
 {
-	int perSM = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor( &perSM, k_solve<THREADS>, THREADS, 0 );
-	int dev = 0;
-	cudaGetDevice( &dev );
-	int sms = 0;
-	cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
-	if ( perSM < 1 )
-		return 0;
-	return sms * ( perSM < perSMWanted ? perSM : perSMWanted );
+	return 16u * (size_t)( 2 + subSteps ) * slots;
 }
 
-int solver_max_blocks( int threads )
+// Co-resident grid of `perSM` blocks per SM.
+template <int THREADS> static int grid_blocks( int perSM )
 {
-	return threads == 256 ? grid_blocks<256>( 2 ) : grid_blocks<512>( 1 );
+	int fit = 0, dev = 0, sms = 0;
+	size_t smem = SOLVER_ROWS_SMEM / perSM;
+	if ( cudaFuncSetAttribute( k_solve<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem ) != cudaSuccess )
+		return 0;
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor( &fit, k_solve<THREADS>, THREADS, smem );
+	cudaGetDevice( &dev );
+	cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
+	int blocks = sms * ( fit < perSM ? fit : perSM );
+	return blocks < SOLVER_MAX_PARTS ? blocks : SOLVER_MAX_PARTS;
+}
+
+int solver_max_blocks( int perSM )
+{
+	return perSM == 2 ? grid_blocks<SOLVER_THREADS / 2>( 2 ) : grid_blocks<SOLVER_THREADS>( 1 );
+}
+
+// The bodies' spatial order and cleared tables, on a stream of their own
+// beside the collide phase: they need the leaf order and the last step's
+// colours only.
+void launch_solver_order( DWorld& w, StepScratch& s, cudaStream_t st )
+{
+	int tiles = ( w.shapeCap + ORDER_TILE - 1 ) / ORDER_TILE;
+	cudaMemsetAsync( w.orderState, 0, sizeof( unsigned long long ) * (size_t)( tiles + 2 ), st );
+	cudaMemsetAsync( w.bodyPos, 0xff, sizeof( int ) * (size_t)w.bodyCount, st );
+	k_body_order<<<tiles, ORDER_THREADS, 0, st>>>( w );
+	cudaMemsetAsync( w.binContacts, 0, sizeof( int ) * SOLVER_MAX_PARTS * ( 2 * F2D_OVERFLOW + 1 ), st );
+	cudaMemsetAsync( w.bodyOrd, 0, sizeof( int4 ) * (size_t)w.bodyCount, st );
+	cudaMemsetAsync( w.dsub, 0xff, sizeof( float4 ) * (size_t)w.bodyCount * ( s.subSteps < FLOW_SUBSTEPS ? s.subSteps : FLOW_SUBSTEPS ), st );
 }
 
 void launch_solver( DWorld& w, StepScratch& s, cudaStream_t st, float dt, int subSteps )
@@ -1575,55 +1411,41 @@ void launch_solver( DWorld& w, StepScratch& s, cudaStream_t st, float dt, int su
 	p.maxLinearSpeed = w.maxLinearSpeed;
 	p.maxAngularSpeed = F2D_MAX_ROTATION * p.inv_dt;
 	p.gravity = w.gravity;
-	p.subSteps = subSteps;
 	p.enableWarmStarting = w.enableWarmStarting;
+	p.subSteps = subSteps < FLOW_SUBSTEPS ? subSteps : FLOW_SUBSTEPS;
 
-	int* fill = s.tmpA; // F2D_COLORS ints
-	k_zero_ints<<<1, 32, 0, st>>>( fill, F2D_COLORS );
-	k_count_colors<<<grid_for( w.contactCap ), 256, 0, st>>>( w, fill );
-	k_color_offsets<<<1, 1, 0, st>>>( w, fill );
-	k_fill_slots<<<grid_for( w.contactCap ), 256, 0, st>>>( w, fill );
-	k_prepare_contacts<<<grid_for( w.contactCap ), 256, 0, st>>>( w, p );
+	const bool two = s.solverVariant == SOLVER_TWO_PER_SM && s.solverBlocks2 > 0;
+	p.parts = two ? s.solverBlocks2 : s.solverBlocks;
+	p.minChunk = s.smallParts ? SOLVER_SMALL_CHUNK : SOLVER_MIN_CHUNK;
+	p.onePart = s.smallParts ? 0 : ( s.solverVariant == SOLVER_FEW_PARTS ? 4 * SOLVER_ONE_PART : SOLVER_ONE_PART );
+	int fit = ( two ? SOLVER_ROWS_SMEM / 2 : SOLVER_ROWS_SMEM ) / ( 16 * ( 2 + p.subSteps ) );
+	int want = ( w.bodyCount + p.parts - 1 ) / p.parts;
+	want = want > p.minChunk ? want : p.minChunk;
+	want = want > p.onePart ? want : p.onePart;
+	want = want < w.bodyCount ? want : w.bodyCount;
+	p.slots = want < fit ? want : fit;
+
+	k_solver_count<<<grid_for( w.contactCap ), 256, 0, st>>>( w, p );
+	size_t binSmem = sizeof( int ) * (size_t)p.parts * ( 2 * F2D_OVERFLOW + 1 );
+	k_solver_prepare<<<grid_for( w.contactCap ), 256, binSmem, st>>>( w, p );
+	if ( w.jointCount > 0 )
+		launch_prepare_joints( w, st, p.h, p.jointSoft );
 	if ( w.learnMode & 2 )
 		launch_learned_warm_start( w, st );
-	launch_prepare_joints( w, s, st, p.h, p.inv_h, p.jointSoft );
-
-	int* jointSlots = s.tmpB;
-	int* jointStart = s.tmpB + w.jointCap;
-	void* args[] = { &w, &p, &jointSlots, &jointStart };
-	// Small worlds solve on one cluster (all stages in distributed shared
-	// memory and under the hardware cluster barrier); beyond about 2e4
-	// bodies the cluster's 16 SMs no longer hold the constraints in registers
-	// and the grid-wide solver is faster (measured: pyramid 0.11 vs 0.17 ms,
-	// 25k pile equal, 100k pile 0.75 vs 0.26 ms).
-	bool useCluster = s.clusterCapacity > 0 && w.bodyCount <= s.clusterCapacity &&
-					  ( s.solverVariant == SOLVER_CLUSTER ||
-						( s.solverVariant == SOLVER_AUTO && w.bodyCount <= CLUSTER_SOLVER_MAX_BODIES ) );
-	if ( useCluster )
-	{
-		int slots = ( w.bodyCount + F2D_CLUSTER - 1 ) / F2D_CLUSTER;
-		cudaLaunchConfig_t cfg = {};
-		cfg.gridDim = dim3( F2D_CLUSTER );
-		cfg.blockDim = dim3( CLUSTER_THREADS );
-		cfg.dynamicSmemBytes = (size_t)( slots > 0 ? slots : 1 ) * 32;
-		cfg.stream = st;
-		cudaLaunchAttribute attr;
-		attr.id = cudaLaunchAttributeClusterDimension;
-		attr.val.clusterDim.x = F2D_CLUSTER;
-		attr.val.clusterDim.y = 1;
-		attr.val.clusterDim.z = 1;
-		cfg.attrs = &attr;
-		cfg.numAttrs = 1;
-		if ( s.evSolveStart )
-			cudaEventRecord( s.evSolveStart, st );
-		cudaLaunchKernelEx( &cfg, k_solve_cluster, w, p, (const int*)jointSlots, (const int*)jointStart );
-		return;
-	}
-	cudaMemsetAsync( &w.sc->barrierCount, 0, sizeof( unsigned ), st );
 	if ( s.evSolveStart )
 		cudaEventRecord( s.evSolveStart, st );
-	if ( s.solverVariant == SOLVER_GRID256 && s.solverBlocks256 > 0 )
-		cudaLaunchCooperativeKernel( (void*)k_solve<256>, dim3( s.solverBlocks256 ), dim3( 256 ), args, 0, st );
-	else
-		cudaLaunchCooperativeKernel( (void*)k_solve<512>, dim3( s.solverBlocks ), dim3( 512 ), args, 0, st );
+	for ( int done = 0; done < subSteps; done += p.subSteps )
+	{
+		p.subSteps = subSteps - done < FLOW_SUBSTEPS ? subSteps - done : FLOW_SUBSTEPS;
+		p.restitution = done + p.subSteps == subSteps;
+		if ( done > 0 )
+			k_solver_refill<<<grid_for( w.bodyCount ), 256, 0, st>>>( w, p.subSteps );
+		void* args[] = { &w, &p };
+		size_t smem = solver_smem( p.slots, p.subSteps );
+		if ( two )
+			cudaLaunchCooperativeKernel( (void*)k_solve<SOLVER_THREADS / 2>, dim3( p.parts ), dim3( SOLVER_THREADS / 2 ), args,
+										 smem, st );
+		else
+			cudaLaunchCooperativeKernel( (void*)k_solve<SOLVER_THREADS>, dim3( p.parts ), dim3( SOLVER_THREADS ), args, smem, st );
+	}
 }

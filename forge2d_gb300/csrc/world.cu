@@ -156,9 +156,9 @@ struct HostWorld
 	// autotuner choice of the tree's leaf-order period (0: default)
 	int orderPeriod = 0;
 
-	// solve on the grid-wide cooperative kernel even when the world fits a
-	// thread-block cluster (F2D_NO_CLUSTER_SOLVER set at world creation)
-	bool gridSolverOnly = false;
+	// the solver deals the bodies of small worlds to many blocks too
+	// (F2D_NO_CLUSTER_SOLVER set at world creation)
+	bool smallParts = false;
 
 	// state of the host mirror of device-changed body rows (MIRROR_*)
 	int bodyMirror = 0;
@@ -233,16 +233,49 @@ static void alloc_scratch( HostWorld* W )
 		bits += 1;
 	s.shapeIdBits = bits;
 	d.pairKeyBits = bits;
-	dfree( d.ovfOwner );
-	dfree( d.ovfLevel );
-	dfree( d.ovfOrder );
-	dgrow( d.ovfOwner, 0, (size_t)d.bodyCap );
-	dgrow( d.ovfLevel, 0, (size_t)d.contactCap + d.jointCap );
-	dgrow( d.ovfOrder, 0, (size_t)d.contactCap + d.jointCap );
-	s.solverThreads = 512;
-	s.solverBlocks = solver_max_blocks( 512 );
-	s.solverBlocks256 = solver_max_blocks( 256 );
-	s.clusterCapacity = W->gridSolverOnly ? 0 : solver_cluster_capacity();
+	size_t constraints = (size_t)d.contactCap + d.jointCap;
+	// constraint slots: every part and colour rounds up to whole groups
+	int parts = std::min( SOLVER_MAX_PARTS, d.bodyCap / ( W->smallParts ? SOLVER_SMALL_CHUNK : SOLVER_MIN_CHUNK ) + 2 );
+	d.slotCap = 32 * ( ( d.contactCap + 31 ) / 32 + parts * F2D_OVERFLOW + 1 );
+	dfree( d.kRow );
+	dgrow( d.kRow, 0, (size_t)KROWS * d.slotCap );
+	dfree( d.orderState );
+	dgrow( d.orderState, 0, (size_t)d.shapeCap / 4096 + 8 );
+	dfree( d.bodyPos );
+	dgrow( d.bodyPos, 0, (size_t)d.bodyCap );
+	dfree( d.bodyAt );
+	dgrow( d.bodyAt, 0, (size_t)d.bodyCap );
+	dfree( d.bodyOrd );
+	dgrow( d.bodyOrd, 0, (size_t)d.bodyCap );
+	dfree( d.bodyInt );
+	dgrow( d.bodyInt, 0, 2 * (size_t)d.bodyCap );
+	dfree( d.dsub );
+	dgrow( d.dsub, 0, FLOW_SUBSTEPS * (size_t)d.bodyCap );
+	dfree( d.jointPlace );
+	dgrow( d.jointPlace, 0, (size_t)d.jointCap );
+	dfree( d.jointSlots );
+	dgrow( d.jointSlots, 0, (size_t)d.jointCap );
+	dfree( d.ovfItems );
+	dgrow( d.ovfItems, 0, constraints );
+	dfree( d.ovfSorted );
+	dgrow( d.ovfSorted, 0, constraints );
+	dfree( d.ovfRank );
+	dgrow( d.ovfRank, 0, constraints );
+	dfree( d.ovfNext );
+	dgrow( d.ovfNext, 0, 2 * constraints );
+	// counts and starts per part: contacts, joints, overflow
+	size_t bins = (size_t)SOLVER_MAX_PARTS * F2D_OVERFLOW;
+	dfree( d.binContacts );
+	dgrow( d.binContacts, 0, 2 * bins + SOLVER_MAX_PARTS );
+	d.binJoints = d.binContacts + bins;
+	d.binOverflow = d.binJoints + bins;
+	dfree( d.binContactStart );
+	dgrow( d.binContactStart, 0, 2 * bins + SOLVER_MAX_PARTS );
+	d.binJointStart = d.binContactStart + bins;
+	d.binOverflowStart = d.binJointStart + bins;
+	s.solverBlocks = solver_max_blocks( 1 );
+	s.solverBlocks2 = solver_max_blocks( 2 );
+	s.smallParts = W->smallParts;
 	s.ptBlocks = pt_large_blocks();
 }
 
@@ -298,20 +331,9 @@ static void grow_contacts( HostWorld* W, int cap )
 	dgrow( d.opDone, 0, cap );
 	dgrow( d.opBodies, 0, cap );
 	dgrow( d.opScan, 0, (size_t)OPS_SCAN_WORDS( cap ) );
-	dgrow( d.slotContact, 0, cap );
 	dgrow( d.overflowList, o, cap );
+	dgrow( d.slotPlace, 0, cap );
 	dgrow( d.npBucket, 0, (size_t)NP_CLASSES * cap );
-	dgrow( d.kIndex, 0, cap );
-	dgrow( d.kMass, 0, cap );
-	dgrow( d.kNormal, 0, cap );
-	dgrow( d.kMisc, 0, cap );
-	dgrow( d.kSoft, 0, cap );
-	dgrow( d.kAnch1, 0, cap );
-	dgrow( d.kAnch2, 0, cap );
-	dgrow( d.kP1, 0, cap );
-	dgrow( d.kP2, 0, cap );
-	dgrow( d.kImp, 0, cap );
-	dgrow( d.kTot, 0, cap );
 	dgrow( d.beginEv, 0, 2 * (size_t)cap );
 	dgrow( d.beginEvF, 0, 9 * (size_t)cap );
 	dgrow( d.endEv, 0, 2 * (size_t)cap );
@@ -1126,7 +1148,7 @@ extern "C" F2D_API int32_t f2d_create_world( const f2d_world_def* def )
 	W->used = true;
 	W->generation = (uint16_t)( gen + 1 );
 	W->index = slot;
-	W->gridSolverOnly = getenv( "F2D_NO_CLUSTER_SOLVER" ) != nullptr;
+	W->smallParts = getenv( "F2D_NO_CLUSTER_SOLVER" ) != nullptr;
 	DWorld& d = W->d;
 	memset( &d, 0, sizeof( d ) );
 	d.gravity = mk( (float)def->gravityX, (float)def->gravityY );
@@ -1189,10 +1211,11 @@ static void free_world( HostWorld* W )
 	F( cmass ); F( mnorm ); F( csimplex ); F( mpA ); F( mpB ); F( mpI ); F( contactFree ); F( pairHash ); F( mortonKeys );
 	F( mortonKeysAlt ); F( leafShape ); F( leafShapeAlt ); F( nodeLeft ); F( nodeRight ); F( nodeParent ); F( nodeBox );
 	F( nodeVisit ); F( sortHist ); F( pairKeys ); F( pairKeysAlt ); F( pairVal ); F( pairValAlt ); F( planIds );
-	F( planKeys ); F( opContact ); F( opKind ); F( opColor ); F( opDone ); F( opBodies ); F( opScan ); F( slotContact ); F( overflowList );
-	F( kIndex ); F( kMass ); F( kNormal ); F( kMisc ); F( kSoft ); F( kAnch1 ); F( kAnch2 ); F( kP1 ); F( kP2 );
-	F( kImp ); F( kTot ); F( jbody ); F( jflags ); F( jcolor ); F( jcolorSet ); F( jnext ); F( jdef0 ); F( jdef1 ); F( jdef2 ); F( jdef3 );
-	F( jimp ); F( jimp2 ); F( jprep0 ); F( jprep1 ); F( jprep2 ); F( jprep3 ); F( jprepM ); F( jindex ); F( overflowJoints ); F( npBucket ); F( ovfOwner ); F( ovfLevel ); F( ovfOrder );
+	F( planKeys ); F( opContact ); F( opKind ); F( opColor ); F( opDone ); F( opBodies ); F( opScan ); F( overflowList );
+	F( slotPlace ); F( kRow ); F( jbody ); F( jflags ); F( jcolor ); F( jcolorSet ); F( jnext ); F( jdef0 ); F( jdef1 ); F( jdef2 ); F( jdef3 );
+	F( jimp ); F( jimp2 ); F( jprep0 ); F( jprep1 ); F( jprep2 ); F( jprep3 ); F( jprepM ); F( jindex ); F( overflowJoints ); F( npBucket ); F( orderState ); F( bodyPos ); F( bodyAt ); F( bodyOrd );
+	F( bodyInt ); F( dsub ); F( jointPlace ); F( jointSlots ); F( ovfItems ); F( ovfSorted ); F( ovfRank ); F( ovfNext );
+	F( binContacts ); F( binContactStart );
 	F( pendingJointOps ); F( fastBodies ); F( beginEv ); F( beginEvF ); F( endEv ); F( hitEvI ); F( hitEvF ); F( moveEvBody );
 	F( moveEvXf ); F( staticShapes ); F( sensorShapes ); F( sensorKeys ); F( sensorKeysAlt ); F( sensorPrevKeys );
 	F( sensorBeginEv ); F( sensorEndEv ); F( cbList ); F( cbReject ); F( cbManifold ); F( sc ); F( sortTemp ); F( newPoint ); F( newFeat ); F( samples );
@@ -3725,6 +3748,7 @@ static void enqueue_step( HostWorld* W, float dt, int subSteps, int planMode )
 		for ( int i = 0; i < 9; ++i )
 			cudaEventCreate( W->ph + i );
 	W->s.evSolveStart = prof ? W->ph[4] : nullptr;
+	W->s.subSteps = subSteps;
 	launch_reset_counters( d, W->stream );
 	if ( prof )
 		cudaEventRecord( W->ph[0], W->stream );
@@ -3896,11 +3920,10 @@ extern "C" F2D_API int32_t f2d_world_autotune( int32_t worldId, double timeStep,
 	flush_uploads( W );
 	int variants[3];
 	int nv = 0;
-	if ( W->s.clusterCapacity > 0 && W->bodyCount <= W->s.clusterCapacity )
-		variants[nv++] = SOLVER_CLUSTER;
-	variants[nv++] = SOLVER_GRID512;
-	if ( W->s.solverBlocks256 > 0 )
-		variants[nv++] = SOLVER_GRID256;
+	variants[nv++] = SOLVER_FEW_PARTS;
+	variants[nv++] = SOLVER_ONE_PER_SM;
+	if ( W->s.solverBlocks2 > 0 )
+		variants[nv++] = SOLVER_TWO_PER_SM;
 	const int periods[4] = { 4, 8, 16, 32 };
 	int reps = stepsPerCandidate < 1 ? 1 : stepsPerCandidate;
 	int status = 0;
@@ -5046,9 +5069,9 @@ extern "C" F2D_API void f2d_world_get_counters( int32_t worldId, int32_t* out8 )
 	out8[7] = W->jointCount - (int)W->jointFree.size();
 }
 
-// Latency side of the solver's roofline: the grid barriers the last
-// grid-wide solver launch passed (0 after a cluster-solver step) and the
-// measured cost of one barrier on its grid (n barriers timed by events).
+// Grid barriers the solver launch passes (none: its stages are a data flow)
+// and the measured cost of one barrier on its grid (n barriers timed by
+// events).
 extern "C" F2D_API void f2d_world_get_solver_latency( int32_t worldId, int32_t probeBarriers, double* out2 )
 {
 	out2[0] = out2[1] = 0.0;
@@ -5056,9 +5079,6 @@ extern "C" F2D_API void f2d_world_get_solver_latency( int32_t worldId, int32_t p
 	if ( W == nullptr )
 		return;
 	cudaStreamSynchronize( W->stream );
-	int barriers = 0;
-	cudaMemcpy( &barriers, &W->d.sc->solveBarriers, sizeof( int ), cudaMemcpyDeviceToHost );
-	out2[0] = barriers;
 	if ( probeBarriers > 0 && W->s.solverBlocks > 0 )
 	{
 		int* err = W->s.tmpB;

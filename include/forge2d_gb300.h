@@ -658,10 +658,9 @@ F2D_API double f2d_world_get_rebuild_ms( int32_t worldId );
 /* awake bodies, live contacts, touching contacts, overflow contacts, active
  * colours, colouring rounds, shapes, joints (b2Counters, types.h:493-506). */
 F2D_API void f2d_world_get_counters( int32_t worldId, int32_t* out8 );
-/* The grid barriers the last grid-wide solver launch passed (out2[0]; 0 after
- * a step on the cluster solver) and, when probeBarriers > 0, the measured
- * microseconds per grid barrier on that solver's grid (out2[1]): the latency
- * floor of the solver kernel is their product. */
+/* The grid barriers the solver launch passes (out2[0]; 0, its stages are
+ * ordered per body) and, when probeBarriers > 0, the measured microseconds
+ * per grid barrier on that solver's grid (out2[1]). */
 F2D_API void f2d_world_get_solver_latency( int32_t worldId, int32_t probeBarriers, double* out2 );
 /* ---- learned warm start (no reference counterpart) ----------------------
  * A small MLP [12 -> 64 -> 64 -> 2] (BF16 weights, FP32 accumulation,
@@ -700,8 +699,8 @@ F2D_API float f2d_mlp_train( int32_t model, const float* samples14, int32_t n, i
 F2D_API void f2d_mlp_predict( int32_t model, const float* feats12, int32_t n, float* out2 );
 
 /* Autotuner (no reference counterpart). Steps the world through every
- * candidate launch configuration -- solver kernel shape (1 thread-block
- * cluster when the bodies fit, grid-wide with 512- or 256-thread blocks) x
+ * candidate launch configuration -- solver shape (1 larger worlds in one
+ * part, 2 one block per SM, 3 two blocks per SM) x
  * broadphase leaf-order refresh period (4, 8, 16, 32 steps) -- timing each
  * over max(stepsPerCandidate, period) steps, and keeps the fastest. The
  * tuning steps are ordinary steps of the world; no configuration changes any
