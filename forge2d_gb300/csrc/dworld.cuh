@@ -149,6 +149,7 @@ struct DScalars
 	// creation stamp of the next new contact (the bodies' contact lists are
 	// newest first); non-static bodies in the awake set (worlds without
 	// island records); destroy calls: collected contacts, end events
+	unsigned splitBarrier; // the island split's grid barrier
 	int orderTotal; // bodies with a place in the solver's spatial order
 	unsigned long long stampBase;
 	int awakeOrderCount;
@@ -281,6 +282,20 @@ struct DIslands
 	unsigned char* islandBits;
 	int* stack;	   // split scratch, bodyCap
 	int* seeds;	   // split scratch, bodyCap
+	// island split scratch (island.cu): edge rows and push rows by row index,
+	// the rest of long ones; row index per body; marks of
+	// large islands; pop order and its inverse (by row index); islands' first
+	// pops and ids; contacts and joints in list order; joints before each pop;
+	// totals per block
+	int2 *splitRows, *splitPool;
+	int *splitPush, *splitPushPool;
+	int* splitIndex;
+	unsigned char* splitMarks;
+	int *splitOrder, *splitPop;
+	int2* splitIslands;
+	int *splitContacts, *splitJoints, *splitJointAt;
+	int2* splitTotals;
+	int splitPoolCount, splitPushCount, splitSerial, splitIslandCount, splitExtra;
 	int* order;	   // new-contact creation order, contactCap
 	int* flag;		   // per awake island: scan input (bodyCap)
 	int* pos;		   // scan output (bodyCap)

@@ -515,6 +515,7 @@ __global__ void k_reset_step_counters( DWorld w )
 	w.sc->hitCount = 0;
 	w.sc->fastCount = 0;
 	w.sc->newPointCount = 0;
+	w.sc->splitBarrier = 0;
 	for ( int k = 0; k < 8; ++k )
 		w.sc->npCount[k] = 0;
 	int age = w.sc->orderAge;

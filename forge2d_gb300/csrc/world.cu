@@ -466,6 +466,15 @@ static void isl_ensure( HostWorld* W )
 		dgrow( h.islandBits, 0, nb );
 		dgrow( h.stack, 0, nb );
 		dgrow( h.seeds, 0, nb );
+		dgrow( h.splitIndex, 0, nb );
+		dgrow( h.splitMarks, 0, 2 * nb + 8 );
+		dgrow( h.splitRows, 0, 16 * nb );
+		dgrow( h.splitPush, 0, 16 * nb );
+		dgrow( h.splitOrder, 0, nb );
+		dgrow( h.splitPop, 0, 2 * nb );
+		dgrow( h.splitIslands, 0, nb + 1 );
+		dgrow( h.splitJointAt, 0, nb );
+		dgrow( h.splitTotals, 0, 1024 );
 		dgrow( h.flag, 0, nb );
 		dgrow( h.pos, 0, nb );
 		dgrow( h.list, 0, nb );
@@ -507,6 +516,17 @@ static void isl_ensure( HostWorld* W )
 		dgrow( h.ncKeysAlt, 0, 2 * (size_t)d.pairCap );
 		h.ncCap = 2 * d.pairCap;
 	}
+	if ( oc != nc || oj != nj )
+	{
+		dfree( h.splitPool );
+		dgrow( h.splitPool, 0, 2 * ( nc + nj ) );
+		dfree( h.splitPushPool );
+		dgrow( h.splitPushPool, 0, 4 * ( nc + nj ) );
+		dfree( h.splitContacts );
+		dgrow( h.splitContacts, 0, nc );
+		dfree( h.splitJoints );
+		dgrow( h.splitJoints, 0, nj );
+	}
 	if ( h.logCap < d.bodyCap + d.jointCap )
 	{
 		dfree( h.log );
@@ -529,7 +549,9 @@ static void isl_free( HostWorld* W )
 	if ( W->islDev )
 	{
 		int* pi[] = { h.bSet, h.bLocal, h.bIsland, h.bIslandPrev, h.bIslandNext, h.bHeadContact, h.bSetNext, h.bMark,
-					  h.bMoveIndex, h.islandFree, h.setFree, h.awakeBodies, h.awakeIslands, h.stack, h.seeds,
+					  h.bMoveIndex, h.islandFree, h.setFree, h.awakeBodies, h.awakeIslands, h.stack, h.seeds, h.splitIndex,
+					  (int*)h.splitRows, (int*)h.splitPool, h.splitPush, h.splitPushPool, (int*)h.splitMarks, h.splitOrder,
+					  h.splitPop, (int*)h.splitIslands, h.splitContacts, h.splitJoints, h.splitJointAt, (int*)h.splitTotals,
 					  h.moveBody, h.moveAsleep, h.flag, h.pos, h.list, h.cSet, h.cIsland, h.cIslandPrev, h.cIslandNext, h.cSetNext,
 					  h.cMark, h.order, h.jSet, h.jIsland, h.jIslandPrev, h.jIslandNext, h.jSetNext, h.jMark,
 					  h.jOverflowIndex, h.log };
