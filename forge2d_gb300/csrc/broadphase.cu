@@ -468,12 +468,6 @@ __global__ void __launch_bounds__( BP_THREADS ) k_find_pairs( DWorld w )
 	}
 }
 
-__global__ void k_clamp_pairs( DWorld w )
-{
-	if ( w.sc->newPairCount > w.pairCap )
-		w.sc->newPairCount = w.pairCap;
-}
-
 // ---------------------------------------------------------------------------
 // contact creation (contact.c:186-330) in the reference's order: row r of the
 // sorted keys, decoded into (creating proxy's shape, other shape)
@@ -497,7 +491,7 @@ __device__ __forceinline__ int plan_lookup( const DWorld& w, unsigned long long 
 
 __global__ void k_create_contacts( DWorld w, int planMode )
 {
-	int n = w.sc->newPairCount;
+	int n = min( w.sc->newPairCount, w.pairCap );
 	int F = w.sc->contactFreeCount;
 	int base = w.sc->contactIdCount;
 	for ( int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x )
@@ -623,6 +617,22 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 						void* hookContext )
 {
 	int gridS = grid_for( w.shapeCount );
+	// world.c:488-502: the dynamic and kinematic trees are rebuilt over their
+	// enlarged nodes every step, on a stream of their own beside the collide
+	// phase (as the reference's rebuild task runs beside its collide tasks).
+	// Gathering the nodes only reads the trees and starts at once. The rebuild
+	// itself waits for the pair search, which ranks the new pairs in them, and
+	// for the sorts after it: cooperative grids do not share the device, and
+	// behind the rebuild's 130 us at 100k bodies the pair sort ended 85 us later.
+	// Nothing else reads or writes the trees until the world joins that stream
+	// before its persistent solver, which needs the whole GPU.
+	cudaStream_t rs = s.rebuild ? s.rebuild : st;
+	if ( rs != st )
+	{
+		cudaEventRecord( s.rebuildFork, st );
+		cudaStreamWaitEvent( rs, s.rebuildFork, 0 );
+		launch_pt_gather( w, rs );
+	}
 	launch_pt_host_moves( w, s, st );
 	// the pair hash of the live contacts is built beside the leaf ordering,
 	// which does not touch it; both meet before the refit
@@ -643,8 +653,8 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 	k_bounds_partial<<<s.boundsBlocks, BP_THREADS, 0, st>>>( w, s.bounds );
 	k_bounds_final<<<1, BP_THREADS, 0, st>>>( &w.sc->rebuildOrder, s.bounds, s.boundsBlocks );
 	k_morton<<<gridS, BP_THREADS, 0, st>>>( w, s.bounds );
-	sort_coop<unsigned>( w.mortonKeys, w.leafShape, w.mortonKeysAlt, w.leafShapeAlt, &w.sc->treeLeafCount, 30,
-						 w.sortHist, &w.sc->barrierCount, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder );
+	sort_coop<unsigned>( w.mortonKeys, w.leafShape, w.mortonKeysAlt, w.leafShapeAlt, &w.sc->treeLeafCount, w.shapeCap, 30,
+						 w.sortHist, w.sc->sortBarrier + SORT_MORTON, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder );
 	if ( hs != st )
 		cudaStreamWaitEvent( st, s.sideJoin[0], 0 );
 	// the solver's body order follows the leaf order, beside the pair search
@@ -656,36 +666,32 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 	launch_solver_order( w, s, s.side[3] ? s.side[3] : st );
 	k_wide_refit<<<( ( w.shapeCap + WIDE - 1 ) / WIDE + 7 ) / 8, BP_THREADS, 0, st>>>( w );
 	k_find_pairs<<<( w.shapeCap + FIND_WARPS - 1 ) / FIND_WARPS, BP_THREADS, 0, st>>>( w );
-	k_clamp_pairs<<<1, 1, 0, st>>>( w );
 	// keys are unique (one per pair), so the key order alone fixes the result
 	int bits = 2 * w.pairKeyBits + 2;
-	sort_coop<unsigned long long>( w.pairKeys, w.pairVal, w.pairKeysAlt, w.pairValAlt, &w.sc->newPairCount, bits,
-								   w.sortHist, &w.sc->barrierCount, &w.sc->error, s.sortBlocks64, st );
+	sort_coop<unsigned long long>( w.pairKeys, w.pairVal, w.pairKeysAlt, w.pairValAlt, &w.sc->newPairCount, w.pairCap, bits,
+								   w.sortHist, w.sc->sortBarrier + SORT_PAIRS, &w.sc->error, s.sortBlocks64, st );
 	launch_pt_decode( w, st );
-	// world.c:488-502: the dynamic and kinematic trees are rebuilt over
-	// their enlarged nodes every step, once the new pairs have their tree
-	// ranks, beside the rest of the collide phase (as the reference's rebuild
-	// task runs beside its collide tasks); nothing until the solver reads or
-	// writes them, and the world joins the rebuild's stream before its
-	// persistent cooperative solver, which needs the whole GPU
-	if ( s.rebuild )
-	{
-		cudaEventRecord( s.rebuildFork, st );
-		cudaStreamWaitEvent( s.rebuild, s.rebuildFork, 0 );
-		if ( s.rebuildT0 )
-			cudaEventRecord( s.rebuildT0, s.rebuild );
-		launch_pt_rebuild( w, s, s.rebuild );
-		if ( s.rebuildT1 )
-			cudaEventRecord( s.rebuildT1, s.rebuild );
-		cudaEventRecord( s.rebuildJoin, s.rebuild );
-	}
-	else
-		launch_pt_rebuild( w, s, st );
 	// broad_phase.c:267-278: the custom filter sees the new pairs last
 	if ( pairHook )
 		pairHook( hookContext );
 	k_create_contacts<<<grid_for( w.pairCap ), BP_THREADS, 0, st>>>( w, planMode );
 	if ( w.isl )
 		launch_isl_new_contacts( w, s, st, planMode );
+	if ( rs != st )
+	{
+		cudaEventRecord( s.rebuildFork, st );
+		cudaStreamWaitEvent( rs, s.rebuildFork, 0 );
+		if ( s.rebuildT0 )
+			cudaEventRecord( s.rebuildT0, rs );
+		launch_pt_rebuild( w, s, rs );
+		if ( s.rebuildT1 )
+			cudaEventRecord( s.rebuildT1, rs );
+		cudaEventRecord( s.rebuildJoin, rs );
+	}
+	else
+	{
+		launch_pt_gather( w, st );
+		launch_pt_rebuild( w, s, st );
+	}
 	k_after_create<<<gridS, BP_THREADS, 0, st>>>( w, planMode );
 }

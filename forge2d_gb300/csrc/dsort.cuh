@@ -55,14 +55,14 @@ union CSortSmem
 
 template <typename K>
 __global__ void __launch_bounds__( CSORT_THREADS )
-	k_sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, const int* nPtr, int bits, unsigned* hist,
+	k_sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, const int* nPtr, int cap, int bits, unsigned* hist,
 				 unsigned* counter, int* err, const int* enable )
 {
 	__shared__ CSortSmem sm;
 	const int tid = threadIdx.x;
 	if ( enable && *enable == 0 )
 		return;
-	const int n = *nPtr;
+	const int n = min( *nPtr, cap );
 	if ( n <= 1 )
 		return;
 	if ( n <= CSORT_SMALL )
@@ -297,10 +297,11 @@ __global__ void __launch_bounds__( CSORT_THREADS )
 
 // Sorts (keys, vals) by the low `bits` bits of the keys; vals may be null.
 // n from device memory. hist needs 256 * CSORT_MAX_BLOCKS unsigned; counter
-// is a device word used by the grid barrier (zeroed here). When enable is
+// is a device word used by the grid barrier (zero before the launch, one
+// launch per step and word). When enable is
 // non-null the sort runs only if *enable != 0.
 template <typename K>
-static inline void sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, const int* nPtr, int bits,
+static inline void sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, const int* nPtr, int cap, int bits,
 							  unsigned* hist, unsigned* counter, int* err, int blocks, cudaStream_t st,
 							  const int* enable = nullptr )
 {
@@ -308,8 +309,7 @@ static inline void sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, cons
 		blocks = CSORT_MAX_BLOCKS;
 	if ( vals == nullptr )
 		valsAlt = nullptr;
-	cudaMemsetAsync( counter, 0, sizeof( unsigned ), st );
-	void* args[] = { &keys, &vals, &keysAlt, &valsAlt, &nPtr, &bits, &hist, &counter, &err, &enable };
+	void* args[] = { &keys, &vals, &keysAlt, &valsAlt, &nPtr, &cap, &bits, &hist, &counter, &err, &enable };
 	cudaLaunchCooperativeKernel( (void*)k_sort_coop<K>, dim3( blocks ), dim3( CSORT_THREADS ), args, 0, st );
 }
 

@@ -77,3 +77,45 @@ __device__ __forceinline__ bool grid_barrier( unsigned* counter, int* err, unsig
 	__syncthreads();
 	return s_timedOut == 0;
 }
+
+// Decoupled look-back over tiles claimed in launch order, one word per tile
+// (zeroed before the launch): flag << 32 | value, 1 aggregate, 2 inclusive
+// prefix. A tile publishes its aggregate, then one whole warp asks for its
+// exclusive prefix, 32 preceding tiles at a time (a lane per word alone would
+// pay an L2 round trip per tile).
+__device__ __forceinline__ void lookback_publish( unsigned long long* state, int tile, int aggregate )
+{
+	st_release_u64( state + tile, ( tile == 0 ? 2ull << 32 : 1ull << 32 ) | (unsigned)aggregate );
+}
+
+__device__ __forceinline__ int lookback_prefix( unsigned long long* state, int tile, int aggregate, int* err )
+{
+	const int lane = threadIdx.x & 31;
+	int prefix = 0;
+	for ( int end = tile; end > 0; end -= 32 )
+	{
+		const int j = end - 1 - lane;
+		unsigned long long v = 2ull << 32;
+		for ( long long spins = 0; j >= 0; )
+		{
+			v = ld_acquire_u64( state + j );
+			if ( ( v >> 32 ) != 0ull )
+				break;
+			if ( ++spins > F2D_SPIN_LIMIT )
+			{
+				atomicOr( err, F2D_ERR_BARRIER_TIMEOUT );
+				v = 2ull << 32;
+				break;
+			}
+		}
+		__syncwarp();
+		const unsigned done = __ballot_sync( 0xffffffffu, ( v >> 32 ) == 2ull );
+		const int last = done ? __ffs( done ) - 1 : 31;
+		prefix += __reduce_add_sync( 0xffffffffu, lane <= last ? (int)(unsigned)( v & 0xffffffffull ) : 0 );
+		if ( done )
+			break;
+	}
+	if ( lane == 0 && tile > 0 )
+		st_release_u64( state + tile, ( 2ull << 32 ) | (unsigned)( prefix + aggregate ) );
+	return prefix;
+}

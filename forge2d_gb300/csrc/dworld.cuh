@@ -88,6 +88,20 @@
 // (new pairs are sorted by key), so it is refreshed periodically.
 #define ORDER_REBUILD_PERIOD 8
 
+// Tiles of the one-launch compactions, an item per thread: the work behind an
+// item (a walk up a tree, an op's dependent reads) wants as many threads as
+// there are items. With 4 items a thread the moves of 100k bodies ran on 25
+// blocks and took 130 us instead of the 52 us of the launches they replace.
+#define LOOKBACK_TILE 512
+#define LOOKBACK_WORDS( cap ) ( 2 + ( cap ) / LOOKBACK_TILE + 1 )
+
+// Grid-barrier words of the step's sorts.
+#define SORT_MORTON 0
+#define SORT_PAIRS 1
+#define SORT_EDGES 2
+#define SORT_LINKS 3
+#define SORT_SENSORS 4
+
 // Substeps of one solver launch, at most (rows of DWorld::dsub per body).
 #define FLOW_SUBSTEPS 8
 // Blocks of the solver launch, at most, and rows of a contact constraint.
@@ -97,6 +111,14 @@
 // worlds to many blocks).
 #define SOLVER_MIN_CHUNK 64
 #define SOLVER_SMALL_CHUNK 8
+
+// Graph kinds of a state-change op.
+enum
+{
+	OP_NONE = 0,
+	OP_ADD = 1,
+	OP_REMOVE = 2
+};
 
 // Per-step scalars kept in device memory so that no launch needs a host
 // round trip.
@@ -114,8 +136,9 @@ struct DScalars
 	int beginCount, endCount, hitCount, moveCount;
 	int error;
 	int colorRounds;
-	unsigned barrierCount;
-	unsigned ptBarrier; // the tree rebuild's grid barrier (it runs beside other kernels)
+	// grid barriers of the step's one-launch kernels, zeroed at its start: the
+	// tree rebuilds (they run beside other kernels) and the sorts (SORT_*)
+	unsigned ptBarrier[2], sortBarrier[5];
 	unsigned barrierGen;
 	int planCount;
 	int awakeCount;
@@ -440,7 +463,10 @@ struct DWorld
 	int* opColor;	// colour result / colour removed
 	int* opDone;
 	int2* opBodies; // solver body indices of the op's contact (-1 static)
-	unsigned long long* opScan; // look-back state of the op output scans
+	unsigned long long* opScan; // look-back state of the op output scans (zeroed at the step's start, as the next two)
+	unsigned long long* collectScan; // of the state-change ops
+	unsigned long long* moveScan;	 // of the move array
+	int lookbackWords;				 // words of the three together
 
 	// ---------------- constraints (by slot, grouped by colour) ----------------
 	int* overflowList; // contact ids in overflow-array order

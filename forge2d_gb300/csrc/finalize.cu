@@ -228,6 +228,52 @@ __device__ __forceinline__ bool joint_allows( const DWorld& w, int ia, int ib )
 	return true;
 }
 
+// solver.c:1758-1818 hit events
+__device__ __forceinline__ void hit_events( const DWorld& w )
+{
+	int n = w.sc->contactIdCount;
+	for ( int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x )
+	{
+		// contacts in the graph
+		int flags = w.cflags[c];
+		if ( ( flags & CF_USED ) == 0 || ( flags & CF_HIT_EVENT ) == 0 || w.ccolor[c] < 0 )
+			continue;
+		float4 mn = w.mnorm[c];
+		int count = __float_as_int( mn.w );
+		float approach = w.hitEventThreshold;
+		bool hit = false;
+		fv2 point = mk( 0.0f, 0.0f );
+		for ( int j = 0; j < count; ++j )
+		{
+			float4 im = w.mpI[2 * c + j];
+			float s = -im.w;
+			if ( s > approach && im.z > 0.0f )
+			{
+				approach = s;
+				float4 pb = w.mpB[2 * c + j];
+				point = mk( pb.x, pb.y );
+				hit = true;
+			}
+		}
+		if ( hit )
+		{
+			int e = atomicAdd( &w.sc->hitCount, 1 );
+			if ( e < w.eventCap )
+			{
+				int2 s = w.cshape[c];
+				w.hitEvI[2 * e] = s.x;
+				w.hitEvI[2 * e + 1] = s.y;
+				float* o = w.hitEvF + 5 * e;
+				o[0] = point.x;
+				o[1] = point.y;
+				o[2] = mn.x;
+				o[3] = mn.y;
+				o[4] = approach;
+			}
+		}
+	}
+}
+
 // solver.c:390-541: one thread per fast body; candidate static shapes are
 // visited in shape-id order
 #define CCD_LIST_MAX 64
@@ -249,7 +295,9 @@ __device__ __forceinline__ bool ccd_rejected( const DWorld& w, unsigned long lon
 
 // listOnly: with a custom filter, a first pass lists the (static shape,
 // fast shape) candidates that reach the filter (solver.c:270-280) for the
-// host and changes nothing; the second pass skips the ones it rejected.
+// host and changes nothing; the second pass skips the ones it rejected. The
+// hit events, which need the solver's impulses only, are found by the same
+// launch.
 __global__ void k_continuous( DWorld w, int listOnly )
 {
 	int n = w.sc->fastCount;
@@ -462,56 +510,22 @@ __global__ void k_continuous( DWorld w, int listOnly )
 			}
 		}
 	}
+	if ( !listOnly )
+		hit_events( w );
 }
 
-// solver.c:1758-1818 hit events
-__global__ void k_hit_events( DWorld w )
-{
-	int n = w.sc->contactIdCount;
-	for ( int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x )
-	{
-		// contacts in the graph
-		int flags = w.cflags[c];
-		if ( ( flags & CF_USED ) == 0 || ( flags & CF_HIT_EVENT ) == 0 || w.ccolor[c] < 0 )
-			continue;
-		float4 mn = w.mnorm[c];
-		int count = __float_as_int( mn.w );
-		float approach = w.hitEventThreshold;
-		bool hit = false;
-		fv2 point = mk( 0.0f, 0.0f );
-		for ( int j = 0; j < count; ++j )
-		{
-			float4 im = w.mpI[2 * c + j];
-			float s = -im.w;
-			if ( s > approach && im.z > 0.0f )
-			{
-				approach = s;
-				float4 pb = w.mpB[2 * c + j];
-				point = mk( pb.x, pb.y );
-				hit = true;
-			}
-		}
-		if ( hit )
-		{
-			int e = atomicAdd( &w.sc->hitCount, 1 );
-			if ( e < w.eventCap )
-			{
-				int2 s = w.cshape[c];
-				w.hitEvI[2 * e] = s.x;
-				w.hitEvI[2 * e + 1] = s.y;
-				float* o = w.hitEvF + 5 * e;
-				o[0] = point.x;
-				o[1] = point.y;
-				o[2] = mn.x;
-				o[3] = mn.y;
-				o[4] = approach;
-			}
-		}
-	}
-}
-
+// Counters, grid-barrier words and look-back states of the step.
 __global__ void k_reset_step_counters( DWorld w )
 {
+	for ( int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.lookbackWords; i += gridDim.x * blockDim.x )
+		w.opScan[i] = 0ull;
+	if ( blockIdx.x != 0 || threadIdx.x != 0 )
+		return;
+	for ( int k = 0; k < 2; ++k )
+		w.sc->ptBarrier[k] = 0;
+	for ( int k = 0; k < 5; ++k )
+		w.sc->sortBarrier[k] = 0;
+	w.sc->pendingOps = 0;
 	w.sc->hitCount = 0;
 	w.sc->fastCount = 0;
 	w.sc->newPointCount = 0;
@@ -538,16 +552,16 @@ void launch_finalize( DWorld& w, StepScratch& s, cudaStream_t st, float dt, Host
 		k_continuous<<<grid_for( w.bodyCount ), 64, 0, st>>>( w, 1 );
 		ccdHook( hookContext );
 	}
-	k_continuous<<<grid_for( w.bodyCount ), 64, 0, st>>>( w, 0 );
-	k_hit_events<<<grid_for( w.contactCap ), 256, 0, st>>>( w );
+	k_continuous<<<grid_for( w.contactCap > w.bodyCount ? w.contactCap : w.bodyCount ), 64, 0, st>>>( w, 0 );
 	// solver.c:1842-1905: enlarged proxies enter the move array of the next
 	// step in awake order and grow their tree leaves
-	launch_pt_moves( w, s, st );
+	launch_pt_moves( w, st );
 	if ( w.isl )
 		launch_isl_sleep( w, st, s.scanState );
 }
 
 void launch_reset_counters( DWorld& w, cudaStream_t st )
 {
-	k_reset_step_counters<<<1, 1, 0, st>>>( w );
+	int blocks = ( w.lookbackWords + 1023 ) / 1024;
+	k_reset_step_counters<<<blocks < 8 ? blocks : 8, 1024, 0, st>>>( w );
 }

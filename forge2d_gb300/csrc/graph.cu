@@ -29,13 +29,6 @@
 #define OVF_HASH 4096	  // shared-memory hash of overflow-array positions
 #define OVF_LIST_SMEM 2048 // overflow-array length handled in shared memory
 
-enum
-{
-	OP_NONE = 0,
-	OP_ADD = 1,
-	OP_REMOVE = 2
-};
-
 __device__ __forceinline__ int body_solver_index( const DWorld& w, int b )
 {
 	return body_type( w.bflags[b] ) == 0 ? -1 : b;
@@ -45,39 +38,6 @@ __device__ __forceinline__ int op_count( const DWorld& w )
 {
 	int n = w.sc->opCount;
 	return n > w.opCap ? w.opCap : n;
-}
-
-// Graph kind of each op, its solver bodies, and the lock reset of the first
-// round (world.c:586-686 order of cases).
-__global__ void k_op_prepare( DWorld w, int* gkind )
-{
-	int nOps = op_count( w );
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < nOps; k += gridDim.x * blockDim.x )
-	{
-		int c = w.opContact[k];
-		int kind = w.opKind[k];
-		int f = w.cflags[c];
-		int g = OP_NONE;
-		if ( kind == 1 )
-			g = OP_ADD;
-		else if ( ( kind == 2 ) || ( kind == 0 && ( f & CF_TOUCHING ) ) )
-			g = OP_REMOVE;
-		w.opColor[k] = g == OP_REMOVE ? w.ccolor[c] : F2D_NULL;
-		w.opDone[k] = g == OP_NONE ? 1 : 0;
-		gkind[k] = g;
-		int2 ab = make_int2( -1, -1 );
-		if ( g != OP_NONE )
-		{
-			int2 bd = w.cbody[c];
-			ab.x = body_solver_index( w, bd.x );
-			ab.y = body_solver_index( w, bd.y );
-			if ( ab.x >= 0 )
-				w.colorLock[ab.x] = INT_MAX;
-			if ( ab.y >= 0 )
-				w.colorLock[ab.y] = INT_MAX;
-		}
-		w.opBodies[k] = ab;
-	}
 }
 
 __global__ void k_op_lock( DWorld w )
@@ -149,32 +109,35 @@ __device__ __forceinline__ void apply_op( const DWorld& w, int k, int g, int a, 
 	}
 }
 
-// First round, grid-wide: lock owners apply; the rest are flagged pending.
-__global__ void k_op_round( DWorld w, const int* gkind, int* pending )
+// First round, grid-wide: lock owners apply; the rest are listed (the list's
+// order does not matter, the rounds lock by op number).
+__global__ void k_op_round( DWorld w, const int* gkind, int* list )
 {
-	int nOps = op_count( w );
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < nOps; k += gridDim.x * blockDim.x )
+	const int nOps = op_count( w );
+	const unsigned lane = threadIdx.x & 31u;
+	for ( int base = blockIdx.x * blockDim.x; base < nOps; base += gridDim.x * blockDim.x )
 	{
-		int pend = 0;
-		if ( w.opDone[k] == 0 )
+		int k = base + threadIdx.x;
+		bool pend = false;
+		if ( k < nOps && w.opDone[k] == 0 )
 		{
 			int2 ab = w.opBodies[k];
 			bool own = ( ab.x < 0 || w.colorLock[ab.x] == k ) && ( ab.y < 0 || w.colorLock[ab.y] == k );
 			if ( own )
 				apply_op( w, k, gkind[k], ab.x, ab.y );
 			else
-				pend = 1;
+				pend = true;
 		}
-		pending[k] = pend;
+		unsigned mask = __ballot_sync( 0xffffffffu, pend );
+		if ( mask == 0u )
+			continue;
+		int at = 0;
+		if ( lane == 0u )
+			at = atomicAdd( &w.sc->pendingOps, __popc( mask ) );
+		at = __shfl_sync( 0xffffffffu, at, 0 );
+		if ( pend )
+			list[at + __popc( mask & ( ( 1u << lane ) - 1u ) )] = k;
 	}
-}
-
-__global__ void k_op_pending_list( DWorld w, const int* pending, const int* pos, int* list )
-{
-	int nOps = op_count( w );
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < nOps; k += gridDim.x * blockDim.x )
-		if ( pending[k] )
-			list[pos[k]] = k;
 }
 
 // Remaining rounds in one block over the pending list, compacted in place
@@ -581,24 +544,18 @@ __global__ void k_joint_ops( DWorld w, int count )
 void launch_graph( DWorld& w, StepScratch& s, cudaStream_t st )
 {
 	const size_t cap = (size_t)w.opCap;
-	int* gkind = s.tmpA;
-	int* pending = s.tmpA + cap;
-	int* pos = s.tmpB;
+	int* gkind = s.tmpA; // written with the ops (k_op_collect)
+	int* ovOps = s.tmpA + cap;
 	int* list = s.tmpB + cap;
-	int* ovOps = s.tmpA + cap; // reuses the pending flags once the rounds are done
 	int g = grid_for( w.opCap );
-	k_op_prepare<<<g, 256, 0, st>>>( w, gkind );
 	// sleeping worlds: island links and unlinks (island.cu); a step whose
 	// changes wake a sleeping set applies them serially there, colours
 	// included, and leaves no op for the rounds below
 	if ( w.isl )
 		launch_isl_ops( w, s, st, gkind );
 	k_op_lock<<<g, 256, 0, st>>>( w );
-	k_op_round<<<g, 256, 0, st>>>( w, gkind, pending );
-	scan_lookback( pending, pos, &w.sc->opCount, 0, w.opCap, &w.sc->pendingOps, s.scanState, &w.sc->error, st );
-	k_op_pending_list<<<g, 256, 0, st>>>( w, pending, pos, list );
+	k_op_round<<<g, 256, 0, st>>>( w, gkind, list );
 	k_color_rounds<<<1, GRAPH_THREADS, 0, st>>>( w, gkind, list );
-	cudaMemsetAsync( w.opScan, 0, sizeof( unsigned long long ) * (size_t)OPS_SCAN_WORDS( w.opCap ), st );
 	k_op_outputs<<<( w.opCap + OPS_TILE - 1 ) / OPS_TILE, OPS_TILE, 0, st>>>( w, gkind, ovOps, 0 );
 	k_overflow_ops<<<1, GRAPH_THREADS, 0, st>>>( w, gkind, ovOps );
 }

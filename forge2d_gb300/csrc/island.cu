@@ -1947,7 +1947,7 @@ void launch_isl_new_contacts( DWorld& w, StepScratch& s, cudaStream_t st, int pl
 	int* count = (int*)( (char*)I + offsetof( DIslands, ncCount ) );
 	unsigned long long* k0 = w.islNcKeys;
 	unsigned long long* k1 = w.islNcKeysAlt;
-	sort_coop<unsigned long long>( k0, nullptr, k1, nullptr, count, 32 + bodyBits, w.sortHist, &w.sc->barrierCount,
+	sort_coop<unsigned long long>( k0, nullptr, k1, nullptr, count, INT_MAX, 32 + bodyBits, w.sortHist, w.sc->sortBarrier + SORT_EDGES,
 								   &w.sc->error, s.sortBlocks64, st );
 	int g2 = grid_for( 2 * w.pairCap );
 	k_isl_nc_chain<<<g2, 256, 0, st>>>( I );
@@ -2269,8 +2269,8 @@ void launch_isl_ops( DWorld& w, StepScratch& s, cudaStream_t st, const int* gkin
 	while ( ( 1 << islandBits ) < w.bodyCap + 1 )
 		islandBits += 1;
 	sort_coop<unsigned long long>( w.islNcKeys, nullptr, w.islNcKeysAlt, nullptr,
-								   (int*)( (char*)w.isl + offsetof( DIslands, linkCount ) ), 32 + islandBits, w.sortHist,
-								   &w.sc->barrierCount, &w.sc->error, s.sortBlocks64, st );
+								   (int*)( (char*)w.isl + offsetof( DIslands, linkCount ) ), INT_MAX, 32 + islandBits, w.sortHist,
+								   w.sc->sortBarrier + SORT_LINKS, &w.sc->error, s.sortBlocks64, st );
 	k_isl_link_chain<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_link_heads<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_merge_roots<<<grid_for( w.bodyCap ), 256, 0, st>>>( w, w.isl );

@@ -105,5 +105,6 @@ int pt_large_blocks();
 void launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st );
 void launch_pt_decode( DWorld& w, cudaStream_t st );
 void launch_pt_rebuild( DWorld& w, StepScratch& s, cudaStream_t st );
-void launch_pt_moves( DWorld& w, StepScratch& s, cudaStream_t st );
+void launch_pt_moves( DWorld& w, cudaStream_t st );
+void launch_pt_gather( DWorld& w, cudaStream_t st );
 void launch_pt_ranks( DWorld& w, cudaStream_t st, int t );

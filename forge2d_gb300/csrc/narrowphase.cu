@@ -7,9 +7,11 @@
 // (world.c:586-686).
 #include "dnarrow.cuh"
 #include "dscan.cuh"
-#include "dsort.cuh"
+#include "dsync.cuh"
 #include "dworld.cuh"
 #include "kernels.cuh"
+
+#include <climits>
 
 #define NP_THREADS 128
 
@@ -304,39 +306,76 @@ template <int CLS> __global__ void __launch_bounds__( NP_THREADS ) k_narrowphase
 	}
 }
 
-__global__ void k_op_flags( DWorld w, int* flags )
+// The contacts that changed state, in contact-id order, each with its graph
+// kind, colour and solver bodies, and the lock reset of the first colouring
+// round (world.c:586-686 order of cases): one launch, tiles chained by
+// decoupled look-back.
+__global__ void __launch_bounds__( LOOKBACK_TILE ) k_op_collect( DWorld w, int* gkind )
 {
-	int n = w.sc->contactIdCount;
-	for ( int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x )
+	__shared__ int smem[32];
+	__shared__ int s_tile, s_prefix;
+	const int n = w.sc->contactIdCount;
+	if ( threadIdx.x == 0 )
+		s_tile = (int)atomicAdd( (unsigned*)w.collectScan, 1u );
+	__syncthreads();
+	const int tile = s_tile, base = tile * LOOKBACK_TILE;
+	if ( base >= n )
 	{
-		int f = w.cflags[c];
-		flags[c] = ( ( f & CF_USED ) && ( f & ( CF_DISJOINT | CF_STARTED | CF_STOPPED ) ) ) ? 1 : 0;
+		if ( tile == 0 && threadIdx.x == 0 )
+			w.sc->opCount = 0;
+		return;
 	}
-}
-
-__global__ void k_op_compact( DWorld w, const int* flags, const int* offs )
-{
-	int n = w.sc->contactIdCount;
-	for ( int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x )
+	const int c = base + threadIdx.x;
+	int f = c < n ? w.cflags[c] : 0;
+	if ( ( f & CF_USED ) == 0 || ( f & ( CF_DISJOINT | CF_STARTED | CF_STOPPED ) ) == 0 )
+		f = 0;
+	int total;
+	int k = block_exclusive_scan_1024( f != 0 ? 1 : 0, smem, &total );
+	if ( threadIdx.x < 32 )
 	{
-		if ( flags[c] == 0 )
-			continue;
-		int o = offs[c];
-		if ( o >= w.opCap )
+		if ( threadIdx.x == 0 )
+			lookback_publish( w.collectScan + 1, tile, total );
+		__syncwarp();
+		int prefix = lookback_prefix( w.collectScan + 1, tile, total, &w.sc->error );
+		if ( threadIdx.x == 0 )
 		{
-			atomicOr( &w.sc->error, ERR_OP_CAPACITY );
-			continue;
+			s_prefix = prefix;
+			if ( base + LOOKBACK_TILE >= n )
+				w.sc->opCount = min( prefix + total, w.opCap );
 		}
-		int f = w.cflags[c];
-		w.opContact[o] = c;
-		w.opKind[o] = ( f & CF_DISJOINT ) ? 0 : ( ( f & CF_STARTED ) ? 1 : 2 );
 	}
-}
-
-__global__ void k_op_clamp( DWorld w )
-{
-	if ( w.sc->opCount > w.opCap )
-		w.sc->opCount = w.opCap;
+	__syncthreads();
+	if ( f == 0 )
+		return;
+	k += s_prefix;
+	if ( k >= w.opCap )
+	{
+		atomicOr( &w.sc->error, ERR_OP_CAPACITY );
+		return;
+	}
+	const int kind = ( f & CF_DISJOINT ) ? 0 : ( ( f & CF_STARTED ) ? 1 : 2 );
+	int g = OP_NONE;
+	if ( kind == 1 )
+		g = OP_ADD;
+	else if ( kind == 2 || ( f & CF_TOUCHING ) )
+		g = OP_REMOVE;
+	w.opContact[k] = c;
+	w.opKind[k] = kind;
+	w.opColor[k] = g == OP_REMOVE ? w.ccolor[c] : F2D_NULL;
+	w.opDone[k] = g == OP_NONE ? 1 : 0;
+	gkind[k] = g;
+	int2 ab = make_int2( -1, -1 );
+	if ( g != OP_NONE )
+	{
+		int2 bd = w.cbody[c];
+		ab.x = body_type( w.bflags[bd.x] ) == 0 ? -1 : bd.x;
+		ab.y = body_type( w.bflags[bd.y] ) == 0 ? -1 : bd.y;
+		if ( ab.x >= 0 )
+			w.colorLock[ab.x] = INT_MAX;
+		if ( ab.y >= 0 )
+			w.colorLock[ab.y] = INT_MAX;
+	}
+	w.opBodies[k] = ab;
 }
 
 void launch_narrowphase( DWorld& w, StepScratch& s, cudaStream_t st, HostHook preSolveHook, void* hookContext )
@@ -375,9 +414,5 @@ void launch_narrowphase( DWorld& w, StepScratch& s, cudaStream_t st, HostHook pr
 			cudaEventRecord( s.sideJoin[k], s.side[k] );
 			cudaStreamWaitEvent( st, s.sideJoin[k], 0 );
 		}
-	k_op_flags<<<grid_for( w.contactCap ), 256, 0, st>>>( w, s.tmpA );
-	scan_lookback( s.tmpA, s.tmpB, &w.sc->contactIdCount, 0, w.contactCap, &w.sc->opCount, s.scanState, &w.sc->error,
-				   st );
-	k_op_compact<<<grid_for( w.contactCap ), 256, 0, st>>>( w, s.tmpA, s.tmpB );
-	k_op_clamp<<<1, 1, 0, st>>>( w );
+	k_op_collect<<<( w.contactCap + LOOKBACK_TILE - 1 ) / LOOKBACK_TILE, LOOKBACK_TILE, 0, st>>>( w, s.tmpA );
 }

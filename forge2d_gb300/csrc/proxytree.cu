@@ -75,36 +75,34 @@ __device__ __forceinline__ float4 pt_union( float4 a, float4 b )
 	return make_float4( a.x < b.x ? a.x : b.x, a.y < b.y ? a.y : b.y, a.z > b.z ? a.z : b.z, a.w > b.w ? a.w : b.w );
 }
 
-__device__ __forceinline__ bool cas_lower( float* addr, float v )
+// the coordinate `old` (as read) moved down / up to v; true when it changed
+__device__ __forceinline__ bool cas_lower( float* addr, float old, float v )
 {
-	int* ia = (int*)addr;
-	int old = *(volatile int*)ia;
-	while ( v < __int_as_float( old ) )
+	while ( v < old )
 	{
-		int prev = atomicCAS( ia, old, __float_as_int( v ) );
-		if ( prev == old )
+		int prev = atomicCAS( (int*)addr, __float_as_int( old ), __float_as_int( v ) );
+		if ( prev == __float_as_int( old ) )
 			return true;
-		old = prev;
+		old = __int_as_float( prev );
 	}
 	return false;
 }
 
-__device__ __forceinline__ bool cas_upper( float* addr, float v )
+__device__ __forceinline__ bool cas_upper( float* addr, float old, float v )
 {
-	int* ia = (int*)addr;
-	int old = *(volatile int*)ia;
-	while ( __int_as_float( old ) < v )
+	while ( old < v )
 	{
-		int prev = atomicCAS( ia, old, __float_as_int( v ) );
-		if ( prev == old )
+		int prev = atomicCAS( (int*)addr, __float_as_int( old ), __float_as_int( v ) );
+		if ( prev == __float_as_int( old ) )
 			return true;
-		old = prev;
+		old = __int_as_float( prev );
 	}
 	return false;
 }
 
 // dynamic_tree.c:827-866 b2DynamicTree_EnlargeProxy, one proxy of many at
-// once (see the file comment)
+// once (see the file comment). Bound by the dependent reads up the tree: box,
+// marks and parent of an ancestor are read together.
 __device__ void pt_enlarge( const DProxyTree& T, int leaf, float4 b, int* err )
 {
 	T.box[leaf] = b;
@@ -117,14 +115,18 @@ __device__ void pt_enlarge( const DProxyTree& T, int leaf, float4 b, int* err )
 			return;
 		}
 		float* f = (float*)( T.box + p );
-		bool changed = cas_lower( f + 0, b.x );
-		changed |= cas_lower( f + 1, b.y );
-		changed |= cas_upper( f + 2, b.z );
-		changed |= cas_upper( f + 3, b.w );
-		int old = atomicOr( T.flags + p, PT_ENLARGED );
-		if ( !changed && ( old & PT_ENLARGED ) )
+		const float4 o = __ldcg( T.box + p );
+		const int marks = __ldcg( T.flags + p );
+		const int up = __ldcg( T.parent + p );
+		bool changed = cas_lower( f + 0, o.x, b.x );
+		changed |= cas_lower( f + 1, o.y, b.y );
+		changed |= cas_upper( f + 2, o.z, b.z );
+		changed |= cas_upper( f + 3, o.w, b.w );
+		if ( ( marks & PT_ENLARGED ) == 0 )
+			atomicOr( T.flags + p, PT_ENLARGED );
+		else if ( !changed )
 			return;
-		p = *(volatile int*)( T.parent + p );
+		p = up;
 	}
 }
 
@@ -136,45 +138,73 @@ __device__ __forceinline__ bool body_awake_plain( int f )
 	return ( f & ( BF_USED | BF_ENABLED ) ) == ( BF_USED | BF_ENABLED ) && body_type( f ) != 0 && ( f & BF_ASLEEP ) == 0;
 }
 
-// per awake-set position: the body's enlarged shapes
-__global__ void k_pt_move_count( DWorld w, int* cnt )
+// The enlarged proxies of every awake body join the move array in awake
+// order, and their tree leaves are enlarged: one launch, tiles of bodies
+// chained by decoupled look-back. The first warp looks back for the tile's
+// slots while the others already walk up the tree.
+__global__ void __launch_bounds__( LOOKBACK_TILE ) k_pt_moves( DWorld w )
 {
-	int n = w.isl ? w.isl->awakeBodyCount : w.sc->awakeOrderCount;
-	if ( blockIdx.x == 0 && threadIdx.x == 0 )
+	__shared__ int smem[32];
+	__shared__ int s_tile, s_prefix;
+	const int n = w.isl ? w.isl->awakeBodyCount : w.sc->awakeOrderCount;
+	if ( threadIdx.x == 0 )
+		s_tile = (int)atomicAdd( (unsigned*)w.moveScan, 1u );
+	__syncthreads();
+	const int tile = s_tile, base = tile * LOOKBACK_TILE;
+	if ( tile == 0 && threadIdx.x == 0 )
 		w.sc->fastCount = 0;
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x )
+	if ( base >= n )
 	{
-		int b = w.isl ? w.isl->awakeBodies[k] : w.awakeOrder[k];
-		int c = 0;
-		if ( w.isl || body_awake_plain( w.bflags[b] ) )
-			for ( int s = w.headShape[b], guard = 0; s != F2D_NULL && guard < ( 1 << 20 ); s = w.nextShape[s], ++guard )
-				c += ( w.sflags[s] & SF_ENLARGED ) ? 1 : 0;
-		cnt[k] = c;
+		if ( tile == 0 && threadIdx.x == 0 )
+			w.sc->moveArrayCount = 0;
+		return;
 	}
-}
-
-// move-array slots in awake order; the proxies' tree leaves are enlarged
-__global__ void k_pt_move_assign( DWorld w, const int* pos )
-{
-	int n = w.isl ? w.isl->awakeBodyCount : w.sc->awakeOrderCount;
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x )
+	const int k = base + threadIdx.x;
+	int head = F2D_NULL;
+	if ( k < n )
 	{
 		int b = w.isl ? w.isl->awakeBodies[k] : w.awakeOrder[k];
-		if ( !w.isl && !body_awake_plain( w.bflags[b] ) )
-			continue;
-		int slot = pos[k];
-		for ( int s = w.headShape[b], guard = 0; s != F2D_NULL && guard < ( 1 << 20 ); s = w.nextShape[s], ++guard )
+		if ( w.isl || body_awake_plain( w.bflags[b] ) )
+			head = w.headShape[b];
+	}
+	int cnt = 0;
+	for ( int s = head, guard = 0; s != F2D_NULL && guard < ( 1 << 20 ); s = w.nextShape[s], ++guard )
+		cnt += ( w.sflags[s] & SF_ENLARGED ) ? 1 : 0;
+	int total;
+	int slot = block_exclusive_scan_1024( cnt, smem, &total );
+	if ( threadIdx.x < 32 )
+	{
+		if ( threadIdx.x == 0 )
+			lookback_publish( w.moveScan + 1, tile, total );
+		__syncwarp();
+		int prefix = lookback_prefix( w.moveScan + 1, tile, total, &w.sc->error );
+		if ( threadIdx.x == 0 )
 		{
-			int f = w.sflags[s];
-			if ( ( f & SF_ENLARGED ) == 0 )
-				continue;
-			w.moveShape[slot] = s;
-			w.shapeMove[s] = slot;
-			slot += 1;
-			w.sflags[s] = ( f & ~SF_ENLARGED ) | SF_MOVED;
-			int pk = w.proxyKey[s];
-			pt_enlarge( w.pt[pk & 3], pk >> 2, w.fat[s], &w.sc->error );
+			s_prefix = prefix;
+			if ( base + LOOKBACK_TILE >= n )
+				w.sc->moveArrayCount = prefix + total;
 		}
+	}
+	if ( cnt > 0 )
+		for ( int s = head, guard = 0; s != F2D_NULL && guard < ( 1 << 20 ); s = w.nextShape[s], ++guard )
+			if ( w.sflags[s] & SF_ENLARGED )
+			{
+				int pk = w.proxyKey[s];
+				pt_enlarge( w.pt[pk & 3], pk >> 2, w.fat[s], &w.sc->error );
+			}
+	__syncthreads();
+	if ( cnt == 0 )
+		return;
+	slot += s_prefix;
+	for ( int s = head, guard = 0; s != F2D_NULL && guard < ( 1 << 20 ); s = w.nextShape[s], ++guard )
+	{
+		int f = w.sflags[s];
+		if ( ( f & SF_ENLARGED ) == 0 )
+			continue;
+		w.moveShape[slot] = s;
+		w.shapeMove[s] = slot;
+		slot += 1;
+		w.sflags[s] = ( f & ~SF_ENLARGED ) | SF_MOVED;
 	}
 }
 
@@ -221,6 +251,9 @@ __global__ void k_pt_host_done( DWorld w, const int* flag, const int* pos )
 __global__ void k_pt_decode( DWorld w )
 {
 	int n = min( w.sc->newPairCount, w.pairCap );
+	// what follows reads the count as it is kept
+	if ( blockIdx.x == 0 && threadIdx.x == 0 && w.sc->newPairCount > n )
+		w.sc->newPairCount = n;
 	int rb = w.pairKeyBits;
 	for ( int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x )
 		w.pairValAlt[r] = w.moveShape[(int)( w.pairKeys[r] >> ( rb + 2 ) )];
@@ -1175,39 +1208,55 @@ void launch_pt_decode( DWorld& w, cudaStream_t st )
 	k_pt_decode<<<grid_for( w.pairCap ), 256, 0, st>>>( w );
 }
 
+static bool pt_present( const DWorld& w, int t )
+{
+	return w.pt[t].cap > 0 && w.ptProxies[t] > 0;
+}
+
+static void pt_gather( DWorld& w, cudaStream_t st, int t )
+{
+	int g = grid_for( w.pt[t].cap );
+	k_pt_mark<<<g, 256, 0, st>>>( w, t );
+	k_pt_count<<<g, 256, 0, st>>>( w, t );
+	k_pt_gather<<<g, 256, 0, st>>>( w, t );
+}
+
 // collide phase: partial rebuild of the dynamic and kinematic trees
-// (broad_phase.c:488-492)
+// (broad_phase.c:488-492). The first tree's nodes are gathered ahead of the
+// rebuild (the scratch holds one tree's at a time).
+void launch_pt_gather( DWorld& w, cudaStream_t st )
+{
+	int t = pt_present( w, 2 ) ? 2 : 1;
+	if ( pt_present( w, t ) )
+		pt_gather( w, st, t );
+}
+
 void launch_pt_rebuild( DWorld& w, StepScratch& s, cudaStream_t st )
 {
+	bool first = true;
 	for ( int t = 2; t >= 1; --t )
 	{
-		const DProxyTree& T = w.pt[t];
-		if ( T.cap == 0 || w.ptProxies[t] == 0 )
+		if ( !pt_present( w, t ) )
 			continue;
-		int g = grid_for( T.cap );
-		k_pt_mark<<<g, 256, 0, st>>>( w, t );
-		k_pt_count<<<g, 256, 0, st>>>( w, t );
-		k_pt_gather<<<g, 256, 0, st>>>( w, t );
+		if ( !first )
+			pt_gather( w, st, t );
+		first = false;
 		if ( s.ptBlocks > 0 )
 		{
-			unsigned* counter = &w.sc->ptBarrier;
-			cudaMemsetAsync( counter, 0, sizeof( unsigned ), st );
+			unsigned* counter = w.sc->ptBarrier + ( t - 1 );
 			void* args[] = { &w, &t, &counter };
 			cudaLaunchCooperativeKernel( (void*)k_pt_large, dim3( s.ptBlocks ), dim3( PT_THREADS ), args,
 										 sizeof( PtLarge ), st );
 		}
 		k_pt_small<<<F2D_SMS * 2, PT_THREADS, sizeof( PtSmall ), st>>>( w, t );
-		k_pt_refresh<<<g, 256, 0, st>>>( w, t );
+		k_pt_refresh<<<grid_for( w.pt[t].cap ), 256, 0, st>>>( w, t );
 	}
 }
 
 // finalize: the move array in awake order, proxies enlarged
-void launch_pt_moves( DWorld& w, StepScratch& s, cudaStream_t st )
+void launch_pt_moves( DWorld& w, cudaStream_t st )
 {
-	int* count = w.isl ? (int*)( (char*)w.isl + offsetof( DIslands, awakeBodyCount ) ) : &w.sc->awakeOrderCount;
-	k_pt_move_count<<<grid_for( w.bodyCap ), 256, 0, st>>>( w, s.tmpA );
-	scan_lookback( s.tmpA, s.tmpB, count, w.bodyCount, w.bodyCap, &w.sc->moveArrayCount, s.scanState, &w.sc->error, st );
-	k_pt_move_assign<<<grid_for( w.bodyCap ), 256, 0, st>>>( w, s.tmpB );
+	k_pt_moves<<<( w.bodyCap + LOOKBACK_TILE - 1 ) / LOOKBACK_TILE, LOOKBACK_TILE, 0, st>>>( w );
 }
 
 // after a host upload of tree t

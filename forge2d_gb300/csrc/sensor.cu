@@ -200,7 +200,7 @@ void launch_sensors( DWorld& w, StepScratch& s, cudaStream_t st )
 	while ( bits < 64 && ( 1ll << ( bits - 32 ) ) < w.sensorCount )
 		bits += 1;
 	// keys are unique, so their order alone fixes the result
-	sort_coop<unsigned long long>( w.sensorKeys, nullptr, w.sensorKeysAlt, nullptr, &w.sc->sensorCur, bits,
-								   w.sortHist, &w.sc->barrierCount, &w.sc->error, s.sortBlocks64, st );
+	sort_coop<unsigned long long>( w.sensorKeys, nullptr, w.sensorKeysAlt, nullptr, &w.sc->sensorCur, INT_MAX, bits,
+								   w.sortHist, w.sc->sortBarrier + SORT_SENSORS, &w.sc->error, s.sortBlocks64, st );
 	k_sensor_events<<<1, SENSOR_THREADS, 0, st>>>( w );
 }

@@ -233,6 +233,14 @@ static void alloc_scratch( HostWorld* W )
 		bits += 1;
 	s.shapeIdBits = bits;
 	d.pairKeyBits = bits;
+	// look-back states, zeroed together at the step's start
+	size_t opWords = OPS_SCAN_WORDS( (size_t)d.opCap ), collectWords = LOOKBACK_WORDS( (size_t)d.contactCap );
+	size_t moveWords = LOOKBACK_WORDS( (size_t)d.bodyCap );
+	d.lookbackWords = (int)( opWords + collectWords + moveWords );
+	dfree( d.opScan );
+	dgrow( d.opScan, 0, (size_t)d.lookbackWords );
+	d.collectScan = d.opScan + opWords;
+	d.moveScan = d.collectScan + collectWords;
 	size_t constraints = (size_t)d.contactCap + d.jointCap;
 	// constraint slots: every part and colour rounds up to whole groups
 	int parts = std::min( SOLVER_MAX_PARTS, d.bodyCap / ( W->smallParts ? SOLVER_SMALL_CHUNK : SOLVER_MIN_CHUNK ) + 2 );
@@ -330,7 +338,6 @@ static void grow_contacts( HostWorld* W, int cap )
 	dgrow( d.opColor, 0, cap );
 	dgrow( d.opDone, 0, cap );
 	dgrow( d.opBodies, 0, cap );
-	dgrow( d.opScan, 0, (size_t)OPS_SCAN_WORDS( cap ) );
 	dgrow( d.overflowList, o, cap );
 	dgrow( d.slotPlace, 0, cap );
 	dgrow( d.npBucket, 0, (size_t)NP_CLASSES * cap );
