@@ -654,7 +654,8 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 	k_bounds_final<<<1, BP_THREADS, 0, st>>>( &w.sc->rebuildOrder, s.bounds, s.boundsBlocks );
 	k_morton<<<gridS, BP_THREADS, 0, st>>>( w, s.bounds );
 	sort_coop<unsigned>( w.mortonKeys, w.leafShape, w.mortonKeysAlt, w.leafShapeAlt, &w.sc->treeLeafCount, w.shapeCap, 30,
-						 w.sortHist, w.sc->sortBarrier + SORT_MORTON, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder );
+						 w.sortHist, w.sc->sortBarrier + SORT_MORTON, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder,
+						 w.shapeCap > SORT_LARGE_WORLD );
 	if ( hs != st )
 		cudaStreamWaitEvent( st, s.sideJoin[0], 0 );
 	// the solver's body order follows the leaf order, beside the pair search
@@ -666,11 +667,13 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 	launch_solver_order( w, s, s.side[3] ? s.side[3] : st );
 	k_wide_refit<<<( ( w.shapeCap + WIDE - 1 ) / WIDE + 7 ) / 8, BP_THREADS, 0, st>>>( w );
 	k_find_pairs<<<( w.shapeCap + FIND_WARPS - 1 ) / FIND_WARPS, BP_THREADS, 0, st>>>( w );
-	// keys are unique (one per pair), so the key order alone fixes the result
+	// keys are unique (one per pair), so the key order alone fixes the result;
+	// a key's top bits are the creating shape's place in the move array
+	SortDecode dec = { w.pairValAlt, w.moveShape, w.pairKeyBits + 2 };
 	int bits = 2 * w.pairKeyBits + 2;
 	sort_coop<unsigned long long>( w.pairKeys, w.pairVal, w.pairKeysAlt, w.pairValAlt, &w.sc->newPairCount, w.pairCap, bits,
-								   w.sortHist, w.sc->sortBarrier + SORT_PAIRS, &w.sc->error, s.sortBlocks64, st );
-	launch_pt_decode( w, st );
+								   w.sortHist, w.sc->sortBarrier + SORT_PAIRS, &w.sc->error, s.sortBlocks64, st, nullptr,
+								   w.shapeCap > SORT_LARGE_WORLD, dec );
 	// broad_phase.c:267-278: the custom filter sees the new pairs last
 	if ( pairHook )
 		pairHook( hookContext );

@@ -5,11 +5,12 @@
 // itself.
 //
 // * sort_coop: stable LSD radix sort of (key, value) rows by the low `bits`
-//   bits of the key, as ONE cooperative launch: per 8-bit digit, a block
-//   histogram, a grid barrier, per-block digit offsets, a stable scatter
-//   (warp match_any ranks) and another grid barrier. Rows of n <= SMALL are
-//   sorted by block 0 alone in shared memory (bitonic on (key, value), which
-//   is the same order the stable sort gives when the input values ascend).
+//   bits of the key. Up to CSORT_SMALL rows block 0 sorts alone in shared
+//   memory (bitonic on (key, value), which is the same order the stable sort
+//   gives when the input values ascend); up to BSORT_MAX rows, one block with
+//   the rows in registers (k_sort_block); above that, ONE cooperative launch (k_sort_coop):
+//   per 8-bit digit, a block histogram, a grid barrier, per-block digit
+//   offsets, a stable scatter (warp match_any ranks) and another grid barrier.
 // * scan_lookback: exclusive scan of n ints in one launch (decoupled
 //   look-back across tiles claimed in launch order).
 #pragma once
@@ -22,6 +23,7 @@
 #define CSORT_THREADS 1024
 #define CSORT_SMALL 2048
 #define CSORT_MAX_BLOCKS 256
+#define SORT_LARGE_WORLD 4096 // shapes
 #define CSORT_WARPS ( CSORT_THREADS / 32 )
 
 #define LB_THREADS 1024
@@ -33,6 +35,189 @@
 template <typename K> __device__ __forceinline__ bool kv_less( K ka, int va, K kb, int vb )
 {
 	return ka < kb || ( ka == kb && va < vb );
+}
+
+// Optional last step of a sort: made[r] = lookup[key of row r >> shift].
+struct SortDecode
+{
+	int* made;
+	const int* lookup;
+	int shift;
+};
+
+// One block's sort of up to BSORT_MAX rows. Bound by its chain of passes, not
+// by memory (98 KB of keys at most): LSD radix, the rows in registers,
+// BSORT_ITEMS a thread, exchanged through shared memory. A pass costs some 3 us
+// at 12k rows where the cooperative one costs 10 us in grid barriers and L2
+// round trips. The limit is what shared memory holds of 64-bit keys.
+#define BSORT_ITEMS 12
+#define BSORT_MAX ( BSORT_ITEMS * CSORT_THREADS )
+
+struct BSortSmem
+{
+	struct
+	{
+		unsigned long long key[BSORT_MAX];
+		unsigned short row[BSORT_MAX];
+		unsigned hist[CSORT_WARPS][256]; // per-warp digit counts, then first positions
+		unsigned part[4][256];
+		unsigned start[256];
+		int scan[32];
+		unsigned long long any, all;
+	} radix;
+};
+
+template <typename K>
+__global__ void __launch_bounds__( CSORT_THREADS, 1 )
+	k_sort_block( K* keys, int* vals, const int* nPtr, int cap, int bits, const int* enable, SortDecode dec )
+{
+	extern __shared__ __align__( 16 ) unsigned char bsortRaw[];
+	BSortSmem& sm = *reinterpret_cast<BSortSmem*>( bsortRaw );
+	const int tid = threadIdx.x;
+	if ( enable && *enable == 0 )
+		return;
+	const int n = min( *nPtr, cap );
+	if ( n <= CSORT_SMALL || n > BSORT_MAX )
+		return;
+	const int lane = tid & 31, warp = tid >> 5;
+	const int items = ( n + CSORT_THREADS - 1 ) / CSORT_THREADS;
+	const int first = warp * items * 32 + lane; // the thread's rows: first + 32 * item
+	K key[BSORT_ITEMS];
+	unsigned tag[BSORT_ITEMS]; // original row | rank << 16
+	unsigned long long any = 0ull, all = ~0ull;
+#pragma unroll
+	for ( int it = 0; it < BSORT_ITEMS; ++it )
+	{
+		const int r = first + 32 * it;
+		const bool valid = it < items && r < n;
+		key[it] = valid ? keys[r] : (K)0;
+		tag[it] = (unsigned)r;
+		if ( valid )
+		{
+			any |= (unsigned long long)key[it];
+			all &= (unsigned long long)key[it];
+		}
+	}
+	// a digit that every row shares needs no pass
+	if ( tid == 0 )
+	{
+		sm.radix.any = 0ull;
+		sm.radix.all = ~0ull;
+	}
+#pragma unroll
+	for ( int off = 16; off > 0; off >>= 1 )
+	{
+		any |= __shfl_xor_sync( 0xffffffffu, any, off );
+		all &= __shfl_xor_sync( 0xffffffffu, all, off );
+	}
+	__syncthreads();
+	if ( lane == 0 )
+	{
+		atomicOr( &sm.radix.any, any );
+		atomicAnd( &sm.radix.all, all );
+	}
+	__syncthreads();
+	const unsigned long long diff = sm.radix.any ^ sm.radix.all;
+	for ( int shift = 0; shift < bits; shift += 8 )
+	{
+		if ( ( ( diff >> shift ) & 0xffull ) == 0ull )
+			continue;
+		for ( int d = lane; d < 256; d += 32 )
+			sm.radix.hist[warp][d] = 0u;
+		__syncwarp();
+		// ranks within the warp's rows, in row order
+#pragma unroll
+		for ( int it = 0; it < BSORT_ITEMS; ++it )
+		{
+			if ( it >= items )
+				break;
+			const bool valid = first + 32 * it < n;
+			const unsigned d = valid ? (unsigned)( ( key[it] >> shift ) & 0xff ) : 256u;
+			const unsigned peers = __match_any_sync( 0xffffffffu, d );
+			const int leader = __ffs( peers ) - 1;
+			unsigned base = 0u;
+			if ( valid && lane == leader )
+			{
+				base = sm.radix.hist[warp][d];
+				sm.radix.hist[warp][d] = base + __popc( peers );
+			}
+			base = __shfl_sync( 0xffffffffu, base, leader );
+			tag[it] = ( tag[it] & 0xffffu ) | ( ( base + __popc( peers & ( ( 1u << lane ) - 1u ) ) ) << 16 );
+			__syncwarp();
+		}
+		__syncthreads();
+		// first position of every (digit, warp)
+		{
+			const int d = tid & 255, q = tid >> 8;
+			unsigned sum = 0u;
+#pragma unroll
+			for ( int k = 0; k < CSORT_WARPS / 4; ++k )
+				sum += sm.radix.hist[q * ( CSORT_WARPS / 4 ) + k][d];
+			sm.radix.part[q][d] = sum;
+			__syncthreads();
+			unsigned total = 0u;
+			if ( tid < 256 )
+				total = sm.radix.part[0][tid] + sm.radix.part[1][tid] + sm.radix.part[2][tid] + sm.radix.part[3][tid];
+			int dummy;
+			const int begin = block_exclusive_scan_1024( (int)total, sm.radix.scan, &dummy );
+			if ( tid < 256 )
+				sm.radix.start[tid] = (unsigned)begin;
+			__syncthreads();
+			unsigned run = sm.radix.start[d];
+			for ( int k = 0; k < q; ++k )
+				run += sm.radix.part[k][d];
+#pragma unroll
+			for ( int k = 0; k < CSORT_WARPS / 4; ++k )
+			{
+				unsigned* h = &sm.radix.hist[q * ( CSORT_WARPS / 4 ) + k][d];
+				const unsigned v = *h;
+				*h = run;
+				run += v;
+			}
+		}
+		__syncthreads();
+#pragma unroll
+		for ( int it = 0; it < BSORT_ITEMS; ++it )
+			if ( it < items && first + 32 * it < n )
+			{
+				const unsigned dst = sm.radix.hist[warp][(unsigned)( ( key[it] >> shift ) & 0xff )] + ( tag[it] >> 16 );
+				sm.radix.key[dst] = (unsigned long long)key[it];
+				sm.radix.row[dst] = (unsigned short)tag[it];
+			}
+		__syncthreads();
+#pragma unroll
+		for ( int it = 0; it < BSORT_ITEMS; ++it )
+		{
+			const int r = first + 32 * it;
+			if ( it < items && r < n )
+			{
+				key[it] = (K)sm.radix.key[r];
+				tag[it] = sm.radix.row[r];
+			}
+		}
+	}
+	if ( vals )
+	{
+		// the values follow their rows: all read before any is written
+#pragma unroll
+		for ( int it = 0; it < BSORT_ITEMS; ++it )
+			if ( it < items && first + 32 * it < n )
+				tag[it] = (unsigned)__ldcg( vals + ( tag[it] & 0xffffu ) );
+		__syncthreads();
+	}
+#pragma unroll
+	for ( int it = 0; it < BSORT_ITEMS; ++it )
+	{
+		const int r = first + 32 * it;
+		if ( it < items && r < n )
+		{
+			keys[r] = key[it];
+			if ( vals )
+				vals[r] = (int)tag[it];
+			if ( dec.made )
+				dec.made[r] = dec.lookup[key[it] >> dec.shift];
+		}
+	}
 }
 
 // shared memory of k_sort_coop: the bitonic buffers or the radix tables
@@ -55,16 +240,19 @@ union CSortSmem
 
 template <typename K>
 __global__ void __launch_bounds__( CSORT_THREADS )
-	k_sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, const int* nPtr, int cap, int bits, unsigned* hist,
-				 unsigned* counter, int* err, const int* enable )
+	k_sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, int* nPtr, int cap, int bits, unsigned* hist,
+				 unsigned* counter, int* err, const int* enable, int skipUpTo, SortDecode dec )
 {
 	__shared__ CSortSmem sm;
 	const int tid = threadIdx.x;
 	if ( enable && *enable == 0 )
 		return;
 	const int n = min( *nPtr, cap );
-	if ( n <= 1 )
+	if ( n < 1 )
 		return;
+	// the count as it is kept
+	if ( blockIdx.x == 0 && tid == 0 && *nPtr > n )
+		*nPtr = n;
 	if ( n <= CSORT_SMALL )
 	{
 		if ( blockIdx.x != 0 )
@@ -106,9 +294,13 @@ __global__ void __launch_bounds__( CSORT_THREADS )
 			keys[i] = (K)sm.small.key[i];
 			if ( vals )
 				vals[i] = sm.small.val[i];
+			if ( dec.made )
+				dec.made[i] = dec.lookup[keys[i] >> dec.shift];
 		}
 		return;
 	}
+	if ( n <= skipUpTo )
+		return;
 
 	unsigned epoch = 0;
 	const int G = gridDim.x;
@@ -293,23 +485,36 @@ __global__ void __launch_bounds__( CSORT_THREADS )
 				vals[i] = __ldcg( vin + i );
 		}
 	}
+	if ( dec.made )
+		for ( int i = lo + tid; i < hi; i += CSORT_THREADS )
+			dec.made[i] = dec.lookup[__ldcg( kin + i ) >> dec.shift];
 }
 
 // Sorts (keys, vals) by the low `bits` bits of the keys; vals may be null.
-// n from device memory. hist needs 256 * CSORT_MAX_BLOCKS unsigned; counter
+// n from device memory, at most cap rows are sorted. `large`: a world whose
+// sorts commonly pass CSORT_SMALL rows (SORT_LARGE_WORLD) launches the
+// one-block sort ahead of the cooperative one; in a smaller world that launch
+// would be 2.3 us of nothing in every step. hist needs 256 * CSORT_MAX_BLOCKS unsigned; counter
 // is a device word used by the grid barrier (zero before the launch, one
 // launch per step and word). When enable is
 // non-null the sort runs only if *enable != 0.
 template <typename K>
-static inline void sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, const int* nPtr, int cap, int bits,
+static inline void sort_coop( K* keys, int* vals, K* keysAlt, int* valsAlt, int* nPtr, int cap, int bits,
 							  unsigned* hist, unsigned* counter, int* err, int blocks, cudaStream_t st,
-							  const int* enable = nullptr )
+							  const int* enable, bool large, SortDecode dec = { nullptr, nullptr, 0 } )
 {
 	if ( blocks > CSORT_MAX_BLOCKS )
 		blocks = CSORT_MAX_BLOCKS;
 	if ( vals == nullptr )
 		valsAlt = nullptr;
-	void* args[] = { &keys, &vals, &keysAlt, &valsAlt, &nPtr, &cap, &bits, &hist, &counter, &err, &enable };
+	int skipUpTo = 0;
+	if ( large )
+	{
+		cudaFuncSetAttribute( k_sort_block<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof( BSortSmem ) );
+		k_sort_block<K><<<1, CSORT_THREADS, sizeof( BSortSmem ), st>>>( keys, vals, nPtr, cap, bits, enable, dec );
+		skipUpTo = BSORT_MAX;
+	}
+	void* args[] = { &keys, &vals, &keysAlt, &valsAlt, &nPtr, &cap, &bits, &hist, &counter, &err, &enable, &skipUpTo, &dec };
 	cudaLaunchCooperativeKernel( (void*)k_sort_coop<K>, dim3( blocks ), dim3( CSORT_THREADS ), args, 0, st );
 }
 

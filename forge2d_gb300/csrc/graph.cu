@@ -55,8 +55,15 @@ __global__ void k_op_lock( DWorld w )
 	}
 }
 
-// Add to the lowest colour free on both bodies (constraint_graph.c:68-140;
-// no static contacts in colour 0), or clear the removed colour's bits
+// The lowest colour free on both bodies (constraint_graph.c:68-140; no static
+// contacts in colour 0), F2D_OVERFLOW when none is.
+__device__ __forceinline__ int free_color( unsigned ma, unsigned mb, bool both )
+{
+	const unsigned lowest = ~( ma | mb ) & ( ( 1u << F2D_OVERFLOW ) - 1u ) & ( both ? ~0u : ~1u );
+	return lowest ? __ffs( lowest ) - 1 : F2D_OVERFLOW;
+}
+
+// Add to a free colour, or clear the removed colour's bits
 // (constraint_graph.c:184-212).
 __device__ __forceinline__ void apply_op( const DWorld& w, int k, int g, int a, int b )
 {
@@ -64,34 +71,13 @@ __device__ __forceinline__ void apply_op( const DWorld& w, int k, int g, int a, 
 	{
 		unsigned ma = a >= 0 ? __ldcg( w.colorMask + a ) : 0u;
 		unsigned mb = b >= 0 ? __ldcg( w.colorMask + b ) : 0u;
-		int color = F2D_OVERFLOW;
-		if ( a >= 0 && b >= 0 )
+		int color = free_color( ma, mb, a >= 0 && b >= 0 );
+		if ( color != F2D_OVERFLOW )
 		{
-			unsigned used = ma | mb;
-			for ( int i = 0; i < F2D_OVERFLOW; ++i )
-				if ( ( used & ( 1u << i ) ) == 0 )
-				{
-					color = i;
-					break;
-				}
-			if ( color != F2D_OVERFLOW )
-			{
+			if ( a >= 0 )
 				w.colorMask[a] = ma | ( 1u << color );
+			if ( b >= 0 )
 				w.colorMask[b] = mb | ( 1u << color );
-			}
-		}
-		else
-		{
-			int d = a >= 0 ? a : b;
-			unsigned md = a >= 0 ? ma : mb;
-			for ( int i = 1; i < F2D_OVERFLOW; ++i )
-				if ( ( md & ( 1u << i ) ) == 0 )
-				{
-					color = i;
-					break;
-				}
-			if ( color != F2D_OVERFLOW )
-				w.colorMask[d] = md | ( 1u << color );
 		}
 		w.opColor[k] = color;
 	}
@@ -140,14 +126,48 @@ __global__ void k_op_round( DWorld w, const int* gkind, int* list )
 	}
 }
 
-// Remaining rounds in one block over the pending list, compacted in place
-// after every round.
+// Remaining rounds, one block. Bound by the chain of rounds (21 at 100k bodies,
+// some 1500 ops in the first), each a lock, a test and a barrier: through L2 a
+// round took 2.9 us, so once the pending ops fit, their bodies' locks and colour
+// masks move into a hash table in shared memory (60 -> 13 us at 100k bodies).
+// There an op that applies frees its bodies' locks; an op that does not stays
+// the lowest on the body it holds, so a round needs no reset pass.
+#define CR_OPS 3072	  // twice as many bodies at most: 0.75 of the table
+#define CR_TABLE 8192
+struct CrSmem
+{
+	int body[CR_TABLE];
+	int lock[CR_TABLE];
+	unsigned mask[CR_TABLE];
+	int op[CR_OPS];
+	unsigned slots[CR_OPS]; // table slots of the op's bodies, 0xffff none
+	int color[CR_OPS];		// in: colour of a removal, CR_ADD of an add; out: opColor
+	unsigned short list[2][CR_OPS];
+	int count[3];
+};
+#define CR_ADD ( -2 )
+
+// the body's slot (the table is never full)
+__device__ __forceinline__ unsigned cr_slot( CrSmem& sm, int body )
+{
+	unsigned h = ( (unsigned)body * 2654435761u ) >> 19;
+	for ( ;; h = ( h + 1u ) & ( CR_TABLE - 1 ) )
+	{
+		int old = atomicCAS( sm.body + h, -1, body );
+		if ( old == -1 || old == body )
+			return h;
+	}
+}
+
 __global__ void __launch_bounds__( GRAPH_THREADS ) k_color_rounds( DWorld w, const int* gkind, int* list )
 {
+	extern __shared__ __align__( 16 ) unsigned char crRaw[];
+	CrSmem& sm = *reinterpret_cast<CrSmem*>( crRaw );
 	__shared__ int smem[32];
+	const int tid = threadIdx.x;
 	int n = w.sc->pendingOps;
 	int round = 1;
-	for ( ; n > 0 && round < GRAPH_MAX_ROUNDS; ++round )
+	for ( ; n > CR_OPS && round < GRAPH_MAX_ROUNDS; ++round )
 	{
 		for ( int i = threadIdx.x; i < n; i += blockDim.x )
 		{
@@ -193,12 +213,121 @@ __global__ void __launch_bounds__( GRAPH_THREADS ) k_color_rounds( DWorld w, con
 		}
 		n = running;
 	}
+	const int first = round < GRAPH_MAX_ROUNDS ? n : 0;
+	if ( first > 0 )
+	{
+		for ( int i = tid; i < CR_TABLE; i += GRAPH_THREADS )
+		{
+			sm.body[i] = -1;
+			sm.lock[i] = INT_MAX;
+		}
+		if ( tid < 3 )
+			sm.count[tid] = 0;
+		__syncthreads();
+		for ( int i = tid; i < n; i += GRAPH_THREADS )
+		{
+			const int k = list[i];
+			const int2 ab = w.opBodies[k];
+			const int color = gkind[k] == OP_ADD ? CR_ADD : w.opColor[k];
+			unsigned sa = 0xffffu, sb = 0xffffu;
+			if ( ab.x >= 0 )
+			{
+				sa = cr_slot( sm, ab.x );
+				sm.mask[sa] = __ldcg( w.colorMask + ab.x );
+			}
+			if ( ab.y >= 0 )
+			{
+				sb = cr_slot( sm, ab.y );
+				sm.mask[sb] = __ldcg( w.colorMask + ab.y );
+			}
+			sm.op[i] = k;
+			sm.slots[i] = sa | ( sb << 16 );
+			sm.color[i] = color;
+			sm.list[0][i] = (unsigned short)i;
+		}
+		__syncthreads();
+	}
+	for ( int at = 0; n > 0 && n <= CR_OPS && round < GRAPH_MAX_ROUNDS; ++round )
+	{
+		// counts rotate: this round's, the next round's, the one being cleared
+		const unsigned short* in = sm.list[at & 1];
+		unsigned short* out = sm.list[( at & 1 ) ^ 1];
+		int* kept = sm.count + at % 3;
+		for ( int j = tid; j < n; j += GRAPH_THREADS )
+		{
+			const int i = in[j];
+			const unsigned sa = sm.slots[i] & 0xffffu, sb = sm.slots[i] >> 16;
+			if ( sa != 0xffffu )
+				atomicMin( sm.lock + sa, sm.op[i] );
+			if ( sb != 0xffffu )
+				atomicMin( sm.lock + sb, sm.op[i] );
+		}
+		if ( tid == 0 )
+			sm.count[( at + 1 ) % 3] = 0;
+		__syncthreads();
+		for ( int j = tid; j < n; j += GRAPH_THREADS )
+		{
+			const int i = in[j], k = sm.op[i];
+			const unsigned sa = sm.slots[i] & 0xffffu, sb = sm.slots[i] >> 16;
+			const bool own = ( sa == 0xffffu || *(volatile int*)( sm.lock + sa ) == k ) &&
+							 ( sb == 0xffffu || *(volatile int*)( sm.lock + sb ) == k );
+			if ( !own )
+			{
+				out[atomicAdd( kept, 1 )] = (unsigned short)i;
+				continue;
+			}
+			const unsigned ma = sa != 0xffffu ? sm.mask[sa] : 0u, mb = sb != 0xffffu ? sm.mask[sb] : 0u;
+			unsigned na = ma, nb = mb;
+			if ( sm.color[i] == CR_ADD )
+			{
+				const int color = free_color( ma, mb, sa != 0xffffu && sb != 0xffffu );
+				if ( color != F2D_OVERFLOW )
+				{
+					na |= 1u << color;
+					nb |= 1u << color;
+				}
+				sm.color[i] = color;
+			}
+			else if ( sm.color[i] >= 0 && sm.color[i] != F2D_OVERFLOW )
+			{
+				na &= ~( 1u << sm.color[i] );
+				nb &= ~( 1u << sm.color[i] );
+			}
+			if ( sa != 0xffffu )
+			{
+				sm.mask[sa] = na;
+				*(volatile int*)( sm.lock + sa ) = INT_MAX;
+			}
+			if ( sb != 0xffffu )
+			{
+				sm.mask[sb] = nb;
+				*(volatile int*)( sm.lock + sb ) = INT_MAX;
+			}
+		}
+		__syncthreads();
+		n = *kept;
+		at += 1;
+	}
+	if ( first > 0 )
+	{
+		for ( int i = tid; i < first; i += GRAPH_THREADS )
+			w.opColor[sm.op[i]] = sm.color[i];
+		for ( int i = tid; i < CR_TABLE; i += GRAPH_THREADS )
+			if ( sm.body[i] >= 0 )
+				w.colorMask[sm.body[i]] = sm.mask[i];
+	}
 	if ( threadIdx.x == 0 )
 	{
 		w.sc->colorRounds = round;
 		if ( round >= GRAPH_MAX_ROUNDS )
 			atomicOr( &w.sc->error, ERR_COLOR_ROUNDS );
 	}
+}
+
+bool color_rounds_setup()
+{
+	return cudaFuncSetAttribute( k_color_rounds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof( CrSmem ) ) ==
+		   cudaSuccess;
 }
 
 // One look-back chain of k_op_outputs: publish this tile's aggregate, sum
@@ -555,7 +684,7 @@ void launch_graph( DWorld& w, StepScratch& s, cudaStream_t st )
 		launch_isl_ops( w, s, st, gkind );
 	k_op_lock<<<g, 256, 0, st>>>( w );
 	k_op_round<<<g, 256, 0, st>>>( w, gkind, list );
-	k_color_rounds<<<1, GRAPH_THREADS, 0, st>>>( w, gkind, list );
+	k_color_rounds<<<1, GRAPH_THREADS, sizeof( CrSmem ), st>>>( w, gkind, list );
 	k_op_outputs<<<( w.opCap + OPS_TILE - 1 ) / OPS_TILE, OPS_TILE, 0, st>>>( w, gkind, ovOps, 0 );
 	k_overflow_ops<<<1, GRAPH_THREADS, 0, st>>>( w, gkind, ovOps );
 }

@@ -1948,7 +1948,7 @@ void launch_isl_new_contacts( DWorld& w, StepScratch& s, cudaStream_t st, int pl
 	unsigned long long* k0 = w.islNcKeys;
 	unsigned long long* k1 = w.islNcKeysAlt;
 	sort_coop<unsigned long long>( k0, nullptr, k1, nullptr, count, INT_MAX, 32 + bodyBits, w.sortHist, w.sc->sortBarrier + SORT_EDGES,
-								   &w.sc->error, s.sortBlocks64, st );
+								   &w.sc->error, s.sortBlocks64, st, nullptr, w.shapeCap > SORT_LARGE_WORLD );
 	int g2 = grid_for( 2 * w.pairCap );
 	k_isl_nc_chain<<<g2, 256, 0, st>>>( I );
 	k_isl_nc_heads<<<g2, 256, 0, st>>>( I );
@@ -2270,7 +2270,7 @@ void launch_isl_ops( DWorld& w, StepScratch& s, cudaStream_t st, const int* gkin
 		islandBits += 1;
 	sort_coop<unsigned long long>( w.islNcKeys, nullptr, w.islNcKeysAlt, nullptr,
 								   (int*)( (char*)w.isl + offsetof( DIslands, linkCount ) ), INT_MAX, 32 + islandBits, w.sortHist,
-								   w.sc->sortBarrier + SORT_LINKS, &w.sc->error, s.sortBlocks64, st );
+								   w.sc->sortBarrier + SORT_LINKS, &w.sc->error, s.sortBlocks64, st, nullptr, w.shapeCap > SORT_LARGE_WORLD );
 	k_isl_link_chain<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_link_heads<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_merge_roots<<<grid_for( w.bodyCap ), 256, 0, st>>>( w, w.isl );

@@ -245,21 +245,6 @@ __global__ void k_pt_host_done( DWorld w, const int* flag, const int* pos )
 }
 
 // ---------------------------------------------------------------------------
-// new-pair keys -> the creating proxy's shape (the other shape is the
-// sorted value)
-// ---------------------------------------------------------------------------
-__global__ void k_pt_decode( DWorld w )
-{
-	int n = min( w.sc->newPairCount, w.pairCap );
-	// what follows reads the count as it is kept
-	if ( blockIdx.x == 0 && threadIdx.x == 0 && w.sc->newPairCount > n )
-		w.sc->newPairCount = n;
-	int rb = w.pairKeyBits;
-	for ( int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x )
-		w.pairValAlt[r] = w.moveShape[(int)( w.pairKeys[r] >> ( rb + 2 ) )];
-}
-
-// ---------------------------------------------------------------------------
 // partial rebuild
 // ---------------------------------------------------------------------------
 __global__ void k_pt_mark( DWorld w, int t )
@@ -1201,11 +1186,6 @@ void launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st )
 	scan_lookback( s.tmpA, s.tmpB, &w.sc->hostMoveCount, 0, w.shapeCap, nullptr, s.scanState, &w.sc->error, st );
 	k_pt_host_write<<<grid_for( w.shapeCap ), 256, 0, st>>>( w, s.tmpA, s.tmpB );
 	k_pt_host_done<<<1, 1, 0, st>>>( w, s.tmpA, s.tmpB );
-}
-
-void launch_pt_decode( DWorld& w, cudaStream_t st )
-{
-	k_pt_decode<<<grid_for( w.pairCap ), 256, 0, st>>>( w );
 }
 
 static bool pt_present( const DWorld& w, int t )

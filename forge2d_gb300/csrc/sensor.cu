@@ -201,6 +201,6 @@ void launch_sensors( DWorld& w, StepScratch& s, cudaStream_t st )
 		bits += 1;
 	// keys are unique, so their order alone fixes the result
 	sort_coop<unsigned long long>( w.sensorKeys, nullptr, w.sensorKeysAlt, nullptr, &w.sc->sensorCur, INT_MAX, bits,
-								   w.sortHist, w.sc->sortBarrier + SORT_SENSORS, &w.sc->error, s.sortBlocks64, st );
+								   w.sortHist, w.sc->sortBarrier + SORT_SENSORS, &w.sc->error, s.sortBlocks64, st, nullptr, w.shapeCap > SORT_LARGE_WORLD );
 	k_sensor_events<<<1, SENSOR_THREADS, 0, st>>>( w );
 }

@@ -285,6 +285,7 @@ static void alloc_scratch( HostWorld* W )
 	s.solverBlocks2 = solver_max_blocks( 2 );
 	s.smallParts = W->smallParts;
 	s.ptBlocks = pt_large_blocks();
+	color_rounds_setup();
 }
 
 static void grow_bodies( HostWorld* W, int cap )
