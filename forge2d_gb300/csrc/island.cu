@@ -1144,7 +1144,9 @@ __global__ void k_isl_merge_apply( DIslands* Ip )
 //
 // Bound: the traversal's chain, a row read (L1), a mark read and a vote per
 // body. One island of 6e4 bodies and 1.4e5 contacts: 300 ms on one thread,
-// 12 ms here (410 cycles a body).
+// 8 ms here (230 cycles a body: a pop is a chain of a row from the L1, its
+// neighbours' marks, a vote and a shuffle; a branch in it costs 50 to 100
+// cycles, and with five of them a split took 12 ms).
 // ---------------------------------------------------------------------------
 #define SPLIT_THREADS 512
 #define SPLIT_ROW 8			   // int2 per edge row: (edges, body), then up to 7 edges
@@ -1155,14 +1157,15 @@ __global__ void k_isl_merge_apply( DIslands* Ip )
 #define SPLIT_JOINT 0x40000000 // edge key: joint id | this, else contact id
 #define SPLIT_OUTSIDE ( -1 )   // the other body is never pushed (static)
 #define SPLIT_AHEAD 256		   // push rows read ahead around the current body (half as many on either side)
-#define SPLIT_AHEAD_WARPS 8
+#define SPLIT_AHEAD_WARPS 4
 
 struct SplitSmem
 {
 	int stack[SPLIT_STACK];
 	unsigned char marks[SPLIT_BYTES];
 	int scan[32];
-	volatile int at; // the traversal's current row, -1 when it is done
+	int spare; // takes the stores of lanes that push nothing
+	volatile int at; // the traversal's next row, -1 when it is done
 };
 
 // The edges of body b a visit can use: touching contacts not marked before,
@@ -1294,7 +1297,7 @@ template <bool SHARED> struct SplitMarks
 // The pop order of the base island's bodies (as row indices) and, per new
 // island, its id and first pop.
 template <bool SHARED>
-__device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n, SplitMarks<SHARED> marks, SplitSmem& sm )
+__device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n, int noRow, SplitMarks<SHARED> marks, SplitSmem& sm )
 {
 	const unsigned full = 0xffffffffu;
 	const int lane = threadIdx.x & 31;
@@ -1309,9 +1312,11 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 	const int* const pushPool = I.splitPushPool;
 	const int* const seeds = I.seeds;
 	const int none = lane < SPLIT_PUSH ? 0 : -1;
+	const int* const links = I.splitPush + SPLIT_PUSH - 1; // of long rows
 	int popped = 0, islands = 0;
 	int lo = 0; // entries below lo are in global memory
-	const unsigned stack = (unsigned)__cvta_generic_to_shared( sm.stack ), ahead = (unsigned)__cvta_generic_to_shared( (int*)&sm.at );
+	const unsigned stack = (unsigned)__cvta_generic_to_shared( sm.stack ), ahead = (unsigned)__cvta_generic_to_shared( (int*)&sm.at ),
+				   spare = (unsigned)__cvta_generic_to_shared( &sm.spare );
 	auto make_room = [&]( int sp ) {
 		if ( sp + 32 > lo + SPLIT_STACK )
 		{
@@ -1341,41 +1346,49 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 				marks.set( next );
 			}
 			islands += 1;
-			int sp = 0;
-			int other = rowBase[(size_t)SPLIT_PUSH * next] | none;
+			int sp = 0, popping = next;
+			int other = rowBase[(size_t)SPLIT_PUSH * next];
 			for ( ;; )
 			{
-				// the chain of a pop: its row (read below, by the pop before), its
+				unsigned longRow;
+				const int high = lo + SPLIT_STACK - 32, low = lo > 0 ? lo : -1;
+				// The chain of a pop: its row (read below, by the pop before), its
 				// neighbours' marks, the vote, and the next pop's row; everything
-				// else is done while that row is on its way
-				__syncwarp();
-				int below = lds_s32( stack + 4u * (unsigned)( ( sp - 1 ) & ( SPLIT_STACK - 1 ) ) );
-				const bool push = other >= 0 && !marks.get( other );
-				const unsigned pushes = __ballot_sync( full, push );
-				const unsigned longRow = __ballot_sync( full, other <= -2 );
-				const int top = __shfl_sync( full, other, pushes ? 31 - __clz( pushes ) : 0 );
-				const int cur = other, popping = next;
-				const int spNew = sp + __popc( pushes );
-				next = pushes ? top : below;
-				if ( longRow == 0u && spNew > 0 )
-					other = rowBase[(size_t)SPLIT_PUSH * next] | none;
-				if ( push )
+				// else is done while that row is on its way. Nothing in the loop
+				// branches but its end: empty places mean the row that counts as
+				// marked, marking it or a marked row again changes nothing, lanes
+				// that push nothing store to a spare word. A pop ends the loop when
+				// its row is long, the stack's shared part is full or used up, or
+				// the stack is empty.
+				do
 				{
+					__syncwarp();
+					const int below = lds_s32( stack + 4u * (unsigned)( ( sp - 1 ) & ( SPLIT_STACK - 1 ) ) );
+					other |= none;
+					const int cur = (int)min( (unsigned)other, (unsigned)noRow );
+					const bool push = !marks.get( cur );
+					longRow = __ballot_sync( full, other <= -2 );
+					const unsigned pushes = __ballot_sync( full, push );
+					const int top = __shfl_sync( full, cur, 31 - __clz( pushes ) );
+					popping = next;
+					const unsigned slot = stack + 4u * (unsigned)( ( sp + __popc( pushes & lt ) ) & ( SPLIT_STACK - 1 ) );
+					sp += __popc( pushes );
+					next = pushes ? top : below;
+					next = sp > 0 ? next : popping;
+					other = rowBase[(size_t)SPLIT_PUSH * next];
 					marks.set( cur );
-					sts_s32( stack + 4u * (unsigned)( ( sp + __popc( pushes & lt ) ) & ( SPLIT_STACK - 1 ) ), cur );
-				}
-				if ( lane == 0 )
-				{
+					sts_s32( push ? slot : spare, cur );
 					order[popped] = popping;
-					sts_s32( ahead, popping );
-				}
-				popped += 1;
-				sp = spNew;
+					sts_s32( ahead, next );
+					popped += 1;
+					sp -= 1;
+				} while ( ( sp != low ) & ( sp < high ) & ( longRow == 0u ) );
+				sp += 1;
 				make_room( sp );
 				if ( longRow )
 				{
 					// a long row's further bodies, in order
-					const int pool = -2 - __shfl_sync( full, cur, SPLIT_PUSH - 1 ), count = pushPool[pool];
+					const int pool = -2 - links[(size_t)SPLIT_PUSH * popping], count = pushPool[pool];
 					for ( int k0 = 0; k0 < count; k0 += 32 )
 					{
 						int o = k0 + lane < count ? pushPool[pool + 1 + k0 + lane] : -1;
@@ -1393,7 +1406,7 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 						make_room( sp );
 					}
 					if ( sp > 0 )
-						other = rowBase[(size_t)SPLIT_PUSH * next] | none;
+						other = rowBase[(size_t)SPLIT_PUSH * next];
 				}
 				if ( sp == 0 )
 					break;
@@ -1568,9 +1581,9 @@ __global__ void __launch_bounds__( SPLIT_THREADS ) k_isl_split( DWorld w, DIslan
 		if ( threadIdx.x < 32 )
 		{
 			if ( shared )
-				split_traverse( w, I, baseId, n, SplitMarks<true>{ marks, (unsigned)__cvta_generic_to_shared( sm.marks ) }, sm );
+				split_traverse( w, I, baseId, n, rows, SplitMarks<true>{ marks, (unsigned)__cvta_generic_to_shared( sm.marks ) }, sm );
 			else
-				split_traverse( w, I, baseId, n, SplitMarks<false>{ marks, 0u }, sm );
+				split_traverse( w, I, baseId, n, rows, SplitMarks<false>{ marks, 0u }, sm );
 		}
 		else if ( threadIdx.x < 32 + 32 * SPLIT_AHEAD_WARPS )
 			split_read_ahead( I, rows, sm, threadIdx.x - 32 );
