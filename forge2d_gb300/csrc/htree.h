@@ -11,14 +11,51 @@
 
 #include "dworld.cuh"
 
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+#include <new>
 #include <vector>
+
+// Page-locked arrays from PINNED_BYTES up (a tree of 4096 nodes): a tree is
+// edited on the host between two steps, so its arrays go both ways every time.
+// From pageable memory the 3.4 MB of a 20k-body world's tree took some 450 us
+// each way. Below, and without a device, plain memory.
+#define PINNED_BYTES 65536
+template <typename T> struct PinnedAlloc
+{
+	typedef T value_type;
+	PinnedAlloc() = default;
+	template <typename U> PinnedAlloc( const PinnedAlloc<U>& ) {}
+	T* allocate( size_t n )
+	{
+		void* p = nullptr;
+		if ( n * sizeof( T ) >= PINNED_BYTES && cudaMallocHost( &p, n * sizeof( T ) ) == cudaSuccess )
+			return (T*)p;
+		cudaGetLastError();
+		p = malloc( n * sizeof( T ) );
+		if ( p == nullptr )
+			throw std::bad_alloc();
+		return (T*)p;
+	}
+	void deallocate( T* p, size_t n )
+	{
+		if ( n * sizeof( T ) >= PINNED_BYTES && cudaFreeHost( p ) == cudaSuccess )
+			return;
+		cudaGetLastError();
+		free( p );
+	}
+	template <typename U> bool operator==( const PinnedAlloc<U>& ) const { return true; }
+	template <typename U> bool operator!=( const PinnedAlloc<U>& ) const { return false; }
+};
+template <typename T> using PinnedVector = std::vector<T, PinnedAlloc<T>>;
 
 struct HTree
 {
 	// per node id; a free node's `parent` is the next node of the free list
-	std::vector<int> child1, child2, parent, height, flags, shape, leaves;
-	std::vector<float4> box; // lower.x lower.y upper.x upper.y
-	std::vector<unsigned long long> cat;
+	PinnedVector<int> child1, child2, parent, height, flags, shape, leaves;
+	PinnedVector<float4> box; // lower.x lower.y upper.x upper.y
+	PinnedVector<unsigned long long> cat;
 	int cap = 0, count = 0, freeList = -1, root = -1, proxyCount = 0;
 
 	HTree();

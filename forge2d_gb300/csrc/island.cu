@@ -2694,6 +2694,9 @@ __global__ void k_destroy_body_records( DWorld w, DIslands* Ip, int b )
 		I.bHeadContact[b] = ISL_NULL;
 	}
 	w.bflags[b] = 0;
+	w.headShape[b] = F2D_NULL;
+	w.headJoint[b] = F2D_NULL;
+	w.jointCountB[b] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2955,10 +2958,14 @@ void launch_body_enable( DWorld& w, cudaStream_t st, int body )
 }
 
 // broad_phase.c:70-88 b2UnBufferMove: the proxy leaves the move array by
-// swap-remove
-__global__ void k_unbuffer_move( DWorld w, int s )
+// swap-remove; `then`: what becomes of the shape
+__global__ void k_unbuffer_move( DWorld w, int s, int then )
 {
 	int f = w.sflags[s];
+	if ( then )
+		w.proxyKey[s] = F2D_NULL;
+	if ( then == MOVE_FREED )
+		w.sflags[s] = 0;
 	if ( ( f & SF_MOVED ) == 0 )
 		return;
 	int idx = w.shapeMove[s];
@@ -2970,7 +2977,8 @@ __global__ void k_unbuffer_move( DWorld w, int s )
 		w.shapeMove[m] = idx;
 	}
 	w.sc->moveArrayCount = last;
-	w.sflags[s] = f & ~SF_MOVED;
+	if ( then != MOVE_FREED )
+		w.sflags[s] = f & ~SF_MOVED;
 }
 
 void launch_destroy_contacts_of( DWorld& w, cudaStream_t st, int body, int shape, int other, int wake, int* list )
@@ -2990,7 +2998,7 @@ void launch_destroy_body_records( DWorld& w, cudaStream_t st, int body )
 	k_destroy_body_records<<<1, 1, 0, st>>>( w, w.isl, body );
 }
 
-void launch_unbuffer_move( DWorld& w, cudaStream_t st, int shape )
+void launch_unbuffer_move( DWorld& w, cudaStream_t st, int shape, int then )
 {
-	k_unbuffer_move<<<1, 1, 0, st>>>( w, shape );
+	k_unbuffer_move<<<1, 1, 0, st>>>( w, shape, then );
 }

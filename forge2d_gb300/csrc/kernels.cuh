@@ -1,6 +1,7 @@
 // Shared launch helpers and the per-phase launch entry points of the step.
 #pragma once
 
+#include <mutex>
 #include "dworld.cuh"
 
 #include <cuda_runtime.h>
@@ -86,7 +87,9 @@ void launch_destroy_body_records( DWorld& w, cudaStream_t st, int body );
 void launch_body_set_type( DWorld& w, cudaStream_t st, int body, int type );
 void launch_body_disable( DWorld& w, cudaStream_t st, int body );
 void launch_body_enable( DWorld& w, cudaStream_t st, int body );
-void launch_unbuffer_move( DWorld& w, cudaStream_t st, int shape );
+#define MOVE_NO_PROXY 1 // and the shape has no proxy from now on
+#define MOVE_FREED 2	// and the shape id is free
+void launch_unbuffer_move( DWorld& w, cudaStream_t st, int shape, int then );
 // microseconds per grid barrier on the grid-wide solver's grid (n barriers timed)
 float solver_barrier_probe( StepScratch& s, cudaStream_t st, unsigned* counter, int* err, int n );
 // b2Shape_TestPoint on the device row of one shape; *out (device) = 0 or 1
@@ -108,3 +111,51 @@ void launch_pt_rebuild( DWorld& w, StepScratch& s, cudaStream_t st );
 void launch_pt_moves( DWorld& w, cudaStream_t st );
 void launch_pt_gather( DWorld& w, cudaStream_t st );
 void launch_pt_ranks( DWorld& w, cudaStream_t st, int t );
+
+// rows by value (rows.cu)
+#define ROW_BATCH 8
+#define ROWS_BY_VALUE 32
+struct BodyRow
+{
+	float4 xf, vel, delta, sweep0, massv, damp, force;
+	float2 center, localCenter, gravity;
+	int id, flags, headShape, headJoint, jointCount;
+};
+struct BodyRows
+{
+	BodyRow row[ROW_BATCH];
+	int n;
+};
+struct ShapeRow
+{
+	float4 geom[GEOM_F4], aabb, fat, mat;
+	unsigned long long cat, mask;
+	int id, group, body, sub, flags, proxyKey, next;
+};
+struct ShapeRows
+{
+	ShapeRow row[ROW_BATCH];
+	int n;
+};
+struct FewMoves
+{
+	int shape[32];
+	int n;
+};
+void launch_body_rows( DWorld& w, const BodyRows& rows, cudaStream_t st );
+void launch_shape_rows( DWorld& w, const ShapeRows& rows, cudaStream_t st );
+void launch_few_moves( DWorld& w, const FewMoves& moves, cudaStream_t st );
+
+// A world's workspace for ray and box queries: allocated once, guarded for
+// calls from several threads, freed with the world.
+#define QUERY_HOST_IDS 2048 // ids that reach the host without a copy of their own
+struct QueryScratch
+{
+	std::mutex lock;
+	unsigned long long* best = nullptr; // closest ray: fraction bits << 32 | shape; ~0 between calls
+	int* count = nullptr;				// blocks done, hits; 0 between calls
+	int* ids = nullptr;					// device: every hit of a box query
+	int idCap = 0;
+	float* ray = nullptr;	 // pinned, written by the kernel
+	int* found = nullptr;	 // pinned: hits, then up to QUERY_HOST_IDS ids
+};

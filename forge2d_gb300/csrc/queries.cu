@@ -340,8 +340,12 @@ __device__ __forceinline__ float ray_box_enter( fbox b, fv2 o, fv2 t )
 	return tmin;
 }
 
+// One launch: the last block to finish evaluates the winner again and writes
+// the answer where the host reads it; the workspace is then as it was found.
+__device__ void ray_result( const DWorld& w, fv2 origin, fv2 translation, unsigned long long key, float* out );
+
 __global__ void k_ray_closest( DWorld w, fv2 origin, fv2 translation, unsigned long long cat, unsigned long long msk,
-							   unsigned long long* best )
+							   unsigned long long* best, int* done, float* out )
 {
 	for ( int s = blockIdx.x * blockDim.x + threadIdx.x; s < w.shapeCount; s += gridDim.x * blockDim.x )
 	{
@@ -378,11 +382,20 @@ __global__ void k_ray_closest( DWorld w, fv2 origin, fv2 translation, unsigned l
 		unsigned long long key = ( (unsigned long long)__float_as_uint( h.fraction ) << 32 ) | (unsigned)s;
 		atomicMin( best, key );
 	}
+	__syncthreads();
+	if ( threadIdx.x != 0 )
+		return;
+	__threadfence();
+	if ( atomicAdd( done, 1 ) != (int)gridDim.x - 1 )
+		return;
+	__threadfence();
+	ray_result( w, origin, translation, __ldcg( best ), out );
+	*best = ~0ull;
+	*done = 0;
 }
 
-__global__ void k_ray_result( DWorld w, fv2 origin, fv2 translation, const unsigned long long* best, float* out )
+__device__ void ray_result( const DWorld& w, fv2 origin, fv2 translation, unsigned long long key, float* out )
 {
-	unsigned long long key = *best;
 	if ( key == ~0ull )
 	{
 		out[5] = -1.0f;
@@ -419,9 +432,13 @@ __global__ void k_ray_result( DWorld w, fv2 origin, fv2 translation, const unsig
 	out[5] = __int_as_float( s );
 }
 
-__global__ void k_overlap( DWorld w, fbox box, unsigned long long cat, unsigned long long msk, int* out, int* count,
-						   int cap )
+// Every hit to `out`, the first QUERY_HOST_IDS also to the host's list; the
+// last block hands over the count and leaves the counters at zero.
+__global__ void k_overlap( DWorld w, fbox box, unsigned long long cat, unsigned long long msk, int* out, int* counters,
+						   int cap, int* host )
 {
+	int* done = counters;
+	int* count = counters + 1;
 	for ( int s = blockIdx.x * blockDim.x + threadIdx.x; s < w.shapeCount; s += gridDim.x * blockDim.x )
 	{
 		int f = w.sflags[s];
@@ -434,7 +451,18 @@ __global__ void k_overlap( DWorld w, fbox box, unsigned long long cat, unsigned 
 		int k = atomicAdd( count, 1 );
 		if ( k < cap )
 			out[k] = s;
+		if ( k < QUERY_HOST_IDS )
+			host[1 + k] = s;
 	}
+	__syncthreads();
+	if ( threadIdx.x != 0 )
+		return;
+	__threadfence();
+	if ( atomicAdd( done, 1 ) != (int)gridDim.x - 1 )
+		return;
+	host[0] = *(volatile int*)count;
+	*count = 0;
+	*done = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -443,6 +471,8 @@ __global__ void k_overlap( DWorld w, fbox box, unsigned long long cat, unsigned 
 DWorld* f2d_internal_world( int32_t worldId, cudaStream_t* st, int* gens, int genCap );
 uint16_t f2d_internal_shape_gen( int32_t worldId, int shape );
 int32_t f2d_internal_world0( int32_t worldId );
+QueryScratch* f2d_internal_query( int32_t worldId );
+bool f2d_internal_query_ready( QueryScratch* q, int shapes, cudaStream_t st );
 
 extern "C" F2D_API int32_t f2d_world_cast_ray_closest( int32_t worldId, double ox, double oy, double tx, double ty,
 													   int64_t categoryBits, int64_t maskBits, int32_t* shape2,
@@ -452,20 +482,18 @@ extern "C" F2D_API int32_t f2d_world_cast_ray_closest( int32_t worldId, double o
 	DWorld* w = f2d_internal_world( worldId, &st, nullptr, 0 );
 	if ( w == nullptr )
 		return 0;
-	unsigned long long* best = nullptr;
-	float* res = nullptr;
-	cudaMalloc( (void**)&best, sizeof( unsigned long long ) );
-	cudaMalloc( (void**)&res, 6 * sizeof( float ) );
-	cudaMemsetAsync( best, 0xff, sizeof( unsigned long long ), st );
+	// the workspace is the world's (with an allocation, a memset, two launches
+	// and a copy per ray, a ray through 20k shapes took 40 us)
+	QueryScratch* scratch = f2d_internal_query( worldId );
+	std::lock_guard<std::mutex> hold( scratch->lock );
+	if ( !f2d_internal_query_ready( scratch, 0, st ) )
+		return 0;
 	fv2 o = mk( (float)ox, (float)oy ), t = mk( (float)tx, (float)ty );
+	float* h = scratch->ray;
+	h[5] = -1.0f;
 	k_ray_closest<<<grid_for( w->shapeCount ), 256, 0, st>>>( *w, o, t, (unsigned long long)categoryBits,
-															   (unsigned long long)maskBits, best );
-	k_ray_result<<<1, 1, 0, st>>>( *w, o, t, best, res );
-	float h[6];
-	cudaMemcpyAsync( h, res, sizeof( h ), cudaMemcpyDeviceToHost, st );
+															   (unsigned long long)maskBits, scratch->best, scratch->count, h );
 	cudaStreamSynchronize( st );
-	cudaFree( best );
-	cudaFree( res );
 	if ( h[5] == -1.0f )
 		return 0;
 	int s;
@@ -604,24 +632,25 @@ extern "C" F2D_API int32_t f2d_world_overlap_aabb( int32_t worldId, double lx, d
 	if ( w == nullptr )
 		return 0;
 	int cap = w->shapeCount > 0 ? w->shapeCount : 1;
-	int* out = nullptr;
-	int* count = nullptr;
-	cudaMalloc( (void**)&out, sizeof( int ) * cap );
-	cudaMalloc( (void**)&count, sizeof( int ) );
-	cudaMemsetAsync( count, 0, sizeof( int ), st );
+	QueryScratch* scratch = f2d_internal_query( worldId );
+	std::lock_guard<std::mutex> hold( scratch->lock );
+	if ( !f2d_internal_query_ready( scratch, cap, st ) )
+		return 0;
 	fbox box;
 	box.lo = mk( (float)lx, (float)ly );
 	box.hi = mk( (float)ux, (float)uy );
+	scratch->found[0] = 0;
 	k_overlap<<<grid_for( w->shapeCount ), 256, 0, st>>>( *w, box, (unsigned long long)categoryBits,
-														   (unsigned long long)maskBits, out, count, cap );
-	int n = 0;
-	cudaMemcpyAsync( &n, count, sizeof( int ), cudaMemcpyDeviceToHost, st );
+														   (unsigned long long)maskBits, scratch->ids, scratch->count, cap,
+														   scratch->found );
 	cudaStreamSynchronize( st );
-	std::vector<int> ids( std::min( n, cap ) );
-	if ( !ids.empty() )
-		cudaMemcpy( ids.data(), out, sizeof( int ) * ids.size(), cudaMemcpyDeviceToHost );
-	cudaFree( out );
-	cudaFree( count );
+	const int n = scratch->found[0];
+	std::vector<int> ids( scratch->found + 1, scratch->found + 1 + std::min( n, QUERY_HOST_IDS ) );
+	if ( n > QUERY_HOST_IDS )
+	{
+		ids.resize( (size_t)std::min( n, cap ) );
+		cudaMemcpy( ids.data(), scratch->ids, sizeof( int ) * ids.size(), cudaMemcpyDeviceToHost );
+	}
 	std::sort( ids.begin(), ids.end() );
 	int world0 = f2d_internal_world0( worldId );
 	for ( int i = 0; i < (int)ids.size() && i < capacity; ++i )

@@ -45,6 +45,8 @@ struct HostWorld
 	cudaStream_t stream2 = nullptr;
 	cudaEvent_t evFork = nullptr, evJoin = nullptr;
 	int* hostError = nullptr; // pinned
+	int* hostEnd = nullptr;	  // pinned: end events of a destroy call (count, then up to HOST_END pairs)
+	QueryScratch* query = nullptr;
 	int statusAccum = 0;
 	bool stepped = false;
 	float lastStepMs = 0.0f;
@@ -200,6 +202,22 @@ template <typename T> static void dfree( T*& p )
 	if ( p )
 		cudaFree( p );
 	p = nullptr;
+}
+
+#define HOST_END 64
+
+static void query_free( HostWorld* W )
+{
+	QueryScratch* q = W->query;
+	if ( q == nullptr )
+		return;
+	dfree( q->best );
+	dfree( q->count );
+	dfree( q->ids );
+	cudaFreeHost( q->ray );
+	cudaFreeHost( q->found );
+	delete q;
+	W->query = nullptr;
 }
 
 // ---------------------------------------------------------------------------
@@ -685,12 +703,19 @@ static int32_t pack_wg( HostWorld* W, int gen )
 // ---------------------------------------------------------------------------
 // device row sync
 // ---------------------------------------------------------------------------
-template <typename T> static void up( T* dptr, const std::vector<T>& h, int lo, int hi, cudaStream_t st, int stride = 1 )
+template <typename T, typename A> static void up( T* dptr, const std::vector<T, A>& h, int lo, int hi, cudaStream_t st, int stride = 1 )
 {
 	if ( hi <= lo )
 		return;
 	cudaMemcpyAsync( dptr + (size_t)lo * stride, h.data() + (size_t)lo * stride, sizeof( T ) * (size_t)( hi - lo ) * stride,
 					 cudaMemcpyHostToDevice, st );
+}
+
+// whole array of n, without waiting
+template <typename T, typename A> static void down_async( std::vector<T, A>& h, const T* dptr, int n, cudaStream_t st )
+{
+	if ( n > 0 )
+		cudaMemcpyAsync( h.data(), dptr, sizeof( T ) * (size_t)n, cudaMemcpyDeviceToHost, st );
 }
 
 template <typename T> static void down( std::vector<T>& h, const T* dptr, int lo, int hi, int stride = 1 )
@@ -719,6 +744,66 @@ static void upload_body_rows( HostWorld* W, int lo, int hi )
 	up( d.headShape, W->headShape, lo, hi, st );
 	up( d.headJoint, W->headJoint, lo, hi, st );
 	up( d.jointCountB, W->jointCountB, lo, hi, st );
+}
+
+// the rows get(0..n-1) in launches of ROW_BATCH (rows.cu)
+template <typename F> static void send_body_rows( HostWorld* W, int n, F get )
+{
+	for ( int k = 0; k < n; k += ROW_BATCH )
+	{
+		BodyRows rows;
+		rows.n = std::min( ROW_BATCH, n - k );
+		for ( int i = 0; i < rows.n; ++i )
+		{
+			int b = get( k + i );
+			BodyRow& r = rows.row[i];
+			r.id = b;
+			r.xf = W->xf[b];
+			r.vel = W->vel[b];
+			r.delta = W->delta[b];
+			r.center = W->center[b];
+			r.sweep0 = W->sweep0[b];
+			r.localCenter = W->localCenter[b];
+			r.massv = W->massv[b];
+			r.damp = W->damp[b];
+			r.gravity = W->bgrav[b];
+			r.force = W->force[b];
+			r.flags = W->bflags[b];
+			r.headShape = W->headShape[b];
+			r.headJoint = W->headJoint[b];
+			r.jointCount = W->jointCountB[b];
+		}
+		launch_body_rows( W->d, rows, W->stream );
+	}
+}
+
+template <typename F> static void send_shape_rows( HostWorld* W, int n, F get )
+{
+	for ( int k = 0; k < n; k += ROW_BATCH )
+	{
+		ShapeRows rows;
+		rows.n = std::min( ROW_BATCH, n - k );
+		for ( int i = 0; i < rows.n; ++i )
+		{
+			int s = get( k + i );
+			ShapeRow& r = rows.row[i];
+			r.id = s;
+			for ( int j = 0; j < GEOM_F4; ++j )
+				r.geom[j] = W->geom[(size_t)s * GEOM_F4 + j];
+			r.aabb = W->aabb[s];
+			r.fat = W->fat[s];
+			r.mat = W->mat[s];
+			r.cat = W->cat[s];
+			r.mask = W->mask[s];
+			r.group = W->group[s];
+			r.body = W->shapeBody[s];
+			r.sub = W->ssub[s];
+			r.flags = W->sflags[s];
+			r.proxyKey = W->proxyKey[s];
+			r.next = W->nextShape[s];
+		}
+		launch_shape_rows( W->d, rows, W->stream );
+	}
 }
 
 static void upload_shape_rows( HostWorld* W, int lo, int hi )
@@ -977,18 +1062,19 @@ static void tree_pull( HostWorld* W, int t )
 		return;
 	HTree& h = W->trees[t];
 	const DProxyTree& T = W->d.pt[t];
-	cudaStreamSynchronize( W->stream );
-	int n = h.cap;
-	down( h.child1, T.child1, 0, n );
-	down( h.child2, T.child2, 0, n );
-	down( h.parent, T.parent, 0, n );
-	down( h.height, T.height, 0, n );
-	down( h.flags, T.flags, 0, n );
-	down( h.shape, T.shape, 0, n );
-	down( h.leaves, T.leaves, 0, n );
-	down( h.box, T.box, 0, n );
-	down( h.cat, T.cat, 0, n );
-	cudaMemcpy( &h.root, &W->d.sc->treeRoot[t], sizeof( int ), cudaMemcpyDeviceToHost );
+	const int n = h.cap;
+	cudaStream_t st = W->stream;
+	down_async( h.child1, T.child1, n, st );
+	down_async( h.child2, T.child2, n, st );
+	down_async( h.parent, T.parent, n, st );
+	down_async( h.height, T.height, n, st );
+	down_async( h.flags, T.flags, n, st );
+	down_async( h.shape, T.shape, n, st );
+	down_async( h.leaves, T.leaves, n, st );
+	down_async( h.box, T.box, n, st );
+	down_async( h.cat, T.cat, n, st );
+	cudaMemcpyAsync( &h.root, &W->d.sc->treeRoot[t], sizeof( int ), cudaMemcpyDeviceToHost, st );
+	cudaStreamSynchronize( st );
 	W->treeStale[t] = false;
 }
 
@@ -1003,12 +1089,27 @@ static void host_move( HostWorld* W, int s )
 	W->hostMoves.push_back( s );
 }
 
-// the buffered proxies go to the device for the step about to be enqueued
-static void upload_host_moves( HostWorld* W )
+// The buffered proxies go to the device for the step about to be enqueued; a
+// few join the move array here and now. True when the step's host-move chain
+// has them to place.
+static bool upload_host_moves( HostWorld* W )
 {
 	int n = (int)W->hostMoves.size();
 	if ( n == 0 )
-		return;
+		return false;
+	FewMoves few;
+	if ( n <= 32 )
+	{
+		few.n = n;
+		for ( int k = 0; k < n; ++k )
+		{
+			few.shape[k] = W->hostMoves[k];
+			W->hostMoved[W->hostMoves[k]] = 0;
+		}
+		W->hostMoves.clear();
+		launch_few_moves( W->d, few, W->stream );
+		return false;
+	}
 	cudaMemcpyAsync( W->d.hostMoves, W->hostMoves.data(), sizeof( int ) * (size_t)n, cudaMemcpyHostToDevice,
 					 W->stream );
 	W->hostMoveCount = n;
@@ -1017,32 +1118,42 @@ static void upload_host_moves( HostWorld* W )
 	for ( int sh : W->hostMoves )
 		W->hostMoved[sh] = 0;
 	W->hostMoves.clear();
+	return true;
 }
 
-static void flush_uploads( HostWorld* W )
+// `trees`: the broadphase trees too (a step and an explosion read them; a run
+// of destroy calls between two steps sends each edited tree once).
+static void flush_uploads( HostWorld* W, bool trees = true )
 {
 	ensure_capacity( W );
 	if ( W->bodyUploaded < W->bodyCount )
 	{
-		upload_body_rows( W, W->bodyUploaded, W->bodyCount );
+		const int lo = W->bodyUploaded, n = W->bodyCount - lo;
+		if ( n <= ROWS_BY_VALUE )
+			send_body_rows( W, n, [&]( int k ) { return lo + k; } );
+		else
+			upload_body_rows( W, lo, W->bodyCount );
 		W->bodyUploaded = W->bodyCount;
 		W->islBodiesUploaded = true;
 	}
+	send_body_rows( W, (int)W->bodyDirty.size(), [&]( int k ) { return W->bodyDirty[(size_t)k]; } );
 	for ( int b : W->bodyDirty )
 	{
-		upload_body_rows( W, b, b + 1 );
 		W->bodyIsDirty[b] = 0;
 		W->islBodiesUploaded = true;
 	}
 	W->bodyDirty.clear();
 	if ( W->shapeUploaded < W->shapeCount )
 	{
-		upload_shape_rows( W, W->shapeUploaded, W->shapeCount );
+		const int lo = W->shapeUploaded, n = W->shapeCount - lo;
+		if ( n <= ROWS_BY_VALUE )
+			send_shape_rows( W, n, [&]( int k ) { return lo + k; } );
+		else
+			upload_shape_rows( W, lo, W->shapeCount );
 		W->shapeUploaded = W->shapeCount;
 		W->forceRebuild = true;
 	}
-	for ( int s : W->shapeDirty )
-		upload_shape_rows( W, s, s + 1 );
+	send_shape_rows( W, (int)W->shapeDirty.size(), [&]( int k ) { return W->shapeDirty[(size_t)k]; } );
 	if ( !W->shapeDirty.empty() )
 		W->forceRebuild = true;
 	W->shapeDirty.clear();
@@ -1143,7 +1254,7 @@ static void flush_uploads( HostWorld* W )
 		W->pendingJoints.clear();
 		W->graphDirty = true;
 	}
-	for ( int t = 0; t < 3; ++t )
+	for ( int t = 0; t < 3 && trees; ++t )
 		if ( W->treeDirty[t] )
 			tree_upload( W, t );
 	// counts are kernel parameters of the captured step: a change re-captures
@@ -1211,6 +1322,8 @@ extern "C" F2D_API int32_t f2d_create_world( const f2d_world_def* def )
 	}
 	cudaMallocHost( (void**)&W->hostError, sizeof( int ) );
 	*W->hostError = 0;
+	W->query = new QueryScratch;
+	cudaMallocHost( (void**)&W->hostEnd, sizeof( int ) * ( 1 + 2 * HOST_END ) );
 	cudaMalloc( (void**)&d.sc, sizeof( DScalars ) );
 	cudaMemset( d.sc, 0, sizeof( DScalars ) );
 	grow_bodies( W, 1024 );
@@ -1264,6 +1377,9 @@ static void free_world( HostWorld* W )
 	W->packedCap = 0;
 	dfree( W->s.bounds );
 	cudaFreeHost( W->hostError );
+	cudaFreeHost( W->hostEnd );
+	W->hostEnd = nullptr;
+	query_free( W );
 	cudaEventDestroy( W->evStart );
 	cudaEventDestroy( W->evStop );
 	cudaEventDestroy( W->evFork );
@@ -1367,8 +1483,7 @@ extern "C" F2D_API int32_t f2d_create_body( int32_t worldId, const f2d_body_def*
 	if ( !W->bodyFree.empty() )
 	{
 		id = W->bodyFree.back();
-		W->bodyFree.pop_back();
-		pull_body( W, id );
+		W->bodyFree.pop_back(); // (every field is set below, the device's row is not wanted)
 	}
 	else
 		id = W->bodyCount++;
@@ -2288,28 +2403,28 @@ static bool chain_live( const HostWorld* W, int c, int32_t wg )
 // join the move array (after the finalize moves, as b2BufferMove appends)
 static void destroy_begin( HostWorld* W )
 {
-	flush_uploads( W );
-	if ( !W->hostMoves.empty() )
-	{
-		upload_host_moves( W );
+	flush_uploads( W, false );
+	if ( upload_host_moves( W ) )
 		launch_pt_host_moves( W->d, W->s, W->stream );
-	}
-	cudaMemsetAsync( &W->d.sc->apiEndCount, 0, sizeof( int ), W->stream );
-	cudaMemsetAsync( &W->d.sc->apiCount, 0, sizeof( int ), W->stream );
+	cudaMemsetAsync( &W->d.sc->apiCount, 0, 2 * sizeof( int ), W->stream ); // and apiEndCount
 }
 
 // end events of the contacts destroyed since destroy_begin, with the shape
 // ids as they are now, for the next step's events
 static void destroy_end( HostWorld* W )
 {
+	W->hostEnd[0] = 0;
+	cudaMemcpyAsync( W->hostEnd, &W->d.sc->apiEndCount, sizeof( int ), cudaMemcpyDeviceToHost, W->stream );
+	cudaMemcpyAsync( W->hostEnd + 1, W->d.apiEndEv, sizeof( int ) * 2 * (size_t)std::min( HOST_END, W->d.contactCap ),
+					 cudaMemcpyDeviceToHost, W->stream );
 	cudaStreamSynchronize( W->stream );
-	int n = 0;
-	cudaMemcpy( &n, &W->d.sc->apiEndCount, sizeof( int ), cudaMemcpyDeviceToHost );
-	n = std::min( n, W->d.contactCap );
+	int n = std::min( W->hostEnd[0], W->d.contactCap );
 	if ( n > 0 )
 	{
-		std::vector<int> ev( 2 * (size_t)n );
-		cudaMemcpy( ev.data(), W->d.apiEndEv, sizeof( int ) * 2 * (size_t)n, cudaMemcpyDeviceToHost );
+		std::vector<int> ev( W->hostEnd + 1, W->hostEnd + 1 + 2 * std::min( n, HOST_END ) );
+		ev.resize( 2 * (size_t)n );
+		if ( n > HOST_END )
+			cudaMemcpy( ev.data(), W->d.apiEndEv, sizeof( int ) * 2 * (size_t)n, cudaMemcpyDeviceToHost );
 		for ( int i = 0; i < n; ++i )
 		{
 			int a = ev[2 * i], b = ev[2 * i + 1];
@@ -2362,12 +2477,12 @@ static void destroy_joint_host( HostWorld* W, int j, int wake )
 }
 
 // broad_phase.c:105-114: out of the move array, then out of its tree
-static void destroy_proxy_host( HostWorld* W, int s )
+static void destroy_proxy_host( HostWorld* W, int s, bool freed = false )
 {
 	int pk = W->proxyKey[s];
 	if ( pk == F2D_NULL )
 		return;
-	launch_unbuffer_move( W->d, W->stream, s );
+	launch_unbuffer_move( W->d, W->stream, s, freed ? MOVE_FREED : MOVE_NO_PROXY );
 	int t = pk & 3;
 	tree_pull( W, t );
 	W->trees[t].destroy_proxy( pk >> 2 );
@@ -2375,7 +2490,6 @@ static void destroy_proxy_host( HostWorld* W, int s )
 	if ( t == 0 )
 		W->staticDirty = true;
 	W->proxyKey[s] = F2D_NULL;
-	up( W->d.proxyKey, W->proxyKey, s, s + 1, W->stream );
 }
 
 // sensor.c:353-380: an end event per current visitor (the last step's
@@ -2494,8 +2608,14 @@ static void destroy_body_host( HostWorld* W, int b )
 	{
 		if ( W->sflags[s] & SF_SENSOR )
 			destroy_sensor_host( W, s );
-		destroy_proxy_host( W, s );
-		free_shape_host( W, s );
+		if ( W->proxyKey[s] != F2D_NULL )
+		{
+			destroy_proxy_host( W, s, true );
+			W->sflags[s] = 0;
+			W->shapeFree.push_back( s );
+		}
+		else
+			free_shape_host( W, s );
 	}
 	for ( int c = W->headChain[b]; c != F2D_NULL; c = W->chainNext[c] )
 	{
@@ -2519,9 +2639,6 @@ static void destroy_body_host( HostWorld* W, int b )
 	W->headShape[b] = F2D_NULL;
 	W->headJoint[b] = F2D_NULL;
 	W->jointCountB[b] = 0;
-	up( W->d.headShape, W->headShape, b, b + 1, W->stream );
-	up( W->d.headJoint, W->headJoint, b, b + 1, W->stream );
-	up( W->d.jointCountB, W->jointCountB, b, b + 1, W->stream );
 	W->bodyFree.push_back( b );
 }
 
@@ -3173,7 +3290,7 @@ extern "C" F2D_API void f2d_shape_set_filter( int32_t index1, int32_t wg, int64_
 		tree_pull( W, t );
 		if ( destroyProxy )
 		{
-			launch_unbuffer_move( W->d, W->stream, s );
+			launch_unbuffer_move( W->d, W->stream, s, 0 );
 			W->trees[t].destroy_proxy( pk >> 2 );
 			int proxyId = W->trees[t].create_proxy( W->fat[s], cat, s );
 			W->proxyKey[s] = ( proxyId << 2 ) | t;
@@ -5131,6 +5248,38 @@ DWorld* f2d_internal_world( int32_t worldId, cudaStream_t* st, int* gens, int ge
 	cudaStreamSynchronize( W->stream );
 	*st = W->stream;
 	return &W->d;
+}
+
+// The world's query workspace, its id list as long as the world has shapes
+// (the caller holds the lock), or nullptr.
+QueryScratch* f2d_internal_query( int32_t worldId )
+{
+	HostWorld* W = world_from_id( worldId );
+	return W ? W->query : nullptr;
+}
+
+bool f2d_internal_query_ready( QueryScratch* q, int shapes, cudaStream_t st )
+{
+	if ( q->best == nullptr )
+	{
+		if ( cudaMalloc( (void**)&q->best, sizeof( unsigned long long ) ) != cudaSuccess ||
+			 cudaMalloc( (void**)&q->count, 2 * sizeof( int ) ) != cudaSuccess ||
+			 cudaMallocHost( (void**)&q->ray, 8 * sizeof( float ) ) != cudaSuccess ||
+			 cudaMallocHost( (void**)&q->found, ( 1 + QUERY_HOST_IDS ) * sizeof( int ) ) != cudaSuccess )
+			return false;
+		cudaMemsetAsync( q->best, 0xff, sizeof( unsigned long long ), st );
+		cudaMemsetAsync( q->count, 0, 2 * sizeof( int ), st );
+	}
+	if ( shapes > q->idCap )
+	{
+		dfree( q->ids );
+		q->idCap = 0;
+		int cap = std::max( 1024, 2 * shapes );
+		if ( cudaMalloc( (void**)&q->ids, sizeof( int ) * (size_t)cap ) != cudaSuccess )
+			return false;
+		q->idCap = cap;
+	}
+	return true;
 }
 
 // For the allocation-free queries: the world's device rows after pending
