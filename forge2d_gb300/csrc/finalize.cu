@@ -274,9 +274,20 @@ __device__ __forceinline__ void hit_events( const DWorld& w )
 	}
 }
 
-// solver.c:390-541: one thread per fast body; candidate static shapes are
-// visited in shape-id order
+// solver.c:390-541: candidate static shapes are visited in the static tree's
+// order. A thread per fast body, or (WARP) a warp, whose lanes test the boxes
+// of the static list 128 at a time, coalesced, and take the hits in order.
+//
+// Bound by dependent reads either way. The list of up to CCD_LIST_MAX shapes is
+// scanned by the thread itself: with 3 statics and 100k bodies a warp each
+// would be 20 waves of warps for one box test per lane. Above, a thread has to
+// walk the pair tree down through every moving shape around its body; the
+// warp's scan replaces that up to CCD_WARP_MAX shapes, where a scan costs what
+// a walk does. Whole finalize phase, walk and scan: 6k bodies on a terrain of
+// 200 segments 144 and 43 us, 512 batched worlds (700 statics) 140 and 71 us.
 #define CCD_LIST_MAX 64
+#define CCD_WARP_MAX 1024
+#define CCD_WARP_THREADS 128
 #define CCD_CANDIDATES 32
 
 __device__ __forceinline__ bool ccd_rejected( const DWorld& w, unsigned long long key )
@@ -298,11 +309,13 @@ __device__ __forceinline__ bool ccd_rejected( const DWorld& w, unsigned long lon
 // host and changes nothing; the second pass skips the ones it rejected. The
 // hit events, which need the solver's impulses only, are found by the same
 // launch.
-__global__ void k_continuous( DWorld w, int listOnly )
+template <bool WARP> __global__ void __launch_bounds__( CCD_WARP_THREADS ) k_continuous( DWorld w, int listOnly )
 {
-	int n = w.sc->fastCount;
-	for ( int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x )
+	const int n = w.sc->fastCount;
+	const int lane = threadIdx.x & 31, width = WARP ? 32 : 1;
+	for ( int i = ( blockIdx.x * blockDim.x + threadIdx.x ) / width; i < n; i += gridDim.x * blockDim.x / width )
 	{
+		// (a warp's lanes all follow one body; lane 0 alone writes)
 		int b = w.fastBodies[i];
 		float4 s0 = w.sweep0[b];
 		float2 c2 = w.center[b];
@@ -331,7 +344,9 @@ __global__ void k_continuous( DWorld w, int listOnly )
 			fbox box1 = box_from4( w.aabb[fs] );
 			fbox box2 = shape_aabb( gf, tf, xf2 );
 			fbox box = box_union( box1, box2 );
-			if ( !listOnly )
+			if ( WARP )
+				__syncwarp();
+			if ( !listOnly && ( !WARP || lane == 0 ) )
 				w.aabb[fs] = box_to4( box2 );
 			if ( sff & SF_SENSOR )
 				continue;
@@ -431,6 +446,26 @@ __global__ void k_continuous( DWorld w, int listOnly )
 			// left-to-right rank), as the reference's query meets them: the
 			// static list (kept in that order) when it is short, else the
 			// static leaves of the pair tree overlapping the sweep box
+			if ( WARP )
+			{
+				for ( int base = 0; base < w.staticCount; base += 128 )
+				{
+					int ss[4];
+					float4 fat[4];
+#pragma unroll
+					for ( int j = 0; j < 4; ++j )
+						ss[j] = base + 32 * j + lane < w.staticCount ? w.staticShapes[base + 32 * j + lane] : -1;
+#pragma unroll
+					for ( int j = 0; j < 4; ++j )
+						fat[j] = ss[j] >= 0 ? w.fat[ss[j]] : make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
+#pragma unroll
+					for ( int j = 0; j < 4; ++j )
+						for ( unsigned hits = __ballot_sync( 0xffffffffu, ss[j] >= 0 && box_overlaps( box_from4( fat[j] ), box ) );
+							  hits != 0u; hits &= hits - 1u )
+							consider( __shfl_sync( 0xffffffffu, ss[j], __ffs( hits ) - 1 ) );
+				}
+				continue;
+			}
 			bool scanList = w.staticCount <= CCD_LIST_MAX;
 			int cand[CCD_CANDIDATES];
 			int nc = 0;
@@ -468,7 +503,7 @@ __global__ void k_continuous( DWorld w, int listOnly )
 					consider( cand[k] );
 			}
 		}
-		if ( listOnly )
+		if ( listOnly || ( WARP && lane != 0 ) )
 			continue;
 		if ( fraction < 1.0f )
 		{
@@ -549,10 +584,13 @@ void launch_finalize( DWorld& w, StepScratch& s, cudaStream_t st, float dt, Host
 	if ( ccdHook )
 	{
 		cudaMemsetAsync( &w.sc->cbList, 0, sizeof( int ), st );
-		k_continuous<<<grid_for( w.bodyCount ), 64, 0, st>>>( w, 1 );
+		k_continuous<false><<<grid_for( w.bodyCount ), 64, 0, st>>>( w, 1 );
 		ccdHook( hookContext );
 	}
-	k_continuous<<<grid_for( w.contactCap > w.bodyCount ? w.contactCap : w.bodyCount ), 64, 0, st>>>( w, 0 );
+	if ( w.staticCount > CCD_LIST_MAX && w.staticCount <= CCD_WARP_MAX )
+		k_continuous<true><<<F2D_SMS * 8, CCD_WARP_THREADS, 0, st>>>( w, 0 );
+	else
+		k_continuous<false><<<grid_for( w.contactCap > w.bodyCount ? w.contactCap : w.bodyCount ), 64, 0, st>>>( w, 0 );
 	// solver.c:1842-1905: enlarged proxies enter the move array of the next
 	// step in awake order and grow their tree leaves
 	launch_pt_moves( w, st );
