@@ -613,6 +613,23 @@ __global__ void k_after_create( DWorld w, int planMode )
 // ---------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------
+// The leaves' spatial order, every few steps and after edits
+// (k_reset_step_counters says when; otherwise every launch here returns).
+static void launch_leaf_order( DWorld& w, StepScratch& s, cudaStream_t st )
+{
+	int gridS = grid_for( w.shapeCount );
+	k_leaf_flags<<<gridS, BP_THREADS, 0, st>>>( w, s.tmpA );
+	scan_lookback( s.tmpA, s.tmpB, nullptr, w.shapeCount, w.shapeCap, &w.sc->treeLeafCount, s.scanState, &w.sc->error,
+				   st, &w.sc->rebuildOrder );
+	k_leaf_compact<<<gridS, BP_THREADS, 0, st>>>( w, s.tmpA, s.tmpB );
+	k_bounds_partial<<<s.boundsBlocks, BP_THREADS, 0, st>>>( w, s.bounds );
+	k_bounds_final<<<1, BP_THREADS, 0, st>>>( &w.sc->rebuildOrder, s.bounds, s.boundsBlocks );
+	k_morton<<<gridS, BP_THREADS, 0, st>>>( w, s.bounds );
+	sort_coop<unsigned>( w.mortonKeys, w.leafShape, w.mortonKeysAlt, w.leafShapeAlt, &w.sc->treeLeafCount, w.shapeCap, 30,
+						 w.sortHist, w.sc->sortBarrier + SORT_MORTON, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder,
+						 w.shapeCap > SORT_LARGE_WORLD );
+}
+
 void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode, HostHook pairHook,
 						void* hookContext )
 {
@@ -633,9 +650,8 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 		cudaStreamWaitEvent( rs, s.rebuildFork, 0 );
 		launch_pt_gather( w, rs );
 	}
-	launch_pt_host_moves( w, s, st );
-	// the pair hash of the live contacts is built beside the leaf ordering,
-	// which does not touch it; both meet before the refit
+	// the pair hash of the live contacts is built beside the leaf ordering and
+	// the refit, which do not touch it; both meet before the pair search
 	cudaStream_t hs = s.side[0] ? s.side[0] : st;
 	if ( hs != st )
 	{
@@ -646,18 +662,8 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 	k_hash_insert<<<grid_for( w.contactCap ), BP_THREADS, 0, hs>>>( w );
 	if ( hs != st )
 		cudaEventRecord( s.sideJoin[0], hs );
-	k_leaf_flags<<<gridS, BP_THREADS, 0, st>>>( w, s.tmpA );
-	scan_lookback( s.tmpA, s.tmpB, nullptr, w.shapeCount, w.shapeCap, &w.sc->treeLeafCount, s.scanState, &w.sc->error,
-				   st, &w.sc->rebuildOrder );
-	k_leaf_compact<<<gridS, BP_THREADS, 0, st>>>( w, s.tmpA, s.tmpB );
-	k_bounds_partial<<<s.boundsBlocks, BP_THREADS, 0, st>>>( w, s.bounds );
-	k_bounds_final<<<1, BP_THREADS, 0, st>>>( &w.sc->rebuildOrder, s.bounds, s.boundsBlocks );
-	k_morton<<<gridS, BP_THREADS, 0, st>>>( w, s.bounds );
-	sort_coop<unsigned>( w.mortonKeys, w.leafShape, w.mortonKeysAlt, w.leafShapeAlt, &w.sc->treeLeafCount, w.shapeCap, 30,
-						 w.sortHist, w.sc->sortBarrier + SORT_MORTON, &w.sc->error, s.sortBlocks32, st, &w.sc->rebuildOrder,
-						 w.shapeCap > SORT_LARGE_WORLD );
-	if ( hs != st )
-		cudaStreamWaitEvent( st, s.sideJoin[0], 0 );
+	if ( !s.lean )
+		launch_leaf_order( w, s, st );
 	// the solver's body order follows the leaf order, beside the pair search
 	if ( s.side[3] )
 	{
@@ -666,6 +672,8 @@ void launch_broadphase( DWorld& w, StepScratch& s, cudaStream_t st, int planMode
 	}
 	launch_solver_order( w, s, s.side[3] ? s.side[3] : st );
 	k_wide_refit<<<( ( w.shapeCap + WIDE - 1 ) / WIDE + 7 ) / 8, BP_THREADS, 0, st>>>( w );
+	if ( hs != st )
+		cudaStreamWaitEvent( st, s.sideJoin[0], 0 );
 	k_find_pairs<<<( w.shapeCap + FIND_WARPS - 1 ) / FIND_WARPS, BP_THREADS, 0, st>>>( w );
 	// keys are unique (one per pair), so the key order alone fixes the result;
 	// a key's top bits are the creating shape's place in the move array

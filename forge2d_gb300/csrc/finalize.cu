@@ -550,7 +550,7 @@ template <bool WARP> __global__ void __launch_bounds__( CCD_WARP_THREADS ) k_con
 }
 
 // Counters, grid-barrier words and look-back states of the step.
-__global__ void k_reset_step_counters( DWorld w )
+__global__ void k_reset_step_counters( DWorld w, int lean )
 {
 	for ( int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.lookbackWords; i += gridDim.x * blockDim.x )
 		w.opScan[i] = 0ull;
@@ -569,7 +569,7 @@ __global__ void k_reset_step_counters( DWorld w )
 		w.sc->npCount[k] = 0;
 	int age = w.sc->orderAge;
 	int period = w.sc->orderPeriod > 0 ? w.sc->orderPeriod : ORDER_REBUILD_PERIOD;
-	int rebuild = ( w.sc->forceRebuild != 0 || age >= period - 1 ) ? 1 : 0;
+	int rebuild = ( lean == 0 && ( w.sc->forceRebuild != 0 || age >= period - 1 ) ) ? 1 : 0;
 	w.sc->rebuildOrder = rebuild;
 	w.sc->orderAge = rebuild ? 0 : age + 1;
 	w.sc->forceRebuild = 0;
@@ -598,8 +598,8 @@ void launch_finalize( DWorld& w, StepScratch& s, cudaStream_t st, float dt, Host
 		launch_isl_sleep( w, st, s.scanState );
 }
 
-void launch_reset_counters( DWorld& w, cudaStream_t st )
+void launch_reset_counters( DWorld& w, cudaStream_t st, bool lean )
 {
 	int blocks = ( w.lookbackWords + 1023 ) / 1024;
-	k_reset_step_counters<<<blocks < 8 ? blocks : 8, 1024, 0, st>>>( w );
+	k_reset_step_counters<<<blocks < 8 ? blocks : 8, 1024, 0, st>>>( w, lean ? 1 : 0 );
 }

@@ -24,6 +24,7 @@ static inline int grid_for( int cap )
 // Step scratch owned by the host world; device pointers only.
 struct StepScratch
 {
+	bool lean;	  // the step being enqueued sorts no leaves
 	int* tmpA;	  // >= max(shapeCap, contactCap, bodyCap) ints
 	int* tmpB;
 	int* scanTmp; // scan tile sums

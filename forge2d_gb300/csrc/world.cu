@@ -27,7 +27,7 @@
 #include <string>
 #include <vector>
 
-void launch_reset_counters( DWorld& w, cudaStream_t st );
+void launch_reset_counters( DWorld& w, cudaStream_t st, bool lean );
 
 
 #define MAX_WORLDS 128
@@ -58,6 +58,11 @@ struct HostWorld
 
 	// graph replay
 	cudaGraphExec_t graphExec = nullptr;
+	// the same step without the leaf ordering, for the steps that do not sort
+	cudaGraphExec_t leanExec = nullptr;
+	int leanKernelNodes = 0;
+	int graphSteps = 0; // steps since the graph was captured
+	int orderAge = 0;	// steps since the leaves were sorted (as the device counts them)
 	float graphDt = 0.0f;
 	int graphSubSteps = 0;
 	int graphKernelNodes = 0;
@@ -1339,6 +1344,8 @@ extern "C" F2D_API int32_t f2d_create_world( const f2d_world_def* def )
 static void free_world( HostWorld* W )
 {
 	cudaStreamSynchronize( W->stream );
+	if ( W->leanExec )
+		cudaGraphExecDestroy( W->leanExec );
 	if ( W->graphExec )
 		cudaGraphExecDestroy( W->graphExec );
 	isl_free( W );
@@ -3887,7 +3894,7 @@ extern "C" F2D_API void f2d_world_set_pre_solve( int32_t worldId, f2d_pre_solve_
 	W->graphDirty = true;
 }
 
-static void enqueue_step( HostWorld* W, float dt, int subSteps, int planMode )
+static void enqueue_step( HostWorld* W, float dt, int subSteps, int planMode, bool lean )
 {
 	DWorld& d = W->d;
 	bool prof = W->profiling;
@@ -3896,7 +3903,8 @@ static void enqueue_step( HostWorld* W, float dt, int subSteps, int planMode )
 			cudaEventCreate( W->ph + i );
 	W->s.evSolveStart = prof ? W->ph[4] : nullptr;
 	W->s.subSteps = subSteps;
-	launch_reset_counters( d, W->stream );
+	W->s.lean = lean;
+	launch_reset_counters( d, W->stream, lean );
 	if ( prof )
 		cudaEventRecord( W->ph[0], W->stream );
 	bool filter = W->customFilter != nullptr, pre = W->preSolve != nullptr;
@@ -3942,6 +3950,31 @@ static int count_kernel_nodes( cudaGraph_t g )
 	return k;
 }
 
+#define LEAN_AFTER 16
+
+// the step as a graph (nullptr when that fails: it is then enqueued each time)
+static void capture_step( HostWorld* W, float dt, int subSteps, bool lean, cudaGraphExec_t* exec, int* nodes )
+{
+	if ( *exec )
+	{
+		cudaGraphExecDestroy( *exec );
+		*exec = nullptr;
+	}
+	cudaGraph_t g;
+	if ( cudaStreamBeginCapture( W->stream, cudaStreamCaptureModeThreadLocal ) == cudaSuccess )
+	{
+		enqueue_step( W, dt, subSteps, 0, lean );
+		if ( cudaStreamEndCapture( W->stream, &g ) == cudaSuccess )
+		{
+			if ( cudaGraphInstantiate( exec, g, 0 ) != cudaSuccess )
+				*exec = nullptr;
+			*nodes = count_kernel_nodes( g );
+			cudaGraphDestroy( g );
+		}
+	}
+	cudaGetLastError();
+}
+
 static void ensure_learning_buffers( HostWorld* W );
 
 extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int32_t subStepCount )
@@ -3969,7 +4002,7 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 	if ( W->stepped && cudaEventQuery( W->evStop ) == cudaSuccess )
 		W->statusAccum |= *W->hostError;
 	flush_uploads( W );
-	upload_host_moves( W );
+	const bool hostMoves = upload_host_moves( W );
 	int planMode = 0;
 	if ( W->planPending )
 	{
@@ -3987,6 +4020,11 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 	if ( W->d.learnMode != 0 )
 		ensure_learning_buffers( W );
 	cudaMemsetAsync( &W->d.sc->error, 0, sizeof( int ), W->stream );
+	if ( hostMoves )
+		launch_pt_host_moves( W->d, W->s, W->stream );
+	const int period = W->orderPeriod > 0 ? W->orderPeriod : ORDER_REBUILD_PERIOD;
+	const bool sorts = W->forceRebuild || W->orderAge >= period - 1;
+	W->orderAge = sorts ? 0 : W->orderAge + 1;
 	if ( W->forceRebuild )
 	{
 		cudaMemsetAsync( &W->d.sc->forceRebuild, 1, 1, W->stream );
@@ -3998,36 +4036,36 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 	bool useGraph = planMode == 0 && !W->profiling && W->d.callbacks == 0;
 	if ( useGraph && ( W->graphDirty || W->graphExec == nullptr || W->graphDt != dt || W->graphSubSteps != subSteps ) )
 	{
-		if ( W->graphExec )
+		if ( W->leanExec )
 		{
-			cudaGraphExecDestroy( W->graphExec );
-			W->graphExec = nullptr;
+			cudaGraphExecDestroy( W->leanExec );
+			W->leanExec = nullptr;
 		}
-		cudaGraph_t g;
-		if ( cudaStreamBeginCapture( W->stream, cudaStreamCaptureModeThreadLocal ) == cudaSuccess )
-		{
-			enqueue_step( W, dt, subSteps, 0 );
-			if ( cudaStreamEndCapture( W->stream, &g ) == cudaSuccess )
-			{
-				if ( cudaGraphInstantiate( &W->graphExec, g, 0 ) != cudaSuccess )
-					W->graphExec = nullptr;
-				W->graphKernelNodes = count_kernel_nodes( g );
-				cudaGraphDestroy( g );
-			}
-		}
-		cudaGetLastError();
+		W->graphSteps = 0;
+		capture_step( W, dt, subSteps, false, &W->graphExec, &W->graphKernelNodes );
 		W->graphDt = dt;
 		W->graphSubSteps = subSteps;
 		W->graphDirty = false;
 	}
-	if ( useGraph && W->graphExec )
+	// A step that sorts no leaves is 8 launches of nothing shorter without the
+	// ordering, some 20 us; capturing that form costs some 0.4 ms, so it is done
+	// once the world has kept its graph for LEAN_AFTER steps.
+	const bool lean = useGraph && !sorts && W->graphExec != nullptr;
+	if ( lean && W->leanExec == nullptr && ++W->graphSteps == LEAN_AFTER )
+		capture_step( W, dt, subSteps, true, &W->leanExec, &W->leanKernelNodes );
+	if ( lean && W->leanExec )
+	{
+		cudaGraphLaunch( W->leanExec, W->stream );
+		W->lastLaunches = W->leanKernelNodes;
+	}
+	else if ( useGraph && W->graphExec )
 	{
 		cudaGraphLaunch( W->graphExec, W->stream );
 		W->lastLaunches = W->graphKernelNodes;
 	}
 	else
 	{
-		enqueue_step( W, dt, subSteps, planMode );
+		enqueue_step( W, dt, subSteps, planMode, false );
 		W->lastLaunches = W->graphKernelNodes;
 	}
 	cudaEventRecord( W->evStop, W->stream );

@@ -57,3 +57,27 @@ def test_queries_equal_port(gpu_lib, count):
         assert str(a) == str(b), ray
     g.close()
     p.close()
+
+
+@pytest.mark.parametrize("edit", [14, 15, 16, 17, 24])
+def test_replayed_forms_equal_port(gpu_lib, edit):
+    """The step is replayed in two forms, with and without the leaf ordering,
+    the second from the 16th unchanged step that sorts nothing: an edit around
+    there, and a change of the substeps after it."""
+    from forge2d_gb300.world import GpuWorld
+    from oracle.oracle import PortWorld
+    wd = scenes.world_def(enableSleep=0)
+    g, p = GpuWorld(wd), PortWorld(wd)
+    for b in (g, p):
+        scenes.build(b, "pile", count=60, width=12.0, height=12.0, seed=3)
+    for frame in range(60):
+        for b in (g, p):
+            if frame == edit:
+                body = b.create_body(scenes.body_def(type=scenes.DYNAMIC, positionX=0.5, positionY=14.0))
+                b.create_circle(body, scenes.shape_def(), 0.0, 0.0, 0.3)
+            b.step(1.0 / 60.0, 4 if frame < edit + 25 else 3)
+        assert g.sync() == 0
+        x, y = g.bodies()[:, :9], p.bodies()[:, :9]
+        assert np.array_equal(x.view(np.uint32), y.view(np.uint32)), (frame, np.argwhere(x != y)[:4].tolist())
+    g.close()
+    p.close()
