@@ -45,6 +45,7 @@
 
 #define PT_THREADS 256
 #define PT_SMALL 1024
+#define PT_SMALL_THREADS 1024
 #define PT_CHUNK 1024
 #define PT_ITEMS ( PT_CHUNK / PT_THREADS )
 #define PT_WARPS ( PT_THREADS / 32 )
@@ -828,7 +829,11 @@ __device__ __forceinline__ void pt_refresh_node( const DProxyTree& T, int p, int
 // centre of [s, s + below) that is not below the pivot swaps with the k-th
 // centre of [s + below, e) that is, counted from the end), the same pairs as
 // the warp form. Returns the split (nodes on the left).
-#define PT_SERIAL 32
+// A segment's levels are short chains and its blocks are few (some 60 at 25k
+// bodies): a thread takes items of up to 8 nodes, a warp each larger one, 32
+// warps a block. With 8 warps and threads for up to 32 nodes the rebuild took
+// 158 us at 25k bodies instead of 147, 120 us at 6k instead of 105.
+#define PT_SERIAL 8
 __device__ __forceinline__ int pt_partition_serial( int* idx, float2* cen, int s, int e )
 {
 	int cnt = e - s;
@@ -873,7 +878,7 @@ __device__ __forceinline__ int pt_partition_serial( int* idx, float2* cen, int s
 	return below;
 }
 
-__global__ void __launch_bounds__( PT_THREADS ) k_pt_small( DWorld w, int t )
+__global__ void __launch_bounds__( PT_SMALL_THREADS ) k_pt_small( DWorld w, int t )
 {
 	extern __shared__ __align__( 16 ) unsigned char ptSmem[];
 	PtSmall& sm = *reinterpret_cast<PtSmall*>( ptSmem );
@@ -931,7 +936,7 @@ __global__ void __launch_bounds__( PT_THREADS ) k_pt_small( DWorld w, int t )
 					sSplit[it] = pt_partition_serial( sIdx, sCen, item.x, item.y );
 			}
 			// larger items: a warp each
-			for ( int it = wid; it < m; it += PT_WARPS )
+			for ( int it = wid; it < m; it += ( PT_SMALL_THREADS / 32 ) )
 			{
 				int4 item = sItem[cur][it];
 				int s = item.x, e = item.y, cnt = e - s;
@@ -1228,7 +1233,7 @@ void launch_pt_rebuild( DWorld& w, StepScratch& s, cudaStream_t st )
 			cudaLaunchCooperativeKernel( (void*)k_pt_large, dim3( s.ptBlocks ), dim3( PT_THREADS ), args,
 										 sizeof( PtLarge ), st );
 		}
-		k_pt_small<<<F2D_SMS * 2, PT_THREADS, sizeof( PtSmall ), st>>>( w, t );
+		k_pt_small<<<F2D_SMS * 2, PT_SMALL_THREADS, sizeof( PtSmall ), st>>>( w, t );
 		k_pt_refresh<<<grid_for( w.pt[t].cap ), 256, 0, st>>>( w, t );
 	}
 }
