@@ -572,16 +572,18 @@ struct DWorld
 // depth-first query visits overlapping leaves in descending position)
 __device__ __forceinline__ int tree_leaf_rank( const DProxyTree& T, int leaf )
 {
-	int r = 0, c = leaf;
-	for ( int guard = 0; guard < ( 1 << 16 ); ++guard )
+	// bound by the chain of parents: an ancestor's links are read together and
+	// the left leaves are added a level late (a level is one round trip)
+	int r = 0, late = 0, c = leaf, p = T.parent[leaf];
+	for ( int guard = 0; guard < ( 1 << 16 ) && p >= 0 && p < T.cap; ++guard )
 	{
-		int p = T.parent[c];
-		if ( p < 0 || p >= T.cap )
-			break;
-		if ( T.child2[p] == c )
-			r += T.leaves[T.child1[p]];
+		const int up = T.parent[p], left = T.child1[p], right = T.child2[p];
+		r += late;
+		late = right == c ? T.leaves[left] : 0;
 		c = p;
+		p = up;
 	}
+	r += late;
 	return r;
 }
 #endif

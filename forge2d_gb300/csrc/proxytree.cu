@@ -288,7 +288,7 @@ __global__ void k_pt_count( DWorld w, int t )
 		int p = T.parent[i];
 		if ( p < 0 || R.doomed[p] == 0 )
 			continue;
-		int c = i;
+		int c = i, mine = 1; // gathered nodes below c
 		for ( int guard = 0;; ++guard )
 		{
 			if ( guard > PT_GUARD )
@@ -296,22 +296,23 @@ __global__ void k_pt_count( DWorld w, int t )
 				atomicOr( &w.sc->error, ERR_TREE );
 				break;
 			}
-			p = T.parent[c];
 			if ( p < 0 || p >= T.cap )
 			{
 				atomicOr( &w.sc->error, ERR_TREE );
 				break;
 			}
+			// the links are on their way while the arrival is counted
+			const int a = T.child1[p], b = T.child2[p], up = T.parent[p];
 			if ( pt_atom_add( R.cnt + p, 1 ) == 0 )
 				break;
-			int a = T.child1[p], b = T.child2[p];
-			int va = R.doomed[a] ? __ldcg( R.rlc + a ) : 1;
-			int vb = R.doomed[b] ? __ldcg( R.rlc + b ) : 1;
-			__stcg( R.rlc + p, va + vb );
+			const int sibling = a == c ? b : a;
+			mine += R.doomed[sibling] ? __ldcg( R.rlc + sibling ) : 1;
+			__stcg( R.rlc + p, mine );
 			__threadfence();
 			if ( p == root )
 				break;
 			c = p;
+			p = up;
 		}
 	}
 }
@@ -334,26 +335,29 @@ __global__ void k_pt_gather( DWorld w, int t )
 		bool gathered = !dm && pi >= 0 && R.doomed[pi] != 0;
 		if ( !dm && !gathered )
 			continue;
-		int acc = 0, c1 = 0, c = i;
+		// a level of the climb is one round trip: the links are read together,
+		// the left subtree's count is added a level late
+		int acc = 0, c1 = 0, c = i, p = pi;
+		int late = 0, lateDoomed = 0, lateCount = 0;
 		bool ok = true;
 		for ( int guard = 0; c != root; ++guard )
 		{
-			int p = T.parent[c];
 			if ( guard > PT_GUARD || p < 0 || p >= T.cap )
 			{
 				atomicOr( &w.sc->error, ERR_TREE );
 				ok = false;
 				break;
 			}
-			if ( T.child2[p] == c )
-			{
-				int a = T.child1[p];
-				acc += R.doomed[a] ? R.rlc[a] : 1;
-			}
-			else
-				c1 += 1;
+			const int up = T.parent[p], left = T.child1[p], right = T.child2[p];
+			acc += late ? ( lateDoomed ? lateCount : 1 ) : 0;
+			late = right == c ? 1 : 0;
+			lateDoomed = R.doomed[left];
+			lateCount = R.rlc[left];
+			c1 += late ^ 1;
 			c = p;
+			p = up;
 		}
+		acc += late ? ( lateDoomed ? lateCount : 1 ) : 0;
 		int total = R.rlc[root];
 		if ( !ok || ( dm ? acc + c1 >= total - 1 : acc >= total ) )
 		{
@@ -1144,21 +1148,7 @@ __global__ void k_pt_ranks( DWorld w, int t, int onlyAfterRebuild )
 	{
 		if ( ( T.flags[i] & ( PT_ALLOCATED | PT_LEAF ) ) != ( PT_ALLOCATED | PT_LEAF ) )
 			continue;
-		int r = 0, c = i;
-		for ( int guard = 0;; ++guard )
-		{
-			if ( guard > PT_GUARD )
-			{
-				atomicOr( &w.sc->error, ERR_TREE );
-				break;
-			}
-			int p = T.parent[c];
-			if ( p < 0 || p >= T.cap )
-				break;
-			if ( T.child2[p] == c )
-				r += T.leaves[T.child1[p]];
-			c = p;
-		}
+		const int r = tree_leaf_rank( T, i );
 		T.rank[i] = r;
 		if ( r >= 0 && r < T.cap )
 			T.rankShape[r] = T.shape[i];
