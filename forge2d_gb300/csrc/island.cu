@@ -1142,11 +1142,12 @@ __global__ void k_isl_merge_apply( DIslands* Ip )
 //   after: the pop ranks decide which body of a contact lists it, prefix sums
 //     over the pop order give every list's order, and the links follow.
 //
-// Bound: the traversal's chain, a row read (L1), a mark read and a vote per
-// body. One island of 6e4 bodies and 1.4e5 contacts: 300 ms on one thread,
-// 8 ms here (230 cycles a body: a pop is a chain of a row from the L1, its
-// neighbours' marks, a vote and a shuffle; a branch in it costs 50 to 100
-// cycles, and with five of them a split took 12 ms).
+// Bound: the traversal's chain: rows from the L1, marks, votes, the stack. One
+// island of 6e4 bodies and 1.4e5 contacts: 300 ms on one thread, 7 ms here, an
+// iteration of 440 cycles for 1.9 pops. A branch in it costs 50 to 100 cycles
+// (with five of them a split took 13 ms), a pop at a time took 8 ms, without
+// the rows read ahead 12 ms; marks as bits instead of bytes cost a shared
+// atomic each and 20 ms.
 // ---------------------------------------------------------------------------
 #define SPLIT_THREADS 512
 #define SPLIT_ROW 8			   // int2 per edge row: (edges, body), then up to 7 edges
@@ -1156,6 +1157,7 @@ __global__ void k_isl_merge_apply( DIslands* Ip )
 #define SPLIT_BYTES 114688	   // mark bytes in shared memory (larger islands: global)
 #define SPLIT_JOINT 0x40000000 // edge key: joint id | this, else contact id
 #define SPLIT_OUTSIDE ( -1 )   // the other body is never pushed (static)
+#define SPLIT_GROUPS ( 32 / SPLIT_PUSH )
 #define SPLIT_AHEAD 256		   // push rows read ahead around the current body (half as many on either side)
 #define SPLIT_AHEAD_WARPS 4
 
@@ -1308,10 +1310,11 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 	// (the record is global memory: its pointers are read once)
 	int* const gstack = I.stack;
 	int* const order = I.splitOrder;
-	const int* const rowBase = I.splitPush + ( lane < SPLIT_PUSH ? lane : 0 );
+	// the warp looks at the SPLIT_GROUPS next pops at once, eight lanes each
+	const int group = lane / SPLIT_PUSH;
+	const int* const rowBase = I.splitPush + lane % SPLIT_PUSH;
 	const int* const pushPool = I.splitPushPool;
 	const int* const seeds = I.seeds;
-	const int none = lane < SPLIT_PUSH ? 0 : -1;
 	const int* const links = I.splitPush + SPLIT_PUSH - 1; // of long rows
 	int popped = 0, islands = 0;
 	int lo = 0; // entries below lo are in global memory
@@ -1346,44 +1349,61 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 				marks.set( next );
 			}
 			islands += 1;
-			int sp = 0, popping = next;
-			int other = rowBase[(size_t)SPLIT_PUSH * next];
+			// entries not popped yet: [0, sp), those below lo in global memory
+			__syncwarp();
+			if ( lane == 0 )
+				sts_s32( stack + 4u * (unsigned)( lo & ( SPLIT_STACK - 1 ) ), next );
+			int sp = lo + 1;
+			const int bottom = lo;
+			__syncwarp();
 			for ( ;; )
 			{
 				unsigned longRow;
-				const int high = lo + SPLIT_STACK - 32, low = lo > 0 ? lo : -1;
-				// The chain of a pop: its row (read below, by the pop before), its
-				// neighbours' marks, the vote, and the next pop's row; everything
-				// else is done while that row is on its way. Nothing in the loop
+				int body, popping;
+				const int high = lo + SPLIT_STACK - 32;
+				int at = sp - 1 - group;
+				body = lds_s32( stack + 4u * (unsigned)( ( at >= lo ? at : sp - 1 ) & ( SPLIT_STACK - 1 ) ) );
+				int other = rowBase[(size_t)SPLIT_PUSH * body];
+				// The chain of a pop: the rows of the next pops, their neighbours'
+				// marks, the votes, the stack and the rows again. The first pops that
+				// push nothing (about half do) change nothing, so they are done
+				// together with the first one that pushes. Nothing in the loop
 				// branches but its end: empty places mean the row that counts as
-				// marked, marking it or a marked row again changes nothing, lanes
-				// that push nothing store to a spare word. A pop ends the loop when
-				// its row is long, the stack's shared part is full or used up, or
-				// the stack is empty.
+				// marked, marking it again changes nothing, lanes that push nothing
+				// store to a spare word, order rows past the pops are written again.
+				// A pop ends the loop when its row is long or when the stack's shared
+				// part is full or used up.
 				do
 				{
-					__syncwarp();
-					const int below = lds_s32( stack + 4u * (unsigned)( ( sp - 1 ) & ( SPLIT_STACK - 1 ) ) );
-					other |= none;
+					other = at >= lo ? other : -1;
 					const int cur = (int)min( (unsigned)other, (unsigned)noRow );
 					const bool push = !marks.get( cur );
-					longRow = __ballot_sync( full, other <= -2 );
-					const unsigned pushes = __ballot_sync( full, push );
-					const int top = __shfl_sync( full, cur, 31 - __clz( pushes ) );
-					popping = next;
-					const unsigned slot = stack + 4u * (unsigned)( ( sp + __popc( pushes & lt ) ) & ( SPLIT_STACK - 1 ) );
+					const unsigned longRows = __ballot_sync( full, other <= -2 );
+					const unsigned votes = __ballot_sync( full, push );
+					const unsigned busy = votes | longRows;
+					const int valid = min( sp - lo, SPLIT_GROUPS );
+					// (no busy lane: past the last group)
+					const int k = min( (int)( ( (unsigned)__ffs( busy ) - 1u ) & 63u ) >> 3, valid );
+					const unsigned pushes = k < valid ? ( votes >> ( SPLIT_PUSH * k ) ) & ( ( 1u << SPLIT_PUSH ) - 1u ) : 0u;
+					longRow = k < valid ? ( longRows >> ( SPLIT_PUSH * k ) ) & ( ( 1u << SPLIT_PUSH ) - 1u ) : 0u;
+					const int pops = min( k + 1, valid );
+					const bool mine = group == k;
+					order[popped + group] = body;
+					popping = body;
+					popped += pops;
+					sp -= pops;
+					const unsigned slot = stack + 4u * (unsigned)( ( sp + __popc( pushes & ( ( 1u << ( lane % SPLIT_PUSH ) ) - 1u ) ) ) & ( SPLIT_STACK - 1 ) );
+					marks.set( mine ? cur : noRow );
+					sts_s32( mine && push ? slot : spare, cur );
 					sp += __popc( pushes );
-					next = pushes ? top : below;
-					next = sp > 0 ? next : popping;
-					other = rowBase[(size_t)SPLIT_PUSH * next];
-					marks.set( cur );
-					sts_s32( push ? slot : spare, cur );
-					order[popped] = popping;
-					sts_s32( ahead, next );
-					popped += 1;
-					sp -= 1;
-				} while ( ( sp != low ) & ( sp < high ) & ( longRow == 0u ) );
-				sp += 1;
+					__syncwarp();
+					at = sp - 1 - group;
+					body = lds_s32( stack + 4u * (unsigned)( ( at >= lo ? at : max( sp - 1, lo ) ) & ( SPLIT_STACK - 1 ) ) );
+					body = sp > lo ? body : popping;
+					other = rowBase[(size_t)SPLIT_PUSH * body];
+					sts_s32( lane == 0 ? ahead : spare, body );
+					popping = __shfl_sync( full, popping, ( SPLIT_PUSH * k ) & 31 );
+				} while ( ( sp > lo ) & ( sp <= high ) & ( longRow == 0u ) );
 				make_room( sp );
 				if ( longRow )
 				{
@@ -1400,24 +1420,20 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 							marks.set( o );
 							sts_s32( stack + 4u * (unsigned)( ( sp + __popc( pm & lt ) ) & ( SPLIT_STACK - 1 ) ), o );
 						}
-						if ( pm )
-							next = __shfl_sync( full, o, 31 - __clz( pm ) );
 						sp += __popc( pm );
 						make_room( sp );
 					}
-					if ( sp > 0 )
-						other = rowBase[(size_t)SPLIT_PUSH * next];
 				}
-				if ( sp == 0 )
+				if ( sp == bottom )
 					break;
-				sp -= 1;
-				if ( sp == lo && lo > 0 )
+				if ( sp == lo )
 				{
 					__syncwarp();
 					lo -= SPLIT_SPILL;
 					for ( int k = lane; k < SPLIT_SPILL; k += 32 )
 						sts_s32( stack + 4u * (unsigned)( ( lo + k ) & ( SPLIT_STACK - 1 ) ), gstack[lo + k] );
 				}
+				__syncwarp();
 			}
 		}
 	}

@@ -501,7 +501,7 @@ static void isl_ensure( HostWorld* W )
 		dgrow( h.splitMarks, 0, 2 * nb + 8 );
 		dgrow( h.splitRows, 0, 16 * nb );
 		dgrow( h.splitPush, 0, 16 * nb );
-		dgrow( h.splitOrder, 0, nb );
+		dgrow( h.splitOrder, 0, nb + 8 );
 		dgrow( h.splitPop, 0, 2 * nb );
 		dgrow( h.splitIslands, 0, nb + 1 );
 		dgrow( h.splitJointAt, 0, nb );
