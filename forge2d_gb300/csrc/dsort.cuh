@@ -17,6 +17,7 @@
 
 #include "dscan.cuh"
 #include "dsync.cuh"
+#include "dworld.cuh"
 
 #include <climits>
 
@@ -528,6 +529,52 @@ template <typename K> static inline int sort_coop_blocks()
 	cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
 	int b = perSM >= 1 ? sms : 0;
 	return b > CSORT_MAX_BLOCKS ? CSORT_MAX_BLOCKS : b;
+}
+
+// Compaction in one launch: blocks of LOOKBACK_TILE threads, an item each, tiles
+// chained by decoupled look-back (state zeroed before the launch, one launch
+// per step and state). Calls place( item, slot ) for the wanted items, slots in
+// item order, and finish( count ) once.
+template <typename Want, typename Place, typename Finish>
+__device__ __forceinline__ void compact_items( unsigned long long* state, int n, int* err, Want want, Place place, Finish finish )
+{
+	__shared__ int smem[32];
+	__shared__ int s_tile, s_prefix;
+	if ( threadIdx.x == 0 )
+		s_tile = (int)atomicAdd( (unsigned*)state, 1u );
+	__syncthreads();
+	const int tile = s_tile, base = tile * LOOKBACK_TILE;
+	if ( base >= n )
+	{
+		if ( tile == 0 && threadIdx.x == 0 )
+			finish( 0 );
+		return;
+	}
+	const int item = base + threadIdx.x;
+	const bool wanted = item < n && want( item );
+	int total;
+	const int slot = block_exclusive_scan_1024( wanted ? 1 : 0, smem, &total );
+	if ( threadIdx.x < 32 )
+	{
+		if ( threadIdx.x == 0 )
+			lookback_publish( state + 1, tile, total );
+		__syncwarp();
+		const int prefix = lookback_prefix( state + 1, tile, total, err );
+		if ( threadIdx.x == 0 )
+		{
+			s_prefix = prefix;
+			if ( base + LOOKBACK_TILE >= n )
+				finish( prefix + total );
+		}
+	}
+	__syncthreads();
+	if ( wanted )
+		place( item, s_prefix + slot );
+}
+
+static inline int compact_blocks( int cap )
+{
+	return ( cap + LOOKBACK_TILE - 1 ) / LOOKBACK_TILE;
 }
 
 // ---------------------------------------------------------------------------

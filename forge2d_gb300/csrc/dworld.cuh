@@ -463,10 +463,12 @@ struct DWorld
 	int* opColor;	// colour result / colour removed
 	int* opDone;
 	int2* opBodies; // solver body indices of the op's contact (-1 static)
-	unsigned long long* opScan; // look-back state of the op output scans (zeroed at the step's start, as the next two)
+	unsigned long long* opScan; // look-back state of the op output scans (zeroed at the step's start, as the next ones)
 	unsigned long long* collectScan; // of the state-change ops
 	unsigned long long* moveScan;	 // of the move array
-	int lookbackWords;				 // words of the three together
+	// of the islands' new contacts, links, merged and sleeping islands
+	unsigned long long *ncScan, *linkScan, *mergeScan, *sleepScan;
+	int lookbackWords; // words of all of them together
 
 	// ---------------- constraints (by slot, grouped by colour) ----------------
 	int* overflowList; // contact ids in overflow-array order

@@ -561,6 +561,8 @@ __global__ void k_reset_step_counters( DWorld w, int lean )
 	for ( int k = 0; k < 5; ++k )
 		w.sc->sortBarrier[k] = 0;
 	w.sc->pendingOps = 0;
+	if ( w.isl )
+		w.isl->serialOps = 0;
 	w.sc->hitCount = 0;
 	w.sc->fastCount = 0;
 	w.sc->newPointCount = 0;
@@ -595,7 +597,7 @@ void launch_finalize( DWorld& w, StepScratch& s, cudaStream_t st, float dt, Host
 	// step in awake order and grow their tree leaves
 	launch_pt_moves( w, st );
 	if ( w.isl )
-		launch_isl_sleep( w, st, s.scanState );
+		launch_isl_sleep( w, st );
 }
 
 void launch_reset_counters( DWorld& w, cudaStream_t st, bool lean )

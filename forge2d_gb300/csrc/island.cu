@@ -1081,13 +1081,12 @@ __global__ void k_isl_merge_roots( DWorld w, DIslands* Ip )
 	}
 }
 
-__global__ void k_isl_list( DIslands* Ip, const int* count )
+__global__ void __launch_bounds__( LOOKBACK_TILE ) k_isl_list( DWorld w, DIslands* Ip, unsigned long long* scan )
 {
 	DIslands& I = *Ip;
-	int n = *count;
-	for ( int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x )
-		if ( I.flag[i] )
-			I.list[I.pos[i]] = I.awakeIslands[i];
+	compact_items(
+		scan, I.awakeIslandCount, &w.sc->error, [&]( int i ) { return I.flag[i] != 0; },
+		[&]( int i, int slot ) { I.list[slot] = I.awakeIslands[i]; }, [&]( int count ) { I.listCount = count; } );
 }
 
 // island.c:539-600 members of merged islands: every body, contact and joint
@@ -1870,43 +1869,32 @@ void launch_isl_create( DWorld& w, cudaStream_t st )
 // creation order; their set records start in parallel and their body edges,
 // sorted by (body, creation rank), are prepended in rank order per body --
 // the list the serial prepends (contact.c:227-262) give.
-__global__ void k_isl_nc_flags( DWorld w, int* ids, int* flag )
-{
-	int n = min( w.sc->newPairCount, w.pairCap );
-	int F = w.sc->contactFreeCount;
-	int base = w.sc->contactIdCount;
-	for ( int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x )
-	{
-		int id = r < F ? w.contactFree[F - 1 - r] : base + ( r - F );
-		bool ok = id >= 0 && id < w.contactCap && ( w.cflags[id] & CF_USED ) != 0;
-		ids[r] = id;
-		flag[r] = ok ? 1 : 0;
-	}
-}
 
-__global__ void k_isl_nc_init( DWorld w, DIslands* Ip, const int* ids, const int* flag, const int* pos )
+__global__ void __launch_bounds__( LOOKBACK_TILE ) k_isl_nc_init( DWorld w, DIslands* Ip )
 {
 	DIslands& I = *Ip;
-	int n = min( w.sc->newPairCount, w.pairCap );
-	for ( int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x )
-	{
-		if ( !flag[r] )
-			continue;
-		int i = pos[r];
-		int c = ids[r];
-		I.order[i] = c;
-		int2 bd = w.cbody[c];
-		bool awake = I.bSet[bd.x] == SET_AWAKE || I.bSet[bd.y] == SET_AWAKE;
-		I.cSet[c] = awake ? SET_AWAKE : SET_DISABLED;
-		I.cIsland[c] = I.cIslandPrev[c] = I.cIslandNext[c] = ISL_NULL;
-		I.cMark[c] = 0;
-		if ( !awake )
-			w.cflags[c] |= CF_INACTIVE;
-		I.ncKeys[2 * i] = ( (unsigned long long)(unsigned)bd.x << 32 ) | (unsigned)( 2 * i );
-		I.ncKeys[2 * i + 1] = ( (unsigned long long)(unsigned)bd.y << 32 ) | (unsigned)( 2 * i + 1 );
-	}
-	if ( blockIdx.x == 0 && threadIdx.x == 0 )
-		I.ncCount = 2 * ( n > 0 ? pos[n - 1] + flag[n - 1] : 0 );
+	const int F = w.sc->contactFreeCount, base = w.sc->contactIdCount;
+	auto contact = [&]( int r ) { return r < F ? w.contactFree[F - 1 - r] : base + ( r - F ); };
+	compact_items(
+		w.ncScan, min( w.sc->newPairCount, w.pairCap ), &w.sc->error,
+		[&]( int r ) {
+			const int id = contact( r );
+			return id >= 0 && id < w.contactCap && ( w.cflags[id] & CF_USED ) != 0;
+		},
+		[&]( int r, int i ) {
+			const int c = contact( r );
+			I.order[i] = c;
+			const int2 bd = w.cbody[c];
+			const bool awake = I.bSet[bd.x] == SET_AWAKE || I.bSet[bd.y] == SET_AWAKE;
+			I.cSet[c] = awake ? SET_AWAKE : SET_DISABLED;
+			I.cIsland[c] = I.cIslandPrev[c] = I.cIslandNext[c] = ISL_NULL;
+			I.cMark[c] = 0;
+			if ( !awake )
+				w.cflags[c] |= CF_INACTIVE;
+			I.ncKeys[2 * i] = ( (unsigned long long)(unsigned)bd.x << 32 ) | (unsigned)( 2 * i );
+			I.ncKeys[2 * i + 1] = ( (unsigned long long)(unsigned)bd.y << 32 ) | (unsigned)( 2 * i + 1 );
+		},
+		[&]( int count ) { I.ncCount = 2 * count; } );
 }
 
 // edge key of sorted row p: (contact << 1) | edge
@@ -1963,13 +1951,7 @@ void launch_isl_new_contacts( DWorld& w, StepScratch& s, cudaStream_t st, int pl
 		return;
 	}
 	DIslands* I = w.isl;
-	int* ids = s.tmpA;
-	int* flag = s.tmpA + w.pairCap;
-	int* pos = s.tmpB;
-	int g = grid_for( w.pairCap );
-	k_isl_nc_flags<<<g, 256, 0, st>>>( w, ids, flag );
-	scan_lookback( flag, pos, &w.sc->newPairCount, 0, w.pairCap, nullptr, s.scanState, &w.sc->error, st );
-	k_isl_nc_init<<<g, 256, 0, st>>>( w, I, ids, flag, pos );
+	k_isl_nc_init<<<compact_blocks( w.pairCap ), LOOKBACK_TILE, 0, st>>>( w, I );
 	int bodyBits = 1;
 	while ( ( 1 << bodyBits ) < w.bodyCap )
 		bodyBits += 1;
@@ -1988,12 +1970,9 @@ static int* isl_field( DIslands* I, size_t offset )
 	return (int*)( (char*)I + offset );
 }
 
-static void isl_list( DWorld& w, unsigned long long* scanState, cudaStream_t st )
+static void isl_list( DWorld& w, unsigned long long* scan, cudaStream_t st )
 {
-	int* count = isl_field( w.isl, offsetof( DIslands, awakeIslandCount ) );
-	int* total = isl_field( w.isl, offsetof( DIslands, listCount ) );
-	scan_lookback( w.islFlag, w.islPos, count, 0, w.bodyCap, total, scanState, &w.sc->error, st );
-	k_isl_list<<<grid_for( w.bodyCap ), 256, 0, st>>>( w.isl, count );
+	k_isl_list<<<compact_blocks( w.bodyCap ), LOOKBACK_TILE, 0, st>>>( w, w.isl, scan );
 }
 
 // parallel form, step 1: mark the contacts that leave an island list (end
@@ -2110,7 +2089,7 @@ __global__ void k_isl_unlink_clear( DWorld w, DIslands* Ip )
 // child of the A root as it goes). The prepends themselves then run in
 // parallel: sorted by (island, op), each island's new contacts chain in op
 // order in front of its old head.
-__global__ void k_isl_link_flags( DWorld w, DIslands* Ip, int* flag )
+__global__ void k_isl_link_flags( DWorld w, DIslands* Ip )
 {
 	const DIslands& I = *Ip;
 	if ( I.serialOps )
@@ -2128,7 +2107,6 @@ __global__ void k_isl_link_flags( DWorld w, DIslands* Ip, int* flag )
 				target = idA;
 		}
 		I.order[k] = target;
-		flag[k] = link ? 1 : 0;
 	}
 }
 
@@ -2200,22 +2178,19 @@ __global__ void __launch_bounds__( LINK_ROOTS_THREADS ) k_isl_link_roots( DWorld
 	}
 }
 
-__global__ void k_isl_link_keys( DWorld w, DIslands* Ip, const int* flag, const int* pos )
+__global__ void __launch_bounds__( LOOKBACK_TILE ) k_isl_link_keys( DWorld w, DIslands* Ip )
 {
 	DIslands& I = *Ip;
 	if ( I.serialOps )
 		return;
-	int nOps = min( w.sc->opCount, w.opCap );
-	for ( int k = blockIdx.x * blockDim.x + threadIdx.x; k < nOps; k += gridDim.x * blockDim.x )
-	{
-		if ( !flag[k] )
-			continue;
-		int c = w.opContact[k];
-		w.cflags[c] |= CF_TOUCHING;
-		I.ncKeys[pos[k]] = ( (unsigned long long)(unsigned)I.order[k] << 32 ) | (unsigned)k;
-	}
-	if ( blockIdx.x == 0 && threadIdx.x == 0 )
-		Ip->linkCount = nOps > 0 ? pos[nOps - 1] + flag[nOps - 1] : 0;
+	compact_items(
+		w.linkScan, min( w.sc->opCount, w.opCap ), &w.sc->error, [&]( int k ) { return w.opKind[k] == 1; },
+		[&]( int k, int slot ) {
+			const int c = w.opContact[k];
+			w.cflags[c] |= CF_TOUCHING;
+			I.ncKeys[slot] = ( (unsigned long long)(unsigned)I.order[k] << 32 ) | (unsigned)k;
+		},
+		[&]( int count ) { I.linkCount = count; } );
 }
 
 __global__ void k_isl_link_chain( DWorld w, DIslands* Ip )
@@ -2278,22 +2253,17 @@ __global__ void k_isl_link_heads( DWorld w, DIslands* Ip )
 
 void launch_isl_ops( DWorld& w, StepScratch& s, cudaStream_t st, const int* gkind )
 {
-	unsigned long long* scanState = s.scanState;
 	int g = grid_for( w.opCap );
-	cudaMemsetAsync( (char*)w.isl + offsetof( DIslands, serialOps ), 0, sizeof( int ), st );
 	k_isl_op_check<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_ops<<<1, 1, 0, st>>>( w, w.isl, gkind );
 	k_isl_unlink_mark<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_unlink_runs<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_unlink_clear<<<g, 256, 0, st>>>( w, w.isl );
 	// links: flags and same-island targets, the serial unions, then the
-	// prepends sorted by (island, op) (scratch past the op kinds in tmpA)
-	int* flag = s.tmpA + w.opCap;
-	int* pos = s.tmpB;
-	k_isl_link_flags<<<g, 256, 0, st>>>( w, w.isl, flag );
+	// prepends sorted by (island, op)
+	k_isl_link_flags<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_link_roots<<<1, LINK_ROOTS_THREADS, 0, st>>>( w, w.isl );
-	scan_lookback( flag, pos, &w.sc->opCount, 0, w.opCap, nullptr, scanState, &w.sc->error, st );
-	k_isl_link_keys<<<g, 256, 0, st>>>( w, w.isl, flag, pos );
+	k_isl_link_keys<<<compact_blocks( w.opCap ), LOOKBACK_TILE, 0, st>>>( w, w.isl );
 	int islandBits = 1;
 	while ( ( 1 << islandBits ) < w.bodyCap + 1 )
 		islandBits += 1;
@@ -2303,7 +2273,7 @@ void launch_isl_ops( DWorld& w, StepScratch& s, cudaStream_t st, const int* gkin
 	k_isl_link_chain<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_link_heads<<<g, 256, 0, st>>>( w, w.isl );
 	k_isl_merge_roots<<<grid_for( w.bodyCap ), 256, 0, st>>>( w, w.isl );
-	isl_list( w, scanState, st );
+	isl_list( w, w.mergeScan, st );
 	k_isl_merge_remap<<<grid_for( w.bodyCap + w.contactCap + w.jointCap ), 256, 0, st>>>( w, w.isl );
 	k_isl_merge_apply<<<1, 1, 0, st>>>( w.isl );
 }
@@ -2326,11 +2296,11 @@ void launch_isl_split( DWorld& w, cudaStream_t st )
 	k_isl_move_slots<<<grid_for( w.bodyCap ), 256, 0, st>>>( w.isl );
 }
 
-void launch_isl_sleep( DWorld& w, cudaStream_t st, unsigned long long* scanState )
+void launch_isl_sleep( DWorld& w, cudaStream_t st )
 {
 	k_isl_bits<<<grid_for( w.bodyCap ), 256, 0, st>>>( w, w.isl );
 	k_isl_sleep_flags<<<grid_for( w.bodyCap ), 256, 0, st>>>( w.isl );
-	isl_list( w, scanState, st );
+	isl_list( w, w.sleepScan, st );
 	k_isl_sleep<<<1, 1, 0, st>>>( w, w.isl );
 }
 

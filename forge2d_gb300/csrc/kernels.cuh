@@ -75,7 +75,7 @@ void launch_isl_create( DWorld& w, cudaStream_t st );
 void launch_isl_new_contacts( DWorld& w, StepScratch& s, cudaStream_t st, int planMode );
 void launch_isl_ops( DWorld& w, StepScratch& s, cudaStream_t st, const int* gkind );
 void launch_isl_split( DWorld& w, cudaStream_t st );
-void launch_isl_sleep( DWorld& w, cudaStream_t st, unsigned long long* scanState );
+void launch_isl_sleep( DWorld& w, cudaStream_t st );
 void launch_isl_api( DWorld& w, cudaStream_t st, int op, int body );
 // destroy path (island.cu), serial launches between steps: the contacts of a
 // body in its contact-list order (only those of `shape` / with body `other`

@@ -259,11 +259,16 @@ static void alloc_scratch( HostWorld* W )
 	// look-back states, zeroed together at the step's start
 	size_t opWords = OPS_SCAN_WORDS( (size_t)d.opCap ), collectWords = LOOKBACK_WORDS( (size_t)d.contactCap );
 	size_t moveWords = LOOKBACK_WORDS( (size_t)d.bodyCap );
-	d.lookbackWords = (int)( opWords + collectWords + moveWords );
+	size_t pairWords = LOOKBACK_WORDS( (size_t)d.pairCap ), linkWords = LOOKBACK_WORDS( (size_t)d.opCap );
+	d.lookbackWords = (int)( opWords + collectWords + 3 * moveWords + pairWords + linkWords );
 	dfree( d.opScan );
 	dgrow( d.opScan, 0, (size_t)d.lookbackWords );
 	d.collectScan = d.opScan + opWords;
 	d.moveScan = d.collectScan + collectWords;
+	d.mergeScan = d.moveScan + moveWords;
+	d.sleepScan = d.mergeScan + moveWords;
+	d.ncScan = d.sleepScan + moveWords;
+	d.linkScan = d.ncScan + pairWords;
 	size_t constraints = (size_t)d.contactCap + d.jointCap;
 	// constraint slots: every part and colour rounds up to whole groups
 	int parts = std::min( SOLVER_MAX_PARTS, d.bodyCap / ( W->smallParts ? SOLVER_SMALL_CHUNK : SOLVER_MIN_CHUNK ) + 2 );
