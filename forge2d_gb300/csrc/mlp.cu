@@ -264,7 +264,7 @@ __global__ void __launch_bounds__( MLP_THREADS )
 		{
 			int i = tile * 16 + lane;
 			bool valid = i < count;
-			const float* smp = samples + (size_t)( valid ? order[first + i] : 0 ) * MLP_SAMPLE;
+			const float* smp = samples + (size_t)( !valid ? 0 : ( order ? order[first + i] : first + i ) ) * MLP_SAMPLE;
 			put_features( s, warp, lane, smp, valid );
 			for ( int o = 0; o < MLP_OUT; ++o )
 				s.t[warp][lane * MLP_OUT + o] =
@@ -599,11 +599,11 @@ extern "C" F2D_API int32_t f2d_mlp_create( uint32_t seed )
 	if ( cudaMalloc( (void**)&M.master, sizeof( float ) * P_COUNT ) != cudaSuccess )
 		return 0;
 	cudaMalloc( (void**)&M.wbf, sizeof( __nv_bfloat16 ) * P_B1 );
-	cudaMalloc( (void**)&M.grad, sizeof( float ) * P_COUNT );
+	cudaMalloc( (void**)&M.grad, sizeof( float ) * ( P_COUNT + 1 ) );
+	M.loss = M.grad + P_COUNT;
 	cudaMalloc( (void**)&M.m, sizeof( float ) * P_COUNT );
 	cudaMalloc( (void**)&M.v, sizeof( float ) * P_COUNT );
 	cudaMalloc( (void**)&M.norm, sizeof( float ) * 2 * MLP_SAMPLE );
-	cudaMalloc( (void**)&M.loss, sizeof( float ) );
 	// He-uniform initialisation from a 32-bit LCG, biases zero
 	std::vector<float> p( P_COUNT, 0.0f );
 	uint32_t x = seed * 2654435761u + 12345u;
@@ -647,7 +647,6 @@ extern "C" F2D_API void f2d_mlp_destroy( int32_t handle )
 	cudaFree( M->m );
 	cudaFree( M->v );
 	cudaFree( M->norm );
-	cudaFree( M->loss );
 	memset( M, 0, sizeof( *M ) );
 }
 
@@ -689,30 +688,24 @@ extern "C" F2D_API float f2d_mlp_gradient( int32_t handle, const float* samples1
 	MlpModel* M = model_from( handle );
 	if ( M == nullptr || n <= 0 )
 		return 0.0f;
+	// the samples in their own order: no index list to build and send (64k rows:
+	// 677 -> 652 us for a gradient and a prediction, the rest is the rows' way up)
 	float* ds = nullptr;
-	int* ord = nullptr;
 	cudaMalloc( (void**)&ds, sizeof( float ) * MLP_SAMPLE * (size_t)n );
-	cudaMalloc( (void**)&ord, sizeof( int ) * (size_t)n );
 	cudaMemcpy( ds, samples14, sizeof( float ) * MLP_SAMPLE * (size_t)n, cudaMemcpyHostToDevice );
-	std::vector<int> o( n );
-	for ( int i = 0; i < n; ++i )
-		o[i] = i;
-	cudaMemcpy( ord, o.data(), sizeof( int ) * (size_t)n, cudaMemcpyHostToDevice );
-	cudaMemset( M->grad, 0, sizeof( float ) * P_COUNT );
-	cudaMemset( M->loss, 0, sizeof( float ) );
+	cudaMemset( M->grad, 0, sizeof( float ) * ( P_COUNT + 1 ) ); // and the loss
 	int tiles = ( n + 15 ) / 16;
 	int blocks = ( tiles + MLP_WARPS - 1 ) / MLP_WARPS;
 	if ( blocks > 4 * F2D_SMS )
 		blocks = 4 * F2D_SMS;
 	mlp_grad_setup();
-	k_mlp_grad<<<blocks, MLP_THREADS, MLP_GRAD_SMEM>>>( ds, ord, 0, n, M->wbf, M->master, M->norm, M->grad, M->loss );
-	float loss = 0.0f;
-	cudaMemcpy( grad, M->grad, sizeof( float ) * P_COUNT, cudaMemcpyDeviceToHost );
-	cudaMemcpy( &loss, M->loss, sizeof( float ), cudaMemcpyDeviceToHost );
-	cudaMemset( M->grad, 0, sizeof( float ) * P_COUNT );
+	k_mlp_grad<<<blocks, MLP_THREADS, MLP_GRAD_SMEM>>>( ds, nullptr, 0, n, M->wbf, M->master, M->norm, M->grad, M->loss );
+	float out[P_COUNT + 1];
+	cudaMemcpy( out, M->grad, sizeof( out ), cudaMemcpyDeviceToHost );
+	memcpy( grad, out, sizeof( float ) * P_COUNT );
+	cudaMemsetAsync( M->grad, 0, sizeof( float ) * P_COUNT, 0 );
 	cudaFree( ds );
-	cudaFree( ord );
-	return loss / (float)n;
+	return out[P_COUNT] / (float)n;
 }
 
 // Adam training on the GPU: `epochs` passes over the n samples in shuffled
