@@ -499,8 +499,6 @@ struct DWorld
 	int* overflowJoints;
 	int* npBucket; // narrowphase: contact ids by manifold class, NP_CLASSES x contactCap
 	DIslands* isl;  // islands and solver sets (sleeping worlds only, else null)
-	int* islFlag;	// device copies of isl->flag and isl->pos (scan arguments)
-	int* islPos;
 	unsigned long long *islNcKeys, *islNcKeysAlt; // copies of isl->ncKeys, ncKeysAlt (sort arguments)
 	// solver scratch
 	unsigned long long* orderState; // look-back state of the body order

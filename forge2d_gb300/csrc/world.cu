@@ -572,8 +572,6 @@ static void isl_ensure( HostWorld* W )
 	cudaMemcpyAsync( W->islDev, &h, sizeof( DIslands ), cudaMemcpyHostToDevice, W->stream );
 	cudaStreamSynchronize( W->stream );
 	d.isl = W->islDev;
-	d.islFlag = h.flag;
-	d.islPos = h.pos;
 	d.islNcKeys = h.ncKeys;
 	d.islNcKeysAlt = h.ncKeysAlt;
 	W->graphDirty = true;
@@ -612,7 +610,6 @@ static void isl_free( HostWorld* W )
 	}
 	W->islDev = nullptr;
 	W->d.isl = nullptr;
-	W->d.islFlag = W->d.islPos = nullptr;
 	W->d.islNcKeys = W->d.islNcKeysAlt = nullptr;
 	memset( &h, 0, sizeof( h ) );
 }
@@ -2415,7 +2412,12 @@ static bool chain_live( const HostWorld* W, int c, int32_t wg )
 // join the move array (after the finalize moves, as b2BufferMove appends)
 static void destroy_begin( HostWorld* W )
 {
-	flush_uploads( W, false );
+	// (a tree that outgrew its device copy goes up now: queries that may not
+	// allocate are answered after a destroy call)
+	bool grown = false;
+	for ( int t = 0; t < 3; ++t )
+		grown = grown || ( W->treeDirty[t] && W->trees[t].cap > W->d.pt[t].cap );
+	flush_uploads( W, grown );
 	if ( upload_host_moves( W ) )
 		launch_pt_host_moves( W->d, W->s, W->stream );
 	cudaMemsetAsync( &W->d.sc->apiCount, 0, 2 * sizeof( int ), W->stream ); // and apiEndCount
