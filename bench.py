@@ -296,7 +296,7 @@ def run_gpu(args, rank, world):
         alg_bytes.append(solver_bytes(g.counters()))
     g.set_profiling(False)
     phases /= reps
-    # latency floor of the solver: its grid barriers x the measured cost of one
+    # grid barriers of the solver (none: its constraints wait for bodies) and the measured cost of one
     barriers, us_per_barrier = g.solver_latency(2000)
     solve_avg = sum(solve_ms) / len(solve_ms)
     alg = sum(alg_bytes) / len(alg_bytes)
@@ -349,9 +349,9 @@ def run_gpu(args, rank, world):
                                  "floor_ms": barriers * us_per_barrier * 1e-3,
                                  "floor_frac_of_launch": (barriers * us_per_barrier * 1e-3 / solve_avg)
                                  if solve_avg > 0 else None,
-                                 "what": "the solver's stages are separated by grid-wide barriers; the floor is "
-                                         "their count in the last launch times the cost of one barrier measured "
-                                         "by a launch of 2000 bare barriers on the same grid"}},
+                                 "what": "grid-wide barriers the last solver launch passed (0: a constraint waits "
+                                         "for the bodies it reads, not for the device) times the cost of one, "
+                                         "measured by a launch of 2000 bare barriers on the same grid"}},
         "phases_ms": {"broadphase": phases[0], "narrowphase": phases[1], "colouring": phases[2],
                       "solver_setup": phases[3], "solver_kernel": phases[4], "finalize": phases[5],
                       "tree_rebuild_beside": rebuild},

@@ -249,7 +249,7 @@ __global__ void __launch_bounds__( GRAPH_THREADS ) k_color_rounds( DWorld w, con
 	}
 	for ( int at = 0; n > 0 && n <= CR_OPS && round < GRAPH_MAX_ROUNDS; ++round )
 	{
-		// counts rotate: this round's, the next round's, the one being cleared
+		// counts rotate: the current, the next, the one being cleared
 		const unsigned short* in = sm.list[at & 1];
 		unsigned short* out = sm.list[( at & 1 ) ^ 1];
 		int* kept = sm.count + at % 3;
