@@ -48,9 +48,9 @@ struct SortDecode
 
 // One block's sort of up to BSORT_MAX rows. Bound by its chain of passes, not
 // by memory (98 KB of keys at most): LSD radix, the rows in registers,
-// BSORT_ITEMS a thread, exchanged through shared memory. A pass costs some 3 us
-// at 12k rows where the cooperative one costs 10 us in grid barriers and L2
-// round trips. The limit is what shared memory holds of 64-bit keys.
+// BSORT_ITEMS a thread, exchanged through shared memory. The cooperative
+// sort's passes pay two grid barriers and several L2 round trips each (100k
+// pile's pair sort at its dense frames, caches cold: 48 -> 38 us). The limit is what shared memory holds of 64-bit keys.
 #define BSORT_ITEMS 12
 #define BSORT_MAX ( BSORT_ITEMS * CSORT_THREADS )
 

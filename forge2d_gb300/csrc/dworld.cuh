@@ -91,7 +91,8 @@
 // Tiles of the one-launch compactions, an item per thread: the work behind an
 // item (a walk up a tree, an op's dependent reads) wants as many threads as
 // there are items. With 4 items a thread the moves of 100k bodies ran on 25
-// blocks and took 130 us instead of the 52 us of the launches they replace.
+// blocks (finalize phase 199 us; 82 with one item, 120 with the launches they
+// replace).
 #define LOOKBACK_TILE 512
 #define LOOKBACK_WORDS( cap ) ( 2 + ( cap ) / LOOKBACK_TILE + 1 )
 

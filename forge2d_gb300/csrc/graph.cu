@@ -129,7 +129,8 @@ __global__ void k_op_round( DWorld w, const int* gkind, int* list )
 // Remaining rounds, one block. Bound by the chain of rounds (21 at 100k bodies,
 // some 1500 ops in the first), each a lock, a test and a barrier: through L2 a
 // round took 2.9 us, so once the pending ops fit, their bodies' locks and colour
-// masks move into a hash table in shared memory (60 -> 13 us at 100k bodies).
+// masks move into a hash table in shared memory (88 -> 24 us a launch at the
+// 100k pile's dense frames, caches cold).
 // There an op that applies frees its bodies' locks; an op that does not stays
 // the lowest on the body it holds, so a round needs no reset pass.
 #define CR_OPS 3072	  // twice as many bodies at most: 0.75 of the table

@@ -798,6 +798,9 @@ struct PtSmall
 	int levelStart[PT_SMALL_LEVELS + 1];
 	int count[2];
 	int kidCount;
+	int tailCount; // nodes of the tails, from kid's end down
+	int tails;
+	int4 tail[PT_SMALL / 2]; // an item of at most PT_SERIAL nodes, then (first of its kids, their count)
 	union
 	{
 		struct // the median-split levels
@@ -834,9 +837,11 @@ __device__ __forceinline__ void pt_refresh_node( const DProxyTree& T, int p, int
 // centre of [s + below, e) that is, counted from the end), the same pairs as
 // the warp form. Returns the split (nodes on the left).
 // A segment's levels are short chains and its blocks are few (some 60 at 25k
-// bodies): a thread takes items of up to 8 nodes, a warp each larger one, 32
-// warps a block. With 8 warps and threads for up to 32 nodes the rebuild took
-// 158 us at 25k bodies instead of 147, 120 us at 6k instead of 105.
+// bodies): a warp takes each item of more than 8 nodes, 32 warps a block, and
+// what is left of the segment then, the tails of up to 8 nodes, a thread each
+// in one go instead of in four or five more levels. Rebuild, levels down to two
+// nodes on 8 warps, then 32 warps, then with tails: 62k bodies in stacks and
+// chains 176, 165, 148 us; 512 batched worlds 206, 199, 188; 6k bodies 120, 105, 98.
 #define PT_SERIAL 8
 __device__ __forceinline__ int pt_partition_serial( int* idx, float2* cen, int s, int e )
 {
@@ -916,12 +921,37 @@ __global__ void __launch_bounds__( PT_SMALL_THREADS ) k_pt_small( DWorld w, int 
 		}
 		if ( threadIdx.x == 0 )
 		{
-			sItem[0][0] = make_int4( 0, n, z, 0 );
-			sCount[0] = 1;
+			const bool tail = n <= PT_SERIAL;
+			( tail ? sm.tail[0] : sItem[0][0] ) = make_int4( 0, n, z, 0 );
+			sCount[0] = tail ? 0 : 1;
 			sCount[1] = 0;
 			sm.kidCount = 0;
+			sm.tailCount = 0;
+			sm.tails = tail ? 1 : 0;
 		}
 		__syncthreads();
+		// the node over [s, e) split at le: its links, and its children by local
+		// slot (a gathered node by its position, a new internal node by PT_SMALL +
+		// its freed position) as kid `k`
+		auto link = [&]( int s, int le, int e, int c1, int k ) {
+			int kn = s + c1 - z, kl = s + c1 + 1 - z, kr = le + c1 - z;
+			if ( kn < 0 || kn >= n - 1 || ( le - s > 1 && ( kl < 0 || kl >= n - 1 ) ) ||
+				 ( e - le > 1 && ( kr < 0 || kr >= n - 1 ) ) || le <= s || le >= e )
+			{
+				atomicOr( &sc->error, ERR_TREE );
+				sm.kid[k] = make_int4( 0, 0, 0, 0 );
+				return false;
+			}
+			int node = sFreed[kn];
+			int left = le - s == 1 ? sIdx[s] : sFreed[kl];
+			int right = e - le == 1 ? sIdx[le] : sFreed[kr];
+			T.child1[node] = left;
+			T.child2[node] = right;
+			T.parent[left] = node;
+			T.parent[right] = node;
+			sm.kid[k] = make_int4( kn, le - s == 1 ? s : PT_SMALL + kl, e - le == 1 ? le : PT_SMALL + kr, 0 );
+			return true;
+		};
 		int levels = 0;
 		for ( int level = 0; level < PT_SMALL_LEVELS; ++level )
 		{
@@ -932,20 +962,11 @@ __global__ void __launch_bounds__( PT_SMALL_THREADS ) k_pt_small( DWorld w, int 
 			if ( threadIdx.x == 0 )
 				sm.levelStart[level] = sm.kidCount;
 			levels = level + 1;
-			// items of at most PT_SERIAL nodes: a thread each
-			for ( int it = threadIdx.x; it < m; it += blockDim.x )
-			{
-				int4 item = sItem[cur][it];
-				if ( item.y - item.x <= PT_SERIAL )
-					sSplit[it] = pt_partition_serial( sIdx, sCen, item.x, item.y );
-			}
-			// larger items: a warp each
+			// a warp each
 			for ( int it = wid; it < m; it += ( PT_SMALL_THREADS / 32 ) )
 			{
 				int4 item = sItem[cur][it];
 				int s = item.x, e = item.y, cnt = e - s;
-				if ( cnt <= PT_SERIAL )
-					continue;
 				int split = 1;
 				{
 					float lx = FLT_MAX, ly = FLT_MAX, hx = -FLT_MAX, hy = -FLT_MAX;
@@ -1026,28 +1047,16 @@ __global__ void __launch_bounds__( PT_SMALL_THREADS ) k_pt_small( DWorld w, int 
 				int4 item = sItem[cur][it];
 				int s = item.x, e = item.y, c1 = item.z;
 				int le = s + sSplit[it];
-				int kn = s + c1 - z, kl = s + c1 + 1 - z, kr = le + c1 - z;
-				if ( kn < 0 || kn >= n - 1 || ( le - s > 1 && ( kl < 0 || kl >= n - 1 ) ) ||
-					 ( e - le > 1 && ( kr < 0 || kr >= n - 1 ) ) || le <= s || le >= e )
-				{
-					atomicOr( &sc->error, ERR_TREE );
+				if ( !link( s, le, e, c1, atomicAdd( &sm.kidCount, 1 ) ) )
 					continue;
-				}
-				int node = sFreed[kn];
-				int left = le - s == 1 ? sIdx[s] : sFreed[kl];
-				int right = e - le == 1 ? sIdx[le] : sFreed[kr];
-				T.child1[node] = left;
-				T.child2[node] = right;
-				T.parent[left] = node;
-				T.parent[right] = node;
-				// children by local slot: a gathered node by its position,
-				// a new internal node by PT_SMALL + its freed position
-				sm.kid[atomicAdd( &sm.kidCount, 1 )] =
-					make_int4( kn, le - s == 1 ? s : PT_SMALL + kl, e - le == 1 ? le : PT_SMALL + kr, 0 );
-				if ( le - s >= 2 )
-					sItem[cur ^ 1][atomicAdd( &sCount[cur ^ 1], 1 )] = make_int4( s, le, c1 + 1, 0 );
-				if ( e - le >= 2 )
-					sItem[cur ^ 1][atomicAdd( &sCount[cur ^ 1], 1 )] = make_int4( le, e, c1, 0 );
+				auto queue = [&]( int from, int to, int c ) {
+					if ( to - from > PT_SERIAL )
+						sItem[cur ^ 1][atomicAdd( &sCount[cur ^ 1], 1 )] = make_int4( from, to, c, 0 );
+					else if ( to - from >= 2 )
+						sm.tail[atomicAdd( &sm.tails, 1 )] = make_int4( from, to, c, 0 );
+				};
+				queue( s, le, c1 + 1 );
+				queue( le, e, c1 );
 			}
 			__syncthreads();
 			if ( threadIdx.x == 0 )
@@ -1056,6 +1065,27 @@ __global__ void __launch_bounds__( PT_SMALL_THREADS ) k_pt_small( DWorld w, int 
 		}
 		if ( threadIdx.x == 0 )
 			sm.levelStart[levels] = sm.kidCount;
+		// the tails, a thread each down to their single nodes
+		for ( int q2 = threadIdx.x; q2 < sm.tails; q2 += blockDim.x )
+		{
+			const int4 item = sm.tail[q2];
+			const int nodes = item.y - item.x - 1, first = atomicAdd( &sm.tailCount, nodes );
+			int3 open[PT_SERIAL];
+			int depth = 1, made = 0;
+			open[0] = make_int3( item.x, item.y, item.z );
+			while ( depth > 0 && made < nodes )
+			{
+				const int3 o = open[--depth];
+				const int le = o.x + pt_partition_serial( sIdx, sCen, o.x, o.y );
+				if ( !link( o.x, le, o.y, o.z, PT_SMALL - 1 - ( first + made++ ) ) )
+					break;
+				if ( le - o.x >= 2 )
+					open[depth++] = make_int3( o.x, le, o.z + 1 );
+				if ( o.y - le >= 2 )
+					open[depth++] = make_int3( le, o.y, o.z );
+			}
+			sm.tail[q2] = make_int4( first, made, 0, 0 );
+		}
 		__syncthreads();
 		// boxes, heights, categories and leaf counts bottom up, a level at a
 		// time in shared memory (dynamic_tree.c:1990-2010), each new node
@@ -1068,27 +1098,32 @@ __global__ void __launch_bounds__( PT_SMALL_THREADS ) k_pt_small( DWorld w, int 
 			sm.u.r.hl[i] = make_int2( T.height[g], T.leaves[g] );
 		}
 		__syncthreads();
+		auto raise = [&]( int k ) {
+			int4 kd = sm.kid[k];
+			float4 bx = pt_union( sm.u.r.box[kd.y], sm.u.r.box[kd.z] );
+			unsigned long long ct = sm.u.r.cat[kd.y] | sm.u.r.cat[kd.z];
+			int2 ha = sm.u.r.hl[kd.y], hb = sm.u.r.hl[kd.z];
+			int2 hl = make_int2( 1 + max( ha.x, hb.x ), ha.y + hb.y );
+			int slot = PT_SMALL + kd.x;
+			sm.u.r.box[slot] = bx;
+			sm.u.r.cat[slot] = ct;
+			sm.u.r.hl[slot] = hl;
+			int node = sFreed[kd.x];
+			T.box[node] = bx;
+			T.cat[node] = ct;
+			T.height[node] = hl.x;
+			T.leaves[node] = hl.y;
+			T.flags[node] = PT_ALLOCATED;
+		};
+		for ( int q2 = threadIdx.x; q2 < sm.tails; q2 += blockDim.x )
+			for ( int k = sm.tail[q2].y - 1; k >= 0; --k )
+				raise( PT_SMALL - 1 - ( sm.tail[q2].x + k ) );
+		__syncthreads();
 		for ( int level = levels - 1; level >= 0; --level )
 		{
 			int k0 = sm.levelStart[level], k1 = sm.levelStart[level + 1];
 			for ( int k = k0 + threadIdx.x; k < k1; k += blockDim.x )
-			{
-				int4 kd = sm.kid[k];
-				float4 bx = pt_union( sm.u.r.box[kd.y], sm.u.r.box[kd.z] );
-				unsigned long long ct = sm.u.r.cat[kd.y] | sm.u.r.cat[kd.z];
-				int2 ha = sm.u.r.hl[kd.y], hb = sm.u.r.hl[kd.z];
-				int2 hl = make_int2( 1 + max( ha.x, hb.x ), ha.y + hb.y );
-				int slot = PT_SMALL + kd.x;
-				sm.u.r.box[slot] = bx;
-				sm.u.r.cat[slot] = ct;
-				sm.u.r.hl[slot] = hl;
-				int node = sFreed[kd.x];
-				T.box[node] = bx;
-				T.cat[node] = ct;
-				T.height[node] = hl.x;
-				T.leaves[node] = hl.y;
-				T.flags[node] = PT_ALLOCATED;
-			}
+				raise( k );
 			__syncthreads();
 		}
 	}
