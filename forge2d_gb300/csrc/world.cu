@@ -1374,7 +1374,10 @@ static void free_world( HostWorld* W )
 	F( shapeMove ); F( moveShape ); F( hostMoves ); F( newPairId ); F( cstamp ); F( awakeOrder ); F( apiEndEv );
 #undef F
 	for ( int t = 0; t < 3; ++t )
+	{
 		pt_free( d.pt[t] );
+		W->trees[t] = HTree(); // its page-locked arrays go with the world
+	}
 	rb_free( d.rb );
 	dfree( W->s.tmpA );
 	dfree( W->s.tmpB );
