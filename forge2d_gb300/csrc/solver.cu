@@ -354,7 +354,8 @@ __global__ void __launch_bounds__( 256 ) k_solver_prepare( DWorld w, SolveParams
 		w.ovfItems[sOverflow[pl.x] + pl.y] = e;
 		int2 bd = w.jbody[j];
 		flow_note( w, dynamic_index( w, bd.x ), F2D_OVERFLOW, e, 0, false );
-		flow_note( w, dynamic_index( w, bd.y ), F2D_OVERFLOW, e, 1, false );
+		if ( bd.y != bd.x ) // a body counts a joint at both its ends once
+			flow_note( w, dynamic_index( w, bd.y ), F2D_OVERFLOW, e, 1, false );
 	}
 	float warmStartScale = p.enableWarmStarting ? 1.0f : 0.0f;
 	const int nc = w.sc->contactIdCount;
@@ -623,7 +624,9 @@ struct Rows
 
 // The two bodies of a joint or overflow contact, in registers: what their
 // functions load and store. Static bodies (index < 0) read as the identity
-// state and are never written (contact_solver.c:1184-1222).
+// state and are never written (contact_solver.c:1184-1222). A joint may hold
+// one body at both ends: what is stored for either end is then that body's
+// state, the later store staying, as where the bodies are stored by index.
 struct PairBodies
 {
 	int ia, ib;
@@ -645,7 +648,13 @@ struct PairBodies
 	{
 		if ( i < 0 )
 			return;
-		BState& t = i == ia ? a : b;
+		if ( i == ia )
+			put( a, s );
+		if ( i == ib )
+			put( b, s );
+	}
+	static __device__ __forceinline__ void put( BState& t, const BState& s )
+	{
 		t.vx = s.vx;
 		t.vy = s.vy;
 		t.w = s.w;
@@ -899,18 +908,21 @@ __device__ __forceinline__ void flow_states( const FlowPair& q, const FlowSeen& 
 }
 
 // The velocity rows back with their counts one higher; after a body's last
-// solve of a substep, its new delta.
+// solve of a substep, its new delta. One body at both ends has one row, written
+// once: the body's next constraint may have passed on from it by a second
+// write.
 __device__ __forceinline__ void flow_publish( const DWorld& w, const SolveParams& p, const Rows& rows, const FlowPair& q,
 											  const PairBodies& ba, int wantA, int wantB, int sub, bool solve )
 {
-	if ( q.ia >= 0 )
+	const bool one = q.ia == q.ib;
+	if ( q.ia >= 0 && !one )
 		rows.put_vel( q.ia, q.slotA, make_float4( ba.a.vx, ba.a.vy, ba.a.w, __int_as_float( wantA + 1 ) ) );
 	if ( q.ib >= 0 )
 		rows.put_vel( q.ib, q.slotB, make_float4( ba.b.vx, ba.b.vy, ba.b.w, __int_as_float( wantB + 1 ) ) );
 	if ( solve )
 	{
 		const bool last = sub == p.subSteps - 1;
-		if ( q.ia >= 0 && q.rankA == q.degA - 1 )
+		if ( q.ia >= 0 && !one && q.rankA == q.degA - 1 )
 			rows.put_delta( sub + 1, last, q.ia, q.slotA, integrate_position( w, p, q.ia, ba.a ) );
 		if ( q.ib >= 0 && q.rankB == q.degB - 1 )
 			rows.put_delta( sub + 1, last, q.ib, q.slotB, integrate_position( w, p, q.ib, ba.b ) );
