@@ -1222,11 +1222,14 @@ __device__ void split_row( const DWorld& w, DIslands& I, int baseId, int b, int 
 					other = edge == 0 ? jb.y : jb.x;
 					use = I.jMark[id] == 0 && I.bSet[other] != SET_DISABLED;
 				}
-				if ( !use )
+				// a joint of the body to itself stands in its list twice, one edge after
+				// the other: it is listed with this body and pushes nothing
+				const bool self = other == b;
+				if ( !use || ( self && edge == 0 ) )
 					continue;
-				const bool inside = I.bIsland[other] == baseId;
+				const bool inside = !self && I.bIsland[other] == baseId;
 				// an unmarked body of another island: left to the serial form
-				if ( !inside && ( list == 0 ? I.bSet[other] != SET_STATIC : I.bSet[other] == SET_AWAKE ) )
+				if ( !inside && !self && ( list == 0 ? I.bSet[other] != SET_STATIC : I.bSet[other] == SET_AWAKE ) )
 					I.splitSerial = 1;
 				const int to = inside ? I.splitIndex[other] : SPLIT_OUTSIDE;
 				if ( pass == 0 )
