@@ -518,6 +518,7 @@ struct DWorld
 	// constraints per part and colour, and per part overflow constraints (one
 	// block of memory), and their starts
 	int *binContacts, *binJoints, *binOverflow;
+	int* flowLong; // (of the same block) a body or part has many overflow constraints
 	int *binContactStart, *binJointStart, *binOverflowStart;
 	int* pendingJointOps; // joint ids whose colour must be assigned at next step
 	int pendingJointCount;

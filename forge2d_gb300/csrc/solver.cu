@@ -34,6 +34,12 @@ struct SolveParams
 };
 
 #define FLOW_SENTINEL 0xffffffffu
+// Overflow constraints of one body whose ranks are found by walking its list,
+// and of one part that are ordered by counting, at most: both are quadratic,
+// but their threads run together. Longer ones are ranked in one pass over all
+// overflow constraints (flow_rank_long).
+#define FLOW_WALK 256
+#define FLOW_SORT 1024
 #define FLOW_SPIN_LIMIT ( 1 << 20 )
 #define FLOW_REST_SHIFT 11		  // bodyOrd.x: colour bits, then the bits of colours with restitution,
 #define FLOW_GLOBAL ( 1 << 22 )	  // and whether the body's row is shared between blocks
@@ -177,6 +183,20 @@ __device__ __forceinline__ int dynamic_index( const DWorld& w, int b )
 	return body_type( w.bflags[b] ) == 0 ? -1 : b;
 }
 
+// Counts an overflow constraint on its bodies (a body at both its ends once)
+// and returns its place in its part.
+__device__ __forceinline__ int overflow_place( const DWorld& w, int part, int a, int b )
+{
+	if ( a >= 0 && atomicAdd( (int*)( w.bodyOrd + a ) + 1, 1 ) == FLOW_WALK )
+		*w.flowLong = 1;
+	if ( b >= 0 && b != a && atomicAdd( (int*)( w.bodyOrd + b ) + 1, 1 ) == FLOW_WALK )
+		*w.flowLong = 1;
+	int at = atomicAdd( w.binOverflow + part, 1 );
+	if ( at == FLOW_SORT )
+		*w.flowLong = 1;
+	return at;
+}
+
 // Counts the constraints per part and colour and gives each its place there;
 // per body, the factors of a substep's velocity integration (solver.c:65-130;
 // they are the same in every substep).
@@ -191,14 +211,15 @@ __global__ void k_solver_count( DWorld w, SolveParams p )
 		if ( col < 0 || ( w.cflags[c] & CF_USED ) == 0 )
 			continue;
 		int2 bd = w.cbody[c];
-		int part = constraint_part( w, p, chunk, dynamic_index( w, bd.x ), dynamic_index( w, bd.y ) );
+		const int ia = dynamic_index( w, bd.x ), ib = dynamic_index( w, bd.y );
+		int part = constraint_part( w, p, chunk, ia, ib );
 		if ( col < F2D_OVERFLOW )
 		{
 			int bin = part * F2D_OVERFLOW + col;
 			w.slotPlace[c] = make_int2( bin, atomicAdd( w.binContacts + bin, 1 ) );
 		}
 		else
-			w.slotPlace[c] = make_int2( part, atomicAdd( w.binOverflow + part, 1 ) );
+			w.slotPlace[c] = make_int2( part, overflow_place( w, part, ia, ib ) );
 	}
 	for ( int j = tid; j < w.jointCount; j += stride )
 	{
@@ -206,14 +227,15 @@ __global__ void k_solver_count( DWorld w, SolveParams p )
 		if ( ( w.jflags[j] & JF_USED ) == 0 || col < 0 )
 			continue;
 		int2 bd = w.jbody[j];
-		int part = constraint_part( w, p, chunk, dynamic_index( w, bd.x ), dynamic_index( w, bd.y ) );
+		const int ia = dynamic_index( w, bd.x ), ib = dynamic_index( w, bd.y );
+		int part = constraint_part( w, p, chunk, ia, ib );
 		if ( col < F2D_OVERFLOW )
 		{
 			int bin = part * F2D_OVERFLOW + col;
 			w.jointPlace[j] = make_int2( bin, atomicAdd( w.binJoints + bin, 1 ) );
 		}
 		else
-			w.jointPlace[j] = make_int2( part, atomicAdd( w.binOverflow + part, 1 ) );
+			w.jointPlace[j] = make_int2( part, overflow_place( w, part, ia, ib ) );
 	}
 	for ( int b = tid; b < w.bodyCount; b += stride )
 	{
@@ -279,11 +301,99 @@ __device__ __forceinline__ void flow_note( const DWorld& w, int b, int colour, i
 		atomicOr( o, ( 1 << colour ) | ( restitution ? 1 << ( FLOW_REST_SHIFT + colour ) : 0 ) );
 		return;
 	}
-	atomicAdd( o + 1, 1 );
 	if ( restitution )
 		atomicAdd( o + 2, 1 );
 	// list heads are keys + 1, 0 when empty
 	w.ovfNext[2 * (size_t)e + side] = atomicExch( o + 3, ( ( e << 2 ) | ( restitution ? 2 : 0 ) | side ) + 1 );
+}
+
+// Bodies of overflow constraint e (-1 static), its part, and whether it has
+// restitution.
+__device__ __forceinline__ int4 overflow_constraint( const DWorld& w, int e, int novfJ )
+{
+	if ( e < novfJ )
+	{
+		const int j = w.overflowJoints[e];
+		const int2 bd = w.jbody[j];
+		return make_int4( dynamic_index( w, bd.x ), dynamic_index( w, bd.y ), w.jointPlace[j].x, 0 );
+	}
+	const int c = w.overflowList[e - novfJ];
+	const int2 bd = w.cbody[c];
+	return make_int4( dynamic_index( w, bd.x ), dynamic_index( w, bd.y ), w.slotPlace[c].x, w.cmat[c].y != 0.0f ? 1 : 0 );
+}
+
+// Ranks of overflow constraints on bodies that have more than FLOW_WALK, and
+// the serial order of parts that have more than FLOW_SORT: one warp each over
+// all of them in order (70 ns a constraint, bound by four dependent reads for
+// 16 of them; each of the body's operations that follow, one after another in
+// every stage, takes 0.8 us: 8000 circles on a plank, 0.6 of 76 ms). Walks
+// between the operations made 500 circles 6.3 ms instead of 5.1 and grew with
+// the square. The body's running counts stand in the free words of its bodyInt
+// row.
+__device__ void flow_rank_long( const DWorld& w, int novfJ, int n, int* partAt )
+{
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const unsigned below = ( 1u << lane ) - 1u;
+	if ( warp == 0 )
+		for ( int base = 0; base < n; base += 16 )
+		{
+			const int e = base + ( lane >> 1 ), side = lane & 1;
+			int key = -1 - lane, rest = 0;
+			bool both = false;
+			if ( e < n )
+			{
+				const int4 k = overflow_constraint( w, e, novfJ );
+				const int b = side ? k.y : k.x;
+				both = k.x == k.y;
+				rest = k.w;
+				if ( b >= 0 && !( both && side ) && w.bodyOrd[b].y > FLOW_WALK )
+					key = b;
+			}
+			const unsigned rests = __ballot_sync( 0xffffffffu, rest != 0 );
+			const unsigned peers = __match_any_sync( 0xffffffffu, key );
+			if ( key >= 0 )
+			{
+				int* at = (int*)( w.bodyInt + 2 * (size_t)key + 1 ) + 2;
+				const int all = __ldcg( at ) + __popc( peers & below ), some = __ldcg( at + 1 ) + __popc( peers & rests & below );
+				int* r = (int*)( w.ovfRank + e );
+				r[side] = all;
+				r[2 + side] = some;
+				if ( both )
+				{
+					r[1] = all;
+					r[3] = some;
+				}
+				__syncwarp( peers );
+				if ( ( peers & ~below ) == ( 1u << lane ) ) // the last of them
+				{
+					__stcg( at, all + 1 );
+					__stcg( at + 1, some + rest );
+				}
+			}
+			__syncwarp();
+		}
+	else if ( warp == 1 )
+		for ( int base = 0; base < n; base += 32 )
+		{
+			const int e = base + lane;
+			int part = -1 - lane;
+			if ( e < n )
+			{
+				const int k = overflow_constraint( w, e, novfJ ).z;
+				if ( w.binOverflow[k] > FLOW_SORT )
+					part = k;
+			}
+			const unsigned peers = __match_any_sync( 0xffffffffu, part );
+			if ( part >= 0 )
+			{
+				const int at = partAt[part] + __popc( peers & below );
+				w.ovfSorted[at] = e;
+				__syncwarp( peers );
+				if ( ( peers & ~below ) == ( 1u << lane ) )
+					partAt[part] = at + 1;
+			}
+			__syncwarp();
+		}
 }
 
 // Constraint rows of every contact in the graph (contact_solver.c:1438-1669
@@ -354,7 +464,7 @@ __global__ void __launch_bounds__( 256 ) k_solver_prepare( DWorld w, SolveParams
 		w.ovfItems[sOverflow[pl.x] + pl.y] = e;
 		int2 bd = w.jbody[j];
 		flow_note( w, dynamic_index( w, bd.x ), F2D_OVERFLOW, e, 0, false );
-		if ( bd.y != bd.x ) // a body counts a joint at both its ends once
+		if ( bd.y != bd.x ) // a body lists a joint at both its ends once
 			flow_note( w, dynamic_index( w, bd.y ), F2D_OVERFLOW, e, 1, false );
 	}
 	float warmStartScale = p.enableWarmStarting ? 1.0f : 0.0f;
@@ -484,6 +594,12 @@ __global__ void __launch_bounds__( 256 ) k_solver_prepare( DWorld w, SolveParams
 		row[32 * KR_P2] = pp[1];
 		row[32 * KR_IMP] = make_float4( ni[0], ni[1], ti[0], ti[1] );
 		row[32 * KR_TOT] = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
+	}
+	// a body or a part with many overflow constraints (counted by the launch before)
+	if ( blockIdx.x == gridDim.x - 1 && *w.flowLong )
+	{
+		__syncthreads();
+		flow_rank_long( w, novfJ, novf + novfJ, sOverflow );
 	}
 }
 
@@ -732,6 +848,61 @@ struct FlowPart
 	unsigned char kind[FLOW_LIST];
 };
 
+// Rank of overflow constraint e on body b among the body's overflow
+// constraints, from the body's (unordered) list; .y among those with
+// restitution. False when the list is long: its ranks are there already.
+__device__ __forceinline__ bool overflow_rank( const DWorld& w, int e, int b, int2& r )
+{
+	r = make_int2( 0, 0 );
+	if ( b < 0 )
+		return true;
+	const int4 ord = w.bodyOrd[b];
+	if ( ord.y > FLOW_WALK )
+		return false;
+	int key = ord.w - 1;
+	for ( int guard = 0; key >= 0 && guard < ord.y; ++guard )
+	{
+		if ( ( key >> 2 ) < e )
+		{
+			r.x += 1;
+			r.y += ( key >> 1 ) & 1;
+		}
+		key = w.ovfNext[2 * (size_t)( key >> 2 ) + ( key & 1 )] - 1;
+	}
+	return true;
+}
+
+// Ranks of overflow constraint e on both its bodies.
+__device__ __forceinline__ void overflow_ranks( const DWorld& w, int e )
+{
+	const int novfJ = w.sc->overflowJointCount;
+	int* r = (int*)( w.ovfRank + e );
+	int2 bd;
+	if ( e < novfJ )
+		bd = w.jindex[w.overflowJoints[e]];
+	else
+	{
+		float4 h = *krow( w, e - novfJ, KR_HEAD );
+		bd = make_int2( __float_as_int( h.x ), __float_as_int( h.y ) );
+	}
+	for ( int side = 0; side < 2; ++side )
+	{
+		int2 k;
+		if ( overflow_rank( w, e, side ? bd.y : bd.x, k ) )
+		{
+			r[side] = k.x;
+			r[2 + side] = k.y;
+		}
+	}
+}
+
+// Lanes of a block for `n` overflow constraints: a quarter of the warps at
+// most, whose chains would hold up the colour groups of a warp that had both.
+__device__ __forceinline__ int overflow_lanes( int threads, int n )
+{
+	return 32 * min( threads / 128, n );
+}
+
 __device__ __forceinline__ void flow_part( const DWorld& w, const SolveParams& p, int part, FlowPart& f )
 {
 	const int novf = w.sc->overflowCount + w.sc->overflowJointCount;
@@ -759,13 +930,19 @@ __device__ __forceinline__ void flow_part( const DWorld& w, const SolveParams& p
 		f.groupStart[FLOW_KINDS] = at;
 	}
 	// overflow constraints in their serial order: each counts the smaller ones
-	for ( int i = threadIdx.x; i < f.overflow; i += blockDim.x )
-	{
-		int e = w.ovfItems[f.overflowFirst + i], rank = 0;
-		for ( int j = 0; j < f.overflow; ++j )
-			rank += w.ovfItems[f.overflowFirst + j] < e ? 1 : 0;
-		w.ovfSorted[f.overflowFirst + rank] = e;
-	}
+	if ( f.overflow <= FLOW_SORT )
+		for ( int i = threadIdx.x; i < f.overflow; i += blockDim.x )
+		{
+			int e = w.ovfItems[f.overflowFirst + i], rank = 0;
+			for ( int j = 0; j < f.overflow; ++j )
+				rank += w.ovfItems[f.overflowFirst + j] < e ? 1 : 0;
+			w.ovfSorted[f.overflowFirst + rank] = e;
+		}
+	// more than a lane each: their ranks before any of them starts, as a walk
+	// between two operations would hold up the lanes beside it
+	if ( f.overflow > overflow_lanes( blockDim.x, f.overflow ) )
+		for ( int i = threadIdx.x; i < f.overflow; i += blockDim.x )
+			overflow_ranks( w, w.ovfItems[f.overflowFirst + i] );
 	__syncthreads();
 	for ( int g = threadIdx.x; g < min( f.groupStart[FLOW_KINDS], FLOW_LIST ); g += blockDim.x )
 	{
@@ -775,27 +952,6 @@ __device__ __forceinline__ void flow_part( const DWorld& w, const SolveParams& p
 		f.kind[g] = (unsigned char)k;
 	}
 	__syncthreads();
-}
-
-// Rank of overflow constraint e on body b among the body's overflow
-// constraints, from the body's (unordered) list; .y among those with
-// restitution.
-__device__ __forceinline__ int2 overflow_rank( const DWorld& w, int e, int b, int limit )
-{
-	int2 r = make_int2( 0, 0 );
-	if ( b < 0 )
-		return r;
-	int key = w.bodyOrd[b].w - 1;
-	for ( int guard = 0; key >= 0 && guard < limit; ++guard )
-	{
-		if ( ( key >> 2 ) < e )
-		{
-			r.x += 1;
-			r.y += ( key >> 1 ) & 1;
-		}
-		key = w.ovfNext[2 * (size_t)( key >> 2 ) + ( key & 1 )] - 1;
-	}
-	return r;
 }
 
 // A constraint's view of one body: KR_REF packs the bodies (x, y), their
@@ -1114,7 +1270,7 @@ __device__ __forceinline__ void solve_overflows( const DWorld& w, const SolvePar
 												 const FlowPart& f, int firstPos, int slots, int first, int stride )
 {
 	const int stages = 3 * p.subSteps;
-	const int novfJ = w.sc->overflowJointCount, limit = 2 * ( novfJ + w.sc->overflowCount );
+	const int novfJ = w.sc->overflowJointCount;
 	const bool single = first + stride >= f.overflow;
 	Lane L;
 	float4* row = nullptr;
@@ -1124,6 +1280,8 @@ __device__ __forceinline__ void solve_overflows( const DWorld& w, const SolvePar
 	s.dA = s.dB = make_float4( 0.0f, 0.0f, 1.0f, 0.0f );
 	int i = first, stage = 0;
 	bool act = i < f.overflow, fresh = true;
+	if ( act && f.overflow <= stride )
+		overflow_ranks( w, w.ovfSorted[f.overflowFirst + i] );
 	for ( int spins = 0;; )
 	{
 		const bool rest = stage == stages;
@@ -1161,11 +1319,6 @@ __device__ __forceinline__ void solve_overflows( const DWorld& w, const SolvePar
 				q.slotB = q.ib >= 0 ? body_slot( w, ob, q.ib, firstPos, slots ) : FLOW_NO_SLOT;
 				q.degA = oa.y + __popc( oa.x & FLOW_COLOURS );
 				q.degB = ob.y + __popc( ob.x & FLOW_COLOURS );
-				if ( stage == 0 )
-				{
-					int2 ra = overflow_rank( w, e, q.ia, limit ), rb = overflow_rank( w, e, q.ib, limit );
-					w.ovfRank[e] = make_int4( ra.x, rb.x, ra.y, rb.y );
-				}
 				int4 o = w.ovfRank[e];
 				q.rankA = rest ? o.z : o.x;
 				q.rankB = rest ? o.w : o.y;
@@ -1300,9 +1453,7 @@ __global__ void __launch_bounds__( THREADS ) k_solve( DWorld w, SolveParams p )
 	const Rows rows = { (unsigned)__cvta_generic_to_shared( sbody ), 16u * (unsigned)p.slots, w.vel, w.delta, w.dsub,
 						(size_t)w.bodyCount };
 	const int warp = threadIdx.x >> 5, warps = THREADS / 32;
-	// a quarter of the warps at most is kept for the overflow constraints,
-	// whose chains would hold up the colour groups of a warp that had both
-	const int ovfWarps = min( warps / 4, f.overflow );
+	const int ovfWarps = overflow_lanes( THREADS, f.overflow ) / 32;
 	if ( warp < warps - ovfWarps )
 		solve_colours( w, p, rows, f, firstPos, mine, warp, warps - ovfWarps );
 	else
@@ -1400,8 +1551,8 @@ __global__ void k_order_clear( DWorld w, int tiles, int subSteps )
 	const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
 	for ( int i = tid; i < tiles + 2; i += stride )
 		w.orderState[i] = 0ull;
-	for ( int i = tid; i < SOLVER_MAX_PARTS * ( 2 * F2D_OVERFLOW + 1 ); i += stride )
-		w.binContacts[i] = 0;
+	for ( int i = tid; i < SOLVER_MAX_PARTS * ( 2 * F2D_OVERFLOW + 1 ) + 1; i += stride )
+		w.binContacts[i] = 0; // and flowLong
 	for ( int i = tid; i < w.bodyCount; i += stride )
 	{
 		w.bodyPos[i] = -1;

@@ -302,9 +302,10 @@ static void alloc_scratch( HostWorld* W )
 	// counts and starts per part: contacts, joints, overflow
 	size_t bins = (size_t)SOLVER_MAX_PARTS * F2D_OVERFLOW;
 	dfree( d.binContacts );
-	dgrow( d.binContacts, 0, 2 * bins + SOLVER_MAX_PARTS );
+	dgrow( d.binContacts, 0, 2 * bins + SOLVER_MAX_PARTS + 1 );
 	d.binJoints = d.binContacts + bins;
 	d.binOverflow = d.binJoints + bins;
+	d.flowLong = d.binOverflow + SOLVER_MAX_PARTS;
 	dfree( d.binContactStart );
 	dgrow( d.binContactStart, 0, 2 * bins + SOLVER_MAX_PARTS );
 	d.binJointStart = d.binContactStart + bins;
