@@ -40,7 +40,12 @@ struct SolveParams
 // overflow constraints (flow_rank_long).
 #define FLOW_WALK 256
 #define FLOW_SORT 1024
-#define FLOW_SPIN_LIMIT ( 1 << 20 )
+// Polls without progress before a warp gives up. A warp may rightly wait for a
+// whole stage's chain of one body's overflow constraints (0.8 us each, up to
+// 15 polls), so they count towards it.
+#define FLOW_SPIN_LIMIT ( 1 << 22 )
+#define FLOW_SPIN_OVERFLOW 256
+#define FLOW_OVERFLOW_MOST ( 1 << 21 )
 #define FLOW_REST_SHIFT 11		  // bodyOrd.x: colour bits, then the bits of colours with restitution,
 #define FLOW_GLOBAL ( 1 << 22 )	  // and whether the body's row is shared between blocks
 #define FLOW_COLOURS ( ( 1 << F2D_OVERFLOW ) - 1 )
@@ -649,7 +654,7 @@ __global__ void k_solver_refill( DWorld w, int subSteps )
 // that precede it in that order, and all blocks are resident, so the first
 // unfinished group of that order is always at the head of its warp and its
 // wait ends. Polls are counted all the same: a warp that makes no progress
-// for FLOW_SPIN_LIMIT polls raises the timeout bit and leaves, as do the
+// for flow_spin_limit polls raises the timeout bit and leaves, as do the
 // others when they see the bit.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float4 unpack_row( unsigned long long lo, unsigned long long hi )
@@ -1085,13 +1090,18 @@ __device__ __forceinline__ void flow_publish( const DWorld& w, const SolveParams
 	}
 }
 
+__device__ __forceinline__ int flow_spin_limit( const DWorld& w )
+{
+	return FLOW_SPIN_LIMIT + FLOW_SPIN_OVERFLOW * min( w.sc->overflowCount + w.sc->overflowJointCount, FLOW_OVERFLOW_MOST );
+}
+
 // Counts a poll without progress; true when the wait is to be given up.
 __device__ __forceinline__ bool flow_give_up( const DWorld& w, int& spins )
 {
 	spins += 1;
 	if ( ( spins & 1023 ) != 0 )
 		return false;
-	bool out = spins >= FLOW_SPIN_LIMIT;
+	bool out = spins >= flow_spin_limit( w );
 	if ( out && ( threadIdx.x & 31 ) == 0 )
 		atomicOr( &w.sc->error, F2D_ERR_BARRIER_TIMEOUT );
 	return __any_sync( 0xffffffffu, out || ( ld_relaxed_s32( &w.sc->error ) & F2D_ERR_BARRIER_TIMEOUT ) );

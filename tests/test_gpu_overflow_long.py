@@ -92,3 +92,30 @@ def test_racks_beside_each_other(gpu_lib):
         shelves(b, 300, head="middle", per=60)
         spokes(b, 300)
     _compare(gpu_lib, build, 4, 3)
+
+
+def test_a_wait_as_long_as_the_chain(gpu_lib):
+    """Circles that touch each other wait in their colours for the whole chain
+    of a body under 210 thousand of them, some 170 milliseconds in each stage.
+    (They come in seven frames: a body's new contacts are coloured one by one,
+    100 thousand at most.)"""
+    from forge2d_gb300.world import GpuWorld
+    from oracle.oracle import PortWorld
+    wd = scenes.world_def(enableSleep=0, gravityY=-1.0)
+    g, p = GpuWorld(wd), PortWorld(wd)
+    for b in (g, p):
+        rack = b.create_body(scenes.body_def(type=scenes.KINEMATIC))
+        for r in list(range(1, 400)) + [0]:
+            b.create_box(rack, scenes.shape_def(), 158.0, 0.1, 158.0, 2.0 * r, 1.0, 0.0)
+    for frame in range(7):
+        for b in (g, p):
+            for k in range(30_000 * frame, 30_000 * frame + 30_000):
+                c = b.create_body(scenes.body_def(type=scenes.DYNAMIC, positionX=0.26 + 0.52 * (k % 600), positionY=2.0 * (k // 600) + 0.34))
+                b.create_circle(c, scenes.shape_def(), 0.0, 0.0, 0.25)
+            b.step(1.0 / 60.0, 1)
+        assert g.sync() == 0, frame
+    x, y = g.bodies()[:, :9], p.bodies()[:, :9]
+    assert np.array_equal(x.view(np.uint32), y.view(np.uint32)), np.argwhere(x != y)[:4].tolist()
+    assert g.counters()["overflow"] == 210_000 - 11
+    g.close()
+    p.close()
