@@ -1171,7 +1171,7 @@ struct SplitSmem
 
 // The edges of body b a visit can use: touching contacts not marked before,
 // joints not marked before whose other body is not disabled; and the bodies
-// among them that can be pushed, each once.
+// among them that can be pushed.
 __device__ void split_row( const DWorld& w, DIslands& I, int baseId, int b, int idx, int none )
 {
 	int2* row = I.splitRows + (size_t)SPLIT_ROW * idx;
@@ -1246,13 +1246,16 @@ __device__ void split_row( const DWorld& w, DIslands& I, int baseId, int b, int 
 				at += 1;
 				if ( !inside )
 					continue;
-				// a body met twice is pushed at the first meeting: later places stay
-				// empty (an index past every body, marked from the start)
+				// a body met twice is pushed at the first meeting: later places in the
+				// row stay empty (an index past every body, marked from the start); the
+				// rest of a long row keeps them, the traversal finds them there (a
+				// search through all earlier ones grows with the row's square)
 				int slot = to;
 				const int kept = pushes > SPLIT_PUSH ? SPLIT_PUSH - 1 : SPLIT_PUSH;
-				for ( int k = 0; k < pushAt; ++k )
-					if ( ( k < kept ? push[k] : I.splitPushPool[pushPool + 1 + k - kept] ) == to )
-						slot = none;
+				if ( pushAt < kept )
+					for ( int k = 0; k < pushAt; ++k )
+						if ( push[k] == to )
+							slot = none;
 				if ( pushAt < kept )
 					push[pushAt] = slot;
 				else
@@ -1415,7 +1418,9 @@ __device__ void split_traverse( const DWorld& w, DIslands& I, int baseId, int n,
 					{
 						int o = k0 + lane < count ? pushPool[pool + 1 + k0 + lane] : -1;
 						__syncwarp();
-						bool pu = o >= 0 && !marks.get( o );
+						// (a body twice among these: the first of them)
+						const unsigned same = __match_any_sync( full, o );
+						bool pu = o >= 0 && !marks.get( o ) && ( same & lt ) == 0u;
 						unsigned pm = __ballot_sync( full, pu );
 						if ( pu )
 						{
