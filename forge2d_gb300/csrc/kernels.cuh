@@ -107,7 +107,7 @@ void launch_prepare_joints( DWorld& w, cudaStream_t st, float h, Soft jointSoft 
 // the reference's broadphase trees and the move array (proxytree.cu)
 int pt_large_blocks();
 bool color_rounds_setup();
-void launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st );
+int launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st ); // the launches
 void launch_pt_rebuild( DWorld& w, StepScratch& s, cudaStream_t st );
 void launch_pt_moves( DWorld& w, cudaStream_t st );
 void launch_pt_gather( DWorld& w, cudaStream_t st );

@@ -1210,12 +1210,13 @@ int pt_large_blocks()
 }
 
 // step start: the host's buffered proxies join the move array
-void launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st )
+int launch_pt_host_moves( DWorld& w, StepScratch& s, cudaStream_t st )
 {
 	k_pt_host_flags<<<grid_for( w.shapeCap ), 256, 0, st>>>( w, s.tmpA );
 	scan_lookback( s.tmpA, s.tmpB, &w.sc->hostMoveCount, 0, w.shapeCap, nullptr, s.scanState, &w.sc->error, st );
 	k_pt_host_write<<<grid_for( w.shapeCap ), 256, 0, st>>>( w, s.tmpA, s.tmpB );
 	k_pt_host_done<<<1, 1, 0, st>>>( w, s.tmpA, s.tmpB );
+	return 4;
 }
 
 static bool pt_present( const DWorld& w, int t )

@@ -1097,36 +1097,49 @@ static void host_move( HostWorld* W, int s )
 	W->hostMoves.push_back( s );
 }
 
-// The buffered proxies go to the device for the step about to be enqueued; a
-// few join the move array here and now. True when the step's host-move chain
-// has them to place.
-static bool upload_host_moves( HostWorld* W )
+// The proxies buffered since the last step, taken for place_host_moves: a few by
+// value, more by a copy to the device.
+struct HostMoves
 {
-	int n = (int)W->hostMoves.size();
-	if ( n == 0 )
-		return false;
 	FewMoves few;
-	if ( n <= 32 )
+	bool many;
+};
+
+static void take_host_moves( HostWorld* W, HostMoves& m )
+{
+	const int n = (int)W->hostMoves.size();
+	m.few.n = 0;
+	m.many = n > 32;
+	if ( n == 0 )
+		return;
+	if ( m.many )
 	{
-		few.n = n;
-		for ( int k = 0; k < n; ++k )
-		{
-			few.shape[k] = W->hostMoves[k];
-			W->hostMoved[W->hostMoves[k]] = 0;
-		}
-		W->hostMoves.clear();
-		launch_few_moves( W->d, few, W->stream );
-		return false;
+		cudaMemcpyAsync( W->d.hostMoves, W->hostMoves.data(), sizeof( int ) * (size_t)n, cudaMemcpyHostToDevice,
+						 W->stream );
+		W->hostMoveCount = n;
+		cudaMemcpyAsync( &W->d.sc->hostMoveCount, &W->hostMoveCount, sizeof( int ), cudaMemcpyHostToDevice, W->stream );
+		cudaStreamSynchronize( W->stream );
 	}
-	cudaMemcpyAsync( W->d.hostMoves, W->hostMoves.data(), sizeof( int ) * (size_t)n, cudaMemcpyHostToDevice,
-					 W->stream );
-	W->hostMoveCount = n;
-	cudaMemcpyAsync( &W->d.sc->hostMoveCount, &W->hostMoveCount, sizeof( int ), cudaMemcpyHostToDevice, W->stream );
-	cudaStreamSynchronize( W->stream );
+	else
+	{
+		m.few.n = n;
+		for ( int k = 0; k < n; ++k )
+			m.few.shape[k] = W->hostMoves[k];
+	}
 	for ( int sh : W->hostMoves )
 		W->hostMoved[sh] = 0;
 	W->hostMoves.clear();
-	return true;
+}
+
+// They join the move array in their order. Returns the launches.
+static int place_host_moves( HostWorld* W, const HostMoves& m )
+{
+	if ( m.many )
+		return launch_pt_host_moves( W->d, W->s, W->stream );
+	if ( m.few.n == 0 )
+		return 0;
+	launch_few_moves( W->d, m.few, W->stream );
+	return 1;
 }
 
 // `trees`: the broadphase trees too (a step and an explosion read them; a run
@@ -2422,8 +2435,9 @@ static void destroy_begin( HostWorld* W )
 	for ( int t = 0; t < 3; ++t )
 		grown = grown || ( W->treeDirty[t] && W->trees[t].cap > W->d.pt[t].cap );
 	flush_uploads( W, grown );
-	if ( upload_host_moves( W ) )
-		launch_pt_host_moves( W->d, W->s, W->stream );
+	HostMoves moves;
+	take_host_moves( W, moves );
+	place_host_moves( W, moves );
 	cudaMemsetAsync( &W->d.sc->apiCount, 0, 2 * sizeof( int ), W->stream ); // and apiEndCount
 }
 
@@ -4013,7 +4027,8 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 	if ( W->stepped && cudaEventQuery( W->evStop ) == cudaSuccess )
 		W->statusAccum |= *W->hostError;
 	flush_uploads( W );
-	const bool hostMoves = upload_host_moves( W );
+	HostMoves moves;
+	take_host_moves( W, moves );
 	int planMode = 0;
 	if ( W->planPending )
 	{
@@ -4031,8 +4046,6 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 	if ( W->d.learnMode != 0 )
 		ensure_learning_buffers( W );
 	cudaMemsetAsync( &W->d.sc->error, 0, sizeof( int ), W->stream );
-	if ( hostMoves )
-		launch_pt_host_moves( W->d, W->s, W->stream );
 	const int period = W->orderPeriod > 0 ? W->orderPeriod : ORDER_REBUILD_PERIOD;
 	const bool sorts = W->forceRebuild || W->orderAge >= period - 1;
 	W->orderAge = sorts ? 0 : W->orderAge + 1;
@@ -4042,6 +4055,7 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 		W->forceRebuild = false;
 	}
 	cudaEventRecord( W->evStart, W->stream );
+	const int moveLaunches = place_host_moves( W, moves );
 	if ( W->d.callbacks )
 		cb_ensure( W );
 	bool useGraph = planMode == 0 && !W->profiling && W->d.callbacks == 0;
@@ -4079,6 +4093,7 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 		enqueue_step( W, dt, subSteps, planMode, false );
 		W->lastLaunches = W->graphKernelNodes;
 	}
+	W->lastLaunches += moveLaunches;
 	cudaEventRecord( W->evStop, W->stream );
 	cudaMemcpyAsync( W->hostError, &W->d.sc->error, sizeof( int ), cudaMemcpyDeviceToHost, W->stream );
 	W->stepped = true;
