@@ -4054,8 +4054,6 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 		cudaMemsetAsync( &W->d.sc->forceRebuild, 1, 1, W->stream );
 		W->forceRebuild = false;
 	}
-	cudaEventRecord( W->evStart, W->stream );
-	const int moveLaunches = place_host_moves( W, moves );
 	if ( W->d.callbacks )
 		cb_ensure( W );
 	bool useGraph = planMode == 0 && !W->profiling && W->d.callbacks == 0;
@@ -4078,6 +4076,9 @@ extern "C" F2D_API int32_t f2d_world_step( int32_t worldId, double timeStep, int
 	const bool lean = useGraph && !sorts && W->graphExec != nullptr;
 	if ( lean && W->leanExec == nullptr && ++W->graphSteps == LEAN_AFTER )
 		capture_step( W, dt, subSteps, true, &W->leanExec, &W->leanKernelNodes );
+	// the step's own device time: what the host did for it above is not in it
+	cudaEventRecord( W->evStart, W->stream );
+	const int moveLaunches = place_host_moves( W, moves );
 	if ( lean && W->leanExec )
 	{
 		cudaGraphLaunch( W->leanExec, W->stream );

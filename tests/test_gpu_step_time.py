@@ -1,7 +1,9 @@
 """What a step reports about itself: its launches with those for the proxies
-buffered by edits."""
+buffered by edits, its device time without the host's captures of the step's
+graph."""
 from __future__ import annotations
 
+import numpy as np
 import pytest
 
 from forge2d_gb300 import scenes
@@ -32,3 +34,18 @@ def test_launches_count_the_buffered_proxies(gpu_lib):
     assert counted[33] == counted[0] + 4
     g.close()
 
+
+def test_step_time_holds_no_capture(gpu_lib):
+    """The step is captured at its first step and, without the leaf ordering,
+    some twenty steps later; the host needs several steps' time for each."""
+    worst = []
+    for _ in range(5):
+        g = _world()
+        ms = []
+        for _ in range(40):
+            g.step()
+            assert g.sync() == 0
+            ms.append(g.last_step_ms())
+        worst.append(max(ms[4:]) / np.median(ms))
+        g.close()
+    assert min(worst) < 1.8, worst
