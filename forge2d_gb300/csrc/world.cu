@@ -4123,6 +4123,18 @@ static void apply_tuning( HostWorld* W, int variant, int period )
 	W->graphDirty = true;
 }
 
+// Both forms of the step as it was replayed last, under the present tuning.
+static void capture_forms( HostWorld* W )
+{
+	if ( W->graphExec == nullptr || W->profiling || W->d.callbacks != 0 )
+		return;
+	if ( W->graphDirty )
+		capture_step( W, W->graphDt, W->graphSubSteps, false, &W->graphExec, &W->graphKernelNodes );
+	if ( W->graphDirty || W->leanExec == nullptr )
+		capture_step( W, W->graphDt, W->graphSubSteps, true, &W->leanExec, &W->leanKernelNodes );
+	W->graphDirty = false;
+}
+
 extern "C" F2D_API int32_t f2d_world_autotune( int32_t worldId, double timeStep, int32_t subStepCount,
 											   int32_t stepsPerCandidate, int32_t* chosen3 )
 {
@@ -4147,8 +4159,11 @@ extern "C" F2D_API int32_t f2d_world_autotune( int32_t worldId, double timeStep,
 		{
 			apply_tuning( W, variants[vi], periods[pi] );
 			// the first step re-captures the graph; the leaf order is re-sorted
-			// at least once per period, so a candidate is timed over a period
+			// at least once per period, so a candidate is timed over a period, and
+			// in the forms that a long run replays, the one without the leaf
+			// ordering too
 			status |= f2d_world_step( worldId, timeStep, subStepCount );
+			capture_forms( W );
 			int n = reps > periods[pi] ? reps : periods[pi];
 			taken += 1 + n;
 			double ms = 0.0;
@@ -4166,6 +4181,7 @@ extern "C" F2D_API int32_t f2d_world_autotune( int32_t worldId, double timeStep,
 			}
 		}
 	apply_tuning( W, bestV, bestP );
+	capture_forms( W );
 	if ( chosen3 )
 	{
 		chosen3[0] = bestV;
