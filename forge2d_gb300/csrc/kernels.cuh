@@ -50,9 +50,17 @@ struct StepScratch
 	cudaEvent_t rebuildFork, rebuildJoin, rebuildT0, rebuildT1;
 };
 
+// A world of up to this many bodies with constraints is one part: no body is
+// shared (pyramids of 55, 210, 465 boxes: 66, 76, 104 us as one part; 66, 111,
+// 109 us in parts of 64). Larger worlds take parts of at least SOLVER_MIN_CHUNK = 64 bodies (820
+// boxes: 111 us against 165 us as one part; 2k-6k piles: parts of 64 bodies
+// 138, 139 us, of 256 bodies 150, 152 us).
+#define SOLVER_ONE_PART 400
+#define SOLVER_FEW_MOST 4 // times as many with SOLVER_FEW_PARTS
+
 // solver variants: same arithmetic, different launch shapes
 #define SOLVER_AUTO 0		// one block per SM
-#define SOLVER_FEW_PARTS 1	// the same; worlds of up to four times the size are one part
+#define SOLVER_FEW_PARTS 1	// the same; worlds of up to SOLVER_FEW_MOST times the size are one part
 #define SOLVER_ONE_PER_SM 2 // the same as AUTO
 #define SOLVER_TWO_PER_SM 3 // two blocks of half the threads per SM
 

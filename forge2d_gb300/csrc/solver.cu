@@ -1520,12 +1520,6 @@ float solver_barrier_probe( StepScratch& s, cudaStream_t st, unsigned* counter, 
 // cost registers (spills from 512 on) and issue slots (waiting warps poll);
 // fewer leave too many groups to a warp.
 #define SOLVER_THREADS 384
-// A world of up to this many bodies with constraints is one part: no body is
-// shared (pyramids of 55, 210, 465 boxes: 66, 76, 104 us as one part; 66, 111,
-// 109 us in parts of 64). Larger worlds take parts of at least SOLVER_MIN_CHUNK = 64 bodies (820
-// boxes: 111 us against 165 us as one part; 2k-6k piles: parts of 64 bodies
-// 138, 139 us, of 256 bodies 150, 152 us).
-#define SOLVER_ONE_PART 400
 
 static size_t solver_smem( int slots, int subSteps )
 {
@@ -1606,7 +1600,7 @@ void launch_solver( DWorld& w, StepScratch& s, cudaStream_t st, float dt, int su
 	const bool two = s.solverVariant == SOLVER_TWO_PER_SM && s.solverBlocks2 > 0;
 	p.parts = two ? s.solverBlocks2 : s.solverBlocks;
 	p.minChunk = s.smallParts ? SOLVER_SMALL_CHUNK : SOLVER_MIN_CHUNK;
-	p.onePart = s.smallParts ? 0 : ( s.solverVariant == SOLVER_FEW_PARTS ? 4 * SOLVER_ONE_PART : SOLVER_ONE_PART );
+	p.onePart = s.smallParts ? 0 : ( s.solverVariant == SOLVER_FEW_PARTS ? SOLVER_FEW_MOST * SOLVER_ONE_PART : SOLVER_ONE_PART );
 	int fit = ( two ? SOLVER_ROWS_SMEM / 2 : SOLVER_ROWS_SMEM ) / ( 16 * ( 2 + p.subSteps ) );
 	int want = ( w.bodyCount + p.parts - 1 ) / p.parts;
 	want = want > p.minChunk ? want : p.minChunk;

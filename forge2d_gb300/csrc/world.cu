@@ -4144,7 +4144,16 @@ extern "C" F2D_API int32_t f2d_world_autotune( int32_t worldId, double timeStep,
 	flush_uploads( W );
 	int variants[3];
 	int nv = 0;
-	variants[nv++] = SOLVER_FEW_PARTS;
+	// (in a smaller or larger world few parts are dealt as one per SM: no
+	// candidate of its own)
+	int placed = W->bodyCount;
+	if ( W->stepped )
+	{
+		cudaMemcpyAsync( &placed, &W->d.sc->orderTotal, sizeof( int ), cudaMemcpyDeviceToHost, W->stream );
+		cudaStreamSynchronize( W->stream );
+	}
+	if ( !W->smallParts && W->bodyCount > SOLVER_ONE_PART && placed <= SOLVER_FEW_MOST * SOLVER_ONE_PART )
+		variants[nv++] = SOLVER_FEW_PARTS;
 	variants[nv++] = SOLVER_ONE_PER_SM;
 	if ( W->s.solverBlocks2 > 0 )
 		variants[nv++] = SOLVER_TWO_PER_SM;
