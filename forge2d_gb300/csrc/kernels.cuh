@@ -1,8 +1,8 @@
 // Shared launch helpers and the per-phase launch entry points of the step.
 #pragma once
 
-#include <mutex>
 #include "dworld.cuh"
+#include "hscratch.h"
 
 #include <cuda_runtime.h>
 
@@ -154,17 +154,3 @@ struct FewMoves
 void launch_body_rows( DWorld& w, const BodyRows& rows, cudaStream_t st );
 void launch_shape_rows( DWorld& w, const ShapeRows& rows, cudaStream_t st );
 void launch_few_moves( DWorld& w, const FewMoves& moves, cudaStream_t st );
-
-// A world's workspace for ray and box queries: allocated once, guarded for
-// calls from several threads, freed with the world.
-#define QUERY_HOST_IDS 2048 // ids that reach the host without a copy of their own
-struct QueryScratch
-{
-	std::mutex lock;
-	unsigned long long* best = nullptr; // closest ray: fraction bits << 32 | shape; ~0 between calls
-	int* count = nullptr;				// blocks done, hits; 0 between calls
-	int* ids = nullptr;					// device: every hit of a box query
-	int idCap = 0;
-	float* ray = nullptr;	 // pinned, written by the kernel
-	int* found = nullptr;	 // pinned: hits, then up to QUERY_HOST_IDS ids
-};

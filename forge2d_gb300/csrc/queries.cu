@@ -472,7 +472,6 @@ DWorld* f2d_internal_world( int32_t worldId, cudaStream_t* st, int* gens, int ge
 uint16_t f2d_internal_shape_gen( int32_t worldId, int shape );
 int32_t f2d_internal_world0( int32_t worldId );
 QueryScratch* f2d_internal_query( int32_t worldId );
-bool f2d_internal_query_ready( QueryScratch* q, int shapes, cudaStream_t st );
 
 extern "C" F2D_API int32_t f2d_world_cast_ray_closest( int32_t worldId, double ox, double oy, double tx, double ty,
 													   int64_t categoryBits, int64_t maskBits, int32_t* shape2,
@@ -486,7 +485,7 @@ extern "C" F2D_API int32_t f2d_world_cast_ray_closest( int32_t worldId, double o
 	// and a copy per ray, a ray through 20k shapes took 40 us)
 	QueryScratch* scratch = f2d_internal_query( worldId );
 	std::lock_guard<std::mutex> hold( scratch->lock );
-	if ( !f2d_internal_query_ready( scratch, 0, st ) )
+	if ( !scratch->ready( 0, st ) )
 		return 0;
 	fv2 o = mk( (float)ox, (float)oy ), t = mk( (float)tx, (float)ty );
 	float* h = scratch->ray;
@@ -634,7 +633,7 @@ extern "C" F2D_API int32_t f2d_world_overlap_aabb( int32_t worldId, double lx, d
 	int cap = w->shapeCount > 0 ? w->shapeCount : 1;
 	QueryScratch* scratch = f2d_internal_query( worldId );
 	std::lock_guard<std::mutex> hold( scratch->lock );
-	if ( !f2d_internal_query_ready( scratch, cap, st ) )
+	if ( !scratch->ready( cap, st ) )
 		return 0;
 	fbox box;
 	box.lo = mk( (float)lx, (float)ly );

@@ -211,20 +211,6 @@ template <typename T> static void dfree( T*& p )
 
 #define HOST_END 64
 
-static void query_free( HostWorld* W )
-{
-	QueryScratch* q = W->query;
-	if ( q == nullptr )
-		return;
-	dfree( q->best );
-	dfree( q->count );
-	dfree( q->ids );
-	cudaFreeHost( q->ray );
-	cudaFreeHost( q->found );
-	delete q;
-	W->query = nullptr;
-}
-
 // ---------------------------------------------------------------------------
 // capacities
 // ---------------------------------------------------------------------------
@@ -1405,7 +1391,9 @@ static void free_world( HostWorld* W )
 	cudaFreeHost( W->hostError );
 	cudaFreeHost( W->hostEnd );
 	W->hostEnd = nullptr;
-	query_free( W );
+	W->query->release();
+	delete W->query;
+	W->query = nullptr;
 	cudaEventDestroy( W->evStart );
 	cudaEventDestroy( W->evStop );
 	cudaEventDestroy( W->evFork );
@@ -5340,36 +5328,10 @@ DWorld* f2d_internal_world( int32_t worldId, cudaStream_t* st, int* gens, int ge
 	return &W->d;
 }
 
-// The world's query workspace, its id list as long as the world has shapes
-// (the caller holds the lock), or nullptr.
 QueryScratch* f2d_internal_query( int32_t worldId )
 {
 	HostWorld* W = world_from_id( worldId );
 	return W ? W->query : nullptr;
-}
-
-bool f2d_internal_query_ready( QueryScratch* q, int shapes, cudaStream_t st )
-{
-	if ( q->best == nullptr )
-	{
-		if ( cudaMalloc( (void**)&q->best, sizeof( unsigned long long ) ) != cudaSuccess ||
-			 cudaMalloc( (void**)&q->count, 2 * sizeof( int ) ) != cudaSuccess ||
-			 cudaMallocHost( (void**)&q->ray, 8 * sizeof( float ) ) != cudaSuccess ||
-			 cudaMallocHost( (void**)&q->found, ( 1 + QUERY_HOST_IDS ) * sizeof( int ) ) != cudaSuccess )
-			return false;
-		cudaMemsetAsync( q->best, 0xff, sizeof( unsigned long long ), st );
-		cudaMemsetAsync( q->count, 0, 2 * sizeof( int ), st );
-	}
-	if ( shapes > q->idCap )
-	{
-		dfree( q->ids );
-		q->idCap = 0;
-		int cap = std::max( 1024, 2 * shapes );
-		if ( cudaMalloc( (void**)&q->ids, sizeof( int ) * (size_t)cap ) != cudaSuccess )
-			return false;
-		q->idCap = cap;
-	}
-	return true;
 }
 
 // For the allocation-free queries: the world's device rows after pending

@@ -1,0 +1,90 @@
+"""Host memory of the library against a fake of the CUDA allocation calls that
+fails where it is told to: no GPU, no driver."""
+from __future__ import annotations
+
+import os
+import shutil
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "forge2d_gb300", "csrc")
+
+FAKE = r"""
+#include <cuda_runtime.h>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <set>
+
+// every call counts; call number `failAt` fails (1: the first)
+static int calls = 0, failAt = 0, sets = 0, bad = 0;
+static std::set<void*> live;
+static bool fails() { calls += 1; return calls == failAt; }
+static cudaError_t give( void** p, size_t n )
+{
+	if ( fails() )
+		return cudaErrorMemoryAllocation; // *p stays as it was
+	*p = malloc( n );
+	live.insert( *p );
+	return cudaSuccess;
+}
+static cudaError_t take( void* p )
+{
+	if ( live.erase( p ) == 0 )
+	{
+		bad += 1;
+		return cudaErrorInvalidValue;
+	}
+	free( p );
+	return cudaSuccess;
+}
+extern "C" cudaError_t cudaMalloc( void** p, size_t n ) { return give( p, n ); }
+extern "C" cudaError_t cudaMallocHost( void** p, size_t n ) { return give( p, n ); }
+extern "C" cudaError_t cudaFree( void* p ) { return take( p ); }
+extern "C" cudaError_t cudaFreeHost( void* p ) { return take( p ); }
+extern "C" cudaError_t cudaMemsetAsync( void* p, int v, size_t n, cudaStream_t ) { sets += 1; memset( p, v, n ); return cudaSuccess; }
+#define CHECK( x ) do { if ( !( x ) ) { printf( "line %d: %s\n", __LINE__, #x ); return 1; } } while ( 0 )
+"""
+
+QUERY = FAKE + r"""
+#include "hscratch.h"
+int main()
+{
+	// the allocation that fails: best, count, ray, found, ids; 6: none
+	for ( int k = 1; k <= 6; ++k )
+	{
+		calls = 0;
+		failAt = k;
+		sets = 0;
+		QueryScratch q;
+		CHECK( q.ready( 10, nullptr ) == ( k == 6 ) );
+		failAt = 0;
+		CHECK( q.ready( 10, nullptr ) );
+		CHECK( q.best && q.count && q.ray && q.found && q.ids && q.idCap >= 10 );
+		CHECK( *q.best == ~0ull && q.count[0] == 0 && q.count[1] == 0 && sets == 2 );
+		CHECK( live.size() == 5 );
+		// a list that cannot grow is asked for again
+		failAt = calls + 1;
+		CHECK( !q.ready( 5000, nullptr ) );
+		failAt = 0;
+		CHECK( q.ready( 5000, nullptr ) && q.ids && q.idCap >= 5000 );
+		q.release();
+		CHECK( live.empty() && bad == 0 );
+	}
+	return 0;
+}
+"""
+
+
+def _run(tmp_path, name, source):
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))), "include")
+    path = tmp_path / (name + ".cpp")
+    path.write_text(source)
+    exe = str(tmp_path / name)
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I" + CSRC, "-I" + cuda, str(path), "-o", exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, (r.returncode, r.stdout + r.stderr)
+
+
+def test_query_workspace_survives_failing_allocations(tmp_path):
+    _run(tmp_path, "query", QUERY)
