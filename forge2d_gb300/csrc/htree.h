@@ -10,45 +10,9 @@
 #pragma once
 
 #include "dworld.cuh"
+#include "hpinned.h"
 
-#include <cuda_runtime.h>
-
-#include <cstdlib>
-#include <new>
 #include <vector>
-
-// Page-locked arrays from PINNED_BYTES up (a tree of 4096 nodes): a tree is
-// edited on the host between two steps, so its arrays go both ways every time.
-// From pageable memory the 3.4 MB of a 20k-body world's tree took some 450 us
-// each way. Below, and without a device, plain memory.
-#define PINNED_BYTES 65536
-template <typename T> struct PinnedAlloc
-{
-	typedef T value_type;
-	PinnedAlloc() = default;
-	template <typename U> PinnedAlloc( const PinnedAlloc<U>& ) {}
-	T* allocate( size_t n )
-	{
-		void* p = nullptr;
-		if ( n * sizeof( T ) >= PINNED_BYTES && cudaMallocHost( &p, n * sizeof( T ) ) == cudaSuccess )
-			return (T*)p;
-		cudaGetLastError();
-		p = malloc( n * sizeof( T ) );
-		if ( p == nullptr )
-			throw std::bad_alloc();
-		return (T*)p;
-	}
-	void deallocate( T* p, size_t n )
-	{
-		if ( n * sizeof( T ) >= PINNED_BYTES && cudaFreeHost( p ) == cudaSuccess )
-			return;
-		cudaGetLastError();
-		free( p );
-	}
-	template <typename U> bool operator==( const PinnedAlloc<U>& ) const { return true; }
-	template <typename U> bool operator!=( const PinnedAlloc<U>& ) const { return false; }
-};
-template <typename T> using PinnedVector = std::vector<T, PinnedAlloc<T>>;
 
 struct HTree
 {

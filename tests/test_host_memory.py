@@ -18,11 +18,17 @@ FAKE = r"""
 // every call counts; call number `failAt` fails (1: the first)
 static int calls = 0, failAt = 0, sets = 0, bad = 0;
 static std::set<void*> live;
+static void* fixedBlock = nullptr; // given instead of heap memory, and not taken back
 static bool fails() { calls += 1; return calls == failAt; }
 static cudaError_t give( void** p, size_t n )
 {
 	if ( fails() )
 		return cudaErrorMemoryAllocation; // *p stays as it was
+	if ( fixedBlock )
+	{
+		*p = fixedBlock;
+		return cudaSuccess;
+	}
 	*p = malloc( n );
 	live.insert( *p );
 	return cudaSuccess;
@@ -74,6 +80,50 @@ int main()
 }
 """
 
+PINNED = FAKE.replace("static cudaError_t give", r"""
+static int errors = 0; // reads of the last error
+extern "C" cudaError_t cudaGetLastError() { errors += 1; return cudaSuccess; }
+static cudaError_t give""") + r"""
+#include "hpinned.h"
+struct F4 { float x, y, z, w; };
+template <typename T> static int arrays()
+{
+	const size_t sizes[] = { 1, 64, PINNED_BYTES / sizeof( T ) - 1, PINNED_BYTES / sizeof( T ), 100000 };
+	for ( size_t n : sizes )
+		for ( int refused = 0; refused < 2; ++refused )
+		{
+			calls = 0;
+			failAt = refused;
+			{
+				PinnedVector<T> v( n );
+				CHECK( ( (size_t)v.data() & 15 ) == 0 );
+				CHECK( live.size() == ( n * sizeof( T ) >= PINNED_BYTES && !refused ? 1u : 0u ) );
+				memset( (void*)v.data(), 0x5a, n * sizeof( T ) );
+				PinnedVector<T> u = v;
+				u.resize( 2 * n );
+				CHECK( memcmp( u.data(), v.data(), n * sizeof( T ) ) == 0 );
+				v = std::move( u );
+			}
+			CHECK( live.empty() && bad == 0 );
+		}
+	return 0;
+}
+int main()
+{
+	CHECK( arrays<int>() == 0 && arrays<F4>() == 0 && arrays<unsigned long long>() == 0 );
+	// a page-locked block that cannot be given back: not the heap's
+	static char locked[PINNED_BYTES + 4096];
+	char* at = locked + 64 - ( (size_t)locked & 63 );
+	fixedBlock = at;
+	{
+		PinnedVector<int> v( PINNED_BYTES / sizeof( int ) );
+		CHECK( (char*)v.data() >= at && (char*)( v.data() + v.size() ) <= at + PINNED_BYTES + 1024 );
+	}
+	CHECK( bad == 1 );
+	return 0;
+}
+"""
+
 
 def _run(tmp_path, name, source):
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))), "include")
@@ -88,3 +138,7 @@ def _run(tmp_path, name, source):
 
 def test_query_workspace_survives_failing_allocations(tmp_path):
     _run(tmp_path, "query", QUERY)
+
+
+def test_page_locked_blocks_are_not_the_heaps(tmp_path):
+    _run(tmp_path, "pinned", PINNED)
