@@ -28,12 +28,13 @@ template <typename T> struct PinnedAlloc
 		const size_t bytes = n * sizeof( T ) + ( head ? PINNED_HEAD : 0 );
 		bool locked = false;
 		if ( head )
-			locked = cudaMallocHost( &p, bytes ) == cudaSuccess;
-		if ( !locked )
 		{
-			cudaGetLastError();
-			p = malloc( bytes );
+			locked = cudaMallocHost( &p, bytes ) == cudaSuccess;
+			if ( !locked )
+				cudaGetLastError();
 		}
+		if ( !locked )
+			p = malloc( bytes );
 		if ( p == nullptr )
 			throw std::bad_alloc();
 		if ( !head )

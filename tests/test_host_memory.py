@@ -124,6 +124,21 @@ int main()
 }
 """
 
+LAST_ERROR = PINNED[:PINNED.index("int main()")] + r"""
+int main()
+{
+	{
+		PinnedVector<int> small( 100 ), large( PINNED_BYTES );
+	}
+	CHECK( errors == 0 ); // an error of another call waits for who asks for it
+	calls = 0;
+	failAt = 1;
+	PinnedVector<int> refused( PINNED_BYTES );
+	CHECK( errors == 1 );
+	return 0;
+}
+"""
+
 
 def _run(tmp_path, name, source):
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))), "include")
@@ -142,3 +157,7 @@ def test_query_workspace_survives_failing_allocations(tmp_path):
 
 def test_page_locked_blocks_are_not_the_heaps(tmp_path):
     _run(tmp_path, "pinned", PINNED)
+
+
+def test_other_calls_errors_are_kept(tmp_path):
+    _run(tmp_path, "last_error", LAST_ERROR)
