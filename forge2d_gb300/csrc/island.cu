@@ -1246,16 +1246,18 @@ __device__ void split_row( const DWorld& w, DIslands& I, int baseId, int b, int 
 				at += 1;
 				if ( !inside )
 					continue;
-				// a body met twice is pushed at the first meeting: later places in the
-				// row stay empty (an index past every body, marked from the start); the
-				// rest of a long row keeps them, the traversal finds them there (a
-				// search through all earlier ones grows with the row's square)
+				// a body met twice is pushed at the first meeting: later places stay
+				// empty (an index past every body, marked from the start). The row is
+				// searched whole; past it only the latest places, so that the search
+				// grows with the edges and not with their square, and the traversal
+				// sorts out what repeats are left. (Without a read of the pool here the
+				// compiler gives the traversal 40 registers and spills: 60k-body island
+				// 7.1 ms instead of 6.7.)
 				int slot = to;
 				const int kept = pushes > SPLIT_PUSH ? SPLIT_PUSH - 1 : SPLIT_PUSH;
-				if ( pushAt < kept )
-					for ( int k = 0; k < pushAt; ++k )
-						if ( push[k] == to )
-							slot = none;
+				for ( int k = max( pushAt - SPLIT_PUSH, 0 ); k < pushAt; ++k )
+					if ( ( k < kept ? push[k] : I.splitPushPool[pushPool + 1 + k - kept] ) == to )
+						slot = none;
 				if ( pushAt < kept )
 					push[pushAt] = slot;
 				else
