@@ -140,7 +140,6 @@ struct DScalars
 	// grid barriers of the step's one-launch kernels, zeroed at its start: the
 	// tree rebuilds (they run beside other kernels) and the sorts (SORT_*)
 	unsigned ptBarrier[2], sortBarrier[5];
-	unsigned barrierGen;
 	int planCount;
 	int awakeCount;
 	int treeLeafCount;
