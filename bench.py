@@ -296,8 +296,6 @@ def run_gpu(args, rank, world):
         alg_bytes.append(solver_bytes(g.counters()))
     g.set_profiling(False)
     phases /= reps
-    # grid barriers of the solver (none: its constraints wait for bodies) and the measured cost of one
-    barriers, us_per_barrier = g.solver_latency(2000)
     solve_avg = sum(solve_ms) / len(solve_ms)
     alg = sum(alg_bytes) / len(alg_bytes)
     peak, peak_kind = measured_peaks()
@@ -336,7 +334,8 @@ def run_gpu(args, rank, world):
                 "what": "f2d_world_step + f2d_world_get_bodies (every body row: transform, velocities, "
                         "to a pinned host buffer) on a second copy of the scene over the same frames, host clock",
                 "steps": len(frames)},
-        "roofline": {"kernel": "k_solve (persistent cooperative solver)", "bound": "hbm",
+        "roofline": {"kernel": "k_solve (persistent cooperative solver)",
+                     "bound": "latency", "peak_is": "HBM rate",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                      "peak_source": peak_kind, "algorithmic_bytes_per_launch": alg,
@@ -344,14 +343,7 @@ def run_gpu(args, rank, world):
                      "traffic_source": "ncu dram bytes per algorithmic byte of a captured pile25k launch "
                                        "(profiles/k_solve_pile25k.md) x this run's algorithmic bytes",
                      "profiled_steps": [{"solve_ms": a, "algorithmic_bytes": b}
-                                        for a, b in zip(solve_ms, alg_bytes)],
-                     "latency": {"barriers_per_launch": barriers, "us_per_barrier": us_per_barrier,
-                                 "floor_ms": barriers * us_per_barrier * 1e-3,
-                                 "floor_frac_of_launch": (barriers * us_per_barrier * 1e-3 / solve_avg)
-                                 if solve_avg > 0 else None,
-                                 "what": "grid-wide barriers the last solver launch passed (0: a constraint waits "
-                                         "for the bodies it reads, not for the device) times the cost of one, "
-                                         "measured by a launch of 2000 bare barriers on the same grid"}},
+                                        for a, b in zip(solve_ms, alg_bytes)]},
         "phases_ms": {"broadphase": phases[0], "narrowphase": phases[1], "colouring": phases[2],
                       "solver_setup": phases[3], "solver_kernel": phases[4], "finalize": phases[5],
                       "tree_rebuild_beside": rebuild},

@@ -282,9 +282,12 @@ __device__ __forceinline__ void hit_events( const DWorld& w )
 // scanned by the thread itself: with 3 statics and 100k bodies a warp each
 // would be 20 waves of warps for one box test per lane. Above, a thread has to
 // walk the pair tree down through every moving shape around its body; the
-// warp's scan replaces that up to CCD_WARP_MAX shapes, where a scan costs what
-// a walk does. Whole finalize phase, walk and scan: 6k bodies on a terrain of
-// 200 segments 144 and 43 us, 512 batched worlds (700 statics) 140 and 71 us.
+// warp's scan replaces that up to CCD_WARP_MAX shapes. Its cost grows with
+// them, the walk's hardly does. Whole finalize phase, walk and scan, on terrains
+// of 89, 889, 3529 segments: 500 bodies 76 and 29, 78 and 33, 88 and 45 us; 6k
+// bodies 150 and 43, 150 and 49, 154 and 62; 20k bodies 176 and 59, 179 and 70,
+// 180 and 117. The two meet beyond 3500; the line lies where the scan is at most
+// half of the walk at all of these.
 #define CCD_LIST_MAX 64
 #define CCD_WARP_MAX 1024
 #define CCD_WARP_THREADS 128

@@ -51,10 +51,12 @@ struct StepScratch
 };
 
 // A world of up to this many bodies with constraints is one part: no body is
-// shared (pyramids of 55, 210, 465 boxes: 66, 76, 104 us as one part; 66, 111,
-// 109 us in parts of 64). Larger worlds take parts of at least SOLVER_MIN_CHUNK = 64 bodies (820
-// boxes: 111 us against 165 us as one part; 2k-6k piles: parts of 64 bodies
-// 138, 139 us, of 256 bodies 150, 152 us).
+// shared. Larger worlds take parts of at least SOLVER_MIN_CHUNK = 64 bodies.
+// Pyramids of 55, 210, 351, 465, 595, 820 boxes: 66, 74, 84, 104, 125, 160 us
+// as one part, 66, 113, 111, 109, 119, 113 us in parts of 64; mixed piles of
+// 300, 500, 700, 1000: 82, 98, 123, 175 and 117, 115, 113, 125 us. The two meet
+// between 500 and 600; the line lies below that, where one part is clearly the
+// better. (Piles of 2k and 6k: parts of 64 bodies 138, 139 us, of 256 150, 152.)
 #define SOLVER_ONE_PART 400
 #define SOLVER_FEW_MOST 4 // times as many with SOLVER_FEW_PARTS
 

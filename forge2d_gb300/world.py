@@ -383,8 +383,8 @@ class GpuWorld:
         return float(self.lib.f2d_world_get_rebuild_ms(self.id))
 
     def solver_latency(self, probe_barriers=2000):
-        """(grid barriers of the last grid-wide solver launch, measured
-        microseconds per grid barrier on its grid)."""
+        """(grid barriers a solver launch passes: 0, measured microseconds per
+        grid barrier on its grid)."""
         out = np.zeros(2, np.float64)
         self.lib.f2d_world_get_solver_latency(self.id, probe_barriers, out.ctypes.data_as(C.POINTER(C.c_double)))
         return int(out[0]), float(out[1])

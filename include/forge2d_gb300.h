@@ -700,7 +700,7 @@ F2D_API void f2d_mlp_predict( int32_t model, const float* feats12, int32_t n, fl
 
 /* Autotuner (no reference counterpart). Steps the world through every
  * candidate launch configuration -- solver shape (1 larger worlds in one
- * part, 2 one block per SM, 3 two blocks per SM) x
+ * part, where that differs from 2; 2 one block per SM, 3 two blocks per SM) x
  * broadphase leaf-order refresh period (4, 8, 16, 32 steps) -- timing each
  * over max(stepsPerCandidate, period) steps, and keeps the fastest. The
  * tuning steps are ordinary steps of the world; no configuration changes any
