@@ -190,15 +190,22 @@ static int ceil_pow2( int v )
 	return p;
 }
 
-template <typename T> static void dgrow( T*& p, size_t oldN, size_t newN )
+// A device array of newN zeros with the old one's first oldN, made on the
+// world's stream: that stream does not wait for the default one, so a clear
+// there may come after what the step writes, and a copy before it.
+template <typename T> static void dgrow( HostWorld* W, T*& p, size_t oldN, size_t newN )
 {
 	T* q = nullptr;
-	cudaMalloc( (void**)&q, sizeof( T ) * ( newN > 0 ? newN : 1 ) );
-	cudaMemset( q, 0, sizeof( T ) * ( newN > 0 ? newN : 1 ) );
+	const size_t n = newN > 0 ? newN : 1;
+	cudaMalloc( (void**)&q, sizeof( T ) * n );
+	cudaMemsetAsync( q, 0, sizeof( T ) * n, W->stream );
 	if ( p && oldN > 0 )
-		cudaMemcpy( q, p, sizeof( T ) * std::min( oldN, newN ), cudaMemcpyDeviceToDevice );
+		cudaMemcpyAsync( q, p, sizeof( T ) * std::min( oldN, newN ), cudaMemcpyDeviceToDevice, W->stream );
 	if ( p )
+	{
+		cudaStreamSynchronize( W->stream );
 		cudaFree( p );
+	}
 	p = q;
 }
 
@@ -216,6 +223,7 @@ template <typename T> static void dfree( T*& p )
 // ---------------------------------------------------------------------------
 static void alloc_scratch( HostWorld* W )
 {
+	cudaStreamSynchronize( W->stream ); // steps that use the old arrays
 	DWorld& d = W->d;
 	StepScratch& s = W->s;
 	dfree( s.tmpA );
@@ -224,19 +232,19 @@ static void alloc_scratch( HostWorld* W )
 	dfree( s.bounds );
 	int m = std::max( std::max( d.shapeCap, d.contactCap ), std::max( d.bodyCap, d.pairCap ) );
 	size_t tmpN = 2 * (size_t)m + 64;
-	dgrow( s.tmpA, 0, tmpN );
-	dgrow( s.tmpB, 0, tmpN + d.jointCap + 64 );
+	dgrow( W, s.tmpA, 0, tmpN );
+	dgrow( W, s.tmpB, 0, tmpN + d.jointCap + 64 );
 	int sortBlocks = ( std::max( d.pairCap, d.shapeCap ) + SORT_TILE - 1 ) / SORT_TILE + 1;
 	int scanN = std::max( 256 * sortBlocks, m );
-	dgrow( s.scanTmp, 0, (size_t)( scanN + SCAN_TILE - 1 ) / SCAN_TILE + 64 );
+	dgrow( W, s.scanTmp, 0, (size_t)( scanN + SCAN_TILE - 1 ) / SCAN_TILE + 64 );
 	dfree( d.sortHist );
-	dgrow( d.sortHist, 0, std::max( (size_t)256 * sortBlocks + 256, (size_t)256 * CSORT_MAX_BLOCKS + 256 ) );
+	dgrow( W, d.sortHist, 0, std::max( (size_t)256 * sortBlocks + 256, (size_t)256 * CSORT_MAX_BLOCKS + 256 ) );
 	dfree( s.scanState );
-	dgrow( s.scanState, 0, (size_t)( m + LB_TILE - 1 ) / LB_TILE + 8 );
+	dgrow( W, s.scanState, 0, (size_t)( m + LB_TILE - 1 ) / LB_TILE + 8 );
 	s.sortBlocks32 = sort_coop_blocks<unsigned>();
 	s.sortBlocks64 = sort_coop_blocks<unsigned long long>();
 	s.boundsBlocks = 64;
-	dgrow( s.bounds, 0, (size_t)s.boundsBlocks );
+	dgrow( W, s.bounds, 0, (size_t)s.boundsBlocks );
 	int bits = 1;
 	while ( ( 1 << bits ) < d.shapeCap )
 		bits += 1;
@@ -248,7 +256,7 @@ static void alloc_scratch( HostWorld* W )
 	size_t pairWords = LOOKBACK_WORDS( (size_t)d.pairCap ), linkWords = LOOKBACK_WORDS( (size_t)d.opCap );
 	d.lookbackWords = (int)( opWords + collectWords + 3 * moveWords + pairWords + linkWords );
 	dfree( d.opScan );
-	dgrow( d.opScan, 0, (size_t)d.lookbackWords );
+	dgrow( W, d.opScan, 0, (size_t)d.lookbackWords );
 	d.collectScan = d.opScan + opWords;
 	d.moveScan = d.collectScan + collectWords;
 	d.mergeScan = d.moveScan + moveWords;
@@ -260,40 +268,40 @@ static void alloc_scratch( HostWorld* W )
 	int parts = std::min( SOLVER_MAX_PARTS, d.bodyCap / ( W->smallParts ? SOLVER_SMALL_CHUNK : SOLVER_MIN_CHUNK ) + 2 );
 	d.slotCap = 32 * ( ( d.contactCap + 31 ) / 32 + parts * F2D_OVERFLOW + 1 );
 	dfree( d.kRow );
-	dgrow( d.kRow, 0, (size_t)KROWS * d.slotCap );
+	dgrow( W, d.kRow, 0, (size_t)KROWS * d.slotCap );
 	dfree( d.orderState );
-	dgrow( d.orderState, 0, (size_t)d.shapeCap / 4096 + 8 );
+	dgrow( W, d.orderState, 0, (size_t)d.shapeCap / 4096 + 8 );
 	dfree( d.bodyPos );
-	dgrow( d.bodyPos, 0, (size_t)d.bodyCap );
+	dgrow( W, d.bodyPos, 0, (size_t)d.bodyCap );
 	dfree( d.bodyAt );
-	dgrow( d.bodyAt, 0, (size_t)d.bodyCap );
+	dgrow( W, d.bodyAt, 0, (size_t)d.bodyCap );
 	dfree( d.bodyOrd );
-	dgrow( d.bodyOrd, 0, (size_t)d.bodyCap );
+	dgrow( W, d.bodyOrd, 0, (size_t)d.bodyCap );
 	dfree( d.bodyInt );
-	dgrow( d.bodyInt, 0, 2 * (size_t)d.bodyCap );
+	dgrow( W, d.bodyInt, 0, 2 * (size_t)d.bodyCap );
 	dfree( d.dsub );
-	dgrow( d.dsub, 0, FLOW_SUBSTEPS * (size_t)d.bodyCap );
+	dgrow( W, d.dsub, 0, FLOW_SUBSTEPS * (size_t)d.bodyCap );
 	dfree( d.jointPlace );
-	dgrow( d.jointPlace, 0, (size_t)d.jointCap );
+	dgrow( W, d.jointPlace, 0, (size_t)d.jointCap );
 	dfree( d.jointSlots );
-	dgrow( d.jointSlots, 0, (size_t)d.jointCap );
+	dgrow( W, d.jointSlots, 0, (size_t)d.jointCap );
 	dfree( d.ovfItems );
-	dgrow( d.ovfItems, 0, constraints );
+	dgrow( W, d.ovfItems, 0, constraints );
 	dfree( d.ovfSorted );
-	dgrow( d.ovfSorted, 0, constraints );
+	dgrow( W, d.ovfSorted, 0, constraints );
 	dfree( d.ovfRank );
-	dgrow( d.ovfRank, 0, constraints );
+	dgrow( W, d.ovfRank, 0, constraints );
 	dfree( d.ovfNext );
-	dgrow( d.ovfNext, 0, 2 * constraints );
+	dgrow( W, d.ovfNext, 0, 2 * constraints );
 	// counts and starts per part: contacts, joints, overflow
 	size_t bins = (size_t)SOLVER_MAX_PARTS * F2D_OVERFLOW;
 	dfree( d.binContacts );
-	dgrow( d.binContacts, 0, 2 * bins + SOLVER_MAX_PARTS + 1 );
+	dgrow( W, d.binContacts, 0, 2 * bins + SOLVER_MAX_PARTS + 1 );
 	d.binJoints = d.binContacts + bins;
 	d.binOverflow = d.binJoints + bins;
 	d.flowLong = d.binOverflow + SOLVER_MAX_PARTS;
 	dfree( d.binContactStart );
-	dgrow( d.binContactStart, 0, 2 * bins + SOLVER_MAX_PARTS );
+	dgrow( W, d.binContactStart, 0, 2 * bins + SOLVER_MAX_PARTS );
 	d.binJointStart = d.binContactStart + bins;
 	d.binOverflowStart = d.binJointStart + bins;
 	s.solverBlocks = solver_max_blocks( 1 );
@@ -307,25 +315,25 @@ static void grow_bodies( HostWorld* W, int cap )
 {
 	DWorld& d = W->d;
 	size_t o = d.bodyCap;
-	dgrow( d.xf, o, cap );
-	dgrow( d.vel, o, cap );
-	dgrow( d.delta, o, cap );
-	dgrow( d.center, o, cap );
-	dgrow( d.sweep0, o, cap );
-	dgrow( d.localCenter, o, cap );
-	dgrow( d.massv, o, cap );
-	dgrow( d.damp, o, cap );
-	dgrow( d.bodyGravity, o, cap );
-	dgrow( d.force, o, cap );
-	dgrow( d.bflags, o, cap );
-	dgrow( d.headShape, o, cap );
-	dgrow( d.headJoint, o, cap );
-	dgrow( d.jointCountB, o, cap );
-	dgrow( d.colorMask, o, cap );
-	dgrow( d.colorLock, o, cap );
-	dgrow( d.fastBodies, o, cap );
-	dgrow( d.moveEvXf, o, cap );
-	dgrow( d.awakeOrder, o, cap );
+	dgrow( W, d.xf, o, cap );
+	dgrow( W, d.vel, o, cap );
+	dgrow( W, d.delta, o, cap );
+	dgrow( W, d.center, o, cap );
+	dgrow( W, d.sweep0, o, cap );
+	dgrow( W, d.localCenter, o, cap );
+	dgrow( W, d.massv, o, cap );
+	dgrow( W, d.damp, o, cap );
+	dgrow( W, d.bodyGravity, o, cap );
+	dgrow( W, d.force, o, cap );
+	dgrow( W, d.bflags, o, cap );
+	dgrow( W, d.headShape, o, cap );
+	dgrow( W, d.headJoint, o, cap );
+	dgrow( W, d.jointCountB, o, cap );
+	dgrow( W, d.colorMask, o, cap );
+	dgrow( W, d.colorLock, o, cap );
+	dgrow( W, d.fastBodies, o, cap );
+	dgrow( W, d.moveEvXf, o, cap );
+	dgrow( W, d.awakeOrder, o, cap );
 	d.bodyCap = cap;
 }
 
@@ -333,41 +341,41 @@ static void grow_contacts( HostWorld* W, int cap )
 {
 	DWorld& d = W->d;
 	size_t o = d.contactCap;
-	dgrow( d.cshape, o, cap );
-	dgrow( d.cbody, o, cap );
-	dgrow( d.cflags, o, cap );
-	dgrow( d.ccolor, o, cap );
-	dgrow( d.coverflowIndex, o, cap );
-	dgrow( d.cmat, o, cap );
-	dgrow( d.cmass, o, cap );
-	dgrow( d.mnorm, o, cap );
-	dgrow( d.csimplex, o, cap );
-	dgrow( d.mpA, 2 * o, 2 * (size_t)cap );
-	dgrow( d.mpB, 2 * o, 2 * (size_t)cap );
-	dgrow( d.mpI, 2 * o, 2 * (size_t)cap );
-	dgrow( d.contactFree, o, cap );
-	dgrow( d.cstamp, o, cap );
-	dgrow( d.apiEndEv, 0, 2 * (size_t)cap );
+	dgrow( W, d.cshape, o, cap );
+	dgrow( W, d.cbody, o, cap );
+	dgrow( W, d.cflags, o, cap );
+	dgrow( W, d.ccolor, o, cap );
+	dgrow( W, d.coverflowIndex, o, cap );
+	dgrow( W, d.cmat, o, cap );
+	dgrow( W, d.cmass, o, cap );
+	dgrow( W, d.mnorm, o, cap );
+	dgrow( W, d.csimplex, o, cap );
+	dgrow( W, d.mpA, 2 * o, 2 * (size_t)cap );
+	dgrow( W, d.mpB, 2 * o, 2 * (size_t)cap );
+	dgrow( W, d.mpI, 2 * o, 2 * (size_t)cap );
+	dgrow( W, d.contactFree, o, cap );
+	dgrow( W, d.cstamp, o, cap );
+	dgrow( W, d.apiEndEv, 0, 2 * (size_t)cap );
 	// step scratch sized by contacts (content not preserved)
-	dgrow( d.opContact, 0, cap );
-	dgrow( d.opKind, 0, cap );
-	dgrow( d.opColor, 0, cap );
-	dgrow( d.opDone, 0, cap );
-	dgrow( d.opBodies, 0, cap );
-	dgrow( d.overflowList, o, cap );
-	dgrow( d.slotPlace, 0, cap );
-	dgrow( d.npBucket, 0, (size_t)NP_CLASSES * cap );
-	dgrow( d.beginEv, 0, 2 * (size_t)cap );
-	dgrow( d.beginEvF, 0, 9 * (size_t)cap );
-	dgrow( d.endEv, 0, 2 * (size_t)cap );
-	dgrow( d.hitEvI, 0, 2 * (size_t)cap );
-	dgrow( d.hitEvF, 0, 5 * (size_t)cap );
+	dgrow( W, d.opContact, 0, cap );
+	dgrow( W, d.opKind, 0, cap );
+	dgrow( W, d.opColor, 0, cap );
+	dgrow( W, d.opDone, 0, cap );
+	dgrow( W, d.opBodies, 0, cap );
+	dgrow( W, d.overflowList, o, cap );
+	dgrow( W, d.slotPlace, 0, cap );
+	dgrow( W, d.npBucket, 0, (size_t)NP_CLASSES * cap );
+	dgrow( W, d.beginEv, 0, 2 * (size_t)cap );
+	dgrow( W, d.beginEvF, 0, 9 * (size_t)cap );
+	dgrow( W, d.endEv, 0, 2 * (size_t)cap );
+	dgrow( W, d.hitEvI, 0, 2 * (size_t)cap );
+	dgrow( W, d.hitEvF, 0, 5 * (size_t)cap );
 	d.contactCap = cap;
 	d.opCap = cap;
 	d.eventCap = cap;
 	int hcap = ceil_pow2( 2 * cap );
 	dfree( d.pairHash );
-	dgrow( d.pairHash, 0, hcap );
+	dgrow( W, d.pairHash, 0, hcap );
 	d.hashCap = hcap;
 }
 
@@ -375,41 +383,41 @@ static void grow_shapes( HostWorld* W, int cap )
 {
 	DWorld& d = W->d;
 	size_t o = d.shapeCap;
-	dgrow( d.geom, o * GEOM_F4, (size_t)cap * GEOM_F4 );
-	dgrow( d.aabb, o, cap );
-	dgrow( d.fat, o, cap );
-	dgrow( d.mat, o, cap );
-	dgrow( d.cat, o, cap );
-	dgrow( d.mask, o, cap );
-	dgrow( d.group, o, cap );
-	dgrow( d.shapeBody, o, cap );
-	dgrow( d.shapeSub, o, cap );
-	dgrow( d.sflags, o, cap );
-	dgrow( d.proxyKey, o, cap );
-	dgrow( d.nextShape, o, cap );
-	dgrow( d.staticShapes, 0, cap );
-	dgrow( d.shapeMove, o, cap );
-	dgrow( d.moveShape, 0, cap );
-	dgrow( d.hostMoves, 0, cap );
+	dgrow( W, d.geom, o * GEOM_F4, (size_t)cap * GEOM_F4 );
+	dgrow( W, d.aabb, o, cap );
+	dgrow( W, d.fat, o, cap );
+	dgrow( W, d.mat, o, cap );
+	dgrow( W, d.cat, o, cap );
+	dgrow( W, d.mask, o, cap );
+	dgrow( W, d.group, o, cap );
+	dgrow( W, d.shapeBody, o, cap );
+	dgrow( W, d.shapeSub, o, cap );
+	dgrow( W, d.sflags, o, cap );
+	dgrow( W, d.proxyKey, o, cap );
+	dgrow( W, d.nextShape, o, cap );
+	dgrow( W, d.staticShapes, 0, cap );
+	dgrow( W, d.shapeMove, o, cap );
+	dgrow( W, d.moveShape, 0, cap );
+	dgrow( W, d.hostMoves, 0, cap );
 	// broadphase scratch
-	dgrow( d.mortonKeys, 0, cap );
-	dgrow( d.mortonKeysAlt, 0, cap );
-	dgrow( d.leafShape, 0, cap );
-	dgrow( d.leafShapeAlt, 0, cap );
-	dgrow( d.nodeLeft, 0, cap );
-	dgrow( d.nodeRight, 0, cap );
-	dgrow( d.nodeParent, 0, 2 * (size_t)cap );
-	dgrow( d.nodeBox, 0, 2 * (size_t)cap );
-	dgrow( d.nodeVisit, 0, cap );
+	dgrow( W, d.mortonKeys, 0, cap );
+	dgrow( W, d.mortonKeysAlt, 0, cap );
+	dgrow( W, d.leafShape, 0, cap );
+	dgrow( W, d.leafShapeAlt, 0, cap );
+	dgrow( W, d.nodeLeft, 0, cap );
+	dgrow( W, d.nodeRight, 0, cap );
+	dgrow( W, d.nodeParent, 0, 2 * (size_t)cap );
+	dgrow( W, d.nodeBox, 0, 2 * (size_t)cap );
+	dgrow( W, d.nodeVisit, 0, cap );
 	d.shapeCap = cap;
 	int pc = std::max( 65536, 4 * cap );
-	dgrow( d.pairKeys, 0, pc );
-	dgrow( d.pairKeysAlt, 0, pc );
-	dgrow( d.pairVal, 0, pc );
-	dgrow( d.pairValAlt, 0, pc );
-	dgrow( d.planKeys, 0, pc );
-	dgrow( d.planIds, 0, pc );
-	dgrow( d.newPairId, 0, pc );
+	dgrow( W, d.pairKeys, 0, pc );
+	dgrow( W, d.pairKeysAlt, 0, pc );
+	dgrow( W, d.pairVal, 0, pc );
+	dgrow( W, d.pairValAlt, 0, pc );
+	dgrow( W, d.planKeys, 0, pc );
+	dgrow( W, d.planIds, 0, pc );
+	dgrow( W, d.newPairId, 0, pc );
 	d.pairCap = pc;
 	if ( d.contactCap < 8 * cap )
 		grow_contacts( W, 8 * cap );
@@ -419,25 +427,25 @@ static void grow_joints( HostWorld* W, int cap )
 {
 	DWorld& d = W->d;
 	size_t o = d.jointCap;
-	dgrow( d.jbody, o, cap );
-	dgrow( d.jflags, o, cap );
-	dgrow( d.jcolor, o, cap );
-	dgrow( d.jcolorSet, o, cap );
-	dgrow( d.jnext, 2 * o, 2 * (size_t)cap );
-	dgrow( d.jdef0, o, cap );
-	dgrow( d.jdef1, o, cap );
-	dgrow( d.jdef2, o, cap );
-	dgrow( d.jdef3, o, cap );
-	dgrow( d.jimp, o, cap );
-	dgrow( d.jimp2, o, cap );
-	dgrow( d.jprep0, 0, cap );
-	dgrow( d.jprep1, 0, cap );
-	dgrow( d.jprep2, 0, 2 * (size_t)cap );
-	dgrow( d.jprep3, 0, cap );
-	dgrow( d.jprepM, 0, cap );
-	dgrow( d.jindex, 0, cap );
-	dgrow( d.overflowJoints, o, cap );
-	dgrow( d.pendingJointOps, 0, cap );
+	dgrow( W, d.jbody, o, cap );
+	dgrow( W, d.jflags, o, cap );
+	dgrow( W, d.jcolor, o, cap );
+	dgrow( W, d.jcolorSet, o, cap );
+	dgrow( W, d.jnext, 2 * o, 2 * (size_t)cap );
+	dgrow( W, d.jdef0, o, cap );
+	dgrow( W, d.jdef1, o, cap );
+	dgrow( W, d.jdef2, o, cap );
+	dgrow( W, d.jdef3, o, cap );
+	dgrow( W, d.jimp, o, cap );
+	dgrow( W, d.jimp2, o, cap );
+	dgrow( W, d.jprep0, 0, cap );
+	dgrow( W, d.jprep1, 0, cap );
+	dgrow( W, d.jprep2, 0, 2 * (size_t)cap );
+	dgrow( W, d.jprep3, 0, cap );
+	dgrow( W, d.jprepM, 0, cap );
+	dgrow( W, d.jindex, 0, cap );
+	dgrow( W, d.overflowJoints, o, cap );
+	dgrow( W, d.pendingJointOps, 0, cap );
 	d.jointCap = cap;
 }
 
@@ -471,89 +479,89 @@ static void isl_ensure( HostWorld* W )
 	size_t nb = d.bodyCap, nc = d.contactCap, nj = d.jointCap;
 	if ( ob != nb )
 	{
-		dgrow( h.bSet, ob, nb );
-		dgrow( h.bLocal, ob, nb );
-		dgrow( h.bIsland, ob, nb );
-		dgrow( h.bIslandPrev, ob, nb );
-		dgrow( h.bIslandNext, ob, nb );
-		dgrow( h.bHeadContact, ob, nb );
-		dgrow( h.bSetNext, ob, nb );
-		dgrow( h.bMark, ob, nb );
-		dgrow( h.bMoveIndex, ob, nb );
-		dgrow( h.islands, ob, nb );
-		dgrow( h.islandFree, ob, nb );
-		dgrow( h.sets, ob + ( ob ? 8 : 0 ), nb + 8 );
-		dgrow( h.setFree, ob + ( ob ? 8 : 0 ), nb + 8 );
-		dgrow( h.awakeBodies, ob, nb );
-		dgrow( h.awakeIslands, ob, nb );
-		dgrow( h.islandBits, 0, nb );
-		dgrow( h.stack, 0, nb );
-		dgrow( h.seeds, 0, nb );
-		dgrow( h.splitIndex, 0, nb );
-		dgrow( h.splitMarks, 0, 2 * nb + 8 );
-		dgrow( h.splitRows, 0, 16 * nb );
-		dgrow( h.splitPush, 0, 16 * nb );
-		dgrow( h.splitOrder, 0, nb + 8 );
-		dgrow( h.splitPop, 0, 2 * nb );
-		dgrow( h.splitIslands, 0, nb + 1 );
-		dgrow( h.splitJointAt, 0, nb );
-		dgrow( h.splitTotals, 0, 1024 );
-		dgrow( h.flag, 0, nb );
-		dgrow( h.pos, 0, nb );
-		dgrow( h.list, 0, nb );
-		dgrow( h.moveBody, ob, nb );
-		dgrow( h.moveAsleep, ob, nb );
+		dgrow( W, h.bSet, ob, nb );
+		dgrow( W, h.bLocal, ob, nb );
+		dgrow( W, h.bIsland, ob, nb );
+		dgrow( W, h.bIslandPrev, ob, nb );
+		dgrow( W, h.bIslandNext, ob, nb );
+		dgrow( W, h.bHeadContact, ob, nb );
+		dgrow( W, h.bSetNext, ob, nb );
+		dgrow( W, h.bMark, ob, nb );
+		dgrow( W, h.bMoveIndex, ob, nb );
+		dgrow( W, h.islands, ob, nb );
+		dgrow( W, h.islandFree, ob, nb );
+		dgrow( W, h.sets, ob + ( ob ? 8 : 0 ), nb + 8 );
+		dgrow( W, h.setFree, ob + ( ob ? 8 : 0 ), nb + 8 );
+		dgrow( W, h.awakeBodies, ob, nb );
+		dgrow( W, h.awakeIslands, ob, nb );
+		dgrow( W, h.islandBits, 0, nb );
+		dgrow( W, h.stack, 0, nb );
+		dgrow( W, h.seeds, 0, nb );
+		dgrow( W, h.splitIndex, 0, nb );
+		dgrow( W, h.splitMarks, 0, 2 * nb + 8 );
+		dgrow( W, h.splitRows, 0, 16 * nb );
+		dgrow( W, h.splitPush, 0, 16 * nb );
+		dgrow( W, h.splitOrder, 0, nb + 8 );
+		dgrow( W, h.splitPop, 0, 2 * nb );
+		dgrow( W, h.splitIslands, 0, nb + 1 );
+		dgrow( W, h.splitJointAt, 0, nb );
+		dgrow( W, h.splitTotals, 0, 1024 );
+		dgrow( W, h.flag, 0, nb );
+		dgrow( W, h.pos, 0, nb );
+		dgrow( W, h.list, 0, nb );
+		dgrow( W, h.moveBody, ob, nb );
+		dgrow( W, h.moveAsleep, ob, nb );
 		h.bodyCap = (int)nb;
 		h.islandCap = (int)nb;
 		h.setCap = (int)nb + 8;
 	}
 	if ( oc != nc )
 	{
-		dgrow( h.cSet, oc, nc );
-		dgrow( h.cIsland, oc, nc );
-		dgrow( h.cIslandPrev, oc, nc );
-		dgrow( h.cIslandNext, oc, nc );
-		dgrow( h.cSetNext, oc, nc );
-		dgrow( h.cMark, oc, nc );
-		dgrow( h.cEdge, oc, nc );
-		dgrow( h.order, 0, nc );
-		dgrow( h.cRemoved, 0, nc );
+		dgrow( W, h.cSet, oc, nc );
+		dgrow( W, h.cIsland, oc, nc );
+		dgrow( W, h.cIslandPrev, oc, nc );
+		dgrow( W, h.cIslandNext, oc, nc );
+		dgrow( W, h.cSetNext, oc, nc );
+		dgrow( W, h.cMark, oc, nc );
+		dgrow( W, h.cEdge, oc, nc );
+		dgrow( W, h.order, 0, nc );
+		dgrow( W, h.cRemoved, 0, nc );
 		h.contactCap = (int)nc;
 	}
 	if ( oj != nj )
 	{
-		dgrow( h.jSet, oj, nj );
-		dgrow( h.jIsland, oj, nj );
-		dgrow( h.jIslandPrev, oj, nj );
-		dgrow( h.jIslandNext, oj, nj );
-		dgrow( h.jSetNext, oj, nj );
-		dgrow( h.jMark, oj, nj );
-		dgrow( h.jOverflowIndex, oj, nj );
+		dgrow( W, h.jSet, oj, nj );
+		dgrow( W, h.jIsland, oj, nj );
+		dgrow( W, h.jIslandPrev, oj, nj );
+		dgrow( W, h.jIslandNext, oj, nj );
+		dgrow( W, h.jSetNext, oj, nj );
+		dgrow( W, h.jMark, oj, nj );
+		dgrow( W, h.jOverflowIndex, oj, nj );
 		h.jointCap = (int)nj;
 	}
 	if ( h.ncCap < 2 * d.pairCap )
 	{
 		dfree( h.ncKeys );
 		dfree( h.ncKeysAlt );
-		dgrow( h.ncKeys, 0, 2 * (size_t)d.pairCap );
-		dgrow( h.ncKeysAlt, 0, 2 * (size_t)d.pairCap );
+		dgrow( W, h.ncKeys, 0, 2 * (size_t)d.pairCap );
+		dgrow( W, h.ncKeysAlt, 0, 2 * (size_t)d.pairCap );
 		h.ncCap = 2 * d.pairCap;
 	}
 	if ( oc != nc || oj != nj )
 	{
 		dfree( h.splitPool );
-		dgrow( h.splitPool, 0, 2 * ( nc + nj ) );
+		dgrow( W, h.splitPool, 0, 2 * ( nc + nj ) );
 		dfree( h.splitPushPool );
-		dgrow( h.splitPushPool, 0, 4 * ( nc + nj ) );
+		dgrow( W, h.splitPushPool, 0, 4 * ( nc + nj ) );
 		dfree( h.splitContacts );
-		dgrow( h.splitContacts, 0, nc );
+		dgrow( W, h.splitContacts, 0, nc );
 		dfree( h.splitJoints );
-		dgrow( h.splitJoints, 0, nj );
+		dgrow( W, h.splitJoints, 0, nj );
 	}
 	if ( h.logCap < d.bodyCap + d.jointCap )
 	{
 		dfree( h.log );
-		dgrow( h.log, 0, (size_t)d.bodyCap + d.jointCap );
+		dgrow( W, h.log, 0, (size_t)d.bodyCap + d.jointCap );
 		h.logCap = d.bodyCap + d.jointCap;
 	}
 	cudaMemcpyAsync( W->islDev, &h, sizeof( DIslands ), cudaMemcpyHostToDevice, W->stream );
@@ -978,25 +986,25 @@ static void rb_ensure( HostWorld* W, int cap )
 		return;
 	rb_free( R );
 	size_t n = (size_t)cap;
-	dgrow( R.doomed, 0, n );
-	dgrow( R.cnt, 0, n );
-	dgrow( R.rlc, 0, n );
-	dgrow( R.gIdx, 0, n );
-	dgrow( R.gCen, 0, n );
-	dgrow( R.freed, 0, n );
-	dgrow( R.bl, 0, n );
-	dgrow( R.br, 0, n );
+	dgrow( W, R.doomed, 0, n );
+	dgrow( W, R.cnt, 0, n );
+	dgrow( W, R.rlc, 0, n );
+	dgrow( W, R.gIdx, 0, n );
+	dgrow( W, R.gCen, 0, n );
+	dgrow( W, R.freed, 0, n );
+	dgrow( W, R.bl, 0, n );
+	dgrow( W, R.br, 0, n );
 	R.segCap = cap / 512 + 8;
 	R.chunkCap = cap / 512 + R.segCap + 8;
-	dgrow( R.segA, 0, (size_t)R.segCap );
-	dgrow( R.segB, 0, (size_t)R.segCap );
-	dgrow( R.segSmall, 0, n / 2 + 8 );
-	dgrow( R.chunkBase, 0, (size_t)R.segCap + 1 );
-	dgrow( R.chunkStat, 0, 5 * (size_t)R.chunkCap );
-	dgrow( R.segBounds, 0, 8 * (size_t)R.segCap ); // two level parities
-	dgrow( R.segBelow, 0, 2 * (size_t)R.segCap );
-	dgrow( R.pairBase, 0, (size_t)R.segCap + 1 );
-	dgrow( R.rfStart, 0, n / 2 + 8 );
+	dgrow( W, R.segA, 0, (size_t)R.segCap );
+	dgrow( W, R.segB, 0, (size_t)R.segCap );
+	dgrow( W, R.segSmall, 0, n / 2 + 8 );
+	dgrow( W, R.chunkBase, 0, (size_t)R.segCap + 1 );
+	dgrow( W, R.chunkStat, 0, 5 * (size_t)R.chunkCap );
+	dgrow( W, R.segBounds, 0, 8 * (size_t)R.segCap ); // two level parities
+	dgrow( W, R.segBelow, 0, 2 * (size_t)R.segCap );
+	dgrow( W, R.pairBase, 0, (size_t)R.segCap + 1 );
+	dgrow( W, R.rfStart, 0, n / 2 + 8 );
 	R.cap = cap;
 	W->graphDirty = true;
 }
@@ -1011,17 +1019,17 @@ static void tree_upload( HostWorld* W, int t )
 	{
 		pt_free( T );
 		size_t n = (size_t)h.cap;
-		dgrow( T.child1, 0, n );
-		dgrow( T.child2, 0, n );
-		dgrow( T.parent, 0, n );
-		dgrow( T.height, 0, n );
-		dgrow( T.flags, 0, n );
-		dgrow( T.shape, 0, n );
-		dgrow( T.leaves, 0, n );
-		dgrow( T.box, 0, n );
-		dgrow( T.cat, 0, n );
-		dgrow( T.rank, 0, n );
-		dgrow( T.rankShape, 0, n );
+		dgrow( W, T.child1, 0, n );
+		dgrow( W, T.child2, 0, n );
+		dgrow( W, T.parent, 0, n );
+		dgrow( W, T.height, 0, n );
+		dgrow( W, T.flags, 0, n );
+		dgrow( W, T.shape, 0, n );
+		dgrow( W, T.leaves, 0, n );
+		dgrow( W, T.box, 0, n );
+		dgrow( W, T.cat, 0, n );
+		dgrow( W, T.rank, 0, n );
+		dgrow( W, T.rankShape, 0, n );
 		T.cap = h.cap;
 		W->graphDirty = true;
 	}
@@ -1209,11 +1217,11 @@ static void flush_uploads( HostWorld* W, bool trees = true )
 		if ( cap > d.sensorPairCap )
 		{
 			size_t o = (size_t)d.sensorPairCap;
-			dgrow( d.sensorPrevKeys, o, cap );
-			dgrow( d.sensorKeys, 0, cap );
-			dgrow( d.sensorKeysAlt, 0, cap );
-			dgrow( d.sensorBeginEv, 0, cap );
-			dgrow( d.sensorEndEv, 0, cap );
+			dgrow( W, d.sensorPrevKeys, o, cap );
+			dgrow( W, d.sensorKeys, 0, cap );
+			dgrow( W, d.sensorKeysAlt, 0, cap );
+			dgrow( W, d.sensorBeginEv, 0, cap );
+			dgrow( W, d.sensorEndEv, 0, cap );
 			d.sensorPairCap = cap;
 		}
 		d.sensorCount = S;
@@ -1332,7 +1340,7 @@ extern "C" F2D_API int32_t f2d_create_world( const f2d_world_def* def )
 	W->query = new QueryScratch;
 	cudaMallocHost( (void**)&W->hostEnd, sizeof( int ) * ( 1 + 2 * HOST_END ) );
 	cudaMalloc( (void**)&d.sc, sizeof( DScalars ) );
-	cudaMemset( d.sc, 0, sizeof( DScalars ) );
+	cudaMemsetAsync( d.sc, 0, sizeof( DScalars ), W->stream );
 	grow_bodies( W, 1024 );
 	grow_shapes( W, 1024 );
 	grow_joints( W, 256 );
@@ -3772,9 +3780,9 @@ static void cb_ensure( HostWorld* W )
 	int cap = std::max( 1 << 16, d.contactCap );
 	if ( cap <= d.cbCap )
 		return;
-	dgrow( d.cbList, 0, cap );
-	dgrow( d.cbReject, 0, cap );
-	dgrow( d.cbManifold, 0, 22 * (size_t)cap );
+	dgrow( W, d.cbList, 0, cap );
+	dgrow( W, d.cbReject, 0, cap );
+	dgrow( W, d.cbManifold, 0, 22 * (size_t)cap );
 	d.cbCap = cap;
 	W->graphDirty = true;
 }
@@ -4208,8 +4216,8 @@ static void ensure_learning_buffers( HostWorld* W )
 		cudaStreamSynchronize( W->stream );
 		dfree( d.newPoint );
 		dfree( d.newFeat );
-		dgrow( d.newPoint, 0, (size_t)d.contactCap );
-		dgrow( d.newFeat, 0, (size_t)d.contactCap * 12 );
+		dgrow( W, d.newPoint, 0, (size_t)d.contactCap );
+		dgrow( W, d.newFeat, 0, (size_t)d.contactCap * 12 );
 		d.newPointCap = d.contactCap;
 	}
 }
@@ -4225,7 +4233,7 @@ extern "C" F2D_API void f2d_world_set_sample_recording( int32_t worldId, int32_t
 	d.sampleCap = 0;
 	if ( capacity > 0 )
 	{
-		dgrow( d.samples, 0, (size_t)capacity * 14 );
+		dgrow( W, d.samples, 0, (size_t)capacity * 14 );
 		d.sampleCap = capacity;
 		ensure_learning_buffers( W );
 		d.learnMode |= 1;

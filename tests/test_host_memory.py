@@ -3,6 +3,7 @@ fails where it is told to: no GPU, no driver."""
 from __future__ import annotations
 
 import os
+import re
 import shutil
 import subprocess
 
@@ -161,3 +162,13 @@ def test_page_locked_blocks_are_not_the_heaps(tmp_path):
 
 def test_other_calls_errors_are_kept(tmp_path):
     _run(tmp_path, "last_error", LAST_ERROR)
+
+
+def test_world_memory_is_written_in_stream_order():
+    """A world's streams do not wait for the default stream: clears of and
+    copies to its device memory go through its own, or a step may run ahead
+    of them (synchronous copies to the host follow a wait)."""
+    source = open(os.path.join(CSRC, "world.cu")).read()
+    assert re.findall(r"\bcudaMemset\(", source) == []
+    copies = re.findall(r"\bcudaMemcpy\((?:[^;]*?)\);", source, re.S)
+    assert copies and [c for c in copies if "cudaMemcpyDeviceToHost" not in c] == []
