@@ -2868,13 +2868,15 @@ static void create_proxy_forced( HostWorld* W, int s, int proxyType )
 }
 
 // after the device launch: the body's rows (type, state, flags) come back
-// to the host mirror, then its mass data (b2UpdateBodyMassData)
-static void type_change_end( HostWorld* W, int b )
+// to the host mirror, then, for a change of type, its mass data
+// (b2UpdateBodyMassData, which b2Body_Disable and b2Body_Enable leave alone)
+static void body_change_end( HostWorld* W, int b, bool mass )
 {
 	destroy_end( W );
 	body_rows_changed( W, false );
 	pull_body( W, b );
-	update_mass( W, b );
+	if ( mass )
+		update_mass( W, b );
 	mark_body( W, b );
 }
 
@@ -2911,7 +2913,7 @@ extern "C" F2D_API void f2d_body_set_type( int32_t index1, int32_t wg, int32_t t
 		destroy_proxy_host( W, s );
 		create_proxy_forced( W, s, type );
 	}
-	type_change_end( W, b );
+	body_change_end( W, b, true );
 }
 
 // RawBox2D.bodyDisable (raw_box2d.dart:254) -> b2Body_Disable (body.c:1557)
@@ -2934,7 +2936,7 @@ extern "C" F2D_API void f2d_body_disable( int32_t index1, int32_t wg )
 	launch_body_disable( W->d, W->stream, b );
 	W->bflags[b] &= ~( BF_ENABLED | BF_ASLEEP );
 	awake_order_remove( W, b );
-	type_change_end( W, b );
+	body_change_end( W, b, false );
 }
 
 // RawBox2D.bodyEnable (raw_box2d.dart:258) -> b2Body_Enable (body.c:1628)
@@ -2959,7 +2961,7 @@ extern "C" F2D_API void f2d_body_enable( int32_t index1, int32_t wg )
 		create_proxy_forced( W, s, type );
 		edit_shape_bits( W, s, SF_PROXY, 0 );
 	}
-	type_change_end( W, b );
+	body_change_end( W, b, false );
 }
 
 extern "C" F2D_API double f2d_body_get_param( int32_t index1, int32_t wg, int32_t code )
