@@ -64,6 +64,10 @@ __device__ int isl_graph_add_contact( const DWorld& w, int c )
 			w.colorMask[d] |= 1u << color;
 	}
 	w.ccolor[c] = color;
+	// constraint_graph.c:139-181: the bodies' masses as they are now (a body may
+	// have gained or lost a shape while it was asleep)
+	const float4 ma = w.massv[bd.x], mb = w.massv[bd.y];
+	w.cmass[c] = make_float4( ma.x, ma.y, mb.x, mb.y );
 	if ( color == F2D_OVERFLOW )
 	{
 		int idx = w.sc->overflowCount;
