@@ -2629,7 +2629,8 @@ static void destroy_body_host( HostWorld* W, int b )
 	{
 		int j = key >> 1;
 		key = W->jnext[2 * j + ( key & 1 )];
-		destroy_joint_host( W, j, 1 );
+		if ( W->jflags[j] & JF_USED ) // (a joint of the body to itself is listed twice)
+			destroy_joint_host( W, j, 1 );
 	}
 	launch_destroy_contacts_of( W->d, W->stream, b, -1, -1, 1, W->s.tmpA );
 	for ( int s = W->headShape[b]; s != F2D_NULL; s = W->nextShape[s] )

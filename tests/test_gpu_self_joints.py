@@ -72,3 +72,36 @@ def test_self_joints_equal_port(gpu_lib, kind, spokes, sleep):
         assert np.array_equal(f, h), (kind, f, h)
     g.close()
     p.close()
+
+
+@pytest.mark.parametrize("sleep", [0, 1])
+def test_destroyed_body_frees_its_self_joint_once(gpu_lib, sleep):
+    """Two joints made after it have different ids, and the world goes on as
+    one in which the joint was destroyed first."""
+    from forge2d_gb300.world import GpuWorld
+    worlds = []
+    for first in (True, False):
+        g = GpuWorld(scenes.world_def(enableSleep=sleep))
+        ground = g.create_body(scenes.body_def(positionY=-1.0))
+        g.create_box(ground, scenes.shape_def(), 20.0, 1.0)
+        ids = []
+        for k in range(6):
+            ids.append(g.create_body(scenes.body_def(type=scenes.DYNAMIC, positionX=1.1 * k, positionY=2.0)))
+            g.create_box(ids[-1], scenes.shape_def(), 0.5, 0.5)
+        joint = _self_joint(g, "mouse", ids[2], 2.2, 2.0)
+        for _ in range(5):
+            g.step()
+        if first:
+            g.destroy_joint(joint)
+        g.destroy_body(ids[2])
+        a = g.create_revolute(scenes.revolute_def(bodyA=ids[0], bodyB=ids[1], localAnchorAX=0.55, localAnchorBX=-0.55))
+        b = g.create_revolute(scenes.revolute_def(bodyA=ids[3], bodyB=ids[4], localAnchorAX=0.55, localAnchorBX=-0.55))
+        assert a[0] != b[0]
+        for _ in range(30):
+            g.step()
+        assert g.sync() == 0 and g.counters()["joints"] == 2
+        worlds.append(g)
+    x, y = (g.bodies()[:, :9] for g in worlds)
+    assert np.array_equal(x.view(np.uint32), y.view(np.uint32))
+    for g in worlds:
+        g.close()
