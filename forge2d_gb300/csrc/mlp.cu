@@ -679,6 +679,7 @@ extern "C" F2D_API void f2d_mlp_set_normalization( int32_t handle, const float* 
 		return;
 	cudaMemcpy( M->norm, mean14, sizeof( float ) * MLP_SAMPLE, cudaMemcpyHostToDevice );
 	cudaMemcpy( M->norm + MLP_SAMPLE, invStd14, sizeof( float ) * MLP_SAMPLE, cudaMemcpyHostToDevice );
+	cudaDeviceSynchronize(); // (a world's stream does not wait for the copies)
 }
 
 // Gradient of the batch loss 0.5 * mean ||y - t||^2 over all n samples

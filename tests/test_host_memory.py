@@ -172,3 +172,11 @@ def test_world_memory_is_written_in_stream_order():
     assert re.findall(r"\bcudaMemset\(", source) == []
     copies = re.findall(r"\bcudaMemcpy\((?:[^;]*?)\);", source, re.S)
     assert copies and [c for c in copies if "cudaMemcpyDeviceToHost" not in c] == []
+
+
+def test_model_edits_end_with_a_wait():
+    """A world may read a model on its own stream right after its edit."""
+    source = open(os.path.join(CSRC, "mlp.cu")).read()
+    for name in ("f2d_mlp_create", "f2d_mlp_set_params", "f2d_mlp_set_normalization"):
+        body = source[source.index(" " + name + "("):]
+        assert "cudaDeviceSynchronize()" in body[:body.index("\n}\n")], name
